@@ -26,7 +26,16 @@
 
 namespace mhd {
 
-enum { R_PDM = 1, R_TVD = 2, R_WENO = 3, R_MPWENO = 4, R_TVDMC = 5 };
+// R_PDMG: PDM evaluated as the reference writes the interpolant and the
+// limiter.  R_PDM (interval form) needs a limiter constant pdmb > 0, so carve()
+// picks R_PDMG otherwise; and the FP32 metric mode uses it throughout: its face
+// fluxes are small differences of B.A-sized terms, so that the last bits of a
+// reconstruction appear at 1e-5 to 1e-4 of the weak components (bz of the blast: 5e-5
+// between the two forms, 4e-4 of either against FP64).
+enum { R_PDM = 1, R_TVD = 2, R_WENO = 3, R_MPWENO = 4, R_TVDMC = 5, R_PDMG = 6 };
+template <typename T, bool M> constexpr int pdm_form() {
+  return M && std::is_same<T, float>::value ? R_PDMG : R_PDM;
+}
 enum { BC_PERIODIC = 0, BC_EVEN = 1, BC_REFLECT = 2, BC_OUTFLOW = 3 };
 enum { EMF_LFM = 0, EMF_YEE = 1 };
 
@@ -108,21 +117,206 @@ template <> struct Ops<float> {
   static __device__ __forceinline__ float dvr(float a, float, float rb) { return a * rb; }
 };
 
-// 8-point centred interpolant (interp_pdm, mhd3d3.f90:866-872), operand order kept.
+// 8-point centred interpolant (interp_pdm, mhd3d3.f90:866-872):
+// (-3, 29, -139, 533, 533, -139, 29, -3) / 840, as eight fused operations
+// with the coefficients divided by 840 beforehand, the smallest first.
+// Against the exact sum its rms error is 0.4-0.5 of what the integer
+// coefficients with a final division gave (FP32, smooth and random taps:
+// 0.32-0.51 against 0.79-1.26 units of 2^-24), because the rounding of the
+// large terms happens once, at the end.
+template <typename T> struct Tap {
+  static constexpr T c0 = T(-3.0 / 840.0), c1 = T(29.0 / 840.0), c2 = T(-139.0 / 840.0), c3 = T(533.0 / 840.0);
+};
+__device__ __forceinline__ float fm(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double fm(double a, double b, double c) { return fma(a, b, c); }
 template <typename T>
 __device__ __forceinline__ T tap8(T a0, T a1, T a2, T a3, T a4, T a5, T a6, T a7) {
-  T s = T(-3) * a0;
-  s = s + T(29) * a1;
-  s = s - T(139) * a2;
-  s = s + T(533) * a3;
-  s = s + T(533) * a4;
-  s = s - T(139) * a5;
-  s = s + T(29) * a6;
-  s = s - T(3) * a7;
-  return Div<T>::by(s, T(840));
+  typedef Tap<T> C;
+  T s = fm(C::c0, a7, C::c0 * a0);
+  s = fm(C::c1, a6, fm(C::c1, a1, s));
+  s = fm(C::c2, a5, fm(C::c2, a2, s));
+  return fm(C::c3, a4, fm(C::c3, a3, s));
 }
 
-// PDM2 (mhd3d3.f90:1069-1172): clamp of the interpolant and partial-donor limiter.
+// PDM2 (mhd3d3.f90:1069-1172) for pdmb > 0, without its signs.  With
+// D(c, f) = 2 pdmb (c - f), the limiter's left state is the interpolant
+// clamped to [fm1, f0] and then kept within [fm1, fm1 + D(fm1, fm2)] -- the
+// reference's fii - s0 max(0, |fii - fm1| - |sm + s0| |dfm|) is exactly that:
+// |sm + s0| is 2 where the two slopes agree and 0 where they do not, and in the
+// latter case the two intervals share only fm1.  The right state is the mirror
+// image about f0.  So each state is one value x held within two intervals
+// that share an end c (the near cell):
+//   within(c, far, out, x), far the cell across the face, out = c + D(c, outer).
+// A limited state is one rounding of c + D instead of three, and the branch
+// decisions are minima and maxima.  NaN: the near cells reach the result as in
+// the reference's form (NaN-propagating min / max on the lower end), a NaN
+// that is only in the interpolant is dropped by the clamp there as here.
+//
+// FP32: two- and three-operand FMNMX.  FP64: FP64 comparisons share the FP64
+// pipe (2 lanes per SM and cycle, a 32nd of the integer pipe), so minima and
+// maxima run on order-preserving integer images of the values.
+template <typename T> struct Sel;
+template <> struct Sel<float> {
+  typedef float K;
+  static __device__ __forceinline__ K key(float x) { return x; }
+  static __device__ __forceinline__ float val(K k) { return k; }
+  static __device__ __forceinline__ K mn(K a, K b) { return fminf(a, b); }
+  static __device__ __forceinline__ K mx(K a, K b) { return fmaxf(a, b); }
+  static __device__ __forceinline__ K mn_nan(K a, K b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+  }
+  static __device__ __forceinline__ K mn3(K a, K b, K c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+  }
+  static __device__ __forceinline__ K mx3_nan(K a, K b, K c) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+  }
+  static __device__ __forceinline__ float keep_nan(float r, float) { return r; }
+};
+template <> struct Sel<double> {
+  typedef long long K;  // ordered as the doubles are: negative values with the magnitude bits inverted
+  static __device__ __forceinline__ K flip(K b) { return b ^ ((b >> 63) & 0x7fffffffffffffffLL); }
+  static __device__ __forceinline__ K key(double x) { return flip(__double_as_longlong(x)); }
+  static __device__ __forceinline__ double val(K k) { return __longlong_as_double(flip(k)); }
+  static __device__ __forceinline__ K mn(K a, K b) { return a < b ? a : b; }
+  static __device__ __forceinline__ K mx(K a, K b) { return a > b ? a : b; }
+  static __device__ __forceinline__ K mn_nan(K a, K b) { return mn(a, b); }
+  static __device__ __forceinline__ K mn3(K a, K b, K c) { return mn(mn(a, b), c); }
+  static __device__ __forceinline__ K mx3_nan(K a, K b, K c) { return mx(mx(a, b), c); }
+  // the integer images order a NaN beyond infinity: hand it on instead
+  // (out = c + D(c, outer) is NaN when c or outer is)
+  static __device__ __forceinline__ double keep_nan(double r, double out) {
+    return (__double2hiint(out) & 0x7fffffff) > 0x7ff00000 ? out : r;
+  }
+};
+// x held within [c, far] and [c, out]; lo = min(c, far), hi = max(c, far).
+template <typename T>
+__device__ __forceinline__ T within(typename Sel<T>::K lo, typename Sel<T>::K hi, typename Sel<T>::K c, T out,
+                                    typename Sel<T>::K x) {
+  typedef Sel<T> S;
+  const typename S::K o = S::key(out);
+  return S::keep_nan(S::val(S::mx3_nan(lo, S::mn_nan(c, o), S::mn3(hi, S::mx(c, o), x))), out);
+}
+// Both states of one face, k = 2 pdmb, outl = fm1 + k (fm1 - fm2), outr = f0 + k (f0 - fp1).
+template <typename T>
+__device__ __forceinline__ void pdm_pick(T fm1, T f0, T outl, T outr, T fi, T& fl, T& fr) {
+  typedef Sel<T> S;
+  const typename S::K a = S::key(fm1), b = S::key(f0), x = S::key(fi);
+  const typename S::K lo = S::mn_nan(a, b), hi = S::mx(a, b);
+  fl = within<T>(lo, hi, a, outl, x);
+  fr = within<T>(lo, hi, b, outr, x);
+}
+template <typename T>
+__device__ __forceinline__ void pdm_states(T fm2, T fm1, T f0, T fp1, T fi, T pdmb, T& fl, T& fr) {
+  const T k = pdmb + pdmb;
+  pdm_pick(fm1, f0, fm(k, fm1 - fm2, fm1), fm(k, f0 - fp1, f0), fi, fl, fr);
+}
+
+// ------------------------------------------------ edge EMF forms (FP64)
+// The edge EMF of the FP64 mode keeps the reference's roundings (its CT
+// differences show the last bit of E: a face-B component that is zero at first
+// takes all its value from them), while the face fluxes take the fused forms
+// above.  What the roundings leave free is where the decisions are made:
+// comparisons, minima, signs and absolute values run on the integer pipe, and
+// the division by 840 takes two operations.  FP32 has one form for both.
+//
+// x / 840, correctly rounded: x zh + x zl with zh + zl = 1/840 to twice the
+// precision errs by about 2^-106 of the quotient before its one rounding,
+// while a quotient by 840 = 8 * 105 is never closer than 2^-54 / 105 to the
+// midpoint of two doubles (105 times an odd 54-bit integer has more than 53
+// bits, so no midpoint is a quotient, and the gap is a whole unit of x).
+template <int N> __device__ __forceinline__ double div_by(double x) {
+  constexpr double zh = 1.0 / N;
+  // 1/N - zh = (1 - N zh) / N: N zh is split so that both products are exact
+  constexpr double zt = (zh * 134217729.0) - ((zh * 134217729.0) - zh);  // upper half of zh
+  constexpr double zl = ((1.0 - N * zt) - N * (zh - zt)) / N;
+  return fma(x, zh, x * zl);
+}
+__device__ __forceinline__ double abs_bits(double x) {
+  return __hiloint2double(__double2hiint(x) & 0x7fffffff, __double2loint(x));
+}
+// a >= b for |a|, |b| (integer comparison of the magnitudes)
+__device__ __forceinline__ bool abs_ge(double a, double b) {
+  return (__double_as_longlong(a) & 0x7fffffffffffffffLL) >= (__double_as_longlong(b) & 0x7fffffffffffffffLL);
+}
+__device__ __forceinline__ bool abs_ge(float a, float b) { return fabsf(a) >= fabsf(b); }
+// x >= 0 (-0.0 counts)
+__device__ __forceinline__ bool ge0(double x) { return Sel<double>::key(x) >= -1LL; }
+__device__ __forceinline__ bool ge0(float x) { return x >= 0.0f; }
+
+// Interpolant and limiter states of the edge EMF.
+template <typename T> struct Edge;
+template <> struct Edge<float> {
+  static __device__ __forceinline__ float tap(float a0, float a1, float a2, float a3, float a4, float a5, float a6,
+                                              float a7) {
+    return tap8(a0, a1, a2, a3, a4, a5, a6, a7);
+  }
+  static __device__ __forceinline__ void states(float fm2, float fm1, float f0, float fp1, float fi, float pdmb,
+                                                float& fl, float& fr) {
+    pdm_states(fm2, fm1, f0, fp1, fi, pdmb, fl, fr);
+  }
+};
+template <> struct Edge<double> {
+  typedef Sel<double> S;
+  // interp_pdm's operand order (mhd3d3.f90:866-872)
+  static __device__ __forceinline__ double tap(double a0, double a1, double a2, double a3, double a4, double a5,
+                                               double a6, double a7) {
+    double s = -3.0 * a0;
+    s = s + 29.0 * a1;
+    s = s - 139.0 * a2;
+    s = s + 533.0 * a3;
+    s = s + 533.0 * a4;
+    s = s - 139.0 * a5;
+    s = s + 29.0 * a6;
+    s = s - 3.0 * a7;
+    return div_by<840>(s);
+  }
+  // the clamp of PDM2: x held within [a, b]
+  static __device__ __forceinline__ double clamp(S::K a, S::K b, S::K x) {
+    return S::val(S::mx(S::mn(a, b), S::mn(x, S::mx(a, b))));
+  }
+  // fii -+ max(0, |near - fii| - q |dn|), q = 2 where the slopes towards the
+  // far cell (up) and from the outer one (dn = pdmb (near - outer)) agree, else
+  // 0; - when the far cell is the larger.  2 |dn| is exact, so the fused
+  // difference rounds as the reference's product and difference do.
+  static __device__ __forceinline__ double limited(double near, double fii, double dn, bool up) {
+    const double m = (__double2hiint(dn) >= 0) == up ? abs_bits(dn) : 0.0;
+    const double t = fma(-2.0, m, abs_bits(near - fii));
+    const int h = __double2hiint(t);
+    const bool neg = (unsigned)h - 0x80000000u <= 0x7ff00000u;  // below zero (not NaN)
+    const double x = __hiloint2double(neg ? 0 : (up ? h ^ 0x80000000 : h), neg ? 0 : __double2loint(t));
+    return fii + x;
+  }
+  static __device__ __forceinline__ void states(double fm2, double fm1, double f0, double fp1, double fi, double pdmb,
+                                                double& fl, double& fr) {
+    const S::K a = S::key(fm1), b = S::key(f0);
+    const double fii = clamp(a, b, S::key(fi));
+    fl = limited(fm1, fii, pdmb * (fm1 - fm2), b >= a);
+    fr = limited(f0, fii, pdmb * (f0 - fp1), a > b);
+  }
+};
+
+// interp_pdm in the reference's operand order (R_PDMG; FP32 with FMA
+// contraction and a reciprocal multiply in place of the division).
+__device__ __forceinline__ double tap_ref(double a0, double a1, double a2, double a3, double a4, double a5, double a6,
+                                          double a7) {
+  return Edge<double>::tap(a0, a1, a2, a3, a4, a5, a6, a7);
+}
+__device__ __forceinline__ float tap_ref(float a0, float a1, float a2, float a3, float a4, float a5, float a6, float a7) {
+  float s = fmaf(29.0f, a1, -3.0f * a0);
+  s = fmaf(533.0f, a3, fmaf(-139.0f, a2, s));
+  s = fmaf(-139.0f, a5, fmaf(533.0f, a4, s));
+  s = fmaf(-3.0f, a7, fmaf(29.0f, a6, s));
+  return s * (1.0f / 840.0f);
+}
+
+// PDM2 (mhd3d3.f90:1069-1172) as the reference writes it, for any pdmb (R_PDMG).
 template <typename T>
 __device__ __forceinline__ void pdm2(T fm2, T fm1, T f0, T fp1, T fi, T pdmb, T& fl, T& fr) {
   T maxf = mx(fm1, f0), minf = mn(fm1, f0);
@@ -226,17 +420,20 @@ struct Prm {
 // (reconstruct_3d for dirs 1-3, mhd3d3.f90:833-860).
 // PDM face states from the 8 taps a0..a7 (cells c-4 .. c+3 along the
 // reconstruction axis; the face at the low side of c).
-template <typename T>
+constexpr bool is_pdm(int recon) { return recon == R_PDM || recon == R_PDMG; }
+// EDGE: the face-B reconstruction of the edge EMF.
+template <typename T, int RECON = R_PDM, bool EDGE = false>
 __device__ __forceinline__ void recon_pdm8(T a0, T a1, T a2, T a3, T a4, T a5, T a6, T a7, T pdmb, T& fl, T& fr) {
-  const T fi = tap8(a0, a1, a2, a3, a4, a5, a6, a7);
-  pdm2(a2, a3, a4, a5, fi, pdmb, fl, fr);
+  if (RECON != R_PDM) pdm2(a2, a3, a4, a5, tap_ref(a0, a1, a2, a3, a4, a5, a6, a7), pdmb, fl, fr);
+  else if (EDGE) Edge<T>::states(a2, a3, a4, a5, Edge<T>::tap(a0, a1, a2, a3, a4, a5, a6, a7), pdmb, fl, fr);
+  else pdm_states(a2, a3, a4, a5, tap8(a0, a1, a2, a3, a4, a5, a6, a7), pdmb, fl, fr);
 }
 
-template <typename T, int RECON, typename I>
+template <typename T, int RECON, typename I, bool EDGE = false>
 __device__ __forceinline__ void recon_face(const T* __restrict__ f, I c, I s, const Prm<T>& P, T& fl, T& fr) {
-  if (RECON == R_PDM) {
-    recon_pdm8(f[c - 4 * s], f[c - 3 * s], f[c - 2 * s], f[c - s], f[c], f[c + s], f[c + 2 * s], f[c + 3 * s], P.pdmb,
-               fl, fr);
+  if (is_pdm(RECON)) {
+    recon_pdm8<T, RECON, EDGE>(f[c - 4 * s], f[c - 3 * s], f[c - 2 * s], f[c - s], f[c], f[c + s], f[c + 2 * s],
+                         f[c + 3 * s], P.pdmb, fl, fr);
   } else if (RECON == R_TVD || RECON == R_TVDMC) {
     T fm2 = f[c - 2 * s], fm1 = f[c - s], f0 = f[c], fp1 = f[c + s];
     T fi = (fm1 + f0) / T(2);
@@ -249,6 +446,17 @@ __device__ __forceinline__ void recon_face(const T* __restrict__ f, I c, I s, co
       fr = mp_side(fr, fp2, fp1, f0, fm1, fm2, P.alpha, P.beta);
     }
   }
+}
+
+// The corner interpolant's passes.
+template <typename T, int RECON>
+__device__ __forceinline__ T edge_tap(T a0, T a1, T a2, T a3, T a4, T a5, T a6, T a7) {
+  return RECON == R_PDM ? Edge<T>::tap(a0, a1, a2, a3, a4, a5, a6, a7) : tap_ref(a0, a1, a2, a3, a4, a5, a6, a7);
+}
+// recon_face of the face B in the edge EMF.
+template <typename T, int RECON, typename I>
+__device__ __forceinline__ void recon_edge(const T* __restrict__ f, I c, I s, const Prm<T>& P, T& fl, T& fr) {
+  recon_face<T, RECON, I, true>(f, c, s, P, fl, fr);
 }
 
 // One side of weno_vals: the left state of the stencil (x0..x4) = (fm3..fp1);
@@ -270,12 +478,32 @@ __device__ __forceinline__ void weno_vals(const T* a, const Prm<T>& P, T& fl, T&
   }
 }
 
-// One half of pdm2 in a single form: the clamp pair (lo, hi) = (fm1, f0), the
-// cell `outer` beyond the near end and the side (left: near = fm1, outer =
-// fm2, result fii - s0*X; right: near = f0, outer = fp1, result fii + s0*X).
-// The difference is formed in pdm2's own operand order for each side, so the
-// result has pdm2's bits; the side is data, not control flow, so lanes that
-// pick different sides do not diverge.
+// PDM part of get_vav_center2corner (mhd3d3.f90:1901-1905, 2056-2108) for
+// an edge with upper cell c and transverse axes d1, d2, given the corner
+// interpolant vi.  The reference limits vi with four shifted PDM2 pairs, which
+// leaves each quadrant cell q two one-sided estimates, one along d1 and one
+// along d2, and takes the one whose outward slope is larger (dif >= 0: d1).
+// An estimate is PDM2's state on the side of q, so in the form above it is
+// within(q, far, q + D(q, outer), vi) with far the cell across the edge and outer the
+// one behind q along that axis: the comparison of the two slopes picks (far,
+// q - outer) and one state per quadrant is evaluated.  The edge takes the mean
+// of the four.
+__device__ __forceinline__ float corner_quad(float q, float far1, float far2, float e1, float e2, float pd, float vi) {
+  typedef Sel<float> S;
+  const bool b = abs_ge(e1, e2);  // q - outer along d1 and d2
+  const float far = b ? far1 : far2;
+  return within<float>(S::mn_nan(q, far), S::mx(q, far), q, fm(pd + pd, b ? e1 : e2, q), vi);
+}
+__device__ __forceinline__ double corner_quad(double q, double far1, double far2, double e1, double e2, double pd,
+                                              double vi) {
+  typedef Sel<double> S;
+  const bool b = abs_ge(e1, e2);
+  const S::K c = S::key(q), f = S::key(b ? far1 : far2);
+  return Edge<double>::limited(q, Edge<double>::clamp(c, f, S::key(vi)), pd * (b ? e1 : e2), f > c);
+}
+// The reference's form, for any pdmb (R_PDMG): one half of pdm2 with the clamp
+// pair (lo, hi) = (fm1, f0), the cell `outer` beyond the near end and the side
+// (left: near = fm1, outer = fm2; right: near = f0, outer = fp1).
 template <typename T>
 __device__ __forceinline__ T pdm_half(T lo, T hi, T outer, bool left, T fi, T pdmb) {
   const T fii = mx(mn(lo, hi), mn(fi, mx(lo, hi)));
@@ -287,28 +515,23 @@ __device__ __forceinline__ T pdm_half(T lo, T hi, T outer, bool left, T fi, T pd
   return left ? fii - x : fii + x;
 }
 
-// PDM part of get_vav_center2corner (mhd3d3.f90:1901-1905, 2056-2108) for
-// an edge with upper cell c and transverse strides s1 (d1), s2 (d2), given
-// the corner interpolant vi: the four shifted PDM2 limiters, the quadrant
-// choice by the sign of dif and the 4-quadrant mean.  Each quadrant keeps one
-// of its two one-sided estimates, so the dif signs pick the stencil and the
-// side first and only that half-limiter is evaluated (pdm_half: same bits as
-// evaluating all four pdm2 and selecting).  v may point to global or shared
-// memory.
-// The same on the 12 cells it reads, named by (offset along d1, offset along
-// d2) from the upper cell: mAB = (-A, -B), pAB = (+A, -B) etc.
-template <typename T>
+// The 12 cells an edge reads, named by (offset along d1, offset along d2)
+// from the upper cell: mAB = (-A, -B), pAB = (+A, -B) etc.; quadrant cells
+// m11, m01, m10, c0.
+template <typename T, int RECON = R_PDM>
 __device__ __forceinline__ T corner_pdm_vals(T m11, T m21, T m12, T m01, T p11, T m02, T m10, T m20, T m1p, T c0,
                                              T p10, T p01, T vi, T pd) {
-  // quadrant cells q00 = (-1,-1), q10 = (0,-1), q01 = (-1,0), q11 = (0,0)
+  if (RECON == R_PDM) {
+    const T v00 = corner_quad(m11, m01, m10, m11 - m21, m11 - m12, pd, vi);
+    const T v10 = corner_quad(m01, m11, c0, m01 - p11, m01 - m02, pd, vi);
+    const T v01 = corner_quad(m10, c0, m11, m10 - m20, m10 - m1p, pd, vi);
+    const T v11 = corner_quad(c0, m10, m01, c0 - p10, c0 - p01, pd, vi);
+    return T(0.25) * (v00 + v01 + v10 + v11);
+  }
   const T d00 = fab(m21 - m11) - fab(m12 - m11);
   const T d10 = fab(p11 - m01) - fab(m02 - m01);
   const T d01 = fab(m20 - m10) - fab(m1p - m10);
   const T d11 = fab(p10 - c0) - fab(p01 - c0);
-  // pdm2 #1 on (c-s2-2s1, c-s2-s1, c-s2, c-s2+s1) -> (v00_0, v10_0)
-  // pdm2 #2 on (c-s1-2s2, c-s1-s2, c-s1, c-s1+s2) -> (v00_1, v01_1)
-  // pdm2 #3 on (c-2s2, c-s2, c, c+s2)             -> (v10_1, v11_1)
-  // pdm2 #4 on (c-2s1, c-s1, c, c+s1)             -> (v01_0, v11_0)
   const bool b00 = d00 >= T(0), b10 = d10 >= T(0), b01 = d01 >= T(0), b11 = d11 >= T(0);
   const T v00 = pdm_half(m11, b00 ? m01 : m10, b00 ? m21 : m12, true, vi, pd);
   const T v10 = pdm_half(b10 ? m11 : m01, b10 ? m01 : c0, b10 ? p11 : m02, !b10, vi, pd);
@@ -317,10 +540,11 @@ __device__ __forceinline__ T corner_pdm_vals(T m11, T m21, T m12, T m01, T p11, 
   return T(0.25) * (v00 + v01 + v10 + v11);
 }
 
-template <typename T, typename I>
+template <typename T, int RECON, typename I>
 __device__ __forceinline__ T corner_pdm(const T* __restrict__ v, I c, I s1, I s2, T vi, T pd) {
-  return corner_pdm_vals(v[c - s1 - s2], v[c - 2 * s1 - s2], v[c - s1 - 2 * s2], v[c - s2], v[c + s1 - s2],
-                         v[c - 2 * s2], v[c - s1], v[c - 2 * s1], v[c - s1 + s2], v[c], v[c + s1], v[c + s2], vi, pd);
+  return corner_pdm_vals<T, RECON>(v[c - s1 - s2], v[c - 2 * s1 - s2], v[c - s1 - 2 * s2], v[c - s2],
+                                   v[c + s1 - s2], v[c - 2 * s2], v[c - s1], v[c - 2 * s1], v[c - s1 + s2], v[c],
+                                   v[c + s1], v[c + s2], vi, pd);
 }
 
 // Two values carried together (the v_a1 and v_a2 components of an edge): one
@@ -334,31 +558,72 @@ template <> struct Pr<float> {
   static __device__ __forceinline__ V mk(float a, float b) { return make_float2(a, b); }
   static __device__ __forceinline__ V mul(float k, V a) { return __fmul2_rn(make_float2(k, k), a); }
   static __device__ __forceinline__ V mad(float k, V a, V c) { return __ffma2_rn(make_float2(k, k), a, c); }  // c + k a
-  static __device__ __forceinline__ V by(V a, float b) { return mul(1.0f / b, a); }  // Div<float>::by
+  static __device__ __forceinline__ V sub(V a, V b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }  // one rounding
 };
 template <> struct Pr<double> {
   typedef double2 V;
   static __device__ __forceinline__ V mk(double a, double b) { return make_double2(a, b); }
   static __device__ __forceinline__ V mul(double k, V a) { return make_double2(k * a.x, k * a.y); }
-  static __device__ __forceinline__ V mad(double k, V a, V c) { return make_double2(c.x + k * a.x, c.y + k * a.y); }
-  static __device__ __forceinline__ V by(V a, double b) { return make_double2(a.x / b, a.y / b); }
+  static __device__ __forceinline__ V mad(double k, V a, V c) { return make_double2(fma(k, a.x, c.x), fma(k, a.y, c.y)); }
+  static __device__ __forceinline__ V sub(V a, V b) { return make_double2(a.x - b.x, a.y - b.y); }
 };
 
-// tap8 on pairs (same operand order: s = -3 a0, s + 29 a1, s - 139 a2, ...)
+// edge_tap on pairs (same operations per lane)
+template <int RECON = R_PDM>
+__device__ __forceinline__ float2 tap8p(float2 a0, float2 a1, float2 a2, float2 a3, float2 a4, float2 a5, float2 a6,
+                                        float2 a7) {
+  typedef Pr<float> Q;
+  if (RECON != R_PDM) {
+    float2 s = Q::mad(29.0f, a1, Q::mul(-3.0f, a0));
+    s = Q::mad(533.0f, a3, Q::mad(-139.0f, a2, s));
+    s = Q::mad(-139.0f, a5, Q::mad(533.0f, a4, s));
+    s = Q::mad(-3.0f, a7, Q::mad(29.0f, a6, s));
+    return Q::mul(1.0f / 840.0f, s);
+  }
+  typedef Tap<float> C;
+  float2 s = Q::mad(C::c0, a7, Q::mul(C::c0, a0));
+  s = Q::mad(C::c1, a6, Q::mad(C::c1, a1, s));
+  s = Q::mad(C::c2, a5, Q::mad(C::c2, a2, s));
+  return Q::mad(C::c3, a4, Q::mad(C::c3, a3, s));
+}
+template <int RECON = R_PDM>
+__device__ __forceinline__ double2 tap8p(double2 a0, double2 a1, double2 a2, double2 a3, double2 a4, double2 a5,
+                                         double2 a6, double2 a7) {
+  return make_double2(Edge<double>::tap(a0.x, a1.x, a2.x, a3.x, a4.x, a5.x, a6.x, a7.x),
+                      Edge<double>::tap(a0.y, a1.y, a2.y, a3.y, a4.y, a5.y, a6.y, a7.y));
+}
+
+// corner_quad of both components of a pair.  FP32: the differences and q + D
+// on the packed pipe, the choice and the clamp per lane.
+__device__ __forceinline__ float2 corner_quad2(float2 q, float2 far1, float2 far2, float2 out1, float2 out2, float pd,
+                                               float2 vi) {
+  typedef Pr<float> Q;
+  typedef Sel<float> S;
+  const float2 e1 = Q::sub(q, out1), e2 = Q::sub(q, out2);
+  const bool bx = abs_ge(e1.x, e2.x), by = abs_ge(e1.y, e2.y);
+  const float2 out = Q::mad(pd + pd, make_float2(bx ? e1.x : e2.x, by ? e1.y : e2.y), q);
+  const float fx = bx ? far1.x : far2.x, fy = by ? far1.y : far2.y;
+  return make_float2(within<float>(S::mn_nan(q.x, fx), S::mx(q.x, fx), q.x, out.x, vi.x),
+                     within<float>(S::mn_nan(q.y, fy), S::mx(q.y, fy), q.y, out.y, vi.y));
+}
+__device__ __forceinline__ double2 corner_quad2(double2 q, double2 far1, double2 far2, double2 out1, double2 out2,
+                                                double pd, double2 vi) {
+  return make_double2(corner_quad(q.x, far1.x, far2.x, q.x - out1.x, q.x - out2.x, pd, vi.x),
+                      corner_quad(q.y, far1.y, far2.y, q.y - out1.y, q.y - out2.y, pd, vi.y));
+}
+// corner_pdm_vals<R_PDM> of both components.
 template <typename T>
-__device__ __forceinline__ typename Pr<T>::V tap8p(typename Pr<T>::V a0, typename Pr<T>::V a1, typename Pr<T>::V a2,
-                                                    typename Pr<T>::V a3, typename Pr<T>::V a4, typename Pr<T>::V a5,
-                                                    typename Pr<T>::V a6, typename Pr<T>::V a7) {
-  typedef Pr<T> Q;
-  typename Q::V s = Q::mul(T(-3), a0);
-  s = Q::mad(T(29), a1, s);
-  s = Q::mad(T(-139), a2, s);
-  s = Q::mad(T(533), a3, s);
-  s = Q::mad(T(533), a4, s);
-  s = Q::mad(T(-139), a5, s);
-  s = Q::mad(T(29), a6, s);
-  s = Q::mad(T(-3), a7, s);
-  return Q::by(s, T(840));
+__device__ __forceinline__ void corner_pdm_vals2(
+    typename Pr<T>::V m11, typename Pr<T>::V m21, typename Pr<T>::V m12, typename Pr<T>::V m01, typename Pr<T>::V p11,
+    typename Pr<T>::V m02, typename Pr<T>::V m10, typename Pr<T>::V m20, typename Pr<T>::V m1p, typename Pr<T>::V c0,
+    typename Pr<T>::V p10, typename Pr<T>::V p01, typename Pr<T>::V vi, T pd, T& r0, T& r1) {
+  typedef typename Pr<T>::V V;
+  const V v00 = corner_quad2(m11, m01, m10, m21, m12, pd, vi);
+  const V v10 = corner_quad2(m01, m11, c0, p11, m02, pd, vi);
+  const V v01 = corner_quad2(m10, c0, m11, m20, m1p, pd, vi);
+  const V v11 = corner_quad2(c0, m10, m01, p10, p01, pd, vi);
+  r0 = T(0.25) * (v00.x + v01.x + v10.x + v11.x);
+  r1 = T(0.25) * (v00.y + v01.y + v10.y + v11.y);
 }
 
 // Compile-time knobs: MHD_FLUX_PACKED = 0 keeps the FP32 flux scalar (two
@@ -380,15 +645,21 @@ __device__ __forceinline__ float2 rsq(float2 a) { return make_float2(rsqrtf(a.x)
 }  // namespace p2
 
 // corner_pdm of both components from pair-interleaved shared memory.
-template <typename T>
+template <typename T, int RECON>
 __device__ __forceinline__ void corner_pdm_pair(const typename Pr<T>::V* __restrict__ v, int c, int s1, int s2,
                                                 typename Pr<T>::V vi, T pd, T& r0, T& r1) {
   typedef typename Pr<T>::V V;
   const V m11 = v[c - s1 - s2], m21 = v[c - 2 * s1 - s2], m12 = v[c - s1 - 2 * s2], m01 = v[c - s2];
   const V p11 = v[c + s1 - s2], m02 = v[c - 2 * s2], m10 = v[c - s1], m20 = v[c - 2 * s1];
   const V m1p = v[c - s1 + s2], c0 = v[c], p10 = v[c + s1], p01 = v[c + s2];
-  r0 = corner_pdm_vals(m11.x, m21.x, m12.x, m01.x, p11.x, m02.x, m10.x, m20.x, m1p.x, c0.x, p10.x, p01.x, vi.x, pd);
-  r1 = corner_pdm_vals(m11.y, m21.y, m12.y, m01.y, p11.y, m02.y, m10.y, m20.y, m1p.y, c0.y, p10.y, p01.y, vi.y, pd);
+  if (RECON == R_PDM) {
+    corner_pdm_vals2<T>(m11, m21, m12, m01, p11, m02, m10, m20, m1p, c0, p10, p01, vi, pd, r0, r1);
+    return;
+  }
+  r0 = corner_pdm_vals<T, RECON>(m11.x, m21.x, m12.x, m01.x, p11.x, m02.x, m10.x, m20.x, m1p.x, c0.x, p10.x, p01.x,
+                                 vi.x, pd);
+  r1 = corner_pdm_vals<T, RECON>(m11.y, m21.y, m12.y, m01.y, p11.y, m02.y, m10.y, m20.y, m1p.y, c0.y, p10.y, p01.y,
+                                 vi.y, pd);
 }
 
 // Limited corner value of v at the edge whose two transverse axes have
@@ -399,16 +670,16 @@ template <typename T, int RECON>
 __device__ __forceinline__ T corner_vel(const T* __restrict__ v, long long c, long long s1, long long s2,
                                         const Prm<T>& P) {
   T v00_0, v00_1, v10_0, v10_1, v01_0, v01_1, v11_0, v11_1;
-  if (RECON == R_PDM) {
+  if (is_pdm(RECON)) {
     // interp2_pdm (926-989): 8-tap along d1 at the 8 d2-rows, then along d2
     T g[8];
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
       const T* r = v + c + (long long)(m - 4) * s2;
-      g[m] = tap8(r[-4 * s1], r[-3 * s1], r[-2 * s1], r[-s1], r[0], r[s1], r[2 * s1], r[3 * s1]);
+      g[m] = edge_tap<T, RECON>(r[-4 * s1], r[-3 * s1], r[-2 * s1], r[-s1], r[0], r[s1], r[2 * s1], r[3 * s1]);
     }
-    T vi = tap8(g[0], g[1], g[2], g[3], g[4], g[5], g[6], g[7]);
-    return corner_pdm(v, c, s1, s2, vi, P.pdmb);
+    T vi = edge_tap<T, RECON>(g[0], g[1], g[2], g[3], g[4], g[5], g[6], g[7]);
+    return corner_pdm<T, RECON>(v, c, s1, s2, vi, P.pdmb);
   } else if (RECON == R_TVD || RECON == R_TVDMC) {
     // interp2_tvd (1037-1067) and TVD with (mhd3d2) or without (mhd3d3) shifts
     constexpr bool MC = (RECON == R_TVDMC);
@@ -836,22 +1107,29 @@ template <> struct Moments<float> {
 // kernel (x faces, y / z face tiles and column sweeps, batched or not) goes
 // through these functions, so they agree bit for bit.
 
-// The limiter of pdm2 for one stencil, given the clamped interpolant fii, the
-// one-sided differences dfl = fii - fm1, dfr = f0 - fii and the scaled cell
-// differences dfm, df0, dfp: (left, right) face states.
+// PDM states of two stencils at once (lanes .x and .y, e.g. two fields at one
+// face) from the interpolant pair fi (pdm_states): the one-sided limits on the
+// packed pipe, the clamps per lane.  lr0 / lr1 are the (left, right) states of
+// lane x / lane y.
+__device__ __forceinline__ void pdm2x2(float2 fm2, float2 fm1, float2 f0, float2 fp1, float2 fi, float pdmb,
+                                       float2& lr0, float2& lr1) {
+  const float2 k = p2::K(pdmb + pdmb);
+  const float2 outl = p2::fma(k, p2::sub(fm1, fm2), fm1);
+  const float2 outr = p2::fma(k, p2::sub(f0, fp1), f0);
+  pdm_pick(fm1.x, f0.x, outl.x, outr.x, fi.x, lr0.x, lr0.y);
+  pdm_pick(fm1.y, f0.y, outl.y, outr.y, fi.y, lr1.x, lr1.y);
+}
+
+// pdm2 of two stencils at once (R_PDMG): the differences on the packed pipe,
+// the clamp and the limiter per lane.
 __device__ __forceinline__ float2 pdm_lim(float fii, float dfl, float dfr, float dfm, float df0, float dfp) {
   const float sm = sgn1(dfm), s0 = sgn1(df0), sp = sgn1(dfp);
   const float qm = fabsf(sm + s0), qp = fabsf(s0 + sp);
   return make_float2(fii - s0 * mx(0.0f, fabsf(dfl) - qm * fabsf(dfm)),
                      fii + s0 * mx(0.0f, fabsf(dfr) - qp * fabsf(dfp)));
 }
-
-// PDM2 (mhd3d3.f90:1069-1172) of two stencils at once (lanes .x and .y, e.g.
-// two fields at one face) from the interpolant pair fi: the differences on
-// the packed pipe, the clamp and the limiter per lane.  lr0 / lr1 are the
-// (left, right) states of lane x / lane y.
-__device__ __forceinline__ void pdm2x2(float2 fm2, float2 fm1, float2 f0, float2 fp1, float2 fi, float pdmb,
-                                       float2& lr0, float2& lr1) {
+__device__ __forceinline__ void pdm2x2_ref(float2 fm2, float2 fm1, float2 f0, float2 fp1, float2 fi, float pdmb,
+                                           float2& lr0, float2& lr1) {
   const float2 kp = p2::K(pdmb);
   const float2 dfm = p2::mul(kp, p2::sub(fm1, fm2));
   const float2 df0 = p2::mul(kp, p2::sub(f0, fm1));
@@ -866,9 +1144,11 @@ __device__ __forceinline__ void pdm2x2(float2 fm2, float2 fm1, float2 f0, float2
 
 // PDM face states of two fields from their 8-tap windows (tap m = cell
 // c+m-4 for the face at the low side of cell c), packed as field pairs.
+template <int RECON>
 __device__ __forceinline__ void pdm_pair_states(const float2* a, float pdmb, float2& lr0, float2& lr1) {
-  const float2 fi = tap8p<float>(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7]);
-  pdm2x2(a[2], a[3], a[4], a[5], fi, pdmb, lr0, lr1);
+  const float2 fi = tap8p<RECON>(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7]);
+  if (RECON == R_PDM) pdm2x2(a[2], a[3], a[4], a[5], fi, pdmb, lr0, lr1);
+  else pdm2x2_ref(a[2], a[3], a[4], a[5], fi, pdmb, lr0, lr1);
 }
 
 // 0.5 erfc(-x.x) (left state, + moment) and 0.5 erfc(x.y) (right state, -
@@ -1056,9 +1336,8 @@ __device__ __forceinline__ void any_face_flux(const Dev<T>& d, long long c, cons
 template <typename T, int RECON, int PH>
 __device__ __forceinline__ void recon_win(const T* w, const Prm<T>& P, T& fl, T& fr) {
 #define TAP(m) w[((m) + PH) & 7]
-  if (RECON == R_PDM) {
-    T fi = tap8(TAP(0), TAP(1), TAP(2), TAP(3), TAP(4), TAP(5), TAP(6), TAP(7));
-    pdm2(TAP(2), TAP(3), TAP(4), TAP(5), fi, P.pdmb, fl, fr);
+  if (is_pdm(RECON)) {
+    recon_pdm8<T, RECON>(TAP(0), TAP(1), TAP(2), TAP(3), TAP(4), TAP(5), TAP(6), TAP(7), P.pdmb, fl, fr);
   } else if (RECON == R_TVD || RECON == R_TVDMC) {
     T fi = (TAP(3) + TAP(4)) / T(2);
     tvd<T, RECON == R_TVDMC>(TAP(2), TAP(3), TAP(4), TAP(5), fi, P.eps, fl, fr);
@@ -1076,7 +1355,7 @@ __device__ __forceinline__ void recon_win(const T* w, const Prm<T>& P, T& fl, T&
 // c along stride s (recon_face per field); FP32 PDM on field pairs.
 template <typename T, int RECON, typename I>
 __device__ __forceinline__ void face_states(const T* const* src, I c, I s, const Prm<T>& P, T* L, T* R) {
-  if constexpr (std::is_same<T, float>::value && RECON == R_PDM && MHD_RECON_PACKED) {
+  if constexpr (std::is_same<T, float>::value && is_pdm(RECON) && MHD_RECON_PACKED) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const float *fa = src[2 * q], *fb = src[2 * q + 1];
@@ -1084,7 +1363,7 @@ __device__ __forceinline__ void face_states(const T* const* src, I c, I s, const
 #pragma unroll
       for (int m = 0; m < 8; ++m) a[m] = make_float2(fa[c + (m - 4) * s], fb[c + (m - 4) * s]);
       float2 lr0, lr1;
-      pdm_pair_states(a, P.pdmb, lr0, lr1);
+      pdm_pair_states<RECON>(a, P.pdmb, lr0, lr1);
       L[2 * q] = lr0.x; R[2 * q] = lr0.y;
       L[2 * q + 1] = lr1.x; R[2 * q + 1] = lr1.y;
     }
@@ -1133,9 +1412,9 @@ __device__ __forceinline__ T comb(int form, T c, T xp, T x, T den) {
 // c+m-4 for the face at the low side of cell c) at col[m * RS].
 template <typename T, int RECON, int RS>
 __device__ __forceinline__ void recon_col(const T* col, const Prm<T>& P, T& fl, T& fr) {
-  if (RECON == R_PDM) {
-    T fi = tap8(col[0], col[RS], col[2 * RS], col[3 * RS], col[4 * RS], col[5 * RS], col[6 * RS], col[7 * RS]);
-    pdm2(col[2 * RS], col[3 * RS], col[4 * RS], col[5 * RS], fi, P.pdmb, fl, fr);
+  if (is_pdm(RECON)) {
+    recon_pdm8<T, RECON>(col[0], col[RS], col[2 * RS], col[3 * RS], col[4 * RS], col[5 * RS], col[6 * RS], col[7 * RS],
+                         P.pdmb, fl, fr);
   } else if (RECON == R_TVD || RECON == R_TVDMC) {
     T fi = (col[3 * RS] + col[4 * RS]) / T(2);
     tvd<T, RECON == R_TVDMC>(col[2 * RS], col[3 * RS], col[4 * RS], col[5 * RS], fi, P.eps, fl, fr);
@@ -1179,8 +1458,9 @@ constexpr bool FLUX_STAGED = MHD_FLUX_STAGED != 0;
 // Resident blocks per SM requested for the flux tiles: FP32 trades registers
 // for occupancy (latency-bound); FP64 needs about twice the registers and
 // would spill at the FP32 setting.
-template <typename T> struct FluxMinB { static constexpr int value = MHD_FLUX_MINB; };
-template <> struct FluxMinB<double> { static constexpr int value = 2; };
+// The metric mode's general normal takes more registers as well.
+template <typename T, bool M> struct FluxMinB { static constexpr int value = M ? 4 : MHD_FLUX_MINB; };
+template <bool M> struct FluxMinB<double, M> { static constexpr int value = 2; };
 
 template <typename T, int TDV = TD>
 __host__ __device__ constexpr size_t flux_t_smem() {
@@ -1261,7 +1541,7 @@ __device__ __forceinline__ void cell_update(const Dev<T>& d, int c, int cd, cons
 }
 
 template <typename T, int RECON, int D, bool M, bool B, int TDV = TD>
-__global__ void __launch_bounds__(32 * (TDV + 1), FluxMinB<T>::value)
+__global__ void __launch_bounds__(32 * (TDV + 1), FluxMinB<T, M>::value)
     k_flux_t(KArg<T, B> ka, Inp<T> in0, Prm<T> P, int form, T cw, T den, int ab) {
   constexpr int TD = TDV;
   constexpr int TROWS = TDV + 8;
@@ -1503,7 +1783,7 @@ __global__ void __launch_bounds__(128, kSweepMinB)
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         float2 lr0, lr1;
-        pdm_pair_states(w[q], P.pdmb, lr0, lr1);
+        pdm_pair_states<RECON>(w[q], P.pdmb, lr0, lr1);
         L[2 * q] = lr0.x; R[2 * q] = lr0.y;
         L[2 * q + 1] = lr1.x; R[2 * q + 1] = lr1.y;
       }
@@ -1569,8 +1849,8 @@ __device__ __forceinline__ T eta4(T a, T b, T c, T e) {
 }
 template <typename T, int E, bool M, typename I>
 __device__ __forceinline__ T emf_value(const Dev<T>& d, I c, T v1av, T v2av, T b1l, T b1r, T b2l, T b2r, T eta) {
-  const T b1u = (v2av >= T(0)) ? b1l : b1r;
-  const T b2u = (v1av >= T(0)) ? b2l : b2r;
+  const T b1u = ge0(v2av) ? b1l : b1r;
+  const T b2u = ge0(v1av) ? b2l : b2r;
   const T e = -v1av * b2u + v2av * b1u;
   if (M)  // E.dl: g_e * (convective term) + eta |dl_e| * (resistive term)
     return (T)d.m.ge[E][c] * e + eta * (T)d.m.dl[E][c] * (b1l + b2r - b1r - b2l);
@@ -1588,8 +1868,8 @@ __device__ __forceinline__ void emf_edge(const Dev<T>& d, const Inp<T>& in, cons
   const T v1av = corner_vel<T, RECON>(vel[A1], c, s1, s2, P);
   const T v2av = corner_vel<T, RECON>(vel[A2], c, s1, s2, P);
   T b1l, b1r, b2l, b2r;
-  recon_face<T, RECON>(fb[A1], c, s2, P, b1l, b1r);
-  recon_face<T, RECON>(fb[A2], c, s1, P, b2l, b2r);
+  recon_edge<T, RECON>(fb[A1], c, s2, P, b1l, b1r);
+  recon_edge<T, RECON>(fb[A2], c, s1, P, b2l, b2r);
   const T* vf = d.vf;
   const T eta = eta4(vf[c - s1 - s2], vf[c - s2], vf[c], vf[c - s1]);
   d.E[E][c] = emf_value<T, E, M>(d, c, v1av, v2av, b1l, b1r, b2l, b2r, eta);
@@ -1656,6 +1936,7 @@ inline dim3 emf_grid(int E, const Geom& g, int tx, int ty, int tz) {
 template <typename T, int E, int TX, int TY, int TZ, bool M>
 __device__ __forceinline__ void emf_pdm_tile(const Dev<T>& d, const Inp<T>& in, const Prm<T>& P, int ox, int oy,
                                              int oz) {
+  constexpr int FORM = pdm_form<T, M>();
   constexpr int A1 = (E + 1) % 3, A2 = (E + 2) % 3;
   constexpr int HX = (E == 0) ? 0 : 4, HY = (E == 1) ? 0 : 4, HZ = (E == 2) ? 0 : 4;
   constexpr int SX = TX + 2 * HX, SY = TY + 2 * HY, SZ = TZ + 2 * HZ;
@@ -1711,7 +1992,7 @@ __device__ __forceinline__ void emf_pdm_tile(const Dev<T>& d, const Inp<T>& in, 
     const int b0 = e * SE + f1 * S1 + r2 * S2;
     const int gi = e * GE + f1 * G1 + r2 * G2;
     const V* a = sv + b0;
-    sg[gi] = tap8p<T>(a[0], a[S1], a[2 * S1], a[3 * S1], a[4 * S1], a[5 * S1], a[6 * S1], a[7 * S1]);
+    sg[gi] = tap8p<FORM>(a[0], a[S1], a[2 * S1], a[3 * S1], a[4 * S1], a[5 * S1], a[6 * S1], a[7 * S1]);
   }
   __syncthreads();
   const int n0[3] = {g.nx0, g.ny0, g.nz0};
@@ -1728,14 +2009,14 @@ __device__ __forceinline__ void emf_pdm_tile(const Dev<T>& d, const Inp<T>& in, 
     const int cv = e * SE + (f1 + 4) * S1 + (f2 + 4) * S2;
     const V* gg = sg + e * GE + f1 * G1 + f2 * G2;
     constexpr int GS = G2;
-    const V vi = tap8p<T>(gg[0], gg[GS], gg[2 * GS], gg[3 * GS], gg[4 * GS], gg[5 * GS], gg[6 * GS], gg[7 * GS]);
+    const V vi = tap8p<FORM>(gg[0], gg[GS], gg[2 * GS], gg[3 * GS], gg[4 * GS], gg[5 * GS], gg[6 * GS], gg[7 * GS]);
     T v1av, v2av;
-    corner_pdm_pair<T>(sv, cv, S1, S2, vi, P.pdmb, v1av, v2av);
+    corner_pdm_pair<T, FORM>(sv, cv, S1, S2, vi, P.pdmb, v1av, v2av);
     const int c = gx + g.px * (gy + g.py * gz);
     const int s1 = st[A1], s2 = st[A2];
     T b1l, b1r, b2l, b2r;
-    recon_face<T, R_PDM>(fb[A1], c, s2, P, b1l, b1r);
-    recon_face<T, R_PDM>(fb[A2], c, s1, P, b2l, b2r);
+    recon_edge<T, FORM>(fb[A1], c, s2, P, b1l, b1r);
+    recon_edge<T, FORM>(fb[A2], c, s1, P, b2l, b2r);
     const T* vf = d.vf;
     const T eta = eta4(vf[c - s1 - s2], vf[c - s2], vf[c], vf[c - s1]);
     d.E[E][c] = emf_value<T, E, M>(d, c, v1av, v2av, b1l, b1r, b2l, b2r, eta);
@@ -1750,11 +2031,14 @@ __device__ __forceinline__ void emf_pdm_tile(const Dev<T>& d, const Inp<T>& in, 
 #ifndef MHD_EMF_FULL_OCC
 #define MHD_EMF_FULL_OCC 1
 #endif
+// FP64 takes 1024 (64 registers): its bound is the FP64 pipe, which a few
+// warps fill, and 32 registers spilled 1.4 KB per thread.
+template <typename T>
 constexpr int emf_min_blocks(int E, int NT, bool B) {
-  return !MHD_EMF_FULL_OCC ? 1 : !B ? 2048 / NT : (E == 0 ? 1024 / NT : 1536 / NT);
+  return !MHD_EMF_FULL_OCC ? 1 : sizeof(T) == 8 ? 1024 / NT : !B ? 2048 / NT : (E == 0 ? 1024 / NT : 1536 / NT);
 }
 template <typename T, int E, int TX, int TY, int TZ, int NT, bool M, bool B>
-__global__ void __launch_bounds__(NT, emf_min_blocks(E, NT, B))
+__global__ void __launch_bounds__(NT, emf_min_blocks<T>(E, NT, B))
     k_emf_pdm(KArg<T, B> ka, Inp<T> in0, Prm<T> P) {
   const int4 bb = ka.blk();
   const auto& d = ka.dev(bb);
@@ -1933,7 +2217,7 @@ __global__ void __launch_bounds__(32 * NW, MHD_EMF_STREAM_MINB)
   // first pass along a1 inside slice s (S = a2)
   auto first_a1 = [&](int s) {
     const V* a = vr + vslot(s) * NS + oi;
-    return tap8p<T>(a[-4 * TS], a[-3 * TS], a[-2 * TS], a[-TS], a[0], a[TS], a[2 * TS], a[3 * TS]);
+    return tap8p(a[-4 * TS], a[-3 * TS], a[-2 * TS], a[-TS], a[0], a[TS], a[2 * TS], a[3 * TS]);
   };
   V gw[8];
   if constexpr (SA2) {
@@ -1953,7 +2237,7 @@ __global__ void __launch_bounds__(32 * NW, MHD_EMF_STREAM_MINB)
     asm volatile("cp.async.commit_group;" ::: "memory");
     V vi;
     if constexpr (SA2) {
-      vi = tap8p<T>(gw[0], gw[1], gw[2], gw[3], gw[4], gw[5], gw[6], gw[7]);
+      vi = tap8p(gw[0], gw[1], gw[2], gw[3], gw[4], gw[5], gw[6], gw[7]);
     } else {
       // first pass along a1 = S across the ring into this warp's row
 #pragma unroll
@@ -1961,14 +2245,14 @@ __global__ void __launch_bounds__(32 * NW, MHD_EMF_STREAM_MINB)
         const int r2 = lane + 32 * h;
         if (r2 < C) {
           const int col = warp * C + r2;
-          gr[col] = tap8p<T>(vr[vslot(s - 4) * NS + col], vr[vslot(s - 3) * NS + col], vr[vslot(s - 2) * NS + col],
+          gr[col] = tap8p(vr[vslot(s - 4) * NS + col], vr[vslot(s - 3) * NS + col], vr[vslot(s - 2) * NS + col],
                              vr[vslot(s - 1) * NS + col], vr[vslot(s) * NS + col], vr[vslot(s + 1) * NS + col],
                              vr[vslot(s + 2) * NS + col], vr[vslot(s + 3) * NS + col]);
         }
       }
       __syncwarp();
       const V* gg = gr + warp * C + lane;
-      vi = tap8p<T>(gg[0], gg[1], gg[2], gg[3], gg[4], gg[5], gg[6], gg[7]);
+      vi = tap8p(gg[0], gg[1], gg[2], gg[3], gg[4], gg[5], gg[6], gg[7]);
     }
     // the 12 corner cells, (d1, d2) from the upper cell
     const V* sm2 = vr + vslot(s - 2) * NS + oi;
@@ -1983,16 +2267,14 @@ __global__ void __launch_bounds__(32 * NW, MHD_EMF_STREAM_MINB)
       m11 = sm1[-1]; m21 = sm2[-1]; m12 = sm1[-2]; m01 = s00[-1]; p11 = sp1[-1]; m02 = s00[-2];
       m10 = sm1[0]; m20 = sm2[0]; m1p = sm1[1]; c0 = s00[0]; p10 = sp1[0]; p01 = s00[1];
     }
-    const T v1av = corner_pdm_vals(m11.x, m21.x, m12.x, m01.x, p11.x, m02.x, m10.x, m20.x, m1p.x, c0.x, p10.x, p01.x,
-                                   vi.x, P.pdmb);
-    const T v2av = corner_pdm_vals(m11.y, m21.y, m12.y, m01.y, p11.y, m02.y, m10.y, m20.y, m1p.y, c0.y, p10.y, p01.y,
-                                   vi.y, P.pdmb);
+    T v1av, v2av;
+    corner_pdm_vals2<T>(m11, m21, m12, m01, p11, m02, m10, m20, m1p, c0, p10, p01, vi, P.pdmb, v1av, v2av);
     // face B: across the slice from the staged slice, along S from the window
     constexpr int BS = SA2 ? TS : 1;
     const T* bb = br + (s & 1) * NS + oi;
     T sl, sr, wl, wr;
-    recon_pdm8(bb[-4 * BS], bb[-3 * BS], bb[-2 * BS], bb[-BS], bb[0], bb[BS], bb[2 * BS], bb[3 * BS], P.pdmb, sl, sr);
-    recon_pdm8(bw[0], bw[1], bw[2], bw[3], bw[4], bw[5], bw[6], bw[7], P.pdmb, wl, wr);
+    recon_pdm8<T, R_PDM, true>(bb[-4 * BS], bb[-3 * BS], bb[-2 * BS], bb[-BS], bb[0], bb[BS], bb[2 * BS], bb[3 * BS], P.pdmb, sl, sr);
+    recon_pdm8<T, R_PDM, true>(bw[0], bw[1], bw[2], bw[3], bw[4], bw[5], bw[6], bw[7], P.pdmb, wl, wr);
     const T* f0 = fr + (s & 3) * NS + oi;
     const T* fm = fr + ((s - 1) & 3) * NS + oi;
     T eta;
@@ -2256,8 +2538,8 @@ __global__ void __launch_bounds__(NT) k_emf_weno(Dev<T> d, Inp<T> in, Prm<T> P) 
     const int c = gx + g.px * (gy + g.py * gz);
     const int s1 = st[A1], s2 = st[A2];
     T b1l, b1r, b2l, b2r;
-    recon_face<T, RECON>(fb[A1], c, s2, P, b1l, b1r);
-    recon_face<T, RECON>(fb[A2], c, s1, P, b2l, b2r);
+    recon_edge<T, RECON>(fb[A1], c, s2, P, b1l, b1r);
+    recon_edge<T, RECON>(fb[A2], c, s1, P, b2l, b2r);
     T b1u = (v2av >= T(0)) ? b1l : b1r;
     T b2u = (v1av >= T(0)) ? b2l : b2r;
     T ee = -v1av * b2u + v2av * b1u;
@@ -2873,7 +3155,8 @@ void flux_r(const Dev<T>& d, const Inp<T>& in, cudaStream_t st) {
 template <typename T, bool M>
 void Launch<T, M>::fluxes(const Dev<T>& d, const Inp<T>& in, cudaStream_t st) {
   switch (d.recon) {
-    case R_PDM: flux_r<T, R_PDM, M>(d, in, st); break;
+    case R_PDM: flux_r<T, pdm_form<T, M>(), M>(d, in, st); break;
+    case R_PDMG: flux_r<T, R_PDMG, M>(d, in, st); break;
     case R_TVD: flux_r<T, R_TVD, M>(d, in, st); break;
     case R_WENO: flux_r<T, R_WENO, M>(d, in, st); break;
     case R_MPWENO: flux_r<T, R_MPWENO, M>(d, in, st); break;
@@ -2912,7 +3195,7 @@ inline dim3 sweep_grid(int D, const Geom& g) {
 
 template <typename T, int RECON, int D, bool M>
 void flux_t_any(const Dev<T>& d, const Inp<T>& in, const Prm<T>& P, int form, T c, T den, int ab, cudaStream_t st) {
-  if constexpr (std::is_same<T, float>::value && !M) {
+  if constexpr (std::is_same<T, float>::value && !M && RECON != R_PDMG) {
     if (d.tile_td == kSweepTile) {  // column sweeps (every FP32 Cartesian reconstruction with a register window)
       static PerDevice pref;  // 4 blocks of 27 KB static shared memory
       prefer_carveout(k_flux_sweep<T, D, false, RECON>, 50, pref);
@@ -2948,7 +3231,8 @@ template <typename T, bool M>
 void Launch<T, M>::hydro(const Dev<T>& d, const Inp<T>& in, int part, int form, double c, double den, bool ab,
                          cudaStream_t st) {
   switch (d.recon) {
-    case R_PDM: hydro_r<T, R_PDM, M>(d, in, part, form, c, den, ab, st); break;
+    case R_PDM: hydro_r<T, pdm_form<T, M>(), M>(d, in, part, form, c, den, ab, st); break;
+    case R_PDMG: hydro_r<T, R_PDMG, M>(d, in, part, form, c, den, ab, st); break;
     case R_TVD: hydro_r<T, R_TVD, M>(d, in, part, form, c, den, ab, st); break;
     case R_WENO: hydro_r<T, R_WENO, M>(d, in, part, form, c, den, ab, st); break;
     case R_MPWENO: hydro_r<T, R_MPWENO, M>(d, in, part, form, c, den, ab, st); break;
@@ -3016,8 +3300,8 @@ __global__ void k_emf_yee(Dev<T> d, Prm<T> P) {
   constexpr int DB = (E == 0) ? 2 : (E == 1) ? 0 : 1;
   const int sA = st[DA], sB = st[DB];
   constexpr bool TV = (RECON == R_TVD || RECON == R_TVDMC);
-  constexpr int M0 = (RECON == R_PDM) ? 0 : TV ? 2 : 1;
-  constexpr int M1 = (RECON == R_PDM) ? 7 : TV ? 5 : 6;
+  constexpr int M0 = is_pdm(RECON) ? 0 : TV ? 2 : 1;
+  constexpr int M1 = is_pdm(RECON) ? 7 : TV ? 5 : 6;
   T part[4];
 #pragma unroll
   for (int s = 0; s < 4; ++s) {  // pp, np, pn, nn
@@ -3055,6 +3339,7 @@ template <typename T>
 void emf_yee(const Dev<T>& d, const Inp<T>& in, cudaStream_t st) {
   switch (d.recon) {
     case R_PDM: emf_yee_r<T, R_PDM>(d, in, st); break;
+    case R_PDMG: emf_yee_r<T, R_PDMG>(d, in, st); break;
     case R_TVD: emf_yee_r<T, R_TVD>(d, in, st); break;
     case R_WENO: emf_yee_r<T, R_WENO>(d, in, st); break;
     case R_MPWENO: emf_yee_r<T, R_MPWENO>(d, in, st); break;
@@ -3114,7 +3399,7 @@ void Launch<T, M>::emf(const Dev<T>& d, const Inp<T>& in0, cudaStream_t st) {
     in.vx = d.mw[0]; in.vy = d.mw[1]; in.vz = d.mw[2];
     in.bi = d.mbn[0]; in.bj = d.mbn[1]; in.bk = d.mbn[2];
   }
-  if (d.recon == R_PDM) {
+  if (d.recon == R_PDM || (d.recon == R_PDMG && pdm_form<T, M>() == R_PDMG)) {
     Prm<T> P = prm_of(d);
     if constexpr (std::is_same<T, float>::value && !M) {
       if (d.tile_ey == kEmfStream) {
@@ -3131,6 +3416,7 @@ void Launch<T, M>::emf(const Dev<T>& d, const Inp<T>& in0, cudaStream_t st) {
     return;
   }
   switch (d.recon) {
+    case R_PDMG: emf_r<T, R_PDMG, M>(d, in, st); break;
     case R_TVD: emf_r<T, R_TVD, M>(d, in, st); break;
     case R_WENO: emf_weno<T, R_WENO, M>(d, in, st); break;
     case R_MPWENO: emf_weno<T, R_MPWENO, M>(d, in, st); break;

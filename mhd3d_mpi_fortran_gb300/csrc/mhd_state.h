@@ -218,6 +218,8 @@ int mlp_correct(void* h, Dev<float>& d, cudaStream_t st);
 // MHD_E_TIMEOUT if an MLP kernel recorded a wait that gave up, else MHD_OK.
 int mlp_status(void* h);
 
+// Dev::recon of PDM with pdmb <= 0 (the general limiter; R_PDMG of the kernels).
+constexpr int kReconPdmGeneral = 6;
 // Tile lengths the autotuner tries (FP32 Cartesian PDM).
 constexpr int kSweepTile = 32;  // face-shape value of the column sweeps
 constexpr int kTileTD[4] = {4, 8, 16, kSweepTile};
