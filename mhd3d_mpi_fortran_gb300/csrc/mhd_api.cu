@@ -64,7 +64,7 @@ struct Handle {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   void* buf = nullptr;
   size_t bytes = 0;
-  double* geo = nullptr;       // dx | dy | dz (FP64)
+  double* geo = nullptr;       // FP64: dx | dy | dz, their reciprocals, the Gaussian moment rows (Dev::gtab)
   Scal* sc = nullptr;          // device scalars
   Scal* sc_h = nullptr;        // pinned mirror
   double* diag = nullptr;      // device diagnostics buffer
@@ -250,7 +250,9 @@ void enqueue_any(Handle* h, int& par, cudaStream_t st, Rec* r = nullptr) {
 
 inline void set_widths(Handle* h, Dev<double>& d) {
   d.wx = d.dx; d.wy = d.dy; d.wz = d.dz;
-  d.rwx = d.dx; d.rwy = d.dy; d.rwz = d.dz;
+  const Geom& g = h->g;
+  const double* r = h->geo + g.nx + g.ny + g.nz;
+  d.rwx = r; d.rwy = r + g.nx; d.rwz = r + g.nx + g.ny;
 }
 inline void set_widths(Handle* h, Dev<float>& d) {
   const Geom& g = h->g;
@@ -274,6 +276,7 @@ void carve(Handle* h, Dev<T>& d, char* base) {
   d.dt_mode = h->prm.dt_mode;
   for (int i = 0; i < 3; ++i) d.bc[i] = h->prm.bc[i];
   d.gam = (T)h->prm.gam; d.pdmb = (T)h->prm.pdmb; d.eps = (T)h->prm.eps;
+  d.rgm1 = (T)(1.0 / (h->prm.gam - 1.0));
   d.alpha = (T)h->prm.alpha; d.beta = (T)h->prm.beta; d.cfl = (T)h->prm.cfl;
   d.rho = next(); d.vx = next(); d.vy = next(); d.vz = next(); d.p = next();
   d.bi = next(); d.bj = next(); d.bk = next(); d.bx = next(); d.by = next(); d.bz = next();
@@ -292,6 +295,7 @@ void carve(Handle* h, Dev<T>& d, char* base) {
   d.vf = next();
   d.dx = h->geo; d.dy = h->geo + g.nx; d.dz = h->geo + g.nx + g.ny;
   set_widths(h, d);
+  d.gtab = h->geo + 2 * (g.nx + g.ny + g.nz);
   d.sc = h->sc;
   d.gmap = h->gmap;
   d.partial = nullptr;
@@ -533,6 +537,41 @@ int mhd_device_info(int32_t out[4]) {
   return MHD_OK;
 }
 
+void mhd::gauss_table(double* out) {
+  // With e(z) = exp(-z^2) / (2 sqrt(pi)): e' = -2 z e gives e's Taylor
+  // coefficients about c by a_{n+1} = -2 (c a_n + a_{n-1}) / (n + 1), and
+  // (0.5 erfc)' = -2 e gives those of 0.5 erfc from them.
+  for (unsigned i = 0; i < kGaussRows; ++i) {
+    const long double c = i / 32.0L;
+    long double a[8], prev = 0.0L;
+    a[0] = std::exp(-c * c) / (2.0L * std::sqrt(3.14159265358979323846264338327950288L));
+    for (int n = 0; n < 7; ++n) {
+      a[n + 1] = -2.0L * (c * a[n] + prev) / (n + 1);
+      prev = a[n];
+    }
+    double* h = out + 16 * i;
+    h[0] = (double)(0.5L * std::erfc(c));
+    for (int n = 0; n < 7; ++n) h[n + 1] = (double)(-2.0L * a[n] / (n + 1));
+    for (int n = 0; n < 8; ++n) h[8 + n] = (double)a[n];
+  }
+}
+
+static size_t geo_doubles(const Geom& g) { return 2 * ((size_t)g.nx + g.ny + g.nz) + 16 * (size_t)kGaussRows; }
+
+// Cell widths (dx | dy | dz), their reciprocals and the Gaussian rows to h->geo.
+static bool upload_geo(Handle* h, std::vector<double> geo) {
+  const size_t n = geo.size();
+  geo.resize(geo_doubles(h->g));
+  for (size_t i = 0; i < n; ++i) geo[n + i] = 1.0 / geo[i];
+  static const std::vector<double> rows = [] {
+    std::vector<double> r(16 * (size_t)kGaussRows);
+    gauss_table(r.data());
+    return r;
+  }();
+  std::copy(rows.begin(), rows.end(), geo.begin() + 2 * n);
+  return cudaMemcpy(h->geo, geo.data(), sizeof(double) * geo.size(), cudaMemcpyHostToDevice) == cudaSuccess;
+}
+
 // Handle with its device buffers allocated and cleared, scalars set from prm,
 // but no fields uploaded yet.
 static int create_handle(const mhd_params* prm, const double* dx, const double* dy, const double* dz,
@@ -580,7 +619,7 @@ static int create_handle(const mhd_params* prm, const double* dx, const double* 
   if (cudaMalloc(&h->buf, h->bytes) != cudaSuccess) return bail(MHD_E_NOMEM, "device allocation failed");
   if (metric && cudaMalloc(&h->met, sizeof(double) * kMetricArrays * (size_t)g.vol) != cudaSuccess)
     return bail(MHD_E_NOMEM, "device allocation of the metric failed");
-  if (cudaMalloc(&h->geo, sizeof(double) * (g.nx + g.ny + g.nz)) != cudaSuccess ||
+  if (cudaMalloc(&h->geo, sizeof(double) * geo_doubles(g)) != cudaSuccess ||
       cudaMalloc(&h->sc, sizeof(Scal)) != cudaSuccess ||
       cudaMalloc(&h->diag, sizeof(double) * (8 + 5 * 152 * 2)) != cudaSuccess)
     return bail(MHD_E_NOMEM, "device allocation failed");
@@ -595,8 +634,7 @@ static int create_handle(const mhd_params* prm, const double* dx, const double* 
   std::memcpy(geo.data() + g.nx + g.ny, dz, sizeof(double) * g.nz);
   for (double v : geo)
     if (!(v > 0.0)) return bail(MHD_E_ARG, "cell widths must be positive (diag_geom)");
-  if (cudaMemcpy(h->geo, geo.data(), sizeof(double) * geo.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-    return bail(MHD_E_CUDA, "geometry upload failed");
+  if (!upload_geo(h, geo)) return bail(MHD_E_CUDA, "geometry upload failed");
   {
     // FP32 widths and their reciprocals (1/dx computed in FP64, rounded once)
     std::vector<float> gf(geo.begin(), geo.end());
@@ -828,9 +866,9 @@ int mhd_checkpoint_load(const char* path, void** handle) {
     }
     if (id == 999) {  // cell widths (FP64)
       const size_t ng = (size_t)nx + ny + nz;
-      ok = cudaMemcpy(h->geo, buf.data(), ng * 8, cudaMemcpyHostToDevice) == cudaSuccess;
-      std::vector<float> gf(ng * 2);
       const double* w = (const double*)buf.data();
+      ok = upload_geo(h, std::vector<double>(w, w + ng));
+      std::vector<float> gf(ng * 2);
       for (size_t i = 0; i < ng; ++i) { gf[i] = (float)w[i]; gf[ng + i] = (float)(1.0 / w[i]); }
       ok = ok && cudaMemcpy(h->geoT, gf.data(), gf.size() * 4, cudaMemcpyHostToDevice) == cudaSuccess;
       ++loaded;

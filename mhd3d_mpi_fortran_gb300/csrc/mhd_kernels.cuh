@@ -101,14 +101,22 @@ template <> struct Div<float> {
   static __device__ __forceinline__ float by(float a, float b) { return a * (1.0f / b); }
 };
 
-// Divisions on the hot path: FP64 divides exactly as the reference writes
-// it; FP32 multiplies by a reciprocal (precomputed for the cell widths).
+// Divisions on the hot path.  An FP64 division takes about nine operations of
+// the FP64 pipe, the bound of every FP64 kernel, so it is kept where the
+// quotient is a result by itself (dv); by a cell width it is a multiply by the
+// reciprocal (dw, both precisions), and several quotients by one divisor share
+// its reciprocal (dvr).  FP32 multiplies by a reciprocal throughout.
 template <typename T> struct Ops;
 template <> struct Ops<double> {
-  static __device__ __forceinline__ double dw(double a, double w, double) { return a / w; }  // a / width
+  static __device__ __forceinline__ double dw(double a, double, double rw) { return a * rw; }  // a / width
   static __device__ __forceinline__ double dv(double a, double b) { return a / b; }
-  static __device__ __forceinline__ double rcp(double b) { return b; }  // used with dvr below
-  static __device__ __forceinline__ double dvr(double a, double b, double) { return a / b; }
+  static __device__ __forceinline__ double rcp(double b) { return 1.0 / b; }  // used with dvr below
+  // a / b from rb = 1 / b and one residual correction (Markstein's theorem:
+  // the rounding of the division when a rb is within one unit of it)
+  static __device__ __forceinline__ double dvr(double a, double b, double rb) {
+    const double q = a * rb;
+    return fma(fma(-q, b, a), rb, q);
+  }
 };
 template <> struct Ops<float> {
   static __device__ __forceinline__ float dw(float a, float, float rw) { return a * rw; }
@@ -626,11 +634,7 @@ __device__ __forceinline__ void corner_pdm_vals2(
   r1 = T(0.25) * (v00.y + v01.y + v10.y + v11.y);
 }
 
-// Compile-time knobs: MHD_FLUX_PACKED = 0 keeps the FP32 flux scalar (two
-// independent left / right chains), MHD_RECON_PACKED = 0 the reconstruction.
-#ifndef MHD_FLUX_PACKED
-#define MHD_FLUX_PACKED 1
-#endif
+// Compile-time knob: MHD_RECON_PACKED = 0 keeps the FP32 reconstruction scalar.
 #ifndef MHD_RECON_PACKED
 #define MHD_RECON_PACKED 1
 #endif
@@ -786,6 +790,14 @@ __device__ __forceinline__ void cell_b_metric(const Metric& m, long long c, T lo
   bz = p0 * (T)m.eb[0][2][c] + p1 * (T)m.eb[1][2][c] + p2 * (T)m.eb[2][2][c];
 }
 
+// vf = |v| + |B| / sqrt(rho) of get_eijk_LFM (1766), b2 = |B|^2.  FP64: from
+// the reciprocal of rho, which get_dt of the same cell shares.
+__device__ __forceinline__ float vf_val(float u, float v, float w, float b2, float r0) {
+  return sq(u * u + v * v + w * w) + sq(b2 / r0);
+}
+__device__ __forceinline__ double vf_val(double u, double v, double w, double b2, double r0) {
+  return sqrt(u * u + v * v + w * w) + sqrt(b2 * (1.0 / r0));
+}
 // get_bxyz over all cells (incl. ghosts) and vf = |v| + |B|/sqrt(rho).
 template <typename T, bool M>
 __global__ void k_bxyz_vf(Dev<T> d, int want_vf) {
@@ -808,7 +820,7 @@ __global__ void k_bxyz_vf(Dev<T> d, int want_vf) {
   d.bz[c] = bz;
   if (want_vf) {
     T u = d.vx[c], v = d.vy[c], w = d.vz[c];
-    d.vf[c] = sq(u * u + v * v + w * w) + sq((bx * bx + by * by + bz * bz) / d.rho[c]);
+    d.vf[c] = vf_val(u, v, w, bx * bx + by * by + bz * bz, d.rho[c]);
   }
 }
 
@@ -819,17 +831,26 @@ __global__ void k_bxyz_vf(Dev<T> d, int want_vf) {
 __device__ __forceinline__ double cfl_sqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float cfl_sqrt(float x) { return x > 0.0f ? x * rsqrtf(x) : 0.0f; }
 
+// |v| + fast speed sqrt(B^2 / rho + gam p / rho); FP64 takes one root and one
+// reciprocal for the second term (three roots and two divisions as written in get_dt).
+__device__ __forceinline__ float cfl_speed(float gam, float r0, float p0, float u, float v, float w, float b2) {
+  typedef Ops<float> O;
+  const float vv = cfl_sqrt(u * u + v * v + w * w);
+  const float valf = O::dv(cfl_sqrt(b2), cfl_sqrt(r0));
+  const float vs = cfl_sqrt(O::dv(gam * p0, r0));
+  return vv + cfl_sqrt(valf * valf + vs * vs);
+}
+__device__ __forceinline__ double cfl_speed(double gam, double r0, double p0, double u, double v, double w, double b2) {
+  return sqrt(u * u + v * v + w * w) + sqrt((b2 + gam * p0) * (1.0 / r0));
+}
+
 // get_dt of one cell (mhd3d3.f90:1608-1639) from its primitives and cell B,
 // with the status bits of its values.
 template <typename T, bool M>
 __device__ __forceinline__ T cell_dt(const Dev<T>& d, int c, int i, int j, int k, T r0, T p0, T u, T v, T w, T a,
                                      T b, T cc, unsigned& st) {
   typedef Ops<T> O;
-  T vv = cfl_sqrt(u * u + v * v + w * w);
-  T btot = cfl_sqrt(a * a + b * b + cc * cc);
-  T valf = O::dv(btot, cfl_sqrt(r0));
-  T vs = cfl_sqrt(O::dv(d.gam * p0, r0));
-  T vcfl = vv + cfl_sqrt(valf * valf + vs * vs);
+  const T vcfl = cfl_speed(d.gam, r0, p0, u, v, w, a * a + b * b + cc * cc);
   T dt;
   if (M)  // metric mode: 1/dx_a -> |mean area vector of the a-faces| / V
     dt = O::dv(d.cfl, O::dw(vcfl * (T)d.m.sa[c], (T)d.m.vol[c], (T)d.m.rvol[c]));
@@ -873,6 +894,10 @@ __device__ __forceinline__ void dt_next_accumulate(Scal* sc, T m, unsigned st) {
   }
 }
 
+// p / (gam - 1): FP64 by the reciprocal (Dev::rgm1).
+__device__ __forceinline__ float over_gm1(const Dev<float>& d, float p) { return Ops<float>::dv(p, d.gam - 1.0f); }
+__device__ __forceinline__ double over_gm1(const Dev<double>& d, double p) { return p * d.rgm1; }
+
 // save != 0 also stores U^n of the RK stage combines (advance_previous,
 // 3794-3819) at interior cells and faces, the only places they are read.
 // next != 0: the dt and status go to the next-step accumulators.
@@ -884,8 +909,6 @@ __global__ void __launch_bounds__(256, pass_min_blocks(B)) k_cfl(KArg<T, B> ka, 
   const Geom& g = d.g;
   T m = T(INFINITY);
   unsigned st = 0;
-  const T gm1 = d.gam - T(1);
-  typedef Ops<T> O;
   const int i = bb.y * 32 + (threadIdx.x & 31);
   const int j = bb.z * 8 + (threadIdx.x >> 5);
   const int k1 = min(g.nz, (bb.w + 1) * 8);
@@ -901,7 +924,7 @@ __global__ void __launch_bounds__(256, pass_min_blocks(B)) k_cfl(KArg<T, B> ka, 
         d.q[1][c] = r0 * u;
         d.q[2][c] = r0 * v;
         d.q[3][c] = r0 * w;
-        d.q[4][c] = T(0.5) * r0 * (u * u + v * v + w * w) + O::dv(p0, gm1);
+        d.q[4][c] = T(0.5) * r0 * (u * u + v * v + w * w) + over_gm1(d, p0);
       }
       const bool fx = i >= g.ng && i <= g.ng + g.nx0, fy = j >= g.ng && j <= g.ng + g.ny0,
                  fz = k >= g.ng && k <= g.ng + g.nz0;
@@ -1217,69 +1240,121 @@ __device__ __forceinline__ void face_flux_lr(const float2* X, float gam, float* 
   for (int q = 0; q < 8; ++q) out[q] = f[q].x + f[q].y;
 }
 
+// ------------------------------------------------------- FP64 moments
+// 0.5 erfc(|z|) and exp(-z^2) / (2 sqrt(pi)) from one table of Taylor
+// polynomials (d.gtab: row i about c = i / 32, eight coefficients of each;
+// gauss_table() fills it).  CUDA's erfc and exp take about 60 and 20 operations
+// of the FP64 pipe; here the row index and the offset from its centre take
+// three and each polynomial seven.  The offset is at most 1/64, where the first
+// term left out is below 5e-17 of either function's largest value; beyond
+// |z| = 6.5 both are below 1e-19 and are taken as zero (NaN stays NaN).
+// In v1 = v v0 +- b the two terms cancel in the tails, so that an absolute error of
+// this size is what the moments carried before as well.
+struct GaussArg {
+  const double2* row;
+  double d;
+  int far;  // 0: in the table, 1: beyond it, 2: NaN
+  __device__ __forceinline__ GaussArg(const double* tab, double z) {
+    const double az = abs_bits(z);
+    const double t = fma(az, 32.0, 6755399441055744.0);  // 1.5 * 2^52: the nearest integer in the low word
+    d = fma(t - 6755399441055744.0, -0.03125, az);
+    const int hi = __double2hiint(az);
+    far = hi < 0x401a0000 ? 0 : hi <= 0x7ff00000 ? 1 : 2;
+    const unsigned i = (unsigned)__double2loint(t);
+    row = reinterpret_cast<const double2*>(tab) + (i < kGaussRows ? i : kGaussRows - 1) * 8;
+  }
+  __device__ __forceinline__ double poly(const double2* q, double z) const {
+    const double2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2), e = __ldg(q + 3);
+    double s = fma(e.y, d, e.x);
+    s = fma(fma(s, d, c.y), d, c.x);
+    s = fma(fma(s, d, b.y), d, b.x);
+    s = fma(fma(s, d, a.y), d, a.x);
+    return far == 0 ? s : far == 1 ? 0.0 : z;
+  }
+  // 0.5 erfc(-z) for the left (+ moment) or 0.5 erfc(z) for the right state
+  __device__ __forceinline__ double half_erfc(double z, bool left) const {
+    const double h = poly(row, z);
+    const bool direct = (__double2hiint(z) < 0) == left;
+    return direct ? h : 1.0 - h;
+  }
+  __device__ __forceinline__ double bell(double z) const { return poly(row + 4, z); }
+};
+
+// One side (left: + moments) of the FP64 flux through a face normal to axis D:
+// the formulas of face_flux with sqrt(lam) = rho / sqrt(2 p rho), the shared
+// products formed once and fused operations.  About 85 operations of the
+// FP64 pipe; as written in the reference, with two divisions, a root, an exp
+// and two erfc per side, about 240.
+template <int D>
+__device__ __forceinline__ void face_side64(const double* q, const Dev<double>& dv, bool left, double* f) {
+  const double r = q[0], u = q[1], v = q[2], w = q[3], p = q[4], x = q[5], y = q[6], z = q[7];
+  const double vn = q[1 + D], bn = q[5 + D];
+  const double ke = fma(u, u, fma(v, v, w * w)), p2 = p + p;
+  const double s = rsqrt(p2 * r);
+  const double a = (r * s) * vn;
+  const GaussArg ga(dv.gtab, a);
+  const double v0 = ga.half_erfc(a, left);
+  const double b = (p2 * s) * ga.bell(a);
+  const double v1 = fma(vn, v0, left ? b : -b);
+  const double m = r * v1, pv = p * v0;
+  f[0] = m;
+  f[1] = m * u;
+  f[2] = m * v;
+  f[3] = m * w;
+  f[1 + D] += pv;
+  f[4] = fma(fma(0.5 * ke, r, p * (dv.rgm1 + 0.5)), v1, (0.5 * vn) * pv);
+  const double b2 = fma(x, x, fma(y, y, z * z));
+  const double am = (r * rsqrt((p2 + b2) * r)) * vn;
+  const double m0 = GaussArg(dv.gtab, am).half_erfc(am, left);
+  const double t = -bn * m0;
+  f[5] = x * t;
+  f[6] = y * t;
+  f[7] = z * t;
+  f[5 + D] = fma(0.5 * b2, m0, f[5 + D]);
+}
+
 // Fluxes and magnetic stress through one face normal to axis D from the
 // reconstructed left (l) and right (r) states {rho, vx, vy, vz, p, bx, by, bz}
 // (get_flux_stress, mhd3d3.f90:2385-2560): out = {rho, rvx, rvy, rvz, eng,
 // s_x, s_y, s_z}.  Left state with the + moments, right with the - moments.
 // FP32: on the packed pipe (face_flux_lr).
-template <typename T, int D>
-__device__ __forceinline__ void face_flux(const T* l, const T* r, T gam, T* out) {
-  if constexpr (std::is_same<T, float>::value && MHD_FLUX_PACKED) {
-    float2 X[8];
+// FP64: face_side64 per side.
+template <int D>
+__device__ __forceinline__ void face_flux(const float* l, const float* r, const Dev<float>& d, float* out) {
+  float2 X[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) X[q] = make_float2(l[q], r[q]);
-    face_flux_lr<D>(X, gam, out);
-    return;
-  }
-  typedef Moments<T> M;
-  const T gm1 = gam - T(1);
-  {
-    T rl = l[0], ul = l[1], vl = l[2], wl = l[3], pl = l[4], xl = l[5], yl = l[6], zl = l[7];
-    T vn = l[1 + D];
-    T bn = l[5 + D];
-    T leng = T(0.5) * rl * (ul * ul + vl * vl + wl * wl) + Ops<T>::dv(pl, gm1);
-    T lam = M::div(rl, T(2) * pl);
-    T v0, v1;
-    M::hydro(lam, vn, true, v0, v1);
-    out[0] = rl * v1;
-    out[1] = rl * ul * v1;
-    out[2] = rl * vl * v1;
-    out[3] = rl * wl * v1;
-    out[4] = (leng + T(0.5) * pl) * v1;
-    out[1 + D] = out[1 + D] + pl * v0;
-    out[4] = out[4] + T(0.5) * pl * vn * v0;
-    T lbsq = xl * xl + yl * yl + zl * zl;
-    lam = M::div(rl, T(2) * pl + lbsq);
-    v0 = M::mag(lam, vn, true);
-    out[5] = ((D == 0) ? (T(0.5) * lbsq - xl * xl) : (-xl * bn)) * v0;
-    out[6] = ((D == 1) ? (T(0.5) * lbsq - yl * yl) : (-yl * bn)) * v0;
-    out[7] = ((D == 2) ? (T(0.5) * lbsq - zl * zl) : (-zl * bn)) * v0;
-  }
-  {
-    T rr = r[0], ur = r[1], vr = r[2], wr = r[3], pr = r[4], xr = r[5], yr = r[6], zr = r[7];
-    T vn = r[1 + D];
-    T bn = r[5 + D];
-    T leng = T(0.5) * rr * (ur * ur + vr * vr + wr * wr) + Ops<T>::dv(pr, gm1);
-    T lam = M::div(rr, T(2) * pr);
-    T v0, v1;
-    M::hydro(lam, vn, false, v0, v1);
-    T f[8];
-    f[0] = rr * v1;
-    f[1] = rr * ur * v1;
-    f[2] = rr * vr * v1;
-    f[3] = rr * wr * v1;
-    f[4] = (leng + T(0.5) * pr) * v1;
-    f[1 + D] = f[1 + D] + pr * v0;
-    f[4] = f[4] + T(0.5) * pr * vn * v0;
-    T lbsq = xr * xr + yr * yr + zr * zr;
-    lam = M::div(rr, T(2) * pr + lbsq);
-    v0 = M::mag(lam, vn, false);
-    f[5] = ((D == 0) ? (T(0.5) * lbsq - xr * xr) : (-xr * bn)) * v0;
-    f[6] = ((D == 1) ? (T(0.5) * lbsq - yr * yr) : (-yr * bn)) * v0;
-    f[7] = ((D == 2) ? (T(0.5) * lbsq - zr * zr) : (-zr * bn)) * v0;
+  for (int q = 0; q < 8; ++q) X[q] = make_float2(l[q], r[q]);
+  face_flux_lr<D>(X, d.gam, out);
+}
+template <int D>
+__device__ __forceinline__ void face_flux(const double* l, const double* r, const Dev<double>& d, double* out) {
+  double f[8];
+  face_side64<D>(l, d, true, out);
+  face_side64<D>(r, d, false, f);
 #pragma unroll
-    for (int q = 0; q < 8; ++q) out[q] = out[q] + f[q];
-  }
+  for (int q = 0; q < 8; ++q) out[q] = out[q] + f[q];
+}
+
+// Moments of one face state (get_v_face): lam = rho / (2 p), and for the
+// magnetic stress lam = rho / p2.
+__device__ __forceinline__ void face_moments(const Dev<float>&, float r, float p, float vn, bool left, float& v0,
+                                             float& v1) {
+  Moments<float>::hydro(Moments<float>::div(r, 2.0f * p), vn, left, v0, v1);
+}
+__device__ __forceinline__ float face_moment_mag(const Dev<float>&, float r, float p2, float vn, bool left) {
+  return Moments<float>::mag(Moments<float>::div(r, p2), vn, left);
+}
+__device__ __forceinline__ void face_moments(const Dev<double>& d, double r, double p, double vn, bool left, double& v0,
+                                             double& v1) {
+  const double p2 = p + p, s = rsqrt(p2 * r), a = (r * s) * vn;
+  const GaussArg ga(d.gtab, a);
+  v0 = ga.half_erfc(a, left);
+  const double b = (p2 * s) * ga.bell(a);
+  v1 = fma(vn, v0, left ? b : -b);
+}
+__device__ __forceinline__ double face_moment_mag(const Dev<double>& d, double r, double p2, double vn, bool left) {
+  const double a = (r * rsqrt(p2 * r)) * vn;
+  return GaussArg(d.gtab, a).half_erfc(a, left);
 }
 
 // Metric-mode flux through a face of unit normal n and area am: the
@@ -1287,9 +1362,7 @@ __device__ __forceinline__ void face_flux(const T* l, const T* r, T gam, T* out)
 // momentum and magnetic stress), left with the + moments and right with the
 // - moments, the sum multiplied by am (the oracle's get_flux_stress_metric).
 template <typename T>
-__device__ __forceinline__ void face_flux_n(const T* l, const T* r, T gam, const T* n, T am, T* out) {
-  typedef Moments<T> Mo;
-  const T gm1 = gam - T(1);
+__device__ __forceinline__ void face_flux_n(const T* l, const T* r, const Dev<T>& d, const T* n, T am, T* out) {
   T tot[8];
 #pragma unroll
   for (int side = 0; side < 2; ++side) {
@@ -1297,10 +1370,9 @@ __device__ __forceinline__ void face_flux_n(const T* l, const T* r, T gam, const
     const T rr = s[0], u0 = s[1], u1 = s[2], u2 = s[3], pr = s[4], b0 = s[5], b1 = s[6], b2 = s[7];
     const T vn = u0 * n[0] + u1 * n[1] + u2 * n[2];
     const T bn = b0 * n[0] + b1 * n[1] + b2 * n[2];
-    const T leng = T(0.5) * rr * (u0 * u0 + u1 * u1 + u2 * u2) + Ops<T>::dv(pr, gm1);
-    T lam = Mo::div(rr, T(2) * pr);
+    const T leng = T(0.5) * rr * (u0 * u0 + u1 * u1 + u2 * u2) + over_gm1(d, pr);
     T v0, v1;
-    Mo::hydro(lam, vn, side == 0, v0, v1);
+    face_moments(d, rr, pr, vn, side == 0, v0, v1);
     T f[8];
     f[0] = rr * v1;
     f[1] = rr * u0 * v1 + pr * n[0] * v0;
@@ -1308,8 +1380,7 @@ __device__ __forceinline__ void face_flux_n(const T* l, const T* r, T gam, const
     f[3] = rr * u2 * v1 + pr * n[2] * v0;
     f[4] = (leng + T(0.5) * pr) * v1 + T(0.5) * pr * vn * v0;
     const T lbsq = b0 * b0 + b1 * b1 + b2 * b2;
-    lam = Mo::div(rr, T(2) * pr + lbsq);
-    v0 = Mo::mag(lam, vn, side == 0);
+    v0 = face_moment_mag(d, rr, T(2) * pr + lbsq, vn, side == 0);
     f[5] = (T(0.5) * lbsq * n[0] - b0 * bn) * v0;
     f[6] = (T(0.5) * lbsq * n[1] - b1 * bn) * v0;
     f[7] = (T(0.5) * lbsq * n[2] - b2 * bn) * v0;
@@ -1325,9 +1396,9 @@ template <typename T, int D, bool M>
 __device__ __forceinline__ void any_face_flux(const Dev<T>& d, long long c, const T* L, const T* R, T* out) {
   if (M) {
     const T n[3] = {(T)d.m.nrm[D][0][c], (T)d.m.nrm[D][1][c], (T)d.m.nrm[D][2][c]};
-    face_flux_n<T>(L, R, d.gam, n, (T)d.m.am[D][c], out);
+    face_flux_n<T>(L, R, d, n, (T)d.m.am[D][c], out);
   } else {
-    face_flux<T, D>(L, R, d.gam, out);
+    face_flux<D>(L, R, d, out);
   }
 }
 
@@ -1401,11 +1472,17 @@ __global__ void k_flux(KArg<T, B> ka, Inp<T> in0, Prm<T> P) {
 
 // Stage combine of the RK steps (mhd3d3.f90:3674-3702, 3745-3788):
 // form 0: (Xp+X)/den, 1: (c*Xp+X)/den, 2: (Xp+c*X)/den.
-template <typename T>
-__device__ __forceinline__ T comb(int form, T c, T xp, T x, T den) {
-  if (form == 0) return Ops<T>::dv(xp + x, den);
-  if (form == 1) return Ops<T>::dv(c * xp + x, den);
-  return Ops<T>::dv(xp + c * x, den);
+// FP64: the divisors are 2, 4 and 3 (forms 0, 1, 2), an exact scaling or two
+// operations with the division's rounding (div_by).
+__device__ __forceinline__ float comb(int form, float c, float xp, float x, float den) {
+  if (form == 0) return Ops<float>::dv(xp + x, den);
+  if (form == 1) return Ops<float>::dv(c * xp + x, den);
+  return Ops<float>::dv(xp + c * x, den);
+}
+__device__ __forceinline__ double comb(int form, double c, double xp, double x, double) {
+  if (form == 0) return 0.5 * (xp + x);
+  if (form == 1) return 0.25 * (c * xp + x);
+  return div_by<3>(xp + c * x);
 }
 
 // One-sided states from a column of taps in shared memory: tap m (cell
@@ -1493,7 +1570,7 @@ __device__ __forceinline__ void cell_update_vals(const Dev<T>& d, int c, int cd,
   // get_conserve of the current state (AB: the state, not the prediction)
   T rr = pv[0], u = pv[1], v = pv[2], ww = pv[3], pr = pv[4];
   T rvx0 = rr * u, rvy0 = rr * v, rvz0 = rr * ww;
-  T eng0 = T(0.5) * rr * (u * u + v * v + ww * ww) + Ops<T>::dv(pr, gm1);
+  T eng0 = T(0.5) * rr * (u * u + v * v + ww * ww) + over_gm1(d, pr);
   if (form == FORM_SAVE) {  // U^n of the step (this first stage's input), read by the later stages' combines
     d.q[0][c] = rr;
     d.q[1][c] = rvx0;
@@ -1796,7 +1873,7 @@ __global__ void __launch_bounds__(128, kSweepMinB)
         recon_win<T, RECON, 0>(wv, P, L[v], R[v]);
       }
     }
-    face_flux<T, D>(L, R, d.gam, F);
+    face_flux<D>(L, R, d, F);
     if (cd > c0) {
       const int cc = cd - 1;
       const int c = col + cc * s;
@@ -2794,7 +2871,7 @@ __device__ __forceinline__ T fill_bxyz_elem(const Dev<T>& d, int4 bb, int want_v
     d.bz[c] = bz;
     if (want_vf || want_dt) {
       const T u = d.vx[c], v = d.vy[c], w = d.vz[c], r0 = d.rho[c];
-      if (want_vf) d.vf[c] = sq(u * u + v * v + w * w) + sq((bx * bx + by * by + bz * bz) / r0);
+      if (want_vf) d.vf[c] = vf_val(u, v, w, bx * bx + by * by + bz * bz, r0);
       if (want_dt) return cell_dt<T, M>(d, c, i, j, k, r0, d.p[c], u, v, w, bx, by, bz, st);
     }
     return T(INFINITY);
@@ -2857,7 +2934,7 @@ __device__ __forceinline__ T fill_bxyz_elem(const Dev<T>& d, int4 bb, int want_v
   d.bx[c] = bx;
   d.by[c] = by;
   d.bz[c] = bz;
-  if (want_vf) d.vf[c] = sq(ux * ux + uy * uy + uz * uz) + sq((bx * bx + by * by + bz * bz) / r0);
+  if (want_vf) d.vf[c] = vf_val(ux, uy, uz, bx * bx + by * by + bz * bz, r0);
   return want_dt ? cell_dt<T, M>(d, c, i, j, k, r0, p0, ux, uy, uz, bx, by, bz, st) : T(INFINITY);
 }
 
@@ -2951,7 +3028,7 @@ __global__ void __launch_bounds__(256, pass_min_blocks(B))
     d.bz[c] = bz;
     if (want_vf || want_dt) {
       const T u = d.ovx[c], v = d.ovy[c], w = d.ovz[c], r0 = d.orho[c];
-      if (want_vf) d.vf[c] = sq(u * u + v * v + w * w) + sq((bx * bx + by * by + bz * bz) / r0);
+      if (want_vf) d.vf[c] = vf_val(u, v, w, bx * bx + by * by + bz * bz, r0);
       if (want_dt) m = cell_dt<T, false>(d, c, i, j, k, r0, d.op[c], u, v, w, bx, by, bz, st);
     }
   }
@@ -3553,12 +3630,16 @@ void Batch<T>::parts(const BatchView& v, int sel, int which, int form, double c,
     const Inp<T> none{};
     k_flux<T, R_PDM, 0, false, true><<<v.nblk[BF_FLUX_X], 128, 0, st>>>(KArg<T, true>{tab, v.map[BF_FLUX_X]}, none,
                                                                        P);
-    if (F32 && v.tile_td == kSweepTile) {
-      k_flux_sweep<T, 1, true><<<v.nblk[BF_FLUX_Y], dim3(32, 4), 0, st>>>(KArg<T, true>{tab, v.map[BF_FLUX_Y]}, none,
-                                                                           P, -1, T(0), T(1));
-      k_flux_sweep<T, 2, true><<<v.nblk[BF_FLUX_Z], dim3(32, 4), 0, st>>>(KArg<T, true>{tab, v.map[BF_FLUX_Z]}, none,
-                                                                           P, form, (T)c, (T)den);
-    } else if (F32 && v.tile_td == 4) batch_flux_t<T, F32 ? 4 : TD>(v, tab, P, form, (T)c, (T)den, st);
+    if constexpr (F32) {
+      if (v.tile_td == kSweepTile) {
+        k_flux_sweep<T, 1, true><<<v.nblk[BF_FLUX_Y], dim3(32, 4), 0, st>>>(KArg<T, true>{tab, v.map[BF_FLUX_Y]}, none,
+                                                                             P, -1, T(0), T(1));
+        k_flux_sweep<T, 2, true><<<v.nblk[BF_FLUX_Z], dim3(32, 4), 0, st>>>(KArg<T, true>{tab, v.map[BF_FLUX_Z]}, none,
+                                                                             P, form, (T)c, (T)den);
+        return parts(v, sel, which & 4, form, c, den, st);
+      }
+    }
+    if (F32 && v.tile_td == 4) batch_flux_t<T, F32 ? 4 : TD>(v, tab, P, form, (T)c, (T)den, st);
     else if (F32 && v.tile_td == 16) batch_flux_t<T, F32 ? 16 : TD>(v, tab, P, form, (T)c, (T)den, st);
     else batch_flux_t<T, TD>(v, tab, P, form, (T)c, (T)den, st);
   }
