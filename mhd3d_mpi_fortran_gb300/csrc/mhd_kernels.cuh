@@ -26,16 +26,9 @@
 
 namespace mhd {
 
-// R_PDMG: PDM evaluated as the reference writes the interpolant and the
-// limiter.  R_PDM (interval form) needs a limiter constant pdmb > 0, so carve()
-// picks R_PDMG otherwise; and the FP32 metric mode uses it throughout: its face
-// fluxes are small differences of B.A-sized terms, so that the last bits of a
-// reconstruction appear at 1e-5 to 1e-4 of the weak components (bz of the blast: 5e-5
-// between the two forms, 4e-4 of either against FP64).
+// R_PDMG: PDM with a limiter constant pdmb that is not positive (carve() picks
+// it), evaluated as the reference writes the limiter; R_PDM needs pdmb > 0.
 enum { R_PDM = 1, R_TVD = 2, R_WENO = 3, R_MPWENO = 4, R_TVDMC = 5, R_PDMG = 6 };
-template <typename T, bool M> constexpr int pdm_form() {
-  return M && std::is_same<T, float>::value ? R_PDMG : R_PDM;
-}
 enum { BC_PERIODIC = 0, BC_EVEN = 1, BC_REFLECT = 2, BC_OUTFLOW = 3 };
 enum { EMF_LFM = 0, EMF_YEE = 1 };
 
@@ -104,11 +97,16 @@ template <> struct Div<float> {
 // Divisions on the hot path.  An FP64 division takes about nine operations of
 // the FP64 pipe, the bound of every FP64 kernel, so it is kept where the
 // quotient is a result by itself (dv); by a cell width it is a multiply by the
-// reciprocal (dw, both precisions), and several quotients by one divisor share
-// its reciprocal (dvr).  FP32 multiplies by a reciprocal throughout.
+// reciprocal (dc, both precisions), and several quotients by one divisor share
+// its reciprocal (dvr).  FP32 multiplies by a reciprocal throughout.  The FP64
+// metric mode divides (dw) and keeps the reference's roundings everywhere: its
+// blast is symmetric to the last bit, and where two slopes tie the corner
+// limiter's choice follows the rounding (8 faces of bk move by 1e-7 of 1e-6 in
+// the second step after a change of 1e-16).
 template <typename T> struct Ops;
 template <> struct Ops<double> {
-  static __device__ __forceinline__ double dw(double a, double, double rw) { return a * rw; }  // a / width
+  static __device__ __forceinline__ double dw(double a, double w, double) { return a / w; }     // metric mode: a / V
+  static __device__ __forceinline__ double dc(double a, double, double rw) { return a * rw; }  // a / width
   static __device__ __forceinline__ double dv(double a, double b) { return a / b; }
   static __device__ __forceinline__ double rcp(double b) { return 1.0 / b; }  // used with dvr below
   // a / b from rb = 1 / b and one residual correction (Markstein's theorem:
@@ -120,49 +118,57 @@ template <> struct Ops<double> {
 };
 template <> struct Ops<float> {
   static __device__ __forceinline__ float dw(float a, float, float rw) { return a * rw; }
+  static __device__ __forceinline__ float dc(float a, float, float rw) { return a * rw; }
   static __device__ __forceinline__ float dv(float a, float b) { return __fdividef(a, b); }
   static __device__ __forceinline__ float rcp(float b) { return __frcp_rn(b); }
   static __device__ __forceinline__ float dvr(float a, float, float rb) { return a * rb; }
 };
 
 // 8-point centred interpolant (interp_pdm, mhd3d3.f90:866-872):
-// (-3, 29, -139, 533, 533, -139, 29, -3) / 840, as eight fused operations
-// with the coefficients divided by 840 beforehand, the smallest first.
-// Against the exact sum its rms error is 0.4-0.5 of what the integer
-// coefficients with a final division gave (FP32, smooth and random taps:
-// 0.32-0.51 against 0.79-1.26 units of 2^-24), because the rounding of the
-// large terms happens once, at the end.
-template <typename T> struct Tap {
-  static constexpr T c0 = T(-3.0 / 840.0), c1 = T(29.0 / 840.0), c2 = T(-139.0 / 840.0), c3 = T(533.0 / 840.0);
-};
-__device__ __forceinline__ float fm(float a, float b, float c) { return fmaf(a, b, c); }
-__device__ __forceinline__ double fm(double a, double b, double c) { return fma(a, b, c); }
-template <typename T>
-__device__ __forceinline__ T tap8(T a0, T a1, T a2, T a3, T a4, T a5, T a6, T a7) {
-  typedef Tap<T> C;
-  T s = fm(C::c0, a7, C::c0 * a0);
-  s = fm(C::c1, a6, fm(C::c1, a1, s));
-  s = fm(C::c2, a5, fm(C::c2, a2, s));
-  return fm(C::c3, a4, fm(C::c3, a3, s));
+// (-3, 29, -139, 533, 533, -139, 29, -3) / 840.  tap8: the reference's operand
+// order (FP32 contracted, with a reciprocal multiply in place of the division;
+// FP64 see div_by).  tap8_fused (FP64 face fluxes): eight fused operations with
+// the coefficients divided beforehand, the smallest first, so that the rounding
+// of the large terms happens once, at the end (rms error 0.4 of the reference
+// order's on smooth and random taps).
+__device__ __forceinline__ float tap8(float a0, float a1, float a2, float a3, float a4, float a5, float a6, float a7) {
+  float s = fmaf(29.0f, a1, -3.0f * a0);
+  s = fmaf(533.0f, a3, fmaf(-139.0f, a2, s));
+  s = fmaf(-139.0f, a5, fmaf(533.0f, a4, s));
+  s = fmaf(-3.0f, a7, fmaf(29.0f, a6, s));
+  return s * (1.0f / 840.0f);
+}
+__device__ __forceinline__ double tap8_fused(double a0, double a1, double a2, double a3, double a4, double a5, double a6,
+                                             double a7) {
+  constexpr double c0 = -3.0 / 840.0, c1 = 29.0 / 840.0, c2 = -139.0 / 840.0, c3 = 533.0 / 840.0;
+  double s = fma(c0, a7, c0 * a0);
+  s = fma(c1, a6, fma(c1, a1, s));
+  s = fma(c2, a5, fma(c2, a2, s));
+  return fma(c3, a4, fma(c3, a3, s));
 }
 
-// PDM2 (mhd3d3.f90:1069-1172) for pdmb > 0, without its signs.  With
-// D(c, f) = 2 pdmb (c - f), the limiter's left state is the interpolant
-// clamped to [fm1, f0] and then kept within [fm1, fm1 + D(fm1, fm2)] -- the
-// reference's fii - s0 max(0, |fii - fm1| - |sm + s0| |dfm|) is exactly that:
-// |sm + s0| is 2 where the two slopes agree and 0 where they do not, and in the
-// latter case the two intervals share only fm1.  The right state is the mirror
-// image about f0.  So each state is one value x held within two intervals
-// that share an end c (the near cell):
-//   within(c, far, out, x), far the cell across the face, out = c + D(c, outer).
-// A limited state is one rounding of c + D instead of three, and the branch
-// decisions are minima and maxima.  NaN: the near cells reach the result as in
-// the reference's form (NaN-propagating min / max on the lower end), a NaN
-// that is only in the interpolant is dropped by the clamp there as here.
+// PDM2 (mhd3d3.f90:1069-1172) for pdmb > 0, without its signs: the
+// interpolant fi clamped to the two near cells gives x, and with D(c, f) = 2
+// pdmb (c - f) the left state is x kept within [fm1, fm1 + D(fm1, fm2)] -- the
+// reference's x - s0 max(0, |x - fm1| - |sm + s0| |dfm|) is exactly that: |sm +
+// s0| is 2 where the two slopes agree and 0 where they do not, and in the latter
+// case the two intervals share only fm1.  The right state is the mirror image
+// about f0.
 //
-// FP32: two- and three-operand FMNMX.  FP64: FP64 comparisons share the FP64
-// pipe (2 lanes per SM and cycle, a 32nd of the integer pipe), so minima and
-// maxima run on order-preserving integer images of the values.
+// FP32 keeps the bits of the reference's form (the corner limiter picks the
+// larger of two slopes, so a last bit elsewhere can move a cell by 1e-3 within
+// a hundred steps): the excess of the displacement d = x - near over D, a soft
+// threshold, is d - (d and D of one sign ? the smaller magnitude : 0), the
+// product of signs and the smaller magnitude being one instruction (FMNMX with
+// xorsign); the same roundings as |d| - |sm + s0| |dfm| and the final
+// difference.  24 instructions per state pair and field instead of 35.
+//
+// FP64: comparisons share the FP64 pipe (2 lanes per SM and cycle, a 32nd of the
+// integer pipe), so minima and maxima run on order-preserving integer images
+// of the values, and the face fluxes take the state as x held within the two
+// intervals at once (within(): one rounding of c + D).
+// NaN: the near cells reach the result as in the reference's form, a NaN that
+// is only in the interpolant is dropped by the clamp there as here.
 template <typename T> struct Sel;
 template <> struct Sel<float> {
   typedef float K;
@@ -180,9 +186,14 @@ template <> struct Sel<float> {
     asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
   }
-  static __device__ __forceinline__ K mx3_nan(K a, K b, K c) {
+  static __device__ __forceinline__ K mx3(K a, K b, K c) {
     float r;
-    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+  }
+  static __device__ __forceinline__ K mx_nan(K a, K b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
     return r;
   }
   static __device__ __forceinline__ float keep_nan(float r, float) { return r; }
@@ -196,43 +207,56 @@ template <> struct Sel<double> {
   static __device__ __forceinline__ K mx(K a, K b) { return a > b ? a : b; }
   static __device__ __forceinline__ K mn_nan(K a, K b) { return mn(a, b); }
   static __device__ __forceinline__ K mn3(K a, K b, K c) { return mn(mn(a, b), c); }
-  static __device__ __forceinline__ K mx3_nan(K a, K b, K c) { return mx(mx(a, b), c); }
+  static __device__ __forceinline__ K mx3(K a, K b, K c) { return mx(mx(a, b), c); }
+  static __device__ __forceinline__ K mx_nan(K a, K b) { return mx(a, b); }
   // the integer images order a NaN beyond infinity: hand it on instead
   // (out = c + D(c, outer) is NaN when c or outer is)
   static __device__ __forceinline__ double keep_nan(double r, double out) {
     return (__double2hiint(out) & 0x7fffffff) > 0x7ff00000 ? out : r;
   }
 };
-// x held within [c, far] and [c, out]; lo = min(c, far), hi = max(c, far).
-template <typename T>
-__device__ __forceinline__ T within(typename Sel<T>::K lo, typename Sel<T>::K hi, typename Sel<T>::K c, T out,
-                                    typename Sel<T>::K x) {
-  typedef Sel<T> S;
-  const typename S::K o = S::key(out);
-  return S::keep_nan(S::val(S::mx3_nan(lo, S::mn_nan(c, o), S::mn3(hi, S::mx(c, o), x))), out);
+// FP32: x clamped to [a, b], and the soft threshold.
+__device__ __forceinline__ float clamp2(float a, float b, float x) {
+  typedef Sel<float> S;
+  return S::mx_nan(S::mn_nan(a, b), S::mn(x, S::mx(a, b)));
 }
-// Both states of one face, k = 2 pdmb, outl = fm1 + k (fm1 - fm2), outr = f0 + k (f0 - fp1).
-template <typename T>
-__device__ __forceinline__ void pdm_pick(T fm1, T f0, T outl, T outr, T fi, T& fl, T& fr) {
-  typedef Sel<T> S;
-  const typename S::K a = S::key(fm1), b = S::key(f0), x = S::key(fi);
-  const typename S::K lo = S::mn_nan(a, b), hi = S::mx(a, b);
-  fl = within<T>(lo, hi, a, outl, x);
-  fr = within<T>(lo, hi, b, outr, x);
+__device__ __forceinline__ float shrink(float d, float D) {  // d and D of one sign: the smaller, with the sign of d
+  float m;
+  asm("min.NaN.xorsign.abs.f32 %0, %1, %2;" : "=f"(m) : "f"(d), "f"(D));
+  return copysignf(Sel<float>::mx_nan(m, 0.0f), d);
 }
-template <typename T>
-__device__ __forceinline__ void pdm_states(T fm2, T fm1, T f0, T fp1, T fi, T pdmb, T& fl, T& fr) {
-  const T k = pdmb + pdmb;
-  pdm_pick(fm1, f0, fm(k, fm1 - fm2, fm1), fm(k, f0 - fp1, f0), fi, fl, fr);
+__device__ __forceinline__ void pdm_states(float fm2, float fm1, float f0, float fp1, float fi, float pdmb, float& fl,
+                                           float& fr) {
+  const float k = pdmb + pdmb, x = clamp2(fm1, f0, fi);
+  const float dl = x - fm1, dr = x - f0;
+  fl = x - (dl - shrink(dl, k * (fm1 - fm2)));
+  fr = x - (dr - shrink(dr, k * (f0 - fp1)));
+}
+// FP64 face fluxes: x held within [c, far] and [c, out]; lo = min(c, far), hi = max(c, far).
+__device__ __forceinline__ double within(long long lo, long long hi, long long c, double out, long long x) {
+  typedef Sel<double> S;
+  const long long o = S::key(out);
+  return S::keep_nan(S::val(S::mx3(lo, S::mn(c, o), S::mn3(hi, S::mx(c, o), x))), out);
+}
+__device__ __forceinline__ void pdm_states_fused(double fm2, double fm1, double f0, double fp1, double fi, double pdmb,
+                                                 double& fl, double& fr) {
+  typedef Sel<double> S;
+  const double k = pdmb + pdmb;
+  const long long a = S::key(fm1), b = S::key(f0), x = S::key(fi);
+  const long long lo = S::mn(a, b), hi = S::mx(a, b);
+  fl = within(lo, hi, a, fma(k, fm1 - fm2, fm1), x);
+  fr = within(lo, hi, b, fma(k, f0 - fp1, f0), x);
 }
 
 // ------------------------------------------------ edge EMF forms (FP64)
-// The edge EMF of the FP64 mode keeps the reference's roundings (its CT
-// differences show the last bit of E: a face-B component that is zero at first
-// takes all its value from them), while the face fluxes take the fused forms
-// above.  What the roundings leave free is where the decisions are made:
-// comparisons, minima, signs and absolute values run on the integer pipe, and
-// the division by 840 takes two operations.  FP32 has one form for both.
+// The FP64 edge EMF keeps the reference's roundings, while the face fluxes take
+// the fused forms above: a face-B component that is zero at first takes its
+// value from CT differences of E, so the last bit of E shows in it (corner
+// velocities or face B rounded otherwise, however exactly, move bz of the
+// 12 x 10 x 9 vortex by 1.8e-11 of its own size in 4 steps, the fluxes by 6e-12).
+// What the roundings leave free is where the decisions are made: comparisons,
+// minima, signs and absolute values run on the integer pipe, and the division
+// by 840 takes two operations.  FP32 has one form for both.
 //
 // x / 840, correctly rounded: x zh + x zl with zh + zl = 1/840 to twice the
 // precision errs by about 2^-106 of the quotient before its one rounding,
@@ -258,33 +282,21 @@ __device__ __forceinline__ bool abs_ge(float a, float b) { return fabsf(a) >= fa
 __device__ __forceinline__ bool ge0(double x) { return Sel<double>::key(x) >= -1LL; }
 __device__ __forceinline__ bool ge0(float x) { return x >= 0.0f; }
 
-// Interpolant and limiter states of the edge EMF.
-template <typename T> struct Edge;
-template <> struct Edge<float> {
-  static __device__ __forceinline__ float tap(float a0, float a1, float a2, float a3, float a4, float a5, float a6,
-                                              float a7) {
-    return tap8(a0, a1, a2, a3, a4, a5, a6, a7);
-  }
-  static __device__ __forceinline__ void states(float fm2, float fm1, float f0, float fp1, float fi, float pdmb,
-                                                float& fl, float& fr) {
-    pdm_states(fm2, fm1, f0, fp1, fi, pdmb, fl, fr);
-  }
-};
-template <> struct Edge<double> {
+__device__ __forceinline__ double tap8(double a0, double a1, double a2, double a3, double a4, double a5, double a6,
+                                       double a7) {
+  double s = -3.0 * a0;
+  s = s + 29.0 * a1;
+  s = s - 139.0 * a2;
+  s = s + 533.0 * a3;
+  s = s + 533.0 * a4;
+  s = s - 139.0 * a5;
+  s = s + 29.0 * a6;
+  s = s - 3.0 * a7;
+  return div_by<840>(s);
+}
+// Limiter states of the FP64 edge EMF.
+struct Edge64 {
   typedef Sel<double> S;
-  // interp_pdm's operand order (mhd3d3.f90:866-872)
-  static __device__ __forceinline__ double tap(double a0, double a1, double a2, double a3, double a4, double a5,
-                                               double a6, double a7) {
-    double s = -3.0 * a0;
-    s = s + 29.0 * a1;
-    s = s - 139.0 * a2;
-    s = s + 533.0 * a3;
-    s = s + 533.0 * a4;
-    s = s - 139.0 * a5;
-    s = s + 29.0 * a6;
-    s = s - 3.0 * a7;
-    return div_by<840>(s);
-  }
   // the clamp of PDM2: x held within [a, b]
   static __device__ __forceinline__ double clamp(S::K a, S::K b, S::K x) {
     return S::val(S::mx(S::mn(a, b), S::mn(x, S::mx(a, b))));
@@ -309,20 +321,6 @@ template <> struct Edge<double> {
     fr = limited(f0, fii, pdmb * (f0 - fp1), a > b);
   }
 };
-
-// interp_pdm in the reference's operand order (R_PDMG; FP32 with FMA
-// contraction and a reciprocal multiply in place of the division).
-__device__ __forceinline__ double tap_ref(double a0, double a1, double a2, double a3, double a4, double a5, double a6,
-                                          double a7) {
-  return Edge<double>::tap(a0, a1, a2, a3, a4, a5, a6, a7);
-}
-__device__ __forceinline__ float tap_ref(float a0, float a1, float a2, float a3, float a4, float a5, float a6, float a7) {
-  float s = fmaf(29.0f, a1, -3.0f * a0);
-  s = fmaf(533.0f, a3, fmaf(-139.0f, a2, s));
-  s = fmaf(-139.0f, a5, fmaf(533.0f, a4, s));
-  s = fmaf(-3.0f, a7, fmaf(29.0f, a6, s));
-  return s * (1.0f / 840.0f);
-}
 
 // PDM2 (mhd3d3.f90:1069-1172) as the reference writes it, for any pdmb (R_PDMG).
 template <typename T>
@@ -360,81 +358,230 @@ __device__ __forceinline__ void tvd(T fm2, T fm1, T f0, T fp1, T fi, T eps, T& f
   fr = f0 - b * (f0 - fi);
 }
 
-// WENO5 (mhd3d3.f90:1329-1375), one face.  The right state is the left-state
-// formula on the mirrored stencil (fp2, fp1, f0, fm1, fm2), term for term, so
-// both come from weno5_left.
-template <typename T>
-__device__ __forceinline__ T weno5_left(T fm3, T fm2, T fm1, T f0, T fp1, T eps) {
-  const T c13 = T(13.0) / T(12.0);
-  T h0 = Div<T>::by(T(2) * fm3 - T(7) * fm2 + T(11) * fm1, T(6));
-  T h1 = Div<T>::by(-fm2 + T(5) * fm1 + T(2) * f0, T(6));
-  T h2 = Div<T>::by(T(2) * fm1 + T(5) * f0 - fp1, T(6));
-  T t = fm3 - T(2) * fm2 + fm1, u = fm3 - T(4) * fm2 + T(3) * fm1;
-  T s0 = c13 * (t * t) + T(0.25) * (u * u);
-  t = fm2 - T(2) * fm1 + f0; u = fm2 - f0;
-  T s1 = c13 * (t * t) + T(0.25) * (u * u);
-  t = fm1 - T(2) * f0 + fp1; u = T(3) * fm1 - T(4) * f0 + fp1;
-  T s2 = c13 * (t * t) + T(0.25) * (u * u);
-  s0 = Ops<T>::dv(T(0.1), (eps + s0) * (eps + s0));
-  s1 = Ops<T>::dv(T(0.6), (eps + s1) * (eps + s1));
-  s2 = Ops<T>::dv(T(0.3), (eps + s2) * (eps + s2));
-  T sum = s0 + s1 + s2;
-  return Ops<T>::dv(s0, sum) * h0 + Ops<T>::dv(s1, sum) * h1 + Ops<T>::dv(s2, sum) * h2;
-}
-template <typename T>
-__device__ __forceinline__ void weno5(T fm3, T fm2, T fm1, T f0, T fp1, T fp2, T eps, T& fl, T& fr) {
-  fl = weno5_left(fm3, fm2, fm1, f0, fp1, eps);
-  fr = weno5_left(fp2, fp1, f0, fm1, fm2, eps);
-}
-
-// minmod (mhd3d3.f90:1380-1403): 0.5 (sign(1,a) + sign(1,b)) min(|a|, |b|).
-// The factor is exactly 1, -1 or 0, so one comparison of the two signs and a
-// select give the same value for every finite m = min(|a|, |b|) (NaN operands
-// included: sign(1, NaN) counts as -1 on both forms).
-template <typename T> __device__ __forceinline__ T minmod(T a, T b) {
-  const T m = mn(fab(a), fab(b));
-  const bool pa = a >= T(0), pb = b >= T(0);
-  return (pa == pb) ? (pa ? m : -m) : T(0);
-}
-// Monotonicity-preserving bound of MPWENO5 (mhd3d3.f90:1530-1591) for one
-// side; left state: (a3,a2,a1,b0,b1) = (fm3,fm2,fm1,f0,fp1), right state:
-// (fp2,fp1,f0,fm1,fm2).
-template <typename T>
-__device__ __forceinline__ T mp_side(T w, T a3, T a2, T a1, T b0, T b1, T alpha, T beta) {
-  T h0 = a3 - T(2) * a2 + a1;
-  T h1 = a2 - T(2) * a1 + b0;
-  T h2 = a1 - T(2) * b0 + b1;
-  T s1 = minmod(T(4) * h1 - h2, T(4) * h2 - h1);
-  T s2 = minmod(h1, h2);
-  T s0 = minmod(s1, s2);
-  T w1 = minmod(T(4) * h0 - h1, T(4) * h1 - h0);
-  T w2 = minmod(h0, h1);
-  T w0 = minmod(w1, w2);
-  s1 = a1 + alpha * (a1 - a2);
-  s2 = T(0.5) * (a1 + b0 - s0);
-  s0 = T(0.5) * (T(3) * a1 - a2) + Div<T>::by(beta * w0, T(3));
-  T lo = mx(mn(mn(a1, b0), s2), mn(mn(a1, s1), s0));
-  T hi = mn(mx(mx(a1, b0), s2), mx(mx(a1, s1), s0));
-  return w + minmod(lo - w, hi - w);
-}
-
 template <typename T>
 struct Prm {
   T pdmb, eps, alpha, beta;
   int tvd_shift;
 };
 
+// ------------------------------------------------------------------ WENO
+// WENO5 (mhd3d3.f90:1329-1375) and the monotonicity-preserving bound of MPWENO5
+// (1530-1591).  The right state of a face is the left-state formula on the
+// mirrored stencil.
+//
+// minmod of four (1380-1403, nested): the one nearest zero where all signs
+// agree, else zero, i.e. the median of their minimum, their maximum and zero.
+template <typename T>
+__device__ __forceinline__ T mm4(T a, T b, T c, T d) {
+  typedef Sel<T> S;
+  const typename S::K p = S::key(a), q = S::key(b), r = S::key(c), s = S::key(d);
+  const typename S::K lo = S::mn(S::mn3(p, q, r), s), hi = S::mx(S::mx3(p, q, r), s);
+  return S::val(S::mx(lo, S::mn(hi, S::key(T(0)))));
+}
+// The bounds of the bound: lo = max(min(a1, b0, md), min(a1, ul, lc)), hi = min(max(..), max(..)).
+template <typename T>
+__device__ __forceinline__ void mp_bounds(T a1, T b0, T md, T ul, T lc, typename Sel<T>::K& lo, typename Sel<T>::K& hi) {
+  typedef Sel<T> S;
+  const typename S::K p = S::key(a1), q = S::key(b0), m = S::key(md), u = S::key(ul), c = S::key(lc);
+  lo = S::mx(S::mn3(p, q, m), S::mn3(p, u, c));
+  hi = S::mn(S::mx3(p, q, m), S::mx3(p, u, c));
+}
+
+// FP32: one value, or a pair of values in the packed lanes (two fields of a
+// face, the two velocity components of an edge, the two sides of a face).  Bound
+// by issue and the ALU pipe; the pair halves the arithmetic, the signs, minima
+// and maxima of the bound stay per lane.  Every operation rounds as the
+// contracted scalar code before it did (the same products fused), because the
+// corner velocities choose between two one-sided estimates and a last bit can
+// turn the choice: 128^3 RK3 frames keep their bits.
+template <typename V> struct VOps;
+template <> struct VOps<float> {
+  static __device__ __forceinline__ float k(float a) { return a; }
+  static __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
+  static __device__ __forceinline__ float sub(float a, float b) { return __fadd_rn(a, -b); }
+  static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+  static __device__ __forceinline__ float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+  static __device__ __forceinline__ float quot(float a, float b) { return __fdividef(a, b); }
+  static __device__ __forceinline__ float mm4v(float a, float b, float c, float d) { return mm4(a, b, c, d); }
+  // w + minmod(lo - w, hi - w)
+  static __device__ __forceinline__ float bound(float w, float a1, float b0, float md, float ul, float lc) {
+    float lo, hi;
+    mp_bounds(a1, b0, md, ul, lc, lo, hi);
+    return __fadd_rn(w, shrink(__fadd_rn(lo, -w), __fadd_rn(hi, -w)));
+  }
+};
+template <> struct VOps<float2> {
+  static __device__ __forceinline__ float2 k(float a) { return make_float2(a, a); }
+  static __device__ __forceinline__ float2 add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+  static __device__ __forceinline__ float2 sub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
+  static __device__ __forceinline__ float2 mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+  static __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+  static __device__ __forceinline__ float2 quot(float2 a, float2 b) {
+    return make_float2(__fdividef(a.x, b.x), __fdividef(a.y, b.y));
+  }
+  static __device__ __forceinline__ float2 mm4v(float2 a, float2 b, float2 c, float2 d) {
+    return make_float2(mm4(a.x, b.x, c.x, d.x), mm4(a.y, b.y, c.y, d.y));
+  }
+  static __device__ __forceinline__ float2 bound(float2 w, float2 a1, float2 b0, float2 md, float2 ul, float2 lc) {
+    float2 lo, hi;
+    mp_bounds(a1.x, b0.x, md.x, ul.x, lc.x, lo.x, hi.x);
+    mp_bounds(a1.y, b0.y, md.y, ul.y, lc.y, lo.y, hi.y);
+    const float2 p = sub(lo, w), q = sub(hi, w);
+    return add(w, make_float2(shrink(p.x, q.x), shrink(p.y, q.y)));
+  }
+};
+// State next to the near cell a1 of the stencil (a3, a2, a1 | b0, b1).
+template <typename V, int RECON>
+__device__ __forceinline__ V weno_side(V a3, V a2, V a1, V b0, V b1, const Prm<float>& P) {
+  typedef VOps<V> O;
+  const V c13 = O::k(13.0f / 12.0f), c4 = O::k(0.25f), m4 = O::k(-4.0f), m2 = O::k(-2.0f), eps = O::k(P.eps);
+  const V m3 = O::mul(O::k(3.0f), a1);
+  const V h0 = O::fma(O::k(11.0f), a1, O::fma(O::k(-7.0f), a2, O::add(a3, a3)));
+  const V n1 = O::fma(m2, b0, O::fma(O::k(-5.0f), a1, a2));  // -(-a2 + 5 a1 + 2 b0)
+  const V h2 = O::sub(O::fma(O::k(5.0f), b0, O::add(a1, a1)), b1);
+  const V t0 = O::add(O::fma(m2, a2, a3), a1), t1 = O::add(O::fma(m2, a1, a2), b0);
+  const V t2 = O::add(O::fma(m2, b0, a1), b1);
+  const V u0 = O::add(O::fma(m4, a2, a3), m3), u1 = O::sub(a2, b0), u2 = O::add(O::fma(m4, b0, m3), b1);
+  const V e0 = O::add(eps, O::fma(c13, O::mul(t0, t0), O::mul(c4, O::mul(u0, u0))));
+  const V e1 = O::add(eps, O::fma(c4, O::mul(u1, u1), O::mul(c13, O::mul(t1, t1))));
+  const V e2 = O::add(eps, O::fma(c13, O::mul(t2, t2), O::mul(c4, O::mul(u2, u2))));
+  const V q0 = O::quot(O::k(0.1f), O::mul(e0, e0)), q1 = O::quot(O::k(0.6f), O::mul(e1, e1));
+  const V q2 = O::quot(O::k(0.3f), O::mul(e2, e2));
+  const V rs = O::quot(O::k(1.0f), O::add(O::add(q0, q1), q2)), r6 = O::k(1.0f / 6.0f);
+  const V w = O::fma(O::mul(q2, rs), O::mul(r6, h2),
+                     O::fma(O::mul(q0, rs), O::mul(r6, h0), O::mul(O::mul(q1, rs), O::mul(O::k(-1.0f / 6.0f), n1))));
+  if (RECON != R_MPWENO) return w;
+  const V f1 = O::mul(O::k(4.0f), t1);
+  const V s0 = O::mm4v(O::sub(f1, t2), O::sub(O::mul(O::k(4.0f), t2), t1), t1, t2);
+  const V w0 = O::mm4v(O::sub(O::mul(O::k(4.0f), t0), t1), O::sub(f1, t0), t0, t1);
+  const V ul = O::fma(O::k(P.alpha), O::sub(a1, a2), a1);
+  const V md = O::mul(O::k(0.5f), O::sub(O::add(a1, b0), s0));
+  const V lc = O::fma(O::k(0.5f), O::sub(m3, a2), O::mul(O::k(1.0f / 3.0f), O::mul(O::k(P.beta), w0)));
+  return O::bound(w, a1, b0, md, ul, lc);
+}
+// Both states of the face between fm1 and f0 (one value: the two sides as a pair).
+template <int RECON>
+__device__ __forceinline__ void weno_both(float2 fm3, float2 fm2, float2 fm1, float2 f0, float2 fp1, float2 fp2,
+                                          const Prm<float>& P, float2& fl, float2& fr) {
+  fl = weno_side<float2, RECON>(fm3, fm2, fm1, f0, fp1, P);
+  fr = weno_side<float2, RECON>(fp2, fp1, f0, fm1, fm2, P);
+}
+template <int RECON>
+__device__ __forceinline__ void weno_both(float fm3, float fm2, float fm1, float f0, float fp1, float fp2,
+                                          const Prm<float>& P, float& fl, float& fr) {
+  const float2 r = weno_side<float2, RECON>(make_float2(fm3, fp2), make_float2(fm2, fp1), make_float2(fm1, f0),
+                                                   make_float2(f0, fm1), make_float2(fp1, fm2), P);
+  fl = r.x;
+  fr = r.y;
+}
+
+// FP64 face fluxes: everything from the first differences, which both sides
+// share: the second differences, the slopes of the smoothness indicators, and
+// the candidates as offsets from the near cell, so that a state is that cell
+// plus a small correction (half a unit of rounding).  48 operations of the FP64
+// pipe per state, as the reference writes it about 150: one division instead
+// of nine, the weights 1 : 6 : 3 over e^2 brought to their common denominator
+// after scaling by a power of two (integer pipe).
+__device__ __forceinline__ double weno_mix(double e0, double e1, double e2, double g0, double g1, double g2) {
+  const int x0 = __double2hiint(e0), x1 = __double2hiint(e1), x2 = __double2hiint(e2);
+  const int sh = (max(x0, max(x1, x2)) & 0x7ff00000) - 0x3ff00000;
+  const double s0 = __hiloint2double(max(x0 - sh, 0x00100000), __double2loint(e0));
+  const double s1 = __hiloint2double(max(x1 - sh, 0x00100000), __double2loint(e1));
+  const double s2 = __hiloint2double(max(x2 - sh, 0x00100000), __double2loint(e2));
+  const double d0 = s0 * s0, d1 = s1 * s1, d2 = s2 * s2;
+  const double a0 = d1 * d2, a1 = (6.0 * d0) * d2, a2 = (3.0 * d0) * d1;
+  return fma(a0, g0, fma(a1, g1, a2 * g2)) / (6.0 * (a0 + a1 + a2));
+}
+// S = 1 for the left state, -1 for the right one (the stencil mirrored): near
+// cell a1, the cell b0 across the face, the first differences dm behind a1 and
+// d0 across the face in the direction of increasing index, and the second
+// differences t0, t1, t2 about the cell behind a1, a1 and b0.
+template <int RECON, int S>
+__device__ __forceinline__ double weno_side64(double a1, double b0, double dm, double d0, double t0, double t1,
+                                              double t2, const Prm<double>& P) {
+  const double c = 13.0 / 3.0, eps = 4.0 * P.eps;  // e_i = 4 (eps + s_i)
+  const double u0 = fma(2.0 * S, dm, t0), u1 = dm + d0, u2 = fma(-2.0 * S, d0, t2);
+  const double e0 = fma(c * t0, t0, fma(u0, u0, eps)), e1 = fma(c * t1, t1, fma(u1, u1, eps));
+  const double e2 = fma(c * t2, t2, fma(u2, u2, eps));
+  const double g0 = fma((double)S, u0 + t0, dm), g1 = fma(2.0, d0, dm), g2 = fma(-(double)S, u2, d0);
+  const double w = fma((double)S, weno_mix(e0, e1, e2, g0, g1, g2), a1);
+  if (RECON != R_MPWENO) return w;
+  const double s0 = mm4(fma(4.0, t1, -t2), fma(4.0, t2, -t1), t1, t2);
+  const double w0 = mm4(fma(4.0, t0, -t1), fma(4.0, t1, -t0), t0, t1);
+  typedef Sel<double> K;
+  long long lo, hi;
+  mp_bounds(a1, b0, fma(0.5 * S, d0, fma(-0.5, s0, a1)), fma(S * P.alpha, dm, a1),
+            fma(0.5 * S, dm, fma(P.beta * (1.0 / 3.0), w0, a1)), lo, hi);
+  // w + minmod(lo - w, hi - w): the median of w, lo and hi
+  return K::keep_nan(K::val(K::mx(K::mn(lo, hi), K::mn(K::mx(lo, hi), K::key(w)))), w);
+}
+template <int RECON>
+__device__ __forceinline__ void weno_both(double fm3, double fm2, double fm1, double f0, double fp1, double fp2,
+                                          const Prm<double>& P, double& fl, double& fr) {
+  const double da = fm2 - fm3, db = fm1 - fm2, dc = f0 - fm1, dd = fp1 - f0, de = fp2 - fp1;
+  const double ta = db - da, tb = dc - db, tc = dd - dc, td = de - dd;
+  fl = weno_side64<RECON, 1>(fm1, f0, db, dc, ta, tb, tc, P);
+  fr = weno_side64<RECON, -1>(f0, fm1, dd, dc, td, tc, tb, P);
+}
+
+// The state with the reference's roundings (FP64 edge EMF and metric mode):
+// products by powers of two are fused, constant divisors take two operations
+// and the quotients by the weights' sum share its reciprocal.
+template <int RECON>
+__device__ __forceinline__ double weno_side_ref(double a3, double a2, double a1, double b0, double b1,
+                                                const Prm<double>& P) {
+  const double eps = P.eps, c13 = 13.0 / 12.0;
+  const double h0 = div_by<6>(fma(2.0, a3, -(7.0 * a2)) + 11.0 * a1);
+  const double h1 = div_by<6>(fma(2.0, b0, 5.0 * a1 - a2));
+  const double h2 = div_by<6>(fma(2.0, a1, 5.0 * b0) - b1);
+  const double t0 = fma(-2.0, a2, a3) + a1, t1 = fma(-2.0, a1, a2) + b0, t2 = fma(-2.0, b0, a1) + b1;
+  const double u0 = fma(-4.0, a2, a3) + 3.0 * a1, u1 = a2 - b0, u2 = fma(-4.0, b0, 3.0 * a1) + b1;
+  const double e0 = eps + fma(0.25, u0 * u0, c13 * (t0 * t0)), e1 = eps + fma(0.25, u1 * u1, c13 * (t1 * t1));
+  const double e2 = eps + fma(0.25, u2 * u2, c13 * (t2 * t2));
+  const double s0 = 0.1 / (e0 * e0), s1 = 0.6 / (e1 * e1), s2 = 0.3 / (e2 * e2);
+  typedef Ops<double> O;
+  const double sum = s0 + s1 + s2, rs = O::rcp(sum);
+  const double w = O::dvr(s0, sum, rs) * h0 + O::dvr(s1, sum, rs) * h1 + O::dvr(s2, sum, rs) * h2;
+  if (RECON != R_MPWENO) return w;
+  typedef Sel<double> S;
+  const double m0 = mm4(fma(4.0, t1, -t2), fma(4.0, t2, -t1), t1, t2);
+  const double m1 = mm4(fma(4.0, t0, -t1), fma(4.0, t1, -t0), t0, t1);
+  long long kl, kh;
+  mp_bounds(a1, b0, 0.5 * (a1 + b0 - m0), a1 + P.alpha * (a1 - a2),
+            fma(0.5, 3.0 * a1 - a2, div_by<3>(P.beta * m1)), kl, kh);
+  const long long lo = S::key(S::val(kl) - w), hi = S::key(S::val(kh) - w);
+  return w + S::val(S::mx(S::mn(lo, hi), S::mn(S::mx(lo, hi), S::key(0.0))));
+}
+
+// The two states of the edge EMF's reconstructions.
+template <int RECON>
+__device__ __forceinline__ void weno_edge(double fm3, double fm2, double fm1, double f0, double fp1, double fp2,
+                                          const Prm<double>& P, double& fl, double& fr) {
+  fl = weno_side_ref<RECON>(fm3, fm2, fm1, f0, fp1, P);
+  fr = weno_side_ref<RECON>(fp2, fp1, f0, fm1, fm2, P);
+}
+template <int RECON, typename V>
+__device__ __forceinline__ void weno_edge(V fm3, V fm2, V fm1, V f0, V fp1, V fp2, const Prm<float>& P, V& fl, V& fr) {
+  weno_both<RECON>(fm3, fm2, fm1, f0, fp1, fp2, P, fl, fr);
+}
+
 // One-sided face states of f at the low face of element c along stride s
 // (reconstruct_3d for dirs 1-3, mhd3d3.f90:833-860).
 // PDM face states from the 8 taps a0..a7 (cells c-4 .. c+3 along the
 // reconstruction axis; the face at the low side of c).
+constexpr bool is_weno(int recon) { return recon == R_WENO || recon == R_MPWENO; }
 constexpr bool is_pdm(int recon) { return recon == R_PDM || recon == R_PDMG; }
 // EDGE: the face-B reconstruction of the edge EMF.
 template <typename T, int RECON = R_PDM, bool EDGE = false>
 __device__ __forceinline__ void recon_pdm8(T a0, T a1, T a2, T a3, T a4, T a5, T a6, T a7, T pdmb, T& fl, T& fr) {
-  if (RECON != R_PDM) pdm2(a2, a3, a4, a5, tap_ref(a0, a1, a2, a3, a4, a5, a6, a7), pdmb, fl, fr);
-  else if (EDGE) Edge<T>::states(a2, a3, a4, a5, Edge<T>::tap(a0, a1, a2, a3, a4, a5, a6, a7), pdmb, fl, fr);
-  else pdm_states(a2, a3, a4, a5, tap8(a0, a1, a2, a3, a4, a5, a6, a7), pdmb, fl, fr);
+  if constexpr (RECON == R_PDM && std::is_same<T, double>::value && !EDGE) {
+    pdm_states_fused(a2, a3, a4, a5, tap8_fused(a0, a1, a2, a3, a4, a5, a6, a7), pdmb, fl, fr);
+  } else {
+    const T fi = tap8(a0, a1, a2, a3, a4, a5, a6, a7);
+    if constexpr (RECON != R_PDM) pdm2(a2, a3, a4, a5, fi, pdmb, fl, fr);
+    else if constexpr (std::is_same<T, double>::value) Edge64::states(a2, a3, a4, a5, fi, pdmb, fl, fr);
+    else pdm_states(a2, a3, a4, a5, fi, pdmb, fl, fr);
+  }
 }
 
 template <typename T, int RECON, typename I, bool EDGE = false>
@@ -448,42 +595,15 @@ __device__ __forceinline__ void recon_face(const T* __restrict__ f, I c, I s, co
     tvd<T, RECON == R_TVDMC>(fm2, fm1, f0, fp1, fi, P.eps, fl, fr);
   } else {
     T fm3 = f[c - 3 * s], fm2 = f[c - 2 * s], fm1 = f[c - s], f0 = f[c], fp1 = f[c + s], fp2 = f[c + 2 * s];
-    weno5(fm3, fm2, fm1, f0, fp1, fp2, P.eps, fl, fr);
-    if (RECON == R_MPWENO) {
-      fl = mp_side(fl, fm3, fm2, fm1, f0, fp1, P.alpha, P.beta);
-      fr = mp_side(fr, fp2, fp1, f0, fm1, fm2, P.alpha, P.beta);
-    }
+    if constexpr (EDGE) weno_edge<RECON>(fm3, fm2, fm1, f0, fp1, fp2, P, fl, fr);
+    else weno_both<RECON>(fm3, fm2, fm1, f0, fp1, fp2, P, fl, fr);
   }
 }
 
-// The corner interpolant's passes.
-template <typename T, int RECON>
-__device__ __forceinline__ T edge_tap(T a0, T a1, T a2, T a3, T a4, T a5, T a6, T a7) {
-  return RECON == R_PDM ? Edge<T>::tap(a0, a1, a2, a3, a4, a5, a6, a7) : tap_ref(a0, a1, a2, a3, a4, a5, a6, a7);
-}
 // recon_face of the face B in the edge EMF.
 template <typename T, int RECON, typename I>
 __device__ __forceinline__ void recon_edge(const T* __restrict__ f, I c, I s, const Prm<T>& P, T& fl, T& fr) {
   recon_face<T, RECON, I, true>(f, c, s, P, fl, fr);
-}
-
-// One side of weno_vals: the left state of the stencil (x0..x4) = (fm3..fp1);
-// the right state is this on the mirrored stencil (fp2, fp1, f0, fm1, fm2).
-template <typename T, int RECON>
-__device__ __forceinline__ T weno_one(T x0, T x1, T x2, T x3, T x4, const Prm<T>& P) {
-  T f = weno5_left(x0, x1, x2, x3, x4, P.eps);
-  if (RECON == R_MPWENO) f = mp_side(f, x0, x1, x2, x3, x4, P.alpha, P.beta);
-  return f;
-}
-
-// WENO5/MPWENO5 pair on six values held in registers.
-template <typename T, int RECON>
-__device__ __forceinline__ void weno_vals(const T* a, const Prm<T>& P, T& fl, T& fr) {
-  weno5(a[0], a[1], a[2], a[3], a[4], a[5], P.eps, fl, fr);
-  if (RECON == R_MPWENO) {
-    fl = mp_side(fl, a[0], a[1], a[2], a[3], a[4], P.alpha, P.beta);
-    fr = mp_side(fr, a[5], a[4], a[3], a[2], a[1], P.alpha, P.beta);
-  }
 }
 
 // PDM part of get_vav_center2corner (mhd3d3.f90:1901-1905, 2056-2108) for
@@ -491,23 +611,22 @@ __device__ __forceinline__ void weno_vals(const T* a, const Prm<T>& P, T& fl, T&
 // interpolant vi.  The reference limits vi with four shifted PDM2 pairs, which
 // leaves each quadrant cell q two one-sided estimates, one along d1 and one
 // along d2, and takes the one whose outward slope is larger (dif >= 0: d1).
-// An estimate is PDM2's state on the side of q, so in the form above it is
-// within(q, far, q + D(q, outer), vi) with far the cell across the edge and outer the
-// one behind q along that axis: the comparison of the two slopes picks (far,
-// q - outer) and one state per quadrant is evaluated.  The edge takes the mean
-// of the four.
+// An estimate is PDM2's state on the side of q: vi clamped to [q, far] and kept
+// within [q, q + D(q, outer)], far the cell across the edge and outer the one
+// behind q along that axis.  The comparison of the two slopes picks (far, q -
+// outer) and one state per quadrant is evaluated, by the same instructions on
+// either side.  The edge takes the mean of the four.
 __device__ __forceinline__ float corner_quad(float q, float far1, float far2, float e1, float e2, float pd, float vi) {
-  typedef Sel<float> S;
   const bool b = abs_ge(e1, e2);  // q - outer along d1 and d2
-  const float far = b ? far1 : far2;
-  return within<float>(S::mn_nan(q, far), S::mx(q, far), q, fm(pd + pd, b ? e1 : e2, q), vi);
+  const float x = clamp2(q, b ? far1 : far2, vi), d = x - q;
+  return x - (d - shrink(d, (pd + pd) * (b ? e1 : e2)));
 }
 __device__ __forceinline__ double corner_quad(double q, double far1, double far2, double e1, double e2, double pd,
                                               double vi) {
   typedef Sel<double> S;
   const bool b = abs_ge(e1, e2);
   const S::K c = S::key(q), f = S::key(b ? far1 : far2);
-  return Edge<double>::limited(q, Edge<double>::clamp(c, f, S::key(vi)), pd * (b ? e1 : e2), f > c);
+  return Edge64::limited(q, Edge64::clamp(c, f, S::key(vi)), pd * (b ? e1 : e2), f > c);
 }
 // The reference's form, for any pdmb (R_PDMG): one half of pdm2 with the clamp
 // pair (lo, hi) = (fm1, f0), the cell `outer` beyond the near end and the side
@@ -576,43 +695,33 @@ template <> struct Pr<double> {
   static __device__ __forceinline__ V sub(V a, V b) { return make_double2(a.x - b.x, a.y - b.y); }
 };
 
-// edge_tap on pairs (same operations per lane)
-template <int RECON = R_PDM>
+// tap8 on pairs (same operations per lane)
 __device__ __forceinline__ float2 tap8p(float2 a0, float2 a1, float2 a2, float2 a3, float2 a4, float2 a5, float2 a6,
                                         float2 a7) {
   typedef Pr<float> Q;
-  if (RECON != R_PDM) {
-    float2 s = Q::mad(29.0f, a1, Q::mul(-3.0f, a0));
-    s = Q::mad(533.0f, a3, Q::mad(-139.0f, a2, s));
-    s = Q::mad(-139.0f, a5, Q::mad(533.0f, a4, s));
-    s = Q::mad(-3.0f, a7, Q::mad(29.0f, a6, s));
-    return Q::mul(1.0f / 840.0f, s);
-  }
-  typedef Tap<float> C;
-  float2 s = Q::mad(C::c0, a7, Q::mul(C::c0, a0));
-  s = Q::mad(C::c1, a6, Q::mad(C::c1, a1, s));
-  s = Q::mad(C::c2, a5, Q::mad(C::c2, a2, s));
-  return Q::mad(C::c3, a4, Q::mad(C::c3, a3, s));
+  float2 s = Q::mad(29.0f, a1, Q::mul(-3.0f, a0));
+  s = Q::mad(533.0f, a3, Q::mad(-139.0f, a2, s));
+  s = Q::mad(-139.0f, a5, Q::mad(533.0f, a4, s));
+  s = Q::mad(-3.0f, a7, Q::mad(29.0f, a6, s));
+  return Q::mul(1.0f / 840.0f, s);
 }
-template <int RECON = R_PDM>
 __device__ __forceinline__ double2 tap8p(double2 a0, double2 a1, double2 a2, double2 a3, double2 a4, double2 a5,
                                          double2 a6, double2 a7) {
-  return make_double2(Edge<double>::tap(a0.x, a1.x, a2.x, a3.x, a4.x, a5.x, a6.x, a7.x),
-                      Edge<double>::tap(a0.y, a1.y, a2.y, a3.y, a4.y, a5.y, a6.y, a7.y));
+  return make_double2(tap8(a0.x, a1.x, a2.x, a3.x, a4.x, a5.x, a6.x, a7.x),
+                      tap8(a0.y, a1.y, a2.y, a3.y, a4.y, a5.y, a6.y, a7.y));
 }
 
-// corner_quad of both components of a pair.  FP32: the differences and q + D
-// on the packed pipe, the choice and the clamp per lane.
+// corner_quad of both components of a pair.  FP32: the differences on the
+// packed pipe, the choice, the clamp and the threshold per lane.
 __device__ __forceinline__ float2 corner_quad2(float2 q, float2 far1, float2 far2, float2 out1, float2 out2, float pd,
                                                float2 vi) {
   typedef Pr<float> Q;
-  typedef Sel<float> S;
   const float2 e1 = Q::sub(q, out1), e2 = Q::sub(q, out2);
   const bool bx = abs_ge(e1.x, e2.x), by = abs_ge(e1.y, e2.y);
-  const float2 out = Q::mad(pd + pd, make_float2(bx ? e1.x : e2.x, by ? e1.y : e2.y), q);
-  const float fx = bx ? far1.x : far2.x, fy = by ? far1.y : far2.y;
-  return make_float2(within<float>(S::mn_nan(q.x, fx), S::mx(q.x, fx), q.x, out.x, vi.x),
-                     within<float>(S::mn_nan(q.y, fy), S::mx(q.y, fy), q.y, out.y, vi.y));
+  const float2 D = Q::mul(pd + pd, make_float2(bx ? e1.x : e2.x, by ? e1.y : e2.y));
+  const float2 x = make_float2(clamp2(q.x, bx ? far1.x : far2.x, vi.x), clamp2(q.y, by ? far1.y : far2.y, vi.y));
+  const float2 d = Q::sub(x, q);
+  return Q::sub(x, Q::sub(d, make_float2(shrink(d.x, D.x), shrink(d.y, D.y))));
 }
 __device__ __forceinline__ double2 corner_quad2(double2 q, double2 far1, double2 far2, double2 out1, double2 out2,
                                                 double pd, double2 vi) {
@@ -649,21 +758,14 @@ __device__ __forceinline__ float2 rsq(float2 a) { return make_float2(rsqrtf(a.x)
 }  // namespace p2
 
 // corner_pdm of both components from pair-interleaved shared memory.
-template <typename T, int RECON>
+template <typename T>
 __device__ __forceinline__ void corner_pdm_pair(const typename Pr<T>::V* __restrict__ v, int c, int s1, int s2,
                                                 typename Pr<T>::V vi, T pd, T& r0, T& r1) {
   typedef typename Pr<T>::V V;
   const V m11 = v[c - s1 - s2], m21 = v[c - 2 * s1 - s2], m12 = v[c - s1 - 2 * s2], m01 = v[c - s2];
   const V p11 = v[c + s1 - s2], m02 = v[c - 2 * s2], m10 = v[c - s1], m20 = v[c - 2 * s1];
   const V m1p = v[c - s1 + s2], c0 = v[c], p10 = v[c + s1], p01 = v[c + s2];
-  if (RECON == R_PDM) {
-    corner_pdm_vals2<T>(m11, m21, m12, m01, p11, m02, m10, m20, m1p, c0, p10, p01, vi, pd, r0, r1);
-    return;
-  }
-  r0 = corner_pdm_vals<T, RECON>(m11.x, m21.x, m12.x, m01.x, p11.x, m02.x, m10.x, m20.x, m1p.x, c0.x, p10.x, p01.x,
-                                 vi.x, pd);
-  r1 = corner_pdm_vals<T, RECON>(m11.y, m21.y, m12.y, m01.y, p11.y, m02.y, m10.y, m20.y, m1p.y, c0.y, p10.y, p01.y,
-                                 vi.y, pd);
+  corner_pdm_vals2<T>(m11, m21, m12, m01, p11, m02, m10, m20, m1p, c0, p10, p01, vi, pd, r0, r1);
 }
 
 // Limited corner value of v at the edge whose two transverse axes have
@@ -680,9 +782,9 @@ __device__ __forceinline__ T corner_vel(const T* __restrict__ v, long long c, lo
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
       const T* r = v + c + (long long)(m - 4) * s2;
-      g[m] = edge_tap<T, RECON>(r[-4 * s1], r[-3 * s1], r[-2 * s1], r[-s1], r[0], r[s1], r[2 * s1], r[3 * s1]);
+      g[m] = tap8(r[-4 * s1], r[-3 * s1], r[-2 * s1], r[-s1], r[0], r[s1], r[2 * s1], r[3 * s1]);
     }
-    T vi = edge_tap<T, RECON>(g[0], g[1], g[2], g[3], g[4], g[5], g[6], g[7]);
+    T vi = tap8(g[0], g[1], g[2], g[3], g[4], g[5], g[6], g[7]);
     return corner_pdm<T, RECON>(v, c, s1, s2, vi, P.pdmb);
   } else if (RECON == R_TVD || RECON == R_TVDMC) {
     // interp2_tvd (1037-1067) and TVD with (mhd3d2) or without (mhd3d3) shifts
@@ -703,19 +805,19 @@ __device__ __forceinline__ T corner_vel(const T* __restrict__ v, long long c, lo
       const T* r = v + c + (long long)(m - 3) * s2;
 #pragma unroll
       for (int t = 0; t < 6; ++t) a[t] = r[(long long)(t - 3) * s1];
-      weno_vals<T, RECON>(a, P, L[m], R[m]);
+      weno_edge<RECON>(a[0], a[1], a[2], a[3], a[4], a[5], P, L[m], R[m]);
     }
-    weno_vals<T, RECON>(L, P, v00_1, v01_1);
-    weno_vals<T, RECON>(R, P, v10_1, v11_1);
+    weno_edge<RECON>(L[0], L[1], L[2], L[3], L[4], L[5], P, v00_1, v01_1);
+    weno_edge<RECON>(R[0], R[1], R[2], R[3], R[4], R[5], P, v10_1, v11_1);
 #pragma unroll
     for (int m = 0; m < 6; ++m) {
       const T* r = v + c + (long long)(m - 3) * s1;
 #pragma unroll
       for (int t = 0; t < 6; ++t) a[t] = r[(long long)(t - 3) * s2];
-      weno_vals<T, RECON>(a, P, L[m], R[m]);
+      weno_edge<RECON>(a[0], a[1], a[2], a[3], a[4], a[5], P, L[m], R[m]);
     }
-    weno_vals<T, RECON>(L, P, v00_0, v01_0);
-    weno_vals<T, RECON>(R, P, v10_0, v11_0);
+    weno_edge<RECON>(L[0], L[1], L[2], L[3], L[4], L[5], P, v00_0, v01_0);
+    weno_edge<RECON>(R[0], R[1], R[2], R[3], R[4], R[5], P, v10_0, v11_0);
   }
   // dif signs pick the smoother one-sided estimate per quadrant (2056-2106)
   const long long q00 = c - s1 - s2, q10 = c - s2, q01 = c - s1, q11 = c;
@@ -790,13 +892,11 @@ __device__ __forceinline__ void cell_b_metric(const Metric& m, long long c, T lo
   bz = p0 * (T)m.eb[0][2][c] + p1 * (T)m.eb[1][2][c] + p2 * (T)m.eb[2][2][c];
 }
 
-// vf = |v| + |B| / sqrt(rho) of get_eijk_LFM (1766), b2 = |B|^2.  FP64: from
-// the reciprocal of rho, which get_dt of the same cell shares.
-__device__ __forceinline__ float vf_val(float u, float v, float w, float b2, float r0) {
+// vf = |v| + |B| / sqrt(rho) of get_eijk_LFM (1766), b2 = |B|^2 (in FP64 with
+// the reference's roundings: the edge EMF multiplies the jumps of B by it).
+template <typename T>
+__device__ __forceinline__ T vf_val(T u, T v, T w, T b2, T r0) {
   return sq(u * u + v * v + w * w) + sq(b2 / r0);
-}
-__device__ __forceinline__ double vf_val(double u, double v, double w, double b2, double r0) {
-  return sqrt(u * u + v * v + w * w) + sqrt(b2 * (1.0 / r0));
 }
 // get_bxyz over all cells (incl. ghosts) and vf = |v| + |B|/sqrt(rho).
 template <typename T, bool M>
@@ -833,6 +933,7 @@ __device__ __forceinline__ float cfl_sqrt(float x) { return x > 0.0f ? x * rsqrt
 
 // |v| + fast speed sqrt(B^2 / rho + gam p / rho); FP64 takes one root and one
 // reciprocal for the second term (three roots and two divisions as written in get_dt).
+template <bool M>
 __device__ __forceinline__ float cfl_speed(float gam, float r0, float p0, float u, float v, float w, float b2) {
   typedef Ops<float> O;
   const float vv = cfl_sqrt(u * u + v * v + w * w);
@@ -840,7 +941,12 @@ __device__ __forceinline__ float cfl_speed(float gam, float r0, float p0, float 
   const float vs = cfl_sqrt(O::dv(gam * p0, r0));
   return vv + cfl_sqrt(valf * valf + vs * vs);
 }
+template <bool M>
 __device__ __forceinline__ double cfl_speed(double gam, double r0, double p0, double u, double v, double w, double b2) {
+  if (M) {
+    const double valf = sqrt(b2) / sqrt(r0), vs = sqrt(gam * p0 / r0);
+    return sqrt(u * u + v * v + w * w) + sqrt(valf * valf + vs * vs);
+  }
   return sqrt(u * u + v * v + w * w) + sqrt((b2 + gam * p0) * (1.0 / r0));
 }
 
@@ -850,13 +956,13 @@ template <typename T, bool M>
 __device__ __forceinline__ T cell_dt(const Dev<T>& d, int c, int i, int j, int k, T r0, T p0, T u, T v, T w, T a,
                                      T b, T cc, unsigned& st) {
   typedef Ops<T> O;
-  const T vcfl = cfl_speed(d.gam, r0, p0, u, v, w, a * a + b * b + cc * cc);
+  const T vcfl = cfl_speed<M>(d.gam, r0, p0, u, v, w, a * a + b * b + cc * cc);
   T dt;
   if (M)  // metric mode: 1/dx_a -> |mean area vector of the a-faces| / V
     dt = O::dv(d.cfl, O::dw(vcfl * (T)d.m.sa[c], (T)d.m.vol[c], (T)d.m.rvol[c]));
   else
-    dt = O::dv(d.cfl, O::dw(vcfl, d.wx[i], d.rwx[i]) + O::dw(vcfl, d.wy[j], d.rwy[j]) +
-                          O::dw(vcfl, d.wz[k], d.rwz[k]));
+    dt = O::dv(d.cfl, O::dc(vcfl, d.wx[i], d.rwx[i]) + O::dc(vcfl, d.wy[j], d.rwy[j]) +
+                          O::dc(vcfl, d.wz[k], d.rwz[k]));
   if (isnan(r0) || isnan(p0) || isnan(u) || isnan(v) || isnan(w)) st |= ST_NAN;
   if (r0 < T(0)) st |= ST_NEG_RHO;
   if (p0 < T(0)) st |= ST_NEG_P;
@@ -894,9 +1000,11 @@ __device__ __forceinline__ void dt_next_accumulate(Scal* sc, T m, unsigned st) {
   }
 }
 
-// p / (gam - 1): FP64 by the reciprocal (Dev::rgm1).
+// p / (gam - 1): FP64 by the reciprocal (Dev::rgm1), the metric mode divides.
+template <bool M>
 __device__ __forceinline__ float over_gm1(const Dev<float>& d, float p) { return Ops<float>::dv(p, d.gam - 1.0f); }
-__device__ __forceinline__ double over_gm1(const Dev<double>& d, double p) { return p * d.rgm1; }
+template <bool M>
+__device__ __forceinline__ double over_gm1(const Dev<double>& d, double p) { return M ? p / (d.gam - 1.0) : p * d.rgm1; }
 
 // save != 0 also stores U^n of the RK stage combines (advance_previous,
 // 3794-3819) at interior cells and faces, the only places they are read.
@@ -924,7 +1032,7 @@ __global__ void __launch_bounds__(256, pass_min_blocks(B)) k_cfl(KArg<T, B> ka, 
         d.q[1][c] = r0 * u;
         d.q[2][c] = r0 * v;
         d.q[3][c] = r0 * w;
-        d.q[4][c] = T(0.5) * r0 * (u * u + v * v + w * w) + over_gm1(d, p0);
+        d.q[4][c] = T(0.5) * r0 * (u * u + v * v + w * w) + over_gm1<M>(d, p0);
       }
       const bool fx = i >= g.ng && i <= g.ng + g.nx0, fy = j >= g.ng && j <= g.ng + g.ny0,
                  fz = k >= g.ng && k <= g.ng + g.nz0;
@@ -1130,48 +1238,20 @@ template <> struct Moments<float> {
 // kernel (x faces, y / z face tiles and column sweeps, batched or not) goes
 // through these functions, so they agree bit for bit.
 
-// PDM states of two stencils at once (lanes .x and .y, e.g. two fields at one
-// face) from the interpolant pair fi (pdm_states): the one-sided limits on the
-// packed pipe, the clamps per lane.  lr0 / lr1 are the (left, right) states of
-// lane x / lane y.
-__device__ __forceinline__ void pdm2x2(float2 fm2, float2 fm1, float2 f0, float2 fp1, float2 fi, float pdmb,
-                                       float2& lr0, float2& lr1) {
-  const float2 k = p2::K(pdmb + pdmb);
-  const float2 outl = p2::fma(k, p2::sub(fm1, fm2), fm1);
-  const float2 outr = p2::fma(k, p2::sub(f0, fp1), f0);
-  pdm_pick(fm1.x, f0.x, outl.x, outr.x, fi.x, lr0.x, lr0.y);
-  pdm_pick(fm1.y, f0.y, outl.y, outr.y, fi.y, lr1.x, lr1.y);
-}
-
-// pdm2 of two stencils at once (R_PDMG): the differences on the packed pipe,
-// the clamp and the limiter per lane.
-__device__ __forceinline__ float2 pdm_lim(float fii, float dfl, float dfr, float dfm, float df0, float dfp) {
-  const float sm = sgn1(dfm), s0 = sgn1(df0), sp = sgn1(dfp);
-  const float qm = fabsf(sm + s0), qp = fabsf(s0 + sp);
-  return make_float2(fii - s0 * mx(0.0f, fabsf(dfl) - qm * fabsf(dfm)),
-                     fii + s0 * mx(0.0f, fabsf(dfr) - qp * fabsf(dfp)));
-}
-__device__ __forceinline__ void pdm2x2_ref(float2 fm2, float2 fm1, float2 f0, float2 fp1, float2 fi, float pdmb,
-                                           float2& lr0, float2& lr1) {
-  const float2 kp = p2::K(pdmb);
-  const float2 dfm = p2::mul(kp, p2::sub(fm1, fm2));
-  const float2 df0 = p2::mul(kp, p2::sub(f0, fm1));
-  const float2 dfp = p2::mul(kp, p2::sub(fp1, f0));
-  float2 fii;
-  fii.x = mx(mn(fm1.x, f0.x), mn(fi.x, mx(fm1.x, f0.x)));
-  fii.y = mx(mn(fm1.y, f0.y), mn(fi.y, mx(fm1.y, f0.y)));
-  const float2 dfl = p2::sub(fii, fm1), dfr = p2::sub(f0, fii);
-  lr0 = pdm_lim(fii.x, dfl.x, dfr.x, dfm.x, df0.x, dfp.x);
-  lr1 = pdm_lim(fii.y, dfl.y, dfr.y, dfm.y, df0.y, dfp.y);
-}
-
-// PDM face states of two fields from their 8-tap windows (tap m = cell
-// c+m-4 for the face at the low side of cell c), packed as field pairs.
-template <int RECON>
+// PDM face states of two fields (lanes .x and .y) from their 8-tap windows (tap
+// m = cell c+m-4 for the face at the low side of cell c): pdm_states with the
+// differences on the packed pipe, the clamps and thresholds per lane.  lr0 /
+// lr1 are the (left, right) states of lane x / lane y.
 __device__ __forceinline__ void pdm_pair_states(const float2* a, float pdmb, float2& lr0, float2& lr1) {
-  const float2 fi = tap8p<RECON>(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7]);
-  if (RECON == R_PDM) pdm2x2(a[2], a[3], a[4], a[5], fi, pdmb, lr0, lr1);
-  else pdm2x2_ref(a[2], a[3], a[4], a[5], fi, pdmb, lr0, lr1);
+  const float2 fi = tap8p(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7]);
+  const float2 fm2 = a[2], fm1 = a[3], f0 = a[4], fp1 = a[5], k = p2::K(pdmb + pdmb);
+  const float2 Dl = p2::mul(k, p2::sub(fm1, fm2)), Dr = p2::mul(k, p2::sub(f0, fp1));
+  const float2 x = make_float2(clamp2(fm1.x, f0.x, fi.x), clamp2(fm1.y, f0.y, fi.y));
+  const float2 dl = p2::sub(x, fm1), dr = p2::sub(x, f0);
+  const float2 l = p2::sub(x, p2::sub(dl, make_float2(shrink(dl.x, Dl.x), shrink(dl.y, Dl.y))));
+  const float2 r = p2::sub(x, p2::sub(dr, make_float2(shrink(dr.x, Dr.x), shrink(dr.y, Dr.y))));
+  lr0 = make_float2(l.x, r.x);
+  lr1 = make_float2(l.y, r.y);
 }
 
 // 0.5 erfc(-x.x) (left state, + moment) and 0.5 erfc(x.y) (right state, -
@@ -1335,34 +1415,13 @@ __device__ __forceinline__ void face_flux(const double* l, const double* r, cons
   for (int q = 0; q < 8; ++q) out[q] = out[q] + f[q];
 }
 
-// Moments of one face state (get_v_face): lam = rho / (2 p), and for the
-// magnetic stress lam = rho / p2.
-__device__ __forceinline__ void face_moments(const Dev<float>&, float r, float p, float vn, bool left, float& v0,
-                                             float& v1) {
-  Moments<float>::hydro(Moments<float>::div(r, 2.0f * p), vn, left, v0, v1);
-}
-__device__ __forceinline__ float face_moment_mag(const Dev<float>&, float r, float p2, float vn, bool left) {
-  return Moments<float>::mag(Moments<float>::div(r, p2), vn, left);
-}
-__device__ __forceinline__ void face_moments(const Dev<double>& d, double r, double p, double vn, bool left, double& v0,
-                                             double& v1) {
-  const double p2 = p + p, s = rsqrt(p2 * r), a = (r * s) * vn;
-  const GaussArg ga(d.gtab, a);
-  v0 = ga.half_erfc(a, left);
-  const double b = (p2 * s) * ga.bell(a);
-  v1 = fma(vn, v0, left ? b : -b);
-}
-__device__ __forceinline__ double face_moment_mag(const Dev<double>& d, double r, double p2, double vn, bool left) {
-  const double a = (r * rsqrt(p2 * r)) * vn;
-  return GaussArg(d.gtab, a).half_erfc(a, left);
-}
-
 // Metric-mode flux through a face of unit normal n and area am: the
 // Gaussian-split formulas of face_flux with n in place of the axis (vector
 // momentum and magnetic stress), left with the + moments and right with the
 // - moments, the sum multiplied by am (the oracle's get_flux_stress_metric).
 template <typename T>
 __device__ __forceinline__ void face_flux_n(const T* l, const T* r, const Dev<T>& d, const T* n, T am, T* out) {
+  typedef Moments<T> Mo;
   T tot[8];
 #pragma unroll
   for (int side = 0; side < 2; ++side) {
@@ -1370,9 +1429,10 @@ __device__ __forceinline__ void face_flux_n(const T* l, const T* r, const Dev<T>
     const T rr = s[0], u0 = s[1], u1 = s[2], u2 = s[3], pr = s[4], b0 = s[5], b1 = s[6], b2 = s[7];
     const T vn = u0 * n[0] + u1 * n[1] + u2 * n[2];
     const T bn = b0 * n[0] + b1 * n[1] + b2 * n[2];
-    const T leng = T(0.5) * rr * (u0 * u0 + u1 * u1 + u2 * u2) + over_gm1(d, pr);
+    const T leng = T(0.5) * rr * (u0 * u0 + u1 * u1 + u2 * u2) + over_gm1<true>(d, pr);
+    T lam = Mo::div(rr, T(2) * pr);
     T v0, v1;
-    face_moments(d, rr, pr, vn, side == 0, v0, v1);
+    Mo::hydro(lam, vn, side == 0, v0, v1);
     T f[8];
     f[0] = rr * v1;
     f[1] = rr * u0 * v1 + pr * n[0] * v0;
@@ -1380,7 +1440,8 @@ __device__ __forceinline__ void face_flux_n(const T* l, const T* r, const Dev<T>
     f[3] = rr * u2 * v1 + pr * n[2] * v0;
     f[4] = (leng + T(0.5) * pr) * v1 + T(0.5) * pr * vn * v0;
     const T lbsq = b0 * b0 + b1 * b1 + b2 * b2;
-    v0 = face_moment_mag(d, rr, T(2) * pr + lbsq, vn, side == 0);
+    lam = Mo::div(rr, T(2) * pr + lbsq);
+    v0 = Mo::mag(lam, vn, side == 0);
     f[5] = (T(0.5) * lbsq * n[0] - b0 * bn) * v0;
     f[6] = (T(0.5) * lbsq * n[1] - b1 * bn) * v0;
     f[7] = (T(0.5) * lbsq * n[2] - b2 * bn) * v0;
@@ -1413,20 +1474,16 @@ __device__ __forceinline__ void recon_win(const T* w, const Prm<T>& P, T& fl, T&
     T fi = (TAP(3) + TAP(4)) / T(2);
     tvd<T, RECON == R_TVDMC>(TAP(2), TAP(3), TAP(4), TAP(5), fi, P.eps, fl, fr);
   } else {
-    weno5(TAP(1), TAP(2), TAP(3), TAP(4), TAP(5), TAP(6), P.eps, fl, fr);
-    if (RECON == R_MPWENO) {
-      fl = mp_side(fl, TAP(1), TAP(2), TAP(3), TAP(4), TAP(5), P.alpha, P.beta);
-      fr = mp_side(fr, TAP(6), TAP(5), TAP(4), TAP(3), TAP(2), P.alpha, P.beta);
-    }
+    weno_both<RECON>(TAP(1), TAP(2), TAP(3), TAP(4), TAP(5), TAP(6), P, fl, fr);
   }
 #undef TAP
 }
 
 // One-sided states of the 8 cell fields src[0..7] at the low face of element
 // c along stride s (recon_face per field); FP32 PDM on field pairs.
-template <typename T, int RECON, typename I>
+template <typename T, int RECON, bool M, typename I>
 __device__ __forceinline__ void face_states(const T* const* src, I c, I s, const Prm<T>& P, T* L, T* R) {
-  if constexpr (std::is_same<T, float>::value && is_pdm(RECON) && MHD_RECON_PACKED) {
+  if constexpr (std::is_same<T, float>::value && RECON == R_PDM && MHD_RECON_PACKED) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const float *fa = src[2 * q], *fb = src[2 * q + 1];
@@ -1434,13 +1491,24 @@ __device__ __forceinline__ void face_states(const T* const* src, I c, I s, const
 #pragma unroll
       for (int m = 0; m < 8; ++m) a[m] = make_float2(fa[c + (m - 4) * s], fb[c + (m - 4) * s]);
       float2 lr0, lr1;
-      pdm_pair_states<RECON>(a, P.pdmb, lr0, lr1);
+      pdm_pair_states(a, P.pdmb, lr0, lr1);
       L[2 * q] = lr0.x; R[2 * q] = lr0.y;
       L[2 * q + 1] = lr1.x; R[2 * q + 1] = lr1.y;
     }
+  } else if constexpr (std::is_same<T, float>::value && is_weno(RECON)) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float *fa = src[2 * q], *fb = src[2 * q + 1];
+      float2 a[6], l, r;
+#pragma unroll
+      for (int m = 0; m < 6; ++m) a[m] = make_float2(fa[c + (m - 3) * s], fb[c + (m - 3) * s]);
+      weno_both<RECON>(a[0], a[1], a[2], a[3], a[4], a[5], P, l, r);
+      L[2 * q] = l.x; R[2 * q] = r.x;
+      L[2 * q + 1] = l.y; R[2 * q + 1] = r.y;
+    }
   } else {
 #pragma unroll
-    for (int v = 0; v < 8; ++v) recon_face<T, RECON>(src[v], c, s, P, L[v], R[v]);
+    for (int v = 0; v < 8; ++v) recon_face<T, RECON, I, M>(src[v], c, s, P, L[v], R[v]);
   }
 }
 
@@ -1464,7 +1532,7 @@ __global__ void k_flux(KArg<T, B> ka, Inp<T> in0, Prm<T> P) {
   const int s = (D == 0) ? 1 : (D == 1) ? g.px : (int)g.plane;
   const T* src[8] = {in.rho, in.vx, in.vy, in.vz, in.p, in.bx, in.by, in.bz};
   T L[8], R[8], out[8];
-  face_states<T, RECON>(src, c, s, P, L, R);
+  face_states<T, RECON, M>(src, c, s, P, L, R);
   any_face_flux<T, D, M>(d, c, L, R, out);
 #pragma unroll
   for (int q = 0; q < 8; ++q) d.F[D][q][c] = out[q];
@@ -1496,12 +1564,7 @@ __device__ __forceinline__ void recon_col(const T* col, const Prm<T>& P, T& fl, 
     T fi = (col[3 * RS] + col[4 * RS]) / T(2);
     tvd<T, RECON == R_TVDMC>(col[2 * RS], col[3 * RS], col[4 * RS], col[5 * RS], fi, P.eps, fl, fr);
   } else {
-    T a1 = col[RS], a2 = col[2 * RS], a3 = col[3 * RS], a4 = col[4 * RS], a5 = col[5 * RS], a6 = col[6 * RS];
-    weno5(a1, a2, a3, a4, a5, a6, P.eps, fl, fr);
-    if (RECON == R_MPWENO) {
-      fl = mp_side(fl, a1, a2, a3, a4, a5, P.alpha, P.beta);
-      fr = mp_side(fr, a6, a5, a4, a3, a2, P.alpha, P.beta);
-    }
+    weno_both<RECON>(col[RS], col[2 * RS], col[3 * RS], col[4 * RS], col[5 * RS], col[6 * RS], P, fl, fr);
   }
 }
 
@@ -1535,9 +1598,11 @@ constexpr bool FLUX_STAGED = MHD_FLUX_STAGED != 0;
 // Resident blocks per SM requested for the flux tiles: FP32 trades registers
 // for occupancy (latency-bound); FP64 needs about twice the registers and
 // would spill at the FP32 setting.
-// The metric mode's general normal takes more registers as well.
-template <typename T, bool M> struct FluxMinB { static constexpr int value = M ? 4 : MHD_FLUX_MINB; };
-template <bool M> struct FluxMinB<double, M> { static constexpr int value = 2; };
+// The metric mode's general normal takes more registers as well, and so do the
+// packed WENO states (they spilled 0.8 KB at 32).
+template <typename T, bool M, int RECON> struct FluxMinB {
+  static constexpr int value = sizeof(T) == 8 ? 2 : RECON == R_WENO || RECON == R_MPWENO ? 3 : M ? 4 : MHD_FLUX_MINB;
+};
 
 template <typename T, int TDV = TD>
 __host__ __device__ constexpr size_t flux_t_smem() {
@@ -1565,12 +1630,12 @@ __device__ __forceinline__ void cell_update_vals(const Dev<T>& d, int c, int cd,
   } else {
     const T dz = d.wz[cd], rdz = d.rwz[cd];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) dv[q] = du[q] + Ops<T>::dw(dF[q], dz, rdz);
+    for (int q = 0; q < 8; ++q) dv[q] = du[q] + Ops<T>::dc(dF[q], dz, rdz);
   }
   // get_conserve of the current state (AB: the state, not the prediction)
   T rr = pv[0], u = pv[1], v = pv[2], ww = pv[3], pr = pv[4];
   T rvx0 = rr * u, rvy0 = rr * v, rvz0 = rr * ww;
-  T eng0 = T(0.5) * rr * (u * u + v * v + ww * ww) + over_gm1(d, pr);
+  T eng0 = T(0.5) * rr * (u * u + v * v + ww * ww) + over_gm1<M>(d, pr);
   if (form == FORM_SAVE) {  // U^n of the step (this first stage's input), read by the later stages' combines
     d.q[0][c] = rr;
     d.q[1][c] = rvx0;
@@ -1589,8 +1654,10 @@ __device__ __forceinline__ void cell_update_vals(const Dev<T>& d, int c, int cd,
     hz = comb(form, cw, qv[3], rz, den);
     eng1 = comb(form, cw, qv[4], eng1, den);
   }
-  const T rrho = Ops<T>::rcp(rho1);
-  T pn = gm1 * (eng1 - Ops<T>::dvr(T(0.5) * (hx * hx + hy * hy + hz * hz), rho1, rrho));
+  constexpr bool EXACT = M && std::is_same<T, double>::value;
+  const T rrho = EXACT ? T(0) : Ops<T>::rcp(rho1);
+  auto over_rho = [&](T x) { return EXACT ? x / rho1 : Ops<T>::dvr(x, rho1, rrho); };
+  T pn = gm1 * (eng1 - over_rho(T(0.5) * (hx * hx + hy * hy + hz * hz)));
   rx = rx - tau * dv[5];
   ry = ry - tau * dv[6];
   rz = rz - tau * dv[7];
@@ -1601,9 +1668,9 @@ __device__ __forceinline__ void cell_update_vals(const Dev<T>& d, int c, int cd,
   }
   d.orho[c] = rho1;
   d.op[c] = pn;
-  d.ovx[c] = Ops<T>::dvr(rx, rho1, rrho);
-  d.ovy[c] = Ops<T>::dvr(ry, rho1, rrho);
-  d.ovz[c] = Ops<T>::dvr(rz, rho1, rrho);
+  d.ovx[c] = over_rho(rx);
+  d.ovy[c] = over_rho(ry);
+  d.ovz[c] = over_rho(rz);
 }
 
 template <typename T, bool M>
@@ -1618,7 +1685,7 @@ __device__ __forceinline__ void cell_update(const Dev<T>& d, int c, int cd, cons
 }
 
 template <typename T, int RECON, int D, bool M, bool B, int TDV = TD>
-__global__ void __launch_bounds__(32 * (TDV + 1), FluxMinB<T, M>::value)
+__global__ void __launch_bounds__(32 * (TDV + 1), FluxMinB<T, M, RECON>::value)
     k_flux_t(KArg<T, B> ka, Inp<T> in0, Prm<T> P, int form, T cw, T den, int ab) {
   constexpr int TD = TDV;
   constexpr int TROWS = TDV + 8;
@@ -1684,7 +1751,7 @@ __global__ void __launch_bounds__(32 * (TDV + 1), FluxMinB<T, M>::value)
       for (int v = 0; v < 8; ++v) recon_col<T, RECON, 32>(sv + (v * TROWS + r) * 32 + tx, P, L[v], R[v]);
     } else {
       const int cf = rowbase + tx + cd * s;
-      face_states<T, RECON>(src, cf, s, P, L, R);
+      face_states<T, RECON, M>(src, cf, s, P, L, R);
     }
     any_face_flux<T, D, M>(d, rowbase + tx + cd * s, L, R, F);
 #pragma unroll
@@ -1710,7 +1777,7 @@ __global__ void __launch_bounds__(32 * (TDV + 1), FluxMinB<T, M>::value)
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const T* x = sX + (q * TD + r) * 33 + tx;
-      d.dU[q][c] = Ops<T>::dw(x[1] - x[0], dx, rdx) + Ops<T>::dw(dF[q], dy, rdy);
+      d.dU[q][c] = Ops<T>::dc(x[1] - x[0], dx, rdx) + Ops<T>::dc(dF[q], dy, rdy);
     }
     return;
   }
@@ -1860,9 +1927,17 @@ __global__ void __launch_bounds__(128, kSweepMinB)
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         float2 lr0, lr1;
-        pdm_pair_states<RECON>(w[q], P.pdmb, lr0, lr1);
+        pdm_pair_states(w[q], P.pdmb, lr0, lr1);
         L[2 * q] = lr0.x; R[2 * q] = lr0.y;
         L[2 * q + 1] = lr1.x; R[2 * q + 1] = lr1.y;
+      }
+    } else if constexpr (std::is_same<T, float>::value && is_weno(RECON)) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        float2 l, r;
+        weno_both<RECON>(w[q][1], w[q][2], w[q][3], w[q][4], w[q][5], w[q][6], P, l, r);
+        L[2 * q] = l.x; R[2 * q] = r.x;
+        L[2 * q + 1] = l.y; R[2 * q + 1] = r.y;
       }
     } else {
 #pragma unroll
@@ -1888,7 +1963,7 @@ __global__ void __launch_bounds__(128, kSweepMinB)
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
             const T* x = &xs[cc & 1][q][tx];
-            d.dU[q][c] = Ops<T>::dw(x[1] - x[0], dx, rdx) + Ops<T>::dw(dF[q], dy, rdy);
+            d.dU[q][c] = Ops<T>::dc(x[1] - x[0], dx, rdx) + Ops<T>::dc(dF[q], dy, rdy);
           }
         }
       } else {
@@ -2013,7 +2088,6 @@ inline dim3 emf_grid(int E, const Geom& g, int tx, int ty, int tz) {
 template <typename T, int E, int TX, int TY, int TZ, bool M>
 __device__ __forceinline__ void emf_pdm_tile(const Dev<T>& d, const Inp<T>& in, const Prm<T>& P, int ox, int oy,
                                              int oz) {
-  constexpr int FORM = pdm_form<T, M>();
   constexpr int A1 = (E + 1) % 3, A2 = (E + 2) % 3;
   constexpr int HX = (E == 0) ? 0 : 4, HY = (E == 1) ? 0 : 4, HZ = (E == 2) ? 0 : 4;
   constexpr int SX = TX + 2 * HX, SY = TY + 2 * HY, SZ = TZ + 2 * HZ;
@@ -2069,7 +2143,7 @@ __device__ __forceinline__ void emf_pdm_tile(const Dev<T>& d, const Inp<T>& in, 
     const int b0 = e * SE + f1 * S1 + r2 * S2;
     const int gi = e * GE + f1 * G1 + r2 * G2;
     const V* a = sv + b0;
-    sg[gi] = tap8p<FORM>(a[0], a[S1], a[2 * S1], a[3 * S1], a[4 * S1], a[5 * S1], a[6 * S1], a[7 * S1]);
+    sg[gi] = tap8p(a[0], a[S1], a[2 * S1], a[3 * S1], a[4 * S1], a[5 * S1], a[6 * S1], a[7 * S1]);
   }
   __syncthreads();
   const int n0[3] = {g.nx0, g.ny0, g.nz0};
@@ -2086,14 +2160,14 @@ __device__ __forceinline__ void emf_pdm_tile(const Dev<T>& d, const Inp<T>& in, 
     const int cv = e * SE + (f1 + 4) * S1 + (f2 + 4) * S2;
     const V* gg = sg + e * GE + f1 * G1 + f2 * G2;
     constexpr int GS = G2;
-    const V vi = tap8p<FORM>(gg[0], gg[GS], gg[2 * GS], gg[3 * GS], gg[4 * GS], gg[5 * GS], gg[6 * GS], gg[7 * GS]);
+    const V vi = tap8p(gg[0], gg[GS], gg[2 * GS], gg[3 * GS], gg[4 * GS], gg[5 * GS], gg[6 * GS], gg[7 * GS]);
     T v1av, v2av;
-    corner_pdm_pair<T, FORM>(sv, cv, S1, S2, vi, P.pdmb, v1av, v2av);
+    corner_pdm_pair<T>(sv, cv, S1, S2, vi, P.pdmb, v1av, v2av);
     const int c = gx + g.px * (gy + g.py * gz);
     const int s1 = st[A1], s2 = st[A2];
     T b1l, b1r, b2l, b2r;
-    recon_edge<T, FORM>(fb[A1], c, s2, P, b1l, b1r);
-    recon_edge<T, FORM>(fb[A2], c, s1, P, b2l, b2r);
+    recon_edge<T, R_PDM>(fb[A1], c, s2, P, b1l, b1r);
+    recon_edge<T, R_PDM>(fb[A2], c, s1, P, b2l, b2r);
     const T* vf = d.vf;
     const T eta = eta4(vf[c - s1 - s2], vf[c - s2], vf[c], vf[c - s1]);
     d.E[E][c] = emf_value<T, E, M>(d, c, v1av, v2av, b1l, b1r, b2l, b2r, eta);
@@ -2513,9 +2587,10 @@ __global__ void __launch_bounds__(NT) k_emf_weno(Dev<T> d, Inp<T> in, Prm<T> P) 
   typedef typename K::L1 L1;
   typedef typename K::L0 L0;
   constexpr int A1 = K::A1, A2 = K::A2, NV = K::NV, NP = K::NP, N1 = L1::N, N0 = L0::N;
+  typedef typename Pr<T>::V V;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* sv = reinterpret_cast<T*>(smem_raw);
-  T* sp = sv + 2 * NV;
+  V* sv = reinterpret_cast<V*>(smem_raw);  // [NV] (v_a1, v_a2)
+  V* sp = sv + NV;                         // L1, R1 [N1], L0, R0 [N0]
   const Geom& g = d.g;
   const int ox = g.ng + blockIdx.x * TX, oy = g.ng + blockIdx.y * TY, oz = g.ng + blockIdx.z * TZ;
   const T* vel[3] = {in.vx, in.vy, in.vz};
@@ -2531,38 +2606,29 @@ __global__ void __launch_bounds__(NT) k_emf_weno(Dev<T> d, Inp<T> in, Prm<T> P) 
       a = v1[gi];
       b = v2[gi];
     }
-    sv[t] = a;
-    sv[NV + t] = b;
+    sv[t] = Pr<T>::mk(a, b);
   }
   __syncthreads();
   // first pass: every row ("_1") and column ("_0") reconstruction of the
-  // tile for both components; tap q of an entry is the cell at offset q - 3
-  for (int t = threadIdx.x; t < 2 * NP; t += blockDim.x) {
-    const int w = t >= NP;
-    const int u = t - w * NP;
-    const T* src = sv + w * NV;
-    T* dst = sp + w * 2 * NP;
-    int e, f1, f2, base, step, o1, o2;
+  // tile, both components; tap q of an entry is the cell at offset q - 3
+  for (int u = threadIdx.x; u < NP; u += blockDim.x) {
+    int e, f1, f2, step, o1, o2;
     if (u < N1) {  // row f2 - 3 along a2, reconstructed along a1 at the face of cell f1
       L1::coords(u, e, f1, f2);
-      base = e * K::SE + f1 * K::S1 + f2 * K::S2;
       step = K::S1;
       o1 = u;
       o2 = N1 + u;
     } else {  // column f1 - 3 along a1, reconstructed along a2 at the face of cell f2
       L0::coords(u - N1, e, f1, f2);
-      base = e * K::SE + f1 * K::S1 + f2 * K::S2;
       step = K::S2;
       o1 = 2 * N1 + (u - N1);
       o2 = 2 * N1 + N0 + (u - N1);
     }
-    T a[6];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) a[q] = src[base + q * step];
-    T fl, fr;
-    weno_vals<T, RECON>(a, P, fl, fr);
-    dst[o1] = fl;
-    dst[o2] = fr;
+    const V* a = sv + e * K::SE + f1 * K::S1 + f2 * K::S2;
+    V fl, fr;
+    weno_both<RECON>(a[0], a[step], a[2 * step], a[3 * step], a[4 * step], a[5 * step], P, fl, fr);
+    sp[o1] = fl;
+    sp[o2] = fr;
   }
   __syncthreads();
   const int lim[3] = {g.ng + g.nx0 + (E != 0), g.ng + g.ny0 + (E != 1), g.ng + g.nz0 + (E != 2)};
@@ -2575,59 +2641,207 @@ __global__ void __launch_bounds__(NT) k_emf_weno(Dev<T> d, Inp<T> in, Prm<T> P) 
     const int e = (E == 0) ? lx : (E == 1) ? ly : lz;
     const int f1 = (A1 == 0) ? lx : (A1 == 1) ? ly : lz;
     const int f2 = (A2 == 0) ? lx : (A2 == 1) ? ly : lz;
-    T v1av = T(0), v2av = T(0);
-#pragma unroll 1
-    for (int w = 0; w < 2; ++w) {
-      const T* s = sp + w * 2 * NP;
-      // dif signs pick the smoother one-sided estimate per quadrant (2056-2106):
-      // "_0" (columns, second pass along d1) if d >= 0, else "_1" (rows)
-      const T* v = sv + w * NV;
-      const int c = e * K::SE + (f1 + 3) * K::S1 + (f2 + 3) * K::S2;
-      constexpr int s1 = K::S1, s2 = K::S2;
-      const int q00 = c - s1 - s2, q10 = c - s2, q01 = c - s1, q11 = c;
-      const T d00 = fab(v[q00 - s1] - v[q00]) - fab(v[q00 - s2] - v[q00]);
-      const T d10 = fab(v[q10 + s1] - v[q10]) - fab(v[q10 - s2] - v[q10]);
-      const T d01 = fab(v[q01 - s1] - v[q01]) - fab(v[q01 + s2] - v[q01]);
-      const T d11 = fab(v[q11 + s1] - v[q11]) - fab(v[q11 + s2] - v[q11]);
-      // left (L) and right (R) first-pass arrays of the rows ("_1") and columns ("_0")
-      const T* l1 = s + e * L1::GE + f1 * L1::G1 + f2 * L1::G2;           // rows f2 - 3 + m at m * G2
-      const T* l0 = s + 2 * N1 + e * L0::GE + f1 * L0::G1 + f2 * L0::G2;  // columns f1 - 3 + m
-      // only the chosen estimate of each quadrant is evaluated: v_00 / v_10 are
-      // the left states of the L / R stencils, v_01 / v_11 the right states
-      // (the left-state formula on the mirrored stencil)
-      auto pick = [&](bool col, int off) -> const T* { return col ? l0 + off : l1 + off; };
-      const T* a00 = pick(d00 >= T(0), 0);
-      const T* a10 = pick(d10 >= T(0), d10 >= T(0) ? N0 : N1);
-      const T* a01 = pick(d01 >= T(0), 0);
-      const T* a11 = pick(d11 >= T(0), d11 >= T(0) ? N0 : N1);
-      const int g00 = d00 >= T(0) ? L0::G1 : L1::G2, g10 = d10 >= T(0) ? L0::G1 : L1::G2;
-      const int g01 = d01 >= T(0) ? L0::G1 : L1::G2, g11 = d11 >= T(0) ? L0::G1 : L1::G2;
-      const T v00 = weno_one<T, RECON>(a00[0], a00[g00], a00[2 * g00], a00[3 * g00], a00[4 * g00], P);
-      const T v10 = weno_one<T, RECON>(a10[0], a10[g10], a10[2 * g10], a10[3 * g10], a10[4 * g10], P);
-      const T v01 = weno_one<T, RECON>(a01[5 * g01], a01[4 * g01], a01[3 * g01], a01[2 * g01], a01[g01], P);
-      const T v11 = weno_one<T, RECON>(a11[5 * g11], a11[4 * g11], a11[3 * g11], a11[2 * g11], a11[g11], P);
-      const T vc = T(0.25) * (v00 + v01 + v10 + v11);
-      if (w == 0)
-        v1av = vc;
-      else
-        v2av = vc;
-    }
+    // dif signs pick the smoother one-sided estimate per quadrant (2056-2106):
+    // "_0" (columns, second pass along d1) if |slope along d1| is not the
+    // smaller, else "_1" (rows); only that one is evaluated.  v_00 / v_10 are
+    // the left states of the L / R stencils, v_01 / v_11 the right states (the
+    // left-state formula on the mirrored stencil).
+    const V* v = sv + e * K::SE + (f1 + 3) * K::S1 + (f2 + 3) * K::S2;
+    constexpr int t1 = K::S1, t2 = K::S2;
+    const T* l1 = reinterpret_cast<const T*>(sp + e * L1::GE + f1 * L1::G1 + f2 * L1::G2);           // rows f2 - 3 + m
+    const T* l0 = reinterpret_cast<const T*>(sp + 2 * N1 + e * L0::GE + f1 * L0::G1 + f2 * L0::G2);  // columns f1 - 3 + m
+    // one quadrant: cell q, outward cells along d1 and d2, first-pass arrays
+    // (L or R) and the direction the stencil runs
+    auto quad = [&](const V q, const V o1, const V o2, bool rgt, bool mirror) -> V {
+      const bool bx = abs_ge(o1.x - q.x, o2.x - q.x), by = abs_ge(o1.y - q.y, o2.y - q.y);
+      const T* ax = bx ? l0 + (rgt ? 2 * N0 : 0) : l1 + (rgt ? 2 * N1 : 0);
+      const T* ay = (by ? l0 + (rgt ? 2 * N0 : 0) : l1 + (rgt ? 2 * N1 : 0)) + 1;
+      int gx2 = 2 * (bx ? L0::G1 : L1::G2), gy2 = 2 * (by ? L0::G1 : L1::G2);
+      if (mirror) {
+        ax += 5 * gx2; ay += 5 * gy2;
+        gx2 = -gx2; gy2 = -gy2;
+      }
+      return weno_side<V, RECON>(Pr<T>::mk(ax[0], ay[0]), Pr<T>::mk(ax[gx2], ay[gy2]),
+                                Pr<T>::mk(ax[2 * gx2], ay[2 * gy2]), Pr<T>::mk(ax[3 * gx2], ay[3 * gy2]),
+                                Pr<T>::mk(ax[4 * gx2], ay[4 * gy2]), P);
+    };
+    const V v00 = quad(v[-t1 - t2], v[-2 * t1 - t2], v[-t1 - 2 * t2], false, false);
+    const V v10 = quad(v[-t2], v[t1 - t2], v[-2 * t2], true, false);
+    const V v01 = quad(v[-t1], v[-2 * t1], v[-t1 + t2], false, true);
+    const V v11 = quad(v[0], v[t1], v[t2], true, true);
+    const T v1av = T(0.25) * (v00.x + v01.x + v10.x + v11.x);
+    const T v2av = T(0.25) * (v00.y + v01.y + v10.y + v11.y);
     const int c = gx + g.px * (gy + g.py * gz);
     const int s1 = st[A1], s2 = st[A2];
     T b1l, b1r, b2l, b2r;
     recon_edge<T, RECON>(fb[A1], c, s2, P, b1l, b1r);
     recon_edge<T, RECON>(fb[A2], c, s1, P, b2l, b2r);
-    T b1u = (v2av >= T(0)) ? b1l : b1r;
-    T b2u = (v1av >= T(0)) ? b2l : b2r;
-    T ee = -v1av * b2u + v2av * b1u;
     const T* vf = d.vf;
-    T eta = T(0.25) * (vf[c - s1 - s2] + vf[c - s2] + vf[c] + vf[c - s1]);
-    if (M)
-      ee = (T)d.m.ge[E][c] * ee + eta * (T)d.m.dl[E][c] * (b1l + b2r - b1r - b2l);
-    else
-      ee = ee + eta * (b1l + b2r - b1r - b2l);
-    d.E[E][c] = ee;
+    const T eta = eta4(vf[c - s1 - s2], vf[c - s2], vf[c], vf[c - s1]);
+    d.E[E][c] = emf_value<T, E, M>(d, c, v1av, v2av, b1l, b1r, b2l, b2r, eta);
   }
+}
+
+// The same in FP64, where the FP64 pipe (2 lanes per SM and cycle) bounds the
+// kernel and every reconstructed state costs it about 100 operations: the tile
+// sizes are chosen at run time so that no state is computed for padding, and
+// the states of the second pass are spread one per thread.
+//  - Across (a1, a2) a tile has at most kW64 x kW64 edges, the n0 + 1 edges of an
+//    axis split evenly (17 = 9 + 8): the first pass reconstructs
+//    (T2 + 5) / T2 states per edge and direction, 1.6 at 9, 2.3 at the 4 x 4
+//    tiles this replaces.
+//  - Along the edge axis a tile has TE edges without halo: 4, fewer while the
+//    launch has less than three blocks per SM (a 16^3 grid: 1, 192 blocks).
+//  - Second pass: 12 states per edge (4 quadrants of 2 components, 2 states of
+//    2 face-B components), one thread each, gathered per edge.
+constexpr int kW64 = 9;
+struct Weno64Shape {
+  int te, t1, t2;  // edges per tile
+  int ne, n1, n2;  // edges of the family along the edge axis, a1, a2
+  __host__ __device__ Weno64Shape(int E, const Geom& g) {
+    const int n0[3] = {g.nx0, g.ny0, g.nz0};
+    ne = n0[E];
+    n1 = n0[(E + 1) % 3] + 1;
+    n2 = n0[(E + 2) % 3] + 1;
+    t1 = split(n1);
+    t2 = split(n2);
+    te = 4;
+    while (te > 1 && blocks() < 3 * 152) te /= 2;
+  }
+  static __host__ __device__ int split(int n) {
+    const int tiles = (n + kW64 - 1) / kW64;
+    return (n + tiles - 1) / tiles;
+  }
+  __host__ __device__ int be() const { return (ne + te - 1) / te; }
+  __host__ __device__ int b1() const { return (n1 + t1 - 1) / t1; }
+  __host__ __device__ int b2() const { return (n2 + t2 - 1) / t2; }
+  __host__ __device__ int blocks() const { return be() * b1() * b2(); }
+  // doubles of shared memory: cells, first-pass states, second-pass states
+  __host__ __device__ size_t smem() const {
+    return sizeof(double) * (size_t)te *
+           (2 * (t1 + 5) * (t2 + 5) + 4 * (t1 * (t2 + 5) + (t1 + 5) * t2) + 12 * t1 * t2);
+  }
+};
+
+template <int RECON, int E, bool M>
+__global__ void __launch_bounds__(256) k_emf_weno64(Dev<double> d, Inp<double> in, Prm<double> P) {
+  constexpr int A1 = (E + 1) % 3, A2 = (E + 2) % 3;
+  const Geom& g = d.g;
+  const Weno64Shape w(E, g);
+  int blk = blockIdx.x;
+  const int o1 = (blk % w.b1()) * w.t1;
+  blk /= w.b1();
+  const int o2 = (blk % w.b2()) * w.t2, oe = (blk / w.b2()) * w.te;
+  const int te = min(w.te, w.ne - oe), t1 = min(w.t1, w.n1 - o1), t2 = min(w.t2, w.n2 - o2);  // this tile's edges
+  const int c1 = t1 + 5, c2 = t2 + 5;  // staged cells: [-3, t + 2) about the tile's edges
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double* sv = reinterpret_cast<double*>(smem_raw);  // [2][te][c2][c1]
+  const int nv = te * c1 * c2, n1 = te * t1 * c2, n0 = te * c1 * t2, ned = te * t1 * t2;
+  double* s1l = sv + 2 * nv;   // rows along a1: [2][te][c2][t1], left and right
+  double* s1r = s1l + 2 * n1;
+  double* s0l = s1r + 2 * n1;  // columns along a2: [2][te][t2][c1]
+  double* s0r = s0l + 2 * n0;
+  double* sq = s0r + 2 * n0;   // [12][ned]
+  const int st[3] = {1, g.px, (int)g.plane};
+  const int se = st[E], st1 = st[A1], st2 = st[A2];
+  const int org = (g.ng + oe) * se + (g.ng + o1) * st1 + (g.ng + o2) * st2;  // first edge's upper cell
+  const double* vel[3] = {in.vx, in.vy, in.vz};
+  for (int t = threadIdx.x; t < 2 * nv; t += blockDim.x) {
+    const int c = t >= nv, u = t - c * nv;
+    const int i1 = u % c1, r = u / c1, i2 = r % c2, e = r / c2;
+    sv[t] = (c ? vel[A2] : vel[A1])[org + e * se + (i1 - 3) * st1 + (i2 - 3) * st2];
+  }
+  __syncthreads();
+  // first pass, one state per thread: [side][rows of both components, columns of both components]
+  const int half = 2 * (n1 + n0);
+  for (int t = threadIdx.x; t < 2 * half; t += blockDim.x) {
+    const int right = t >= half;
+    int u = t - right * half;
+    const double* a;
+    double* dst;
+    int step;
+    if (u < 2 * n1) {
+      dst = (right ? s1r : s1l) + u;
+      const int c = u >= n1;
+      u -= c * n1;
+      const int f1 = u % t1, r = u / t1;  // r = e c2 + row
+      a = sv + c * nv + r * c1 + f1;
+      step = 1;
+    } else {
+      u -= 2 * n1;
+      dst = (right ? s0r : s0l) + u;
+      const int c = u >= n0;
+      u -= c * n0;
+      const int i1 = u % c1, r = u / c1, f2 = r % t2, e = r / t2;
+      a = sv + c * nv + (e * c2 + f2) * c1 + i1;
+      step = c1;
+    }
+    if (right) {  // the mirrored stencil
+      a += 5 * step;
+      step = -step;
+    }
+    *dst = weno_side_ref<RECON>(a[0], a[step], a[2 * step], a[3 * step], a[4 * step], P);
+  }
+  __syncthreads();
+  // second pass, one state per thread: 0-7 quadrant and component, 8-11 face B
+  const double* fb[3] = {in.bi, in.bj, in.bk};
+  for (int t = threadIdx.x; t < 12 * ned; t += blockDim.x) {
+    const int k = t / ned, u = t - k * ned;
+    const int f1 = u % t1, r = u / t1, f2 = r % t2, e = r / t2;
+    const double* a;
+    int step;
+    bool right;
+    if (k < 8) {
+      const int q = k >> 1, c = k & 1;
+      const bool q1 = q & 1, q2 = q & 2;  // quadrant cell (f1 - 1 + q1, f2 - 1 + q2)
+      const double* v = sv + c * nv + (e * c2 + f2 + 2 + q2) * c1 + f1 + 2 + q1;
+      // the smoother one-sided estimate: columns ("_0") if the outward slope along a1 is not the smaller, else rows
+      const bool col = abs_ge(v[q1 ? 1 : -1] - v[0], v[q2 ? c1 : -c1] - v[0]);
+      // v_10, v_11 (q1) read the R stencils, v_01, v_11 (q2) take the right state
+      if (col) {
+        a = (q1 ? s0r : s0l) + c * n0 + (e * t2 + f2) * c1 + f1;  // columns f1 - 3 ..
+        step = 1;
+      } else {
+        a = (q1 ? s1r : s1l) + c * n1 + (e * c2 + f2) * t1 + f1;  // rows f2 - 3 ..
+        step = t1;
+      }
+      right = q2;
+    } else {  // b_a1 along a2 (8, 9), b_a2 along a1 (10, 11)
+      step = k < 10 ? st2 : st1;
+      a = (k < 10 ? fb[A1] : fb[A2]) + org + e * se + f1 * st1 + f2 * st2 - 3 * step;
+      right = k & 1;
+    }
+    if (right) {
+      a += 5 * step;
+      step = -step;
+    }
+    sq[t] = weno_side_ref<RECON>(a[0], a[step], a[2 * step], a[3 * step], a[4 * step], P);
+  }
+  __syncthreads();
+  for (int u = threadIdx.x; u < ned; u += blockDim.x) {
+    const int f1 = u % t1, r = u / t1, f2 = r % t2, e = r / t2;
+    const double* q = sq + u;
+    // the mean in the reference's order (00, 01, 10, 11); quadrant index q1 + 2 q2
+    const double v1 = 0.25 * (q[0] + q[4 * ned] + q[2 * ned] + q[6 * ned]);
+    const double v2 = 0.25 * (q[ned] + q[5 * ned] + q[3 * ned] + q[7 * ned]);
+    const int c = org + e * se + f1 * st1 + f2 * st2;
+    const double* vf = d.vf;
+    const double eta = eta4(vf[c - st1 - st2], vf[c - st2], vf[c], vf[c - st1]);
+    d.E[E][c] = emf_value<double, E, M>(d, c, v1, v2, q[8 * ned], q[9 * ned], q[10 * ned], q[11 * ned], eta);
+  }
+}
+
+template <int RECON, int E, bool M>
+void launch_emf_weno64(const Dev<double>& d, const Inp<double>& in, const Prm<double>& P, cudaStream_t st) {
+  static PerDevice attr;
+  unsigned long long bit = 0;
+  if (attr.need(bit)) {  // the largest tile: 4 x 9 x 9
+    cudaFuncSetAttribute(k_emf_weno64<RECON, E, M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)(sizeof(double) * 4 * (2 * 14 * 14 + 8 * 9 * 14 + 12 * 81)));
+    attr.mark(bit);
+  }
+  const Weno64Shape w(E, d.g);
+  k_emf_weno64<RECON, E, M><<<w.blocks(), 256, w.smem(), st>>>(d, in, P);
 }
 
 template <typename T, int RECON, int E, int TX, int TY, int TZ, int NT, bool M>
@@ -2708,17 +2922,17 @@ __global__ void k_update_b(KArg<T, B> ka, int form, T cw, T den) {
     return;
   }
   if (in_y && in_z) {
-    T b = d.bi[c] - tau * (O::dw(ek[c + sy] - ek[c], dy, ry) - O::dw(ej[c + sz] - ej[c], dz, rz));
+    T b = d.bi[c] - tau * (O::dc(ek[c + sy] - ek[c], dy, ry) - O::dc(ej[c + sz] - ej[c], dz, rz));
     if (form >= 0) b = comb(form, cw, d.q[5][c], b, den);
     d.obi[c] = b;
   }
   if (in_x && in_z) {
-    T b = d.bj[c] - tau * (O::dw(ei[c + sz] - ei[c], dz, rz) - O::dw(ek[c + 1] - ek[c], dx, rx));
+    T b = d.bj[c] - tau * (O::dc(ei[c + sz] - ei[c], dz, rz) - O::dc(ek[c + 1] - ek[c], dx, rx));
     if (form >= 0) b = comb(form, cw, d.q[6][c], b, den);
     d.obj[c] = b;
   }
   if (in_x && in_y) {
-    T b = d.bk[c] - tau * (O::dw(ej[c + 1] - ej[c], dx, rx) - O::dw(ei[c + sy] - ei[c], dy, ry));
+    T b = d.bk[c] - tau * (O::dc(ej[c + 1] - ej[c], dx, rx) - O::dc(ei[c + sy] - ei[c], dy, ry));
     if (form >= 0) b = comb(form, cw, d.q[7][c], b, den);
     d.obk[c] = b;
   }
@@ -2991,15 +3205,15 @@ __global__ void __launch_bounds__(256, pass_min_blocks(B))
     const T *ei = d.E[0], *ej = d.E[1], *ek = d.E[2];
     typedef Ops<T> O;
     auto new_bi = [&](int f) {
-      T b = d.bi[f] - tau * (O::dw(ek[f + px] - ek[f], dy, ry) - O::dw(ej[f + pl] - ej[f], dz, rz));
+      T b = d.bi[f] - tau * (O::dc(ek[f + px] - ek[f], dy, ry) - O::dc(ej[f + pl] - ej[f], dz, rz));
       return form >= 0 ? comb(form, cw, d.q[5][f], b, den) : b;
     };
     auto new_bj = [&](int f) {
-      T b = d.bj[f] - tau * (O::dw(ei[f + pl] - ei[f], dz, rz) - O::dw(ek[f + 1] - ek[f], dx, rx));
+      T b = d.bj[f] - tau * (O::dc(ei[f + pl] - ei[f], dz, rz) - O::dc(ek[f + 1] - ek[f], dx, rx));
       return form >= 0 ? comb(form, cw, d.q[6][f], b, den) : b;
     };
     auto new_bk = [&](int f) {
-      T b = d.bk[f] - tau * (O::dw(ej[f + 1] - ej[f], dx, rx) - O::dw(ei[f + px] - ei[f], dy, ry));
+      T b = d.bk[f] - tau * (O::dc(ej[f + 1] - ej[f], dx, rx) - O::dc(ei[f + px] - ei[f], dy, ry));
       return form >= 0 ? comb(form, cw, d.q[7][f], b, den) : b;
     };
     const bool lx = i == g.ng + g.nx0 - 1, ly = j == g.ng + g.ny0 - 1, lz = k == g.ng + g.nz0 - 1;
@@ -3232,7 +3446,7 @@ void flux_r(const Dev<T>& d, const Inp<T>& in, cudaStream_t st) {
 template <typename T, bool M>
 void Launch<T, M>::fluxes(const Dev<T>& d, const Inp<T>& in, cudaStream_t st) {
   switch (d.recon) {
-    case R_PDM: flux_r<T, pdm_form<T, M>(), M>(d, in, st); break;
+    case R_PDM: flux_r<T, R_PDM, M>(d, in, st); break;
     case R_PDMG: flux_r<T, R_PDMG, M>(d, in, st); break;
     case R_TVD: flux_r<T, R_TVD, M>(d, in, st); break;
     case R_WENO: flux_r<T, R_WENO, M>(d, in, st); break;
@@ -3308,7 +3522,7 @@ template <typename T, bool M>
 void Launch<T, M>::hydro(const Dev<T>& d, const Inp<T>& in, int part, int form, double c, double den, bool ab,
                          cudaStream_t st) {
   switch (d.recon) {
-    case R_PDM: hydro_r<T, pdm_form<T, M>(), M>(d, in, part, form, c, den, ab, st); break;
+    case R_PDM: hydro_r<T, R_PDM, M>(d, in, part, form, c, den, ab, st); break;
     case R_PDMG: hydro_r<T, R_PDMG, M>(d, in, part, form, c, den, ab, st); break;
     case R_TVD: hydro_r<T, R_TVD, M>(d, in, part, form, c, den, ab, st); break;
     case R_WENO: hydro_r<T, R_WENO, M>(d, in, part, form, c, den, ab, st); break;
@@ -3424,14 +3638,19 @@ void emf_yee(const Dev<T>& d, const Inp<T>& in, cudaStream_t st) {
   }
 }
 
-// ei tiles of 32 (FP32) or 16 (FP64) edges x 4 x 4; ej, ek plane tiles of 32 x 8.
+// FP32: ei tiles of 32 x 4 x 4 edges; ej, ek plane tiles of 32 x 8.
 template <typename T, int RECON, bool M>
 void emf_weno(const Dev<T>& d, const Inp<T>& in, cudaStream_t st) {
   const Prm<T> P = prm_of(d);
-  constexpr int EX = std::is_same<T, float>::value ? 32 : 16;
-  launch_emf_weno<T, RECON, 0, EX, 4, 4, EX * 16, M>(d, in, P, st);
-  launch_emf_weno<T, RECON, 1, 32, 1, 8, 256, M>(d, in, P, st);
-  launch_emf_weno<T, RECON, 2, 32, 8, 1, 256, M>(d, in, P, st);
+  if constexpr (std::is_same<T, double>::value) {
+    launch_emf_weno64<RECON, 0, M>(d, in, P, st);
+    launch_emf_weno64<RECON, 1, M>(d, in, P, st);
+    launch_emf_weno64<RECON, 2, M>(d, in, P, st);
+  } else {
+    launch_emf_weno<T, RECON, 0, 32, 4, 4, 512, M>(d, in, P, st);
+    launch_emf_weno<T, RECON, 1, 32, 1, 8, 256, M>(d, in, P, st);
+    launch_emf_weno<T, RECON, 2, 32, 8, 1, 256, M>(d, in, P, st);
+  }
 }
 
 template <typename T, int RECON, bool M>
@@ -3476,7 +3695,7 @@ void Launch<T, M>::emf(const Dev<T>& d, const Inp<T>& in0, cudaStream_t st) {
     in.vx = d.mw[0]; in.vy = d.mw[1]; in.vz = d.mw[2];
     in.bi = d.mbn[0]; in.bj = d.mbn[1]; in.bk = d.mbn[2];
   }
-  if (d.recon == R_PDM || (d.recon == R_PDMG && pdm_form<T, M>() == R_PDMG)) {
+  if (d.recon == R_PDM) {
     Prm<T> P = prm_of(d);
     if constexpr (std::is_same<T, float>::value && !M) {
       if (d.tile_ey == kEmfStream) {

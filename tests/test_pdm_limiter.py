@@ -1,10 +1,11 @@
-"""The PDM limiter as nested intervals (Sel / within / pdm_states of the kernels).
+"""The PDM limiter without its signs (pdm_states, within and corner_quad of the kernels).
 
-CPU: the interval form against the reference's sign form (PDM2,
+CPU: the soft threshold (FP32 kernels) bit for bit and the nested intervals
+(FP64 face fluxes) to rounding against the reference's sign form (PDM2,
 mhd3d3.f90:1069-1172) for positive pdmb, ties, jumps and values across the
 exponent range included.  GPU: fluxes and EMFs for limiter constants on both
-sides of the rule (pdmb > 0 takes the intervals, anything else the reference's
-form) against the oracle, in every launch shape that reads the limiter.
+sides of the rule (pdmb > 0 takes these forms, anything else the reference's)
+against the oracle, in every launch shape that reads the limiter.
 """
 import numpy as np
 import pytest
@@ -27,16 +28,44 @@ def reference(fm2, fm1, f0, fp1, fi, pdmb):
     return left, right
 
 
-@pytest.mark.parametrize("pdmb", [1e-6, 0.25, 1.0, 4.0, 1e6])
-@pytest.mark.parametrize("kind", ["random", "ties", "wide"])
-def test_interval_form_is_the_reference_limiter(kind, pdmb):
+def threshold(near, x, D):
+    """shrink() and its use: the excess of x - near over D, with the kernels' operations."""
+    d = x - near
+    m = np.minimum(np.abs(d), np.abs(D)) * np.where(np.signbit(d) == np.signbit(D), 1, -1).astype(d.dtype)
+    return x - (d - np.copysign(np.maximum(m, 0), d))
+
+
+def cells(kind):
     rng = np.random.default_rng(3)
     n = 20000
     f = rng.standard_normal((5, n))
     if kind == "ties":  # equal neighbours, zero and signed-zero slopes
         f = rng.integers(-2, 3, size=(5, n)).astype(float) * rng.choice([1.0, -0.0, 0.0], size=(5, n))
     if kind == "wide":
-        f *= 10.0 ** rng.uniform(-30, 30, size=(1, n))
+        f *= 10.0 ** rng.uniform(-15, 15, size=(1, n))
+    return f
+
+
+@pytest.mark.parametrize("pdmb", [0.25, 0.3, 4.0])
+@pytest.mark.parametrize("kind", ["random", "ties", "wide"])
+def test_threshold_has_the_reference_bits_in_fp32(kind, pdmb):
+    f = cells(kind).astype(np.float32)
+    p = np.float32(pdmb)
+    sg = lambda v: np.where(v >= 0, np.float32(1), np.float32(-1))
+    x = np.maximum(np.minimum(f[1], f[2]), np.minimum(f[4], np.maximum(f[1], f[2])))
+    dm, d0, dp = p * (f[1] - f[0]), p * (f[2] - f[1]), p * (f[3] - f[2])
+    zero = np.float32(0)
+    l = x - sg(d0) * np.maximum(zero, np.abs(x - f[1]) - np.abs(sg(dm) + sg(d0)) * np.abs(dm))
+    r = x + sg(d0) * np.maximum(zero, np.abs(f[2] - x) - np.abs(sg(d0) + sg(dp)) * np.abs(dp))
+    k = p + p
+    assert np.array_equal(threshold(f[1], x, k * (f[1] - f[0])), l)
+    assert np.array_equal(threshold(f[2], x, k * (f[2] - f[3])), r)
+
+
+@pytest.mark.parametrize("pdmb", [1e-6, 0.25, 1.0, 4.0, 1e6])
+@pytest.mark.parametrize("kind", ["random", "ties", "wide"])
+def test_interval_form_is_the_reference_limiter(kind, pdmb):
+    f = cells(kind)
     l, r = reference(*f, pdmb)
     a, b = within(f[1], f[2], f[1] + 2 * pdmb * (f[1] - f[0]), f[4]), within(f[2], f[1], f[2] + 2 * pdmb * (f[2] - f[3]), f[4])
     # a few roundings of the largest term: the cells and the slopes times 2 pdmb
