@@ -1538,6 +1538,46 @@ __global__ void k_flux(KArg<T, B> ka, Inp<T> in0, Prm<T> P) {
   for (int q = 0; q < 8; ++q) d.F[D][q][c] = out[q];
 }
 
+// FP64, single grids: the faces of all three axes in one launch, their fluxes
+// to memory, and the conserved update of k_update_faces after it.  The FP64 pipe
+// bounds the faces, so the fluxes' traffic is free, no face is computed twice
+// (the y / z tiles recompute one of nine), the lanes are full whatever the
+// extents (nx0 = 16 left half of a tile's idle), and 16^3 cells are spread over
+// every SM (blocks of 64 faces while there are few).  The y fluxes take the
+// place of dU, the z fluxes the other half's face B, dead until CT writes it, and
+// five arrays of their own (Dev::fz; without them, on a grid that leaves no room,
+// the tiles run).
+template <typename T, int D>
+__device__ __forceinline__ T* face_flux_ptr(const Dev<T>& d, int q) {
+  if (D == 0) return d.F[0][q];
+  if (D == 1) return d.dU[q];
+  return q == 0 ? d.obi : q == 1 ? d.obj : q == 2 ? d.obk : d.fz[q < 3 ? 0 : q - 3];
+}
+template <typename T, int RECON, int D, bool M>
+__device__ __forceinline__ void face_one(const Dev<T>& d, const Inp<T>& in, const Prm<T>& P, int t, int ni, int nj) {
+  const Geom& g = d.g;
+  const int i = t % ni, r = t / ni, j = r % nj, k = r / nj;
+  const int c = i + g.ng + g.px * (j + g.ng + g.py * (k + g.ng));
+  const int s = (D == 0) ? 1 : (D == 1) ? g.px : (int)g.plane;
+  const T* src[8] = {in.rho, in.vx, in.vy, in.vz, in.p, in.bx, in.by, in.bz};
+  T L[8], R[8], out[8];
+  face_states<T, RECON, M>(src, c, s, P, L, R);
+  any_face_flux<T, D, M>(d, c, L, R, out);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) face_flux_ptr<T, D>(d, q)[c] = out[q];
+}
+template <typename T, int RECON, bool M>
+__global__ void __launch_bounds__(128) k_faces(Dev<T> d, Inp<T> in, Prm<T> P) {
+  const Geom& g = d.g;
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int n0 = (g.nx0 + 1) * g.ny0 * g.nz0, n1 = g.nx0 * (g.ny0 + 1) * g.nz0, n2 = g.nx0 * g.ny0 * (g.nz0 + 1);
+  if (t < n0) return face_one<T, RECON, 0, M>(d, in, P, t, g.nx0 + 1, g.ny0);
+  t -= n0;
+  if (t < n1) return face_one<T, RECON, 1, M>(d, in, P, t, g.nx0, g.ny0 + 1);
+  t -= n1;
+  if (t < n2) face_one<T, RECON, 2, M>(d, in, P, t, g.nx0, g.ny0);
+}
+
 // Stage combine of the RK steps (mhd3d3.f90:3674-3702, 3745-3788):
 // form 0: (Xp+X)/den, 1: (c*Xp+X)/den, 2: (Xp+c*X)/den.
 // FP64: the divisors are 2, 4 and 3 (forms 0, 1, 2), an exact scaling or two
@@ -1682,6 +1722,28 @@ __device__ __forceinline__ void cell_update(const Dev<T>& d, int c, int cd, cons
 #pragma unroll
   for (int q = 0; q < 5; ++q) qv[q] = (form >= 0) ? d.q[q][c] : T(0);
   cell_update_vals<T, M>(d, c, cd, dF, du, pv, qv, form, cw, den);
+}
+
+// The update after k_faces: the flux divergence in the tiles' order, then cell_update_vals.
+template <typename T, bool M>
+__global__ void __launch_bounds__(128) k_update_faces(Dev<T> d, int form, T cw, T den) {
+  const Geom& g = d.g;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= g.nx0 * g.ny0 * g.nz0) return;
+  const int i = t % g.nx0 + g.ng, r = t / g.nx0, j = r % g.ny0 + g.ng, k = r / g.ny0 + g.ng;
+  const int c = i + g.px * (j + g.py * k), sy = g.px, sz = (int)g.plane;
+  T du[8], dF[8], pv[5], qv[5];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const T *fx = face_flux_ptr<T, 0>(d, q), *fy = face_flux_ptr<T, 1>(d, q), *fz = face_flux_ptr<T, 2>(d, q);
+    const T dx = fx[c + 1] - fx[c], dy = fy[c + sy] - fy[c];
+    du[q] = M ? dx + dy : Ops<T>::dc(dx, d.wx[i], d.rwx[i]) + Ops<T>::dc(dy, d.wy[j], d.rwy[j]);
+    dF[q] = fz[c + sz] - fz[c];
+  }
+  pv[0] = d.rho[c]; pv[1] = d.vx[c]; pv[2] = d.vy[c]; pv[3] = d.vz[c]; pv[4] = d.p[c];
+#pragma unroll
+  for (int q = 0; q < 5; ++q) qv[q] = (form >= 0) ? d.q[q][c] : T(0);
+  cell_update_vals<T, M>(d, c, k, dF, du, pv, qv, form, cw, den);
 }
 
 template <typename T, int RECON, int D, bool M, bool B, int TDV = TD>
@@ -2682,74 +2744,108 @@ __global__ void __launch_bounds__(NT) k_emf_weno(Dev<T> d, Inp<T> in, Prm<T> P) 
   }
 }
 
-// The same in FP64, where the FP64 pipe (2 lanes per SM and cycle) bounds the
-// kernel and every reconstructed state costs it about 100 operations: the tile
-// sizes are chosen at run time so that no state is computed for padding, and
-// the states of the second pass are spread one per thread.
-//  - Across (a1, a2) a tile has at most kW64 x kW64 edges, the n0 + 1 edges of an
-//    axis split evenly (17 = 9 + 8): the first pass reconstructs
-//    (T2 + 5) / T2 states per edge and direction, 1.6 at 9, 2.3 at the 4 x 4
-//    tiles this replaces.
-//  - Along the edge axis a tile has TE edges without halo: 4, fewer while the
-//    launch has less than three blocks per SM (a 16^3 grid: 1, 192 blocks).
-//  - Second pass: 12 states per edge (4 quadrants of 2 components, 2 states of
-//    2 face-B components), one thread each, gathered per edge.
-constexpr int kW64 = 9;
-struct Weno64Shape {
-  int te, t1, t2;  // edges per tile
-  int ne, n1, n2;  // edges of the family along the edge axis, a1, a2
-  __host__ __device__ Weno64Shape(int E, const Geom& g) {
-    const int n0[3] = {g.nx0, g.ny0, g.nz0};
-    ne = n0[E];
-    n1 = n0[(E + 1) % 3] + 1;
-    n2 = n0[(E + 2) % 3] + 1;
-    t1 = split(n1);
-    t2 = split(n2);
-    te = 4;
-    while (te > 1 && blocks() < 3 * 152) te /= 2;
-  }
-  static __host__ __device__ int split(int n) {
-    const int tiles = (n + kW64 - 1) / kW64;
+// ------------------------------------------------------------- FP64 EMF
+// The FP64 pipe (2 lanes per SM and cycle) bounds the FP64 edge EMF: a WENO
+// state costs it about 100 operations, a PDM interpolant 17.  All three families
+// run as one launch of run-time tiles, so that nothing is computed for padding
+// and a small grid still reaches every SM, and the states of a tile are spread
+// one per thread.
+//  - WENO across (a1, a2): at most 9 x 9 edges (6 x 6 while the launch is short of
+//    blocks), the n0 + 1 edges of an axis split evenly (17 = 9 + 8).  The first
+//    pass reconstructs (t + 5) / t states per edge and direction (1.6 at 9, 2.3
+//    at the 4 x 4 tiles before), the second 12 per edge: 4 quadrants of 2
+//    components, 2 states of 2 face-B components.
+//  - PDM: at most 4 x 33 edges; only the first pass of the interpolant has a halo,
+//    along a2: (t2 + 8) / t2 interpolants per edge, 1.25 at 33 (3 in the 4 x 4 ei
+//    tiles before, 2 in the 8-deep planes).
+//  - Along the edge axis te edges without halo: 4, fewer while there are less
+//    than three blocks per SM.
+struct Tile64 {
+  int te, t1, t2;     // edges per tile along the edge axis, a1, a2
+  int ne, n1, n2;     // edges of the family
+  int be, b1, b2;     // tiles
+};
+struct Tiles64 {
+  Tile64 f[3];
+  int blocks[3];
+  size_t smem;
+  static int split(int n, int most) {
+    const int tiles = (n + most - 1) / most;
     return (n + tiles - 1) / tiles;
   }
-  __host__ __device__ int be() const { return (ne + te - 1) / te; }
-  __host__ __device__ int b1() const { return (n1 + t1 - 1) / t1; }
-  __host__ __device__ int b2() const { return (n2 + t2 - 1) / t2; }
-  __host__ __device__ int blocks() const { return be() * b1() * b2(); }
-  // doubles of shared memory: cells, first-pass states, second-pass states
-  __host__ __device__ size_t smem() const {
-    return sizeof(double) * (size_t)te *
-           (2 * (t1 + 5) * (t2 + 5) + 4 * (t1 * (t2 + 5) + (t1 + 5) * t2) + 12 * t1 * t2);
+  // doubles of shared memory of a tile: cells, first-pass states, second-pass results
+  static size_t words(bool weno, int te, int t1, int t2) {
+    return weno ? (size_t)te * (2 * (t1 + 5) * (t2 + 5) + 4 * (t1 * (t2 + 5) + (t1 + 5) * t2) + 12 * t1 * t2)
+                : (size_t)te * (2 * (t1 + 8) * (t2 + 8) + 2 * t1 * (t2 + 8) + 6 * t1 * t2);
+  }
+  Tiles64(bool weno, const Geom& g) {
+    const int n0[3] = {g.nx0, g.ny0, g.nz0};
+    const int m1[2] = {weno ? 9 : 4, weno ? 6 : 4}, m2[2] = {weno ? 9 : 33, weno ? 6 : 9};
+    int total = 0;
+    for (int small = 0; small < 2; ++small)
+      for (int te = 4; te >= 1; te /= 2) {
+        total = 0;
+        smem = 0;
+        for (int e = 0; e < 3; ++e) {
+          Tile64& t = f[e];
+          t.ne = n0[e];
+          t.n1 = n0[(e + 1) % 3] + 1;
+          t.n2 = n0[(e + 2) % 3] + 1;
+          t.te = te;
+          t.t1 = split(t.n1, m1[small]);
+          t.t2 = split(t.n2, m2[small]);
+          t.be = (t.ne + te - 1) / te;
+          t.b1 = (t.n1 + t.t1 - 1) / t.t1;
+          t.b2 = (t.n2 + t.t2 - 1) / t.t2;
+          total += blocks[e] = t.be * t.b1 * t.b2;
+          const size_t w = sizeof(double) * words(weno, te, t.t1, t.t2);
+          smem = w > smem ? w : smem;
+        }
+        if (total >= 3 * 152) return;
+      }
+  }
+  static size_t max_smem(bool weno) { return sizeof(double) * (weno ? words(true, 4, 9, 9) : words(false, 4, 4, 33)); }
+};
+
+// The tile's place: edges te x t1 x t2 from (oe, o1, o2), org the element index
+// of its first edge's upper cell.
+template <int E>
+struct Place64 {
+  int te, t1, t2, se, s1, s2, org;
+  __device__ __forceinline__ Place64(const Geom& g, const Tile64& w, int blk) {
+    constexpr int A1 = (E + 1) % 3, A2 = (E + 2) % 3;
+    const int o1 = (blk % w.b1) * w.t1;
+    blk /= w.b1;
+    const int o2 = (blk % w.b2) * w.t2, oe = (blk / w.b2) * w.te;
+    te = min(w.te, w.ne - oe);
+    t1 = min(w.t1, w.n1 - o1);
+    t2 = min(w.t2, w.n2 - o2);
+    const int st[3] = {1, g.px, (int)g.plane};
+    se = st[E];
+    s1 = st[A1];
+    s2 = st[A2];
+    org = (g.ng + oe) * se + (g.ng + o1) * s1 + (g.ng + o2) * s2;
   }
 };
 
 template <int RECON, int E, bool M>
-__global__ void __launch_bounds__(256) k_emf_weno64(Dev<double> d, Inp<double> in, Prm<double> P) {
+__device__ __forceinline__ void emf64_weno(const Dev<double>& d, const Inp<double>& in, const Prm<double>& P,
+                                           const Tile64& w, int blk, double* sv) {
   constexpr int A1 = (E + 1) % 3, A2 = (E + 2) % 3;
-  const Geom& g = d.g;
-  const Weno64Shape w(E, g);
-  int blk = blockIdx.x;
-  const int o1 = (blk % w.b1()) * w.t1;
-  blk /= w.b1();
-  const int o2 = (blk % w.b2()) * w.t2, oe = (blk / w.b2()) * w.te;
-  const int te = min(w.te, w.ne - oe), t1 = min(w.t1, w.n1 - o1), t2 = min(w.t2, w.n2 - o2);  // this tile's edges
+  const Place64<E> p(d.g, w, blk);
+  const int te = p.te, t1 = p.t1, t2 = p.t2, st1 = p.s1, st2 = p.s2;
   const int c1 = t1 + 5, c2 = t2 + 5;  // staged cells: [-3, t + 2) about the tile's edges
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* sv = reinterpret_cast<double*>(smem_raw);  // [2][te][c2][c1]
   const int nv = te * c1 * c2, n1 = te * t1 * c2, n0 = te * c1 * t2, ned = te * t1 * t2;
-  double* s1l = sv + 2 * nv;   // rows along a1: [2][te][c2][t1], left and right
+  double* s1l = sv + 2 * nv;   // sv: cells [2][te][c2][c1]; rows along a1: [2][te][c2][t1], left and right
   double* s1r = s1l + 2 * n1;
   double* s0l = s1r + 2 * n1;  // columns along a2: [2][te][t2][c1]
   double* s0r = s0l + 2 * n0;
   double* sq = s0r + 2 * n0;   // [12][ned]
-  const int st[3] = {1, g.px, (int)g.plane};
-  const int se = st[E], st1 = st[A1], st2 = st[A2];
-  const int org = (g.ng + oe) * se + (g.ng + o1) * st1 + (g.ng + o2) * st2;  // first edge's upper cell
   const double* vel[3] = {in.vx, in.vy, in.vz};
   for (int t = threadIdx.x; t < 2 * nv; t += blockDim.x) {
     const int c = t >= nv, u = t - c * nv;
     const int i1 = u % c1, r = u / c1, i2 = r % c2, e = r / c2;
-    sv[t] = (c ? vel[A2] : vel[A1])[org + e * se + (i1 - 3) * st1 + (i2 - 3) * st2];
+    sv[t] = (c ? vel[A2] : vel[A1])[p.org + e * p.se + (i1 - 3) * st1 + (i2 - 3) * st2];
   }
   __syncthreads();
   // first pass, one state per thread: [side][rows of both components, columns of both components]
@@ -2808,7 +2904,7 @@ __global__ void __launch_bounds__(256) k_emf_weno64(Dev<double> d, Inp<double> i
       right = q2;
     } else {  // b_a1 along a2 (8, 9), b_a2 along a1 (10, 11)
       step = k < 10 ? st2 : st1;
-      a = (k < 10 ? fb[A1] : fb[A2]) + org + e * se + f1 * st1 + f2 * st2 - 3 * step;
+      a = (k < 10 ? fb[A1] : fb[A2]) + p.org + e * p.se + f1 * st1 + f2 * st2 - 3 * step;
       right = k & 1;
     }
     if (right) {
@@ -2824,24 +2920,92 @@ __global__ void __launch_bounds__(256) k_emf_weno64(Dev<double> d, Inp<double> i
     // the mean in the reference's order (00, 01, 10, 11); quadrant index q1 + 2 q2
     const double v1 = 0.25 * (q[0] + q[4 * ned] + q[2 * ned] + q[6 * ned]);
     const double v2 = 0.25 * (q[ned] + q[5 * ned] + q[3 * ned] + q[7 * ned]);
-    const int c = org + e * se + f1 * st1 + f2 * st2;
+    const int c = p.org + e * p.se + f1 * st1 + f2 * st2;
     const double* vf = d.vf;
     const double eta = eta4(vf[c - st1 - st2], vf[c - st2], vf[c], vf[c - st1]);
     d.E[E][c] = emf_value<double, E, M>(d, c, v1, v2, q[8 * ned], q[9 * ned], q[10 * ned], q[11 * ned], eta);
   }
 }
 
-template <int RECON, int E, bool M>
-void launch_emf_weno64(const Dev<double>& d, const Inp<double>& in, const Prm<double>& P, cudaStream_t st) {
+template <int E, bool M>
+__device__ __forceinline__ void emf64_pdm(const Dev<double>& d, const Inp<double>& in, const Prm<double>& P,
+                                          const Tile64& w, int blk, double* sv) {
+  constexpr int A1 = (E + 1) % 3, A2 = (E + 2) % 3;
+  const Place64<E> p(d.g, w, blk);
+  const int te = p.te, t1 = p.t1, t2 = p.t2, st1 = p.s1, st2 = p.s2;
+  const int c1 = t1 + 8, c2 = t2 + 8;  // staged cells: [-4, t + 4) about the tile's edges
+  const int nv = te * c1 * c2, ng = te * t1 * c2, ned = te * t1 * t2;
+  double* sg = sv + 2 * nv;  // sv: cells [2][te][c2][c1]; first pass: [2][te][c2][t1]
+  double* sq = sg + 2 * ng;  // [6][ned]
+  const double* vel[3] = {in.vx, in.vy, in.vz};
+  for (int t = threadIdx.x; t < 2 * nv; t += blockDim.x) {
+    const int c = t >= nv, u = t - c * nv;
+    const int i1 = u % c1, r = u / c1, i2 = r % c2, e = r / c2;
+    sv[t] = (c ? vel[A2] : vel[A1])[p.org + e * p.se + (i1 - 4) * st1 + (i2 - 4) * st2];
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < 2 * ng; t += blockDim.x) {
+    const int f1 = t % t1, r = t / t1;  // r = (component te + e) c2 + row
+    const double* a = sv + r * c1 + f1;
+    sg[t] = tap8(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7]);
+  }
+  __syncthreads();
+  // second pass: 0, 1 corner velocity of a component; 2, 3 states of b_a1 along a2, of b_a2 along a1
+  const double* fb[3] = {in.bi, in.bj, in.bk};
+  for (int t = threadIdx.x; t < 4 * ned; t += blockDim.x) {
+    const int k = t / ned, u = t - k * ned;
+    const int f1 = u % t1, r = u / t1, f2 = r % t2, e = r / t2;
+    if (k < 2) {
+      const double* q = sg + ((k * te + e) * c2 + f2) * t1 + f1;
+      const double vi = tap8(q[0], q[t1], q[2 * t1], q[3 * t1], q[4 * t1], q[5 * t1], q[6 * t1], q[7 * t1]);
+      const double* v = sv + ((k * te + e) * c2 + f2 + 4) * c1 + f1 + 4;
+      sq[t] = corner_pdm<double, R_PDM>(v, 0, 1, c1, vi, P.pdmb);
+    } else {
+      const int s = k == 2 ? st2 : st1;
+      double l, rr;
+      recon_edge<double, R_PDM>(k == 2 ? fb[A1] : fb[A2], p.org + e * p.se + f1 * st1 + f2 * st2, s, P, l, rr);
+      sq[(2 * k - 2) * ned + u] = l;
+      sq[(2 * k - 1) * ned + u] = rr;
+    }
+  }
+  __syncthreads();
+  for (int u = threadIdx.x; u < ned; u += blockDim.x) {
+    const int f1 = u % t1, r = u / t1, f2 = r % t2, e = r / t2;
+    const double* q = sq + u;
+    const int c = p.org + e * p.se + f1 * st1 + f2 * st2;
+    const double* vf = d.vf;
+    const double eta = eta4(vf[c - st1 - st2], vf[c - st2], vf[c], vf[c - st1]);
+    d.E[E][c] = emf_value<double, E, M>(d, c, q[0], q[ned], q[2 * ned], q[3 * ned], q[4 * ned], q[5 * ned], eta);
+  }
+}
+
+template <int RECON, bool M>
+__global__ void __launch_bounds__(256) k_emf64(Dev<double> d, Inp<double> in, Prm<double> P, Tiles64 w) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double* sm = reinterpret_cast<double*>(smem_raw);
+  int b = blockIdx.x;
+  auto tile = [&](auto fam, int blk) {
+    constexpr int E = decltype(fam)::value;
+    if constexpr (is_weno(RECON)) emf64_weno<RECON, E, M>(d, in, P, w.f[E], blk, sm);
+    else emf64_pdm<E, M>(d, in, P, w.f[E], blk, sm);
+  };
+  if (b < w.blocks[0]) return tile(std::integral_constant<int, 0>{}, b);
+  b -= w.blocks[0];
+  if (b < w.blocks[1]) return tile(std::integral_constant<int, 1>{}, b);
+  tile(std::integral_constant<int, 2>{}, b - w.blocks[1]);
+}
+
+template <int RECON, bool M>
+void launch_emf64(const Dev<double>& d, const Inp<double>& in, const Prm<double>& P, cudaStream_t st) {
   static PerDevice attr;
   unsigned long long bit = 0;
-  if (attr.need(bit)) {  // the largest tile: 4 x 9 x 9
-    cudaFuncSetAttribute(k_emf_weno64<RECON, E, M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(sizeof(double) * 4 * (2 * 14 * 14 + 8 * 9 * 14 + 12 * 81)));
+  if (attr.need(bit)) {
+    cudaFuncSetAttribute(k_emf64<RECON, M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)Tiles64::max_smem(is_weno(RECON)));
     attr.mark(bit);
   }
-  const Weno64Shape w(E, d.g);
-  k_emf_weno64<RECON, E, M><<<w.blocks(), 256, w.smem(), st>>>(d, in, P);
+  const Tiles64 w(is_weno(RECON), d.g);
+  k_emf64<RECON, M><<<w.blocks[0] + w.blocks[1] + w.blocks[2], 256, w.smem, st>>>(d, in, P, w);
 }
 
 template <typename T, int RECON, int E, int TX, int TY, int TZ, int NT, bool M>
@@ -3506,6 +3670,16 @@ void hydro_r(const Dev<T>& d, const Inp<T>& in, int part, int form, double c, do
              cudaStream_t st) {
   Prm<T> P = prm_of(d);
   const Geom& g = d.g;
+  if (std::is_same<T, double>::value && d.fz[0]) {
+    if (part == 0) {
+      const int n = (g.nx0 + 1) * g.ny0 * g.nz0 + g.nx0 * (g.ny0 + 1) * g.nz0 + g.nx0 * g.ny0 * (g.nz0 + 1);
+      const int nt = n < 4 * 152 * 128 ? 64 : 128;
+      k_faces<T, RECON, M><<<(n + nt - 1) / nt, nt, 0, st>>>(d, in, P);
+    } else if (part == 2) {
+      k_update_faces<T, M><<<(g.nx0 * g.ny0 * g.nz0 + 127) / 128, 128, 0, st>>>(d, form, (T)c, (T)den);
+    }
+    return;
+  }
   if (part == 0) {
     const int n0 = (g.nx0 + 1) * g.ny0 * g.nz0;
     static PerDevice pref;
@@ -3513,7 +3687,7 @@ void hydro_r(const Dev<T>& d, const Inp<T>& in, int part, int form, double c, do
     k_flux<T, RECON, 0, M, false><<<(n0 + 127) / 128, 128, 0, st>>>(one(d), in, P);
   } else if (part == 1) {
     flux_t_any<T, RECON, 1, M>(d, in, P, -1, T(0), T(1), 0, st);
-  } else {
+  } else if (part == 2) {
     flux_t_any<T, RECON, 2, M>(d, in, P, form, (T)c, (T)den, ab ? 1 : 0, st);
   }
 }
@@ -3643,9 +3817,7 @@ template <typename T, int RECON, bool M>
 void emf_weno(const Dev<T>& d, const Inp<T>& in, cudaStream_t st) {
   const Prm<T> P = prm_of(d);
   if constexpr (std::is_same<T, double>::value) {
-    launch_emf_weno64<RECON, 0, M>(d, in, P, st);
-    launch_emf_weno64<RECON, 1, M>(d, in, P, st);
-    launch_emf_weno64<RECON, 2, M>(d, in, P, st);
+    launch_emf64<RECON, M>(d, in, P, st);
   } else {
     launch_emf_weno<T, RECON, 0, 32, 4, 4, 512, M>(d, in, P, st);
     launch_emf_weno<T, RECON, 1, 32, 1, 8, 256, M>(d, in, P, st);
@@ -3703,12 +3875,16 @@ void Launch<T, M>::emf(const Dev<T>& d, const Inp<T>& in0, cudaStream_t st) {
         return;
       }
     }
-    if (std::is_same<T, float>::value && !M && d.tile_ey == 4)
-      launch_emf_pdm<T, 0, 32, 4, 4, 512, M>(d, in, P, st);
-    else
-      launch_emf_pdm<T, 0, ei_x(EiTile<T>::Y), EiTile<T>::Y, EiTile<T>::Y, 512, M>(d, in, P, st);
-    launch_emf_pdm<T, 1, 32, 1, kPT, 32 * kPT, M>(d, in, P, st);
-    launch_emf_pdm<T, 2, 32, kPT, 1, 32 * kPT, M>(d, in, P, st);
+    if constexpr (std::is_same<T, double>::value) {
+      launch_emf64<R_PDM, M>(d, in, P, st);
+    } else {
+      if (!M && d.tile_ey == 4)
+        launch_emf_pdm<T, 0, 32, 4, 4, 512, M>(d, in, P, st);
+      else
+        launch_emf_pdm<T, 0, ei_x(EiTile<T>::Y), EiTile<T>::Y, EiTile<T>::Y, 512, M>(d, in, P, st);
+      launch_emf_pdm<T, 1, 32, 1, kPT, 32 * kPT, M>(d, in, P, st);
+      launch_emf_pdm<T, 2, 32, kPT, 1, 32 * kPT, M>(d, in, P, st);
+    }
     return;
   }
   switch (d.recon) {
