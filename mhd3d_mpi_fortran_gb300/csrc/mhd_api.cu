@@ -84,6 +84,7 @@ struct Handle {
   // batched steps)
   bool prepared = false;
   int tile_td = 8, tile_ey = 8;  // launch shapes (autotuned for FP32 Cartesian PDM)
+  bool tiles_set = false;        // chosen by mhd_set_tiles or an autotuner, not by default
   float* geoT = nullptr;       // FP32 copy of the cell widths
   int* gmap = nullptr;         // ghost-image tables
   bool metric = false;         // curvilinear metric mode (mhd_init_mapped)
@@ -306,6 +307,8 @@ void carve(Handle* h, Dev<T>& d, char* base) {
   d.m = Metric{};
   d.tile_td = h->tile_td;
   d.tile_ey = h->tile_ey;
+  for (int D = 1; D < 3; ++D) d.seg[D - 1] = sweep_seg(D, g, sweep_cols(D, g));
+  for (int E = 0; E < 3; ++E) d.eseg[E] = emf_stream_seg(E, g, emf_stream_cols(E, g));
   for (int a = 0; a < 3; ++a) {
     d.mw[a] = h->metric ? next() : nullptr;
     d.mbn[a] = h->metric ? next() : nullptr;
@@ -593,8 +596,8 @@ static int create_handle(const mhd_params* prm, const double* dx, const double* 
   Geom& g = h->g;
   g.nx0 = prm->nx0; g.ny0 = prm->ny0; g.nz0 = prm->nz0;
   {
-    const long long eb = (long long)((g.nx0 + 31) / 32) * ((g.ny0 + MHD_EMF_NW - 1) / MHD_EMF_NW) *
-                         emf_stream_segs(g.nz0, emf_stream_seg(g.nx0, g.ny0, g.nz0));
+    const int cols = emf_stream_cols(0, g);
+    const long long eb = (long long)cols * emf_stream_segs(g.nz0, emf_stream_seg(0, g, cols));
     h->tile_ey = (h->fp32 && !metric) ? (eb >= 256 ? kEmfStream : 8) : h->fp32 ? 8 : 4;
   }
   g.nord = prm->nord; g.ng = prm->nord / 2;
@@ -1217,19 +1220,46 @@ static bool batchable(Handle* const* hs, int n) {
   return true;
 }
 
+// Segment lengths of the sweeps and EMF streams of every grid of a batch: a
+// launch holds the blocks of all of them.  Returns the blocks of its ei streams.
+template <typename T>
+static long long batch_segments(std::vector<Dev<T>>& ds) {
+  long long cols[5] = {0, 0, 0, 0, 0}, eb = 0;
+  for (const Dev<T>& d : ds) {
+    for (int D = 1; D < 3; ++D) cols[D - 1] += sweep_cols(D, d.g);
+    for (int E = 0; E < 3; ++E) cols[2 + E] += emf_stream_cols(E, d.g);
+  }
+  for (long long& c : cols) c = std::min<long long>(c, INT32_MAX / 2);
+  for (Dev<T>& d : ds) {
+    for (int D = 1; D < 3; ++D) d.seg[D - 1] = sweep_seg(D, d.g, (int)cols[D - 1]);
+    for (int E = 0; E < 3; ++E) d.eseg[E] = emf_stream_seg(E, d.g, (int)cols[2 + E]);
+    eb += (long long)emf_stream_cols(0, d.g) * emf_stream_segs(d.g.nz0, d.eseg[0]);
+  }
+  return eb;
+}
+
+// The batch's launch shapes are those of its first grid; where nobody chose them,
+// the EMF streams take over at 256 blocks of the whole launch, as for one grid.
+// 32 grids of 32^3 to 96^3: 3.06 ms a stage with the ei tiles, 2.66 with the
+// streams; five grids 0.54 and 0.48.
 template <typename T>
 static int build_batch(Handle* const* hs, int n, BatchBufs& b) {
-  std::vector<Dev<T>> tab(2 * (size_t)n);
+  std::vector<Dev<T>> tab(2 * (size_t)n), ds;
+  for (int i = 0; i < n; ++i) ds.push_back(dev<T>(hs[i]));
+  const long long eb = batch_segments(ds);
+  const int td = hs[0]->tile_td;
+  const int ey = hs[0]->tiles_set || !hs[0]->fp32 ? hs[0]->tile_ey : eb >= 256 ? kEmfStream : 8;
   for (int i = 0; i < n; ++i) {
-    tab[i] = at_par(dev<T>(hs[i]), hs[i]->par);
-    tab[n + i] = at_par(dev<T>(hs[i]), hs[i]->par ^ 1);
+    const Dev<T>& d = ds[i];
+    tab[i] = at_par(d, hs[i]->par);
+    tab[n + i] = at_par(d, hs[i]->par ^ 1);
   }
   std::vector<int4> map;
   size_t off[BF_COUNT];
   for (int f = 0; f < BF_COUNT; ++f) {
     off[f] = map.size();
     for (int i = 0; i < n; ++i) {
-      const dim3 dd = Batch<T>::dims(f, hs[i]->g, hs[0]->tile_td, hs[0]->tile_ey);
+      const dim3 dd = Batch<T>::dims(f, ds[i], td, ey);
       for (unsigned z = 0; z < dd.z; ++z)
         for (unsigned y = 0; y < dd.y; ++y)
           for (unsigned x = 0; x < dd.x; ++x) map.push_back(make_int4(i, (int)x, (int)y, (int)z));
@@ -1249,24 +1279,28 @@ static int build_batch(Handle* const* hs, int n, BatchBufs& b) {
   const mhd_params& p = hs[0]->prm;
   b.view.pdmb = p.pdmb; b.view.eps = p.eps; b.view.alpha = p.alpha; b.view.beta = p.beta;
   b.view.tvd_shift = p.tvd_shift;
-  b.view.tile_td = hs[0]->tile_td;
-  b.view.tile_ey = hs[0]->tile_ey;
+  b.view.tile_td = td;
+  b.view.tile_ey = ey;
   return MHD_OK;
 }
 
 // nsteps RK steps of every grid of a batch; returns the number of half swaps.
+// As a single grid's step (enqueue_step): the first stage stores U^n, the last
+// one accumulates the next step's CFL dt, which only the first step computes in
+// a pass of its own, and that only unless every grid comes prepared (the pass
+// took 0.40 of 5.9 ms a step of 32 grids).
 // The EMF families of a stage run on the side stream st2 beside the face
 // fluxes (they read the same stage input and write disjoint arrays), joined
 // before CT, as a single grid's stage runs them.
 template <typename T>
-static int enqueue_batch(const BatchView& v, int stepop, int dt_mode, int nsteps, cudaStream_t st,
+static int enqueue_batch(const BatchView& v, int stepop, int dt_mode, int nsteps, bool prepared, cudaStream_t st,
                          cudaStream_t st2, cudaEvent_t fork, cudaEvent_t join) {
   int flips = 0;
   const int nst = (stepop == MHD_STEP_RK2) ? 2 : 3;
   for (int s = 0; s < nsteps; ++s) {
-    Batch<T>::cfl(v, flips & 1, dt_mode == MHD_DT_CFL ? 1 : 0, st);
+    Batch<T>::cfl(v, flips & 1, dt_mode == MHD_DT_CFL ? 1 : 0, s == 0 && !prepared, st);
     for (int k = 1; k <= nst; ++k) {
-      int form = -1;
+      int form = FORM_SAVE;
       double c = 0.0, den = 1.0;
       if (k > 1) {
         if (nst == 2) { form = 0; den = 2.0; }
@@ -1281,7 +1315,7 @@ static int enqueue_batch(const BatchView& v, int stepop, int dt_mode, int nsteps
       Batch<T>::parts(v, sel, 2, form, c, den, st);
       cudaEventRecord(join, st2);
       cudaStreamWaitEvent(st, join, 0);
-      Batch<T>::parts(v, sel, 4, form, c, den, st);
+      Batch<T>::parts(v, sel, k == nst ? 4 | 8 : 4, form, c, den, st);
       ++flips;
     }
   }
@@ -1290,21 +1324,21 @@ static int enqueue_batch(const BatchView& v, int stepop, int dt_mode, int nsteps
 
 // Graph of nsteps steps of every grid: batched (one launch per kernel family
 // over all grids) when the grids allow it, else one branch per grid.
-static int capture_ensemble(const std::vector<Handle*>& hs, int nsteps, cudaGraphExec_t* ex,
-                            std::vector<int>& pars, BatchBufs& bufs) {
+static int capture_ensemble(const std::vector<Handle*>& hs, int nsteps, bool batched, bool prepared,
+                            cudaGraphExec_t* ex, std::vector<int>& pars, BatchBufs& bufs) {
   Handle* h0 = hs[0];
   const int n = (int)hs.size();
   pars.resize(n);
   cudaGraph_t gr = nullptr;
-  if (batchable(hs.data(), n)) {
+  if (batched) {
     int rc = h0->fp32 ? build_batch<float>(hs.data(), n, bufs) : build_batch<double>(hs.data(), n, bufs);
     if (rc) return rc;
     CK(cudaStreamBeginCapture(h0->st, cudaStreamCaptureModeThreadLocal));
     const int flips =
-        h0->fp32 ? enqueue_batch<float>(bufs.view, h0->prm.stepop, h0->prm.dt_mode, nsteps, h0->st, h0->st2,
-                                        h0->ev_fork, h0->ev_join)
-                 : enqueue_batch<double>(bufs.view, h0->prm.stepop, h0->prm.dt_mode, nsteps, h0->st, h0->st2,
-                                         h0->ev_fork, h0->ev_join);
+        h0->fp32 ? enqueue_batch<float>(bufs.view, h0->prm.stepop, h0->prm.dt_mode, nsteps, prepared, h0->st,
+                                        h0->st2, h0->ev_fork, h0->ev_join)
+                 : enqueue_batch<double>(bufs.view, h0->prm.stepop, h0->prm.dt_mode, nsteps, prepared, h0->st,
+                                         h0->st2, h0->ev_fork, h0->ev_join);
     CK(cudaStreamEndCapture(h0->st, &gr));
     for (int i = 0; i < n; ++i) pars[i] = hs[i]->par ^ (flips & 1);
   } else {
@@ -1317,6 +1351,7 @@ static int capture_ensemble(const std::vector<Handle*>& hs, int nsteps, cudaGrap
     for (int i = 0; i < n; ++i) {
       Handle* h = hs[i];
       int par = h->par;
+      h->prepared = false;
       for (int s = 0; s < nsteps; ++s) {
         if (h->fp32) enqueue_any<float>(h, par, h->st);
         else enqueue_any<double>(h, par, h->st);
@@ -1397,11 +1432,16 @@ static int ens_launch(void** handles, int32_t ngrids, int32_t nsteps, std::vecto
     key.push_back((unsigned long long)h->par);
   }
   key.push_back((unsigned long long)nsteps);
-  key.push_back((unsigned long long)(h0->tile_td * 64 + h0->tile_ey));  // the batch's launch shapes
+  // the batch's launch shapes, and whether its first step runs a dt pass
+  const bool batched = batchable(hs.data(), ngrids);
+  bool prepared = batched;
+  for (Handle* h : hs) prepared = prepared && h->prepared;
+  key.push_back((unsigned long long)(((h0->tile_td * 64 + h0->tile_ey) * 2 + (h0->tiles_set ? 1 : 0)) * 2 +
+                                     (prepared ? 1 : 0)));
   auto it = g_ens_cache.find(key);
   if (it == g_ens_cache.end()) {
     EnsEntry en;
-    int rc = capture_ensemble(hs, nsteps, &en.ex, en.par_end, en.bufs);
+    int rc = capture_ensemble(hs, nsteps, batched, prepared, &en.ex, en.par_end, en.bufs);
     if (rc) {
       ens_release(en);
       return rc;
@@ -1418,7 +1458,7 @@ static int ens_launch(void** handles, int32_t ngrids, int32_t nsteps, std::vecto
   }
   for (int i = 0; i < ngrids; ++i) {
     hs[i]->par = it->second.par_end[i];
-    hs[i]->prepared = false;  // batched steps run their own CFL pass
+    hs[i]->prepared = batched;  // (an unbatched branch starts with its own dt pass)
   }
   if (ev_before) CK(cudaEventRecord(ev_before, h0->st));
   CK(cudaGraphLaunch(it->second.ex, h0->st));
@@ -1523,6 +1563,7 @@ int mhd_autotune(void* handle, int32_t reps, int32_t out[2]) {
     }
     h->tile_td = pick_td;
     h->tile_ey = pick_ey;
+    h->tiles_set = true;
     carve<float>(h, h->df, (char*)h->buf);
     drop_graphs(h);
     CK(cudaGetLastError());
@@ -1548,6 +1589,7 @@ int mhd_set_tiles(void* handle, int32_t face_tile, int32_t ei_tile) {
   if (rc) return rc;
   h->tile_td = face_tile;
   h->tile_ey = ei_tile;
+  h->tiles_set = true;
   carve<float>(h, h->df, (char*)h->buf);
   drop_graphs(h);
   return MHD_OK;
@@ -1572,7 +1614,7 @@ int mhd_ensemble_autotune(void** handles, int32_t ngrids, int32_t reps, int32_t 
     float best = INFINITY;
     for (int td : kTileTD) {
       for (int ey : kTileEY) {
-        for (Handle* h : hs) { h->tile_td = td; h->tile_ey = ey; }
+        for (Handle* h : hs) { h->tile_td = td; h->tile_ey = ey; h->tiles_set = true; }
         BatchBufs b;
         int rc = build_batch<float>(hs.data(), ngrids, b);
         if (rc == MHD_OK) {

@@ -843,7 +843,9 @@ __device__ __forceinline__ Inp<T> state_view(const Dev<T>& d) {
 // B = false: one grid, its Dev by value, block index from blockIdx.
 // B = true: many grids in one flattened 1-D launch; block b takes its grid
 // and block coordinates from map[b] = {grid, bx, by, bz} and its Dev from
-// tab[grid] (by value: a snapshot the compiler keeps in registers).
+// tab[grid], read in place: a copy held the array pointers in registers (x faces
+// 56 instead of 40, CT + bxyz 180 bytes spilled under its budget; a stage of 32
+// grids 2720 -> 2583 us).
 template <typename T, bool B> struct KArg;
 template <typename T> struct KArg<T, false> {
   Dev<T> d;
@@ -856,16 +858,14 @@ template <typename T> struct KArg<T, true> {
   const Dev<T>* __restrict__ tab;
   const int4* __restrict__ map;
   __device__ __forceinline__ int4 blk() const { return map[blockIdx.x]; }
-  __device__ __forceinline__ Dev<T> dev(const int4& b) const { return tab[b.x]; }
+  __device__ __forceinline__ const Dev<T>& dev(const int4& b) const { return tab[b.x]; }
 };
 template <typename T>
 inline KArg<T, false> one(const Dev<T>& d) { return KArg<T, false>{d}; }
 
 // Resident 256-thread blocks per SM requested for the cell passes (CFL, CT +
-// bxyz, fill).  Single grid: none (0; they take 32 registers).  Batched: each
-// thread holds its grid's array pointers in registers (from the grid table,
-// not the constant bank), about 75 registers unbounded, which would leave 3
-// blocks per SM for these latency-bound passes; a budget keeps more resident.
+// bxyz, fill).  Single grid: none (0; they take 32 registers).  Batched: a
+// budget of 40, since these passes wait on memory and live on residency.
 #ifndef MHD_BATCH_MINB
 #define MHD_BATCH_MINB 6
 #endif
@@ -1065,19 +1065,18 @@ __global__ void __launch_bounds__(256, pass_min_blocks(B)) k_cfl(KArg<T, B> ka, 
 }
 
 // Empties the next-step accumulators before a dt pass refills them.
-__global__ inline void k_next_reset(Scal* sc) {
+__device__ __forceinline__ void next_reset(Scal* sc) {
   sc->dtnext_bits = (unsigned long long)__double_as_longlong(INFINITY);
   sc->pend_status = 0;
 }
+__global__ inline void k_next_reset(Scal* sc) { next_reset(sc); }
 
 // tau selection of step_ab (3609) / step_rk2,3 (3656-3661, 3723-3728).
 // mode 0: RK with fixed deck dt; 1: CFL dt every step; 2: AB (CFL dt and the
 // predictor coefficient tau/tau0/2, then tau0=tau).
 // mode | 4: take the dt and status accumulated for this state by the
 // previous step (dtnext_bits, pend_status) and empty them.
-template <typename T>
-__global__ void k_cfl_final(Dev<T> d, int mode) {
-  Scal* s = d.sc;
+__device__ __forceinline__ void select_tau(Scal* s, int mode) {
   double dt;
   if (mode & 4) {
     dt = __longlong_as_double((long long)s->dtnext_bits);
@@ -1103,23 +1102,19 @@ __global__ void k_cfl_final(Dev<T> d, int mode) {
   }
   // mode 3: read-only (diagnostics); tau untouched
 }
+template <typename T>
+__global__ void k_cfl_final(Dev<T> d, int mode) { select_tau(d.sc, mode); }
 
-// k_cfl_final of every grid of a batch (one thread per grid; RK modes 0, 1).
+// The same for every grid of a batch, one thread per grid.
+template <typename T>
+__global__ void k_next_reset_batch(const Dev<T>* __restrict__ tab, int ngrids) {
+  const int gi = blockIdx.x * blockDim.x + threadIdx.x;
+  if (gi < ngrids) next_reset(tab[gi].sc);
+}
 template <typename T>
 __global__ void k_cfl_final_batch(const Dev<T>* __restrict__ tab, int ngrids, int mode) {
   const int gi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gi >= ngrids) return;
-  Scal* s = tab[gi].sc;
-  double dt = __longlong_as_double((long long)s->dtmin_bits);
-  s->dtmin_bits = (unsigned long long)__double_as_longlong(INFINITY);
-  s->dt_cfl = dt;
-  if (mode == 0) {
-    if (dt < s->tau0) s->status |= ST_CFL;
-    s->tau = s->tau0;
-  } else if (mode == 1) {
-    s->tau = dt;
-    s->tau0 = dt;
-  }
+  if (gi < ngrids) select_tau(tab[gi].sc, mode);
 }
 
 // advance_previous for RK (3794-3819): U^n of the stage combines.
@@ -1850,16 +1845,12 @@ __global__ void __launch_bounds__(32 * (TDV + 1), FluxMinB<T, M, RECON>::value)
 // y / z faces by column sweeps: the FP32 Cartesian PDM alternative to the face
 // tiles, one more launch shape for the autotuner.  A thread owns one column of
 // cells along D (x from the lane, the remaining axis from the warp) over a
-// segment of SWEEP_SEG cells and keeps the 8 reconstructed fields of the 8
+// segment of Dev::seg cells (sweep_seg) and keeps the 8 reconstructed fields of the 8
 // cells around its current face in registers: one new cell is loaded per face
 // (issued a face ahead, before that face's arithmetic), every face flux is
 // computed once, and a cell's face-pair difference is the current minus the
 // previous face's flux.  Face arithmetic and epilogues are those of k_flux_t,
 // so the two give the same bits.
-#ifndef MHD_SWEEP_SEG
-#define MHD_SWEEP_SEG 32
-#endif
-constexpr int SWEEP_SEG = MHD_SWEEP_SEG;  // cells per column segment (compile-time knob)
 #ifndef MHD_SWEEP_UNROLL
 #define MHD_SWEEP_UNROLL 1
 #endif
@@ -1878,27 +1869,34 @@ __global__ void __launch_bounds__(128, kSweepMinB)
   const Geom& g = d.g;
   const int n0 = (D == 1) ? g.ny0 : g.nz0;
   const int no = (D == 1) ? g.nz0 : g.ny0;
-  const int o = bb.w * 4 + threadIdx.y + g.ng;  // remaining axis (one per warp): z for y faces, y for z faces
-  if (o >= g.ng + no) return;
-  const int tx = threadIdx.x;
-  // lanes past the last column work on a copy of it and store nothing, so the
-  // whole warp stays in the loop (warp-synchronous copies below)
-  const int i0 = bb.y * 32 + tx + g.ng;
-  const bool xin = i0 < g.ng + g.nx0;
-  const int i = xin ? i0 : g.ng + g.nx0 - 1;
-  const int c0 = g.ng + bb.z * SWEEP_SEG;
-  const int c1 = min(c0 + SWEEP_SEG, g.ng + n0);
+  // columns are numbered x first, then along the remaining axis (z for y
+  // faces, y for z faces), 32 to a warp, so a warp may span rows; lanes past the
+  // last column work on a copy of it and store nothing, so the whole warp stays
+  // in the loop (warp-synchronous copies below)
+  const int tx = threadIdx.x, ncol = g.nx0 * no;
+  const int u = (bb.y * 4 + threadIdx.y) * 32 + tx;
+  if (u - tx >= ncol) return;
+  const bool xin = u < ncol;
+  const int uc = xin ? u : ncol - 1;
+  const int i = uc % g.nx0 + g.ng, o = uc / g.nx0 + g.ng;
+  // y faces: does this lane copy its own x face i + 1 (the next lane holds another row, or there is none)?
+  const bool xlast = tx == 31 || i == g.ng + g.nx0 - 1;
+  const int seg = d.seg[D - 1];
+  const int c0 = g.ng + bb.z * seg;
+  const int c1 = min(c0 + seg, g.ng + n0);
   const int s = (D == 1) ? g.px : (int)g.plane;
   const int col = (D == 1) ? i + (int)g.plane * o : i + g.px * o;  // + cd * s
   const T* src[8] = {in.rho, in.vx, in.vy, in.vz, in.p, in.bx, in.by, in.bz};
   // y faces: the x-face fluxes of the next cell are copied asynchronously into
   // a per-warp double buffer one face ahead of the epilogue that reads them
-  __shared__ __align__(16) T sxf[4][2][8][33];
-  T (*xs)[8][33] = sxf[threadIdx.y];
+  // (the copies that xlast lanes make follow the warp's 32)
+  __shared__ __align__(16) T sxf[D == 1 ? 4 : 1][2][8][64];
+  T (*xs)[8][64] = sxf[D == 1 ? threadIdx.y : 0];
+  const int xh = xlast ? 32 : 1;  // from a lane's low x face to its high one
   // z faces: dU, the state (rho, v, p) and U^n of the next cell, likewise
   // (each lane reads back only what it copied)
-  __shared__ __align__(16) T szf[4][2][18][32];
-  T (*zs)[18][32] = szf[threadIdx.y];
+  __shared__ __align__(16) T szf[D == 2 ? 4 : 1][2][18][32];
+  T (*zs)[18][32] = szf[D == 2 ? threadIdx.y : 0];
   // the window holds the 8 fields as pairs (rho, vx), (vy, vz), (p, bx),
   // (by, bz), the operands of the packed FP32 reconstruction
   typedef typename Pr<T>::V V2;
@@ -1941,10 +1939,7 @@ __global__ void __launch_bounds__(128, kSweepMinB)
     if (D == 1) {
       __syncwarp();  // every lane is done reading the slot refilled here
       if (cd < c1) {
-        // x faces i0 (this lane) and, on lane 31, i0 + 32, clamped to the last
-        // face (a lane past the last column supplies its left neighbour's high face)
-        const int fo = ((D == 1) ? (int)g.plane * o : g.px * o) + cd * s;
-        const int fl = fo + min(i0, g.ng + g.nx0), fh = fo + min(i0 + 1, g.ng + g.nx0);
+        const int fl = col + cd * s;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           const T* fx = d.F[0][q] + fl;
@@ -1953,13 +1948,12 @@ __global__ void __launch_bounds__(128, kSweepMinB)
             asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sp), "l"(fx) : "memory");
           else
             asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sp), "l"(fx) : "memory");
-          if (tx == 31) {
-            const uint32_t sq = (uint32_t)__cvta_generic_to_shared(&xs[cd & 1][q][32]);
-            const T* fy = d.F[0][q] + fh;
+          if (xlast) {
+            const uint32_t sq = (uint32_t)__cvta_generic_to_shared(&xs[cd & 1][q][tx + 32]);
             if (sizeof(T) == 4)
-              asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sq), "l"(fy) : "memory");
+              asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sq), "l"(fx + 1) : "memory");
             else
-              asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sq), "l"(fy) : "memory");
+              asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sq), "l"(fx + 1) : "memory");
           }
         }
       }
@@ -2025,7 +2019,7 @@ __global__ void __launch_bounds__(128, kSweepMinB)
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
             const T* x = &xs[cc & 1][q][tx];
-            d.dU[q][c] = Ops<T>::dc(x[1] - x[0], dx, rdx) + Ops<T>::dc(dF[q], dy, rdy);
+            d.dU[q][c] = Ops<T>::dc(x[xh] - x[0], dx, rdx) + Ops<T>::dc(dF[q], dy, rdy);
           }
         }
       } else {
@@ -2365,7 +2359,7 @@ __global__ void __launch_bounds__(32 * NW, MHD_EMF_STREAM_MINB)
   const int nS0 = (E == 2) ? g.ny0 : g.nz0;     // interior cells along S
   const int nSg = (E == 2) ? g.ny : g.nz;
   const int nW0 = (E == 2) ? g.nz0 : g.ny0;
-  const int seg = emf_stream_seg(g.nx0, nW0, nS0);
+  const int seg = d.eseg[E];
   const int s_lo = g.ng + seg * bb.w;
   const int s_hi = (bb.w == emf_stream_segs(nS0, seg) - 1) ? g.ng + nS0 : s_lo + seg - 1;
   const int SS = (E == 2) ? g.px : (int)g.plane;  // global stride along S
@@ -2556,10 +2550,10 @@ __global__ void __launch_bounds__(256) k_emf_rows(KArg<T, B> ka, Inp<T> in0, Prm
 }
 
 // blocks of streamed family E on one grid (x tiles, warp-axis tiles, segments)
-inline dim3 emf_stream_grid(int E, const Geom& g) {
+inline dim3 emf_stream_grid(int E, const Geom& g, int seg) {
   const int nS0 = (E == 2) ? g.ny0 : g.nz0, nW0 = (E == 2) ? g.nz0 : g.ny0;
   return dim3((g.nx0 + 31) / 32, (nW0 + MHD_EMF_NW - 1) / MHD_EMF_NW,
-              emf_stream_segs(nS0, emf_stream_seg(g.nx0, nW0, nS0)));
+              emf_stream_segs(nS0, seg));
 }
 template <typename T, int E, bool M, bool B>
 void stream_attr() {
@@ -2575,7 +2569,7 @@ template <typename T, int E, bool M>
 void launch_emf_stream(const Dev<T>& d, const Inp<T>& in, const Prm<T>& P, cudaStream_t st) {
   typedef EmfStream<T, E, MHD_EMF_NW> K;
   stream_attr<T, E, M, false>();
-  k_emf_stream<T, E, MHD_EMF_NW, M, false><<<emf_stream_grid(E, d.g), K::NT, K::smem, st>>>(one(d), in, P);
+  k_emf_stream<T, E, MHD_EMF_NW, M, false><<<emf_stream_grid(E, d.g, d.eseg[E]), K::NT, K::smem, st>>>(one(d), in, P);
 }
 
 template <typename T, bool M>
@@ -3325,9 +3319,8 @@ __global__ void __launch_bounds__(256, pass_min_blocks(B))
   const int4 bb = ka.blk();
   const auto& d = ka.dev(bb);
   unsigned st = 0;
-  const bool want_dt = !B && dt_next;  // single grids only (a batch runs its own CFL pass)
-  const T m = fill_bxyz_elem<T, M>(d, bb, want_vf, shell_only, want_dt, st);
-  if (want_dt) dt_next_accumulate(d.sc, m, st);
+  const T m = fill_bxyz_elem<T, M>(d, bb, want_vf, shell_only, dt_next != 0, st);
+  if (dt_next) dt_next_accumulate(d.sc, m, st);
 }
 
 // CT fused with get_bxyz and vf on Cartesian meshes (advance_bijk + combine,
@@ -3356,8 +3349,7 @@ __global__ void __launch_bounds__(256, pass_min_blocks(B))
   const int i = g.ng + bb.y * 32 + (threadIdx.x & 31);
   const int j = g.ng + bb.z * 8 + (threadIdx.x >> 5);
   const int k = g.ng + bb.w;
-  // batched stages neither store U^n nor accumulate the next dt (their CFL pass does both)
-  const bool save = !B && form == FORM_SAVE, want_dt = !B && dt_next;
+  const bool save = form == FORM_SAVE, want_dt = dt_next != 0;
   T m = T(INFINITY);
   unsigned st = 0;
   if (i < g.ng + g.nx0 && j < g.ng + g.ny0) {
@@ -3643,9 +3635,9 @@ constexpr bool tunable() {
   return std::is_same<T, float>::value && RECON == R_PDM && !M;
 }
 
-inline dim3 sweep_grid(int D, const Geom& g) {
+inline dim3 sweep_grid(int D, const Geom& g, int seg) {
   const int n0 = (D == 1) ? g.ny0 : g.nz0, no = (D == 1) ? g.nz0 : g.ny0;
-  return dim3((g.nx0 + 31) / 32, (n0 + SWEEP_SEG - 1) / SWEEP_SEG, (no + 3) / 4);
+  return dim3((g.nx0 * no + 127) / 128, (n0 + seg - 1) / seg);
 }
 
 template <typename T, int RECON, int D, bool M>
@@ -3654,7 +3646,7 @@ void flux_t_any(const Dev<T>& d, const Inp<T>& in, const Prm<T>& P, int form, T 
     if (d.tile_td == kSweepTile) {  // column sweeps (every FP32 Cartesian reconstruction with a register window)
       static PerDevice pref;  // 4 blocks of 27 KB static shared memory
       prefer_carveout(k_flux_sweep<T, D, false, RECON>, 50, pref);
-      k_flux_sweep<T, D, false, RECON><<<sweep_grid(D, d.g), dim3(32, 4), 0, st>>>(one(d), in, P, form, c, den);
+      k_flux_sweep<T, D, false, RECON><<<sweep_grid(D, d.g, d.seg[D - 1]), dim3(32, 4), 0, st>>>(one(d), in, P, form, c, den);
       return;
     }
   }
@@ -3911,18 +3903,19 @@ void Launch<T, M>::fill(const Dev<T>& d, cudaStream_t st) {
 
 // ------------------------------------------------------------ batched ensemble
 template <typename T>
-dim3 Batch<T>::dims(int fam, const Geom& g, int td, int ey) {
+dim3 Batch<T>::dims(int fam, const Dev<T>& d, int td, int ey) {
+  const Geom& g = d.g;
   const bool stream = std::is_same<T, float>::value && ey == kEmfStream;
   const int Y = std::is_same<T, float>::value && !stream ? ey : EiTile<T>::Y;
   if (!std::is_same<T, float>::value) td = TD;
   switch (fam) {
     case BF_CFL: return dim3((g.nx + 31) / 32, (g.ny + 7) / 8, (g.nz + 7) / 8);
     case BF_FLUX_X: return dim3(((g.nx0 + 1) * g.ny0 * g.nz0 + 127) / 128, 1, 1);
-    case BF_FLUX_Y: return td == kSweepTile ? sweep_grid(1, g) : dim3((g.nx0 + 31) / 32, (g.ny0 + td - 1) / td, g.nz0);
-    case BF_FLUX_Z: return td == kSweepTile ? sweep_grid(2, g) : dim3((g.nx0 + 31) / 32, (g.nz0 + td - 1) / td, g.ny0);
-    case BF_EMF_I: return stream ? emf_stream_grid(0, g) : emf_grid(0, g, ei_x(Y), Y, Y);
-    case BF_EMF_J: return stream ? emf_stream_grid(1, g) : emf_grid(1, g, 32, 1, kPT);
-    case BF_EMF_K: return stream ? emf_stream_grid(2, g) : emf_grid(2, g, 32, kPT, 1);
+    case BF_FLUX_Y: return td == kSweepTile ? sweep_grid(1, g, d.seg[0]) : dim3((g.nx0 + 31) / 32, (g.ny0 + td - 1) / td, g.nz0);
+    case BF_FLUX_Z: return td == kSweepTile ? sweep_grid(2, g, d.seg[1]) : dim3((g.nx0 + 31) / 32, (g.nz0 + td - 1) / td, g.ny0);
+    case BF_EMF_I: return stream ? emf_stream_grid(0, g, d.eseg[0]) : emf_grid(0, g, ei_x(Y), Y, Y);
+    case BF_EMF_J: return stream ? emf_stream_grid(1, g, d.eseg[1]) : emf_grid(1, g, 32, 1, kPT);
+    case BF_EMF_K: return stream ? emf_stream_grid(2, g, d.eseg[2]) : emf_grid(2, g, 32, kPT, 1);
     case BF_EMF_R: return stream ? dim3(EmfRows(g).blocks(), 1, 1) : dim3(0, 0, 0);
     case BF_CT: {  // k_ct_fill: the fill's interior tiles
       const FillShape fs(g);
@@ -3933,10 +3926,14 @@ dim3 Batch<T>::dims(int fam, const Geom& g, int td, int ey) {
 }
 
 template <typename T>
-void Batch<T>::cfl(const BatchView& v, int sel, int mode, cudaStream_t st) {
-  KArg<T, true> a{(const Dev<T>*)v.tab[sel], v.map[BF_CFL]};
-  k_cfl<T, false, true><<<v.nblk[BF_CFL], 256, 0, st>>>(a, 1, 0);
-  k_cfl_final_batch<T><<<(v.ngrids + 127) / 128, 128, 0, st>>>((const Dev<T>*)v.tab[sel], v.ngrids, mode);
+void Batch<T>::cfl(const BatchView& v, int sel, int mode, bool recompute, cudaStream_t st) {
+  const Dev<T>* tab = (const Dev<T>*)v.tab[sel];
+  const int nb = (v.ngrids + 127) / 128;
+  if (recompute) {
+    k_next_reset_batch<T><<<nb, 128, 0, st>>>(tab, v.ngrids);
+    k_cfl<T, false, true><<<v.nblk[BF_CFL], 256, 0, st>>>(KArg<T, true>{tab, v.map[BF_CFL]}, 0, 1);
+  }
+  k_cfl_final_batch<T><<<nb, 128, 0, st>>>(tab, v.ngrids, mode | 4);
 }
 
 template <typename K>
@@ -4039,15 +4036,11 @@ void Batch<T>::parts(const BatchView& v, int sel, int which, int form, double c,
     else batch_flux_t<T, TD>(v, tab, P, form, (T)c, (T)den, st);
   }
   if (which & 4) {  // face-B update + bxyz + vf (interior), then the ghost shell of the half the stage wrote
-    k_ct_fill<T, true><<<v.nblk[BF_CT], 256, 0, st>>>(KArg<T, true>{tab, v.map[BF_CT]}, form, (T)c, (T)den, 1, 0);
+    const int dt_next = (which & 8) ? 1 : 0;
+    k_ct_fill<T, true><<<v.nblk[BF_CT], 256, 0, st>>>(KArg<T, true>{tab, v.map[BF_CT]}, form, (T)c, (T)den, 1, dt_next);
     KArg<T, true> fa{(const Dev<T>*)v.tab[sel ^ 1], v.map[BF_FILL]};
-    k_fill_bxyz<T, false, true><<<v.nblk[BF_FILL], 256, 0, st>>>(fa, 1, 1, 0);
+    k_fill_bxyz<T, false, true><<<v.nblk[BF_FILL], 256, 0, st>>>(fa, 1, 1, dt_next);
   }
-}
-
-template <typename T>
-void Batch<T>::stage(const BatchView& v, int sel, int form, double c, double den, cudaStream_t st) {
-  parts(v, sel, 7, form, c, den, st);
 }
 
 template <typename T, bool M>

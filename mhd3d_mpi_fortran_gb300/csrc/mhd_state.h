@@ -113,6 +113,8 @@ struct Dev {
   // tile 4 or 8, or kEmfStream), chosen by the autotuner for the FP32 Cartesian
   // PDM path
   int tile_td, tile_ey;
+  int seg[2];        // cells per column segment of the y / z sweeps (sweep_seg)
+  int eseg[3];       // edges per segment of the streamed EMF families (emf_stream_seg)
   int emf;           // edge EMF scheme: 0 LFM, 1 Yee
   T* ye[12];         // Yee split electric fields, [x, y, z edges][pp, np, pn, nn] (emf = 1)
 };
@@ -199,14 +201,13 @@ struct BatchView {
 template <typename T>
 struct Batch {
   // blocks (x, y, z) of family f for one grid with the given tiles
-  static dim3 dims(int fam, const Geom& g, int td, int ey);
-  // get_dt + advance_previous of every grid (RK); mode as Launch::cfl
-  static void cfl(const BatchView& v, int sel, int mode, cudaStream_t st);
-  // one RK stage of every grid: emf, fluxes + update, ct (on tab[sel]), then
-  // fill + bxyz + vf on tab[sel ^ 1], the half the stage wrote
-  static void stage(const BatchView& v, int sel, int form, double c, double den, cudaStream_t st);
+  static dim3 dims(int fam, const Dev<T>& d, int td, int ey);
+  // tau selection of every grid as Launch::cfl_folded (U^n is stored by the first stage)
+  static void cfl(const BatchView& v, int sel, int mode, bool recompute, cudaStream_t st);
   // parts of a stage, bit mask: 1 EMF, 2 fluxes + conserved update (writes
-  // only scratch and the other half), 4 face-B update + fill (state)
+  // only scratch and the other half), 4 face-B update (on tab[sel]), then fill +
+  // bxyz + vf on tab[sel ^ 1], the half the stage wrote; with 8 these also
+  // accumulate the CFL dt and status of the new state for the next step
   static void parts(const BatchView& v, int sel, int which, int form, double c, double den, cudaStream_t st);
 };
 
@@ -245,16 +246,39 @@ constexpr int kEmfStream = 1;   // EMF-shape value of the slice-streamed EMF fam
 #ifndef MHD_EMF_SEG_MIN
 #define MHD_EMF_SEG_MIN 16
 #endif
-// Edge positions per segment for a family with nx0 x nW0 edge columns and
-// nS0 + 1 edge positions along the stream axis.
-__host__ __device__ inline int emf_stream_seg(int nx0, int nW0, int nS0) {
-  const int cols = ((nx0 + 31) / 32) * ((nW0 + MHD_EMF_NW - 1) / MHD_EMF_NW);
+// Blocks of edge columns of streamed family E of a grid.
+inline int emf_stream_cols(int E, const Geom& g) {
+  return ((g.nx0 + 31) / 32) * (((E == 2 ? g.nz0 : g.ny0) + MHD_EMF_NW - 1) / MHD_EMF_NW);
+}
+// Edge positions per segment of the stream axis, for a launch of `cols` column
+// blocks (of all the grids of a batch).
+inline int emf_stream_seg(int E, const Geom& g, int cols) {
+  const int nS0 = (E == 2) ? g.ny0 : g.nz0;
   const int nseg = (MHD_EMF_BLOCKS + cols / 2) / cols;
   const int seg = (nS0 + 1) / (nseg > 1 ? nseg : 1);
   return seg > MHD_EMF_SEG_MIN ? seg : MHD_EMF_SEG_MIN;
 }
 // Segments along the stream axis: nseg of seg edge positions, the last one taking the rest.
 __host__ __device__ inline int emf_stream_segs(int nS0, int seg) { return (nS0 + 1) / seg > 1 ? (nS0 + 1) / seg : 1; }
+// Blocks of columns (128 a block) of the y (D = 1) or z sweep of a grid.
+inline int sweep_cols(int D, const Geom& g) {
+  return (g.nx0 * (D == 1 ? g.nz0 : g.ny0) + 127) / 128;
+}
+// Cells per column segment of the y / z sweeps, for a launch of `cols` column
+// blocks (of all the grids of a batch).  A block walks its segment serially,
+// about 1 us per face, and a segment costs one face and a window load extra:
+// segments of 32 cells when those fill the chip's 608 block slots (4 per SM),
+// else as many equal segments as the slots take, down to 4 cells (shorter ones
+// measured no faster).  RK stage in us with segments of 32 cells -> the rule's:
+// 32^3 71 -> 27, 64^3 101 -> 59, 113x75x58 (MC) 137 -> 96, 96^3 182 -> 160,
+// 128^3 340 either way; 256^3 2364 (8-cell segments: 2445).
+inline int sweep_seg(int D, const Geom& g, int cols) {
+  const int n0 = (D == 1) ? g.ny0 : g.nz0;
+  int ns = 608 / cols;
+  if (ns > (n0 + 3) / 4) ns = (n0 + 3) / 4;
+  if (ns < (n0 + 31) / 32) ns = (n0 + 31) / 32;
+  return (n0 + ns - 1) / ns;
+}
 constexpr int kTileEY[3] = {4, 8, kEmfStream};
 
 }  // namespace mhd

@@ -1,0 +1,62 @@
+"""Launch shapes that follow the grid: segments and flattened columns of the
+FP32 column sweeps, and the batched step with its dt folded into the last stage."""
+import numpy as np
+import pytest
+
+from mhd3d_mpi_fortran_gb300 import MHDSolver, ensemble_step, ics
+from mhd3d_mpi_fortran_gb300.abi import DT_CFL, FP32, FP64, STEP_RK2, STEP_RK3, Params
+
+pytestmark = pytest.mark.gpu
+FIELDS = ("rho", "vx", "vy", "vz", "p", "bx", "by", "bz", "bi", "bj", "bk")
+
+
+def state(nx, ny, nz, nord, seed):
+    """Smooth waves with seeded noise and a random face field."""
+    g = ics.grid(nx, ny, nz, nord=nord)
+    s = ics.empty_state(g)
+    r = np.random.default_rng(seed)
+    x, y, z = [c.reshape(sh) for c, sh in zip(g.centres(), ((-1, 1, 1), (1, -1, 1), (1, 1, -1)))]
+    s.rho[...] = 1.0 + 0.3 * np.sin(2 * np.pi * (x + y)) + 0.0 * z
+    s.p[...] = 1.0 + 0.2 * np.cos(2 * np.pi * (y + z)) + 0.0 * x
+    for v in (s.vx, s.vy, s.vz, s.bi, s.bj, s.bk):
+        v[...] = 0.2 * r.standard_normal(v.shape)
+    return s
+
+
+@pytest.mark.parametrize("recon,nord", [(1, 8), (3, 6), (5, 4)])
+@pytest.mark.parametrize("shape", [(9, 37, 10), (31, 5, 66), (33, 34, 4), (40, 65, 9), (65, 16, 21)])
+def test_sweeps_equal_face_tiles(shape, recon, nord):
+    """Columns flattened over (x, remaining axis) with rows that end inside a
+    warp, and segments from 4 cells to a ragged last one: the bits of the face tiles."""
+    s = state(*shape, nord, sum(shape))
+    prm = Params(*shape, nord=nord, reconop=recon, stepop=STEP_RK3, precision=FP32, tau=2e-4)
+    out = {}
+    for td in (8, 32):
+        with MHDSolver(prm, s) as g:
+            g.set_tiles(td, 8)
+            g.step(2)
+            out[td] = g.fetch()
+    for k in FIELDS:
+        assert np.array_equal(out[8][k], out[32][k]), k
+
+
+@pytest.mark.parametrize("precision,stepop", [(FP32, STEP_RK2), (FP32, STEP_RK3), (FP64, STEP_RK2)])
+def test_batched_steps_fold_dt_as_single_steps(precision, stepop):
+    """CFL-driven batches, in calls of 1, 2 and 1 steps with single steps of one
+    grid between them (prepared and unprepared starts), against each grid alone."""
+    shapes = [(16, 24, 9), (40, 16, 16), (33, 12, 20), (24, 24, 24)]
+    ss = [state(*n, 8, 3 + m) for m, n in enumerate(shapes)]
+    ps = [Params(*n, precision=precision, stepop=stepop, dt_mode=DT_CFL, tau=1e-4) for n in shapes]
+    batch = [MHDSolver(p, s) for p, s in zip(ps, ss)]
+    alone = [MHDSolver(p, s) for p, s in zip(ps, ss)]
+    for n in (1, 2, 1):
+        ensemble_step(batch, n)
+        for g in alone:
+            g.step(n)
+        assert batch[1].step(1) == alone[1].step(1)  # (tau, status)
+    for a, b in zip(batch, alone):
+        fa, fb = a.fetch(), b.fetch()
+        for k in FIELDS:
+            assert np.array_equal(fa[k], fb[k]), k
+        a.close()
+        b.close()
