@@ -8,6 +8,7 @@
 #include <cuda_bf16.h>
 #include <math.h>
 #include <stdint.h>
+#include <string.h>
 #include <string>
 
 #include "../../include/mhd_gpu.h"
@@ -137,27 +138,7 @@ __device__ __forceinline__ float gelu_t(float z, float& dg) {
   return 0.5f * z * (1.0f + t);
 }
 
-// GELU of the 16 accumulators z[0..16) of row r, columns c0.. (+ bias),
-// rounded to BF16 and stored as two 16-byte core-matrix rows of the K-major
-// [128 x NH] activation tile.
-__device__ __forceinline__ void gelu16_store(unsigned char* tile, int r, int c0, const float* z,
-                                             const float* __restrict__ bias) {
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    uint32_t pk[4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      float d0, d1;
-      const int i = 8 * h + 2 * a;
-      const __nv_bfloat162 v = __floats2bfloat162_rn(gelu_t(z[i] + bias[c0 + i], d0),
-                                                     gelu_t(z[i + 1] + bias[c0 + i + 1], d1));
-      pk[a] = *reinterpret_cast<const uint32_t*>(&v);
-    }
-    *reinterpret_cast<uint4*>(tile + tc::kmaj(r, c0 + 8 * h, NH)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-  }
-}
-
-// The inference epilogue of gelu16_store on the packed FP32 pipe: GELU (tanh
+// The inference epilogue on the packed FP32 pipe: GELU (tanh
 // form) of two accumulators plus their biases (bias pairs from shared memory),
 // rounded to BF16 as one pair.  gelu_t's value with its constants folded:
 // u = c z + (c a) z^3 = z (c + (c a) z^2), GELU = h z + h z t (h = 1/2).
@@ -212,37 +193,100 @@ __device__ __forceinline__ void gemm(uint32_t d, uint32_t a, uint32_t b, int N, 
     tc::mma(d, tc::tile_desc(a, K, kk), tc::tile_desc(b, K, kk), id, (acc || kk > 0) ? 1u : 0u);
 }
 
-// One training pass over `count` samples idx[0..count): accumulates the
-// gradient of loss = mean over samples and outputs of (y - t)^2 into grad
-// (FP32, parameter layout) and the loss sum into *loss.  Persistent CTAs of
-// 128 threads, one 128-sample tile at a time; thread r owns sample row r and
-// reads TMEM lane r.
-__global__ void __launch_bounds__(128, 1)
+// 8 x 8 blocks of a warp's BF16 tile, transposed: four core matrices at
+// src, src + ss, .. go to dst, dst + ds, .. (each 128 contiguous bytes, so both
+// sides are free of bank conflicts).  Every lane calls it.
+__device__ __forceinline__ void transpose4(uint32_t dst, uint32_t ds, uint32_t src, uint32_t ss) {
+  const uint32_t m = (threadIdx.x >> 3) & 3, row = (threadIdx.x & 7) << 4;
+  uint32_t a, b, c, d;
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(a), "=r"(b), "=r"(c), "=r"(d)
+               : "r"(src + m * ss + row)
+               : "memory");
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(dst + m * ds + row), "r"(a),
+               "r"(b), "r"(c), "r"(d)
+               : "memory");
+}
+// 16 consecutive columns of row r, rounded to BF16, into a K-major tile of K columns.
+__device__ __forceinline__ void store16_bf16(unsigned char* tile, int r, int c0, int K, const float* v) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t pk[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      const __nv_bfloat162 x = __floats2bfloat162_rn(v[8 * h + 2 * a], v[8 * h + 2 * a + 1]);
+      pk[a] = *reinterpret_cast<const uint32_t*>(&x);
+    }
+    *reinterpret_cast<uint4*>(tile + tc::kmaj(r, c0 + 8 * h, K)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+  }
+}
+
+// One training pass over `count` samples (idx[0..count), or off .. off + count - 1
+// when idx is null): accumulates the gradient of loss = mean over samples and
+// outputs of (y - t)^2 into grad (FP32, parameter layout) and the loss sum into
+// *loss.  Persistent CTAs of 256 threads, one 128-sample tile at a time.  Thread
+// (q, half, lane) owns sample row 32 q + lane (TMEM lane of its warp's quarter)
+// and half of the columns of each layer.
+//
+// A tile is a chain of six GEMMs with an epilogue between each, so its time is
+// latency and shared-memory traffic, not bytes (67 MB of features: 10 us) or
+// tensor rate.  The contractions over samples need X, H, dZ and dY with samples
+// contiguous: those transposes go through ldmatrix / stmatrix on whole core
+// matrices (2-byte stores ran with up to 32 lanes on a bank), activations and
+// deltas are stored 16 bytes at a time, GELU's derivative stays in registers for
+// the way back, bias gradients are summed in registers over all tiles of the CTA
+// (shuffles per column and tile before), and the next tile is copied while the
+// weight gradient of layer 1 runs.  131072 samples: 256 -> 86 us.
+__global__ void __launch_bounds__(256, 1)
     k_mlp_train(const __nv_bfloat16* __restrict__ X, const float* __restrict__ T, const int* __restrict__ idx,
-                int count, float gscale, MlpW w, float* __restrict__ grad, float* __restrict__ loss, int* err) {
+                long long off, int count, float gscale, MlpW w, float* __restrict__ grad, float* __restrict__ loss,
+                int* err) {
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t tslot;
-  __shared__ float red[4][NH], red1[4][NH];  // per-warp bias-gradient sums (dZ2, dZ1 phases)
-  const int tid = threadIdx.x, q = tid >> 5, lane = tid & 31;
-  if (q == 0) tc::tmem_alloc(&tslot, T_COLS);
+  const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, q = wid & 3, half = wid >> 2;
+  const int row = 32 * q + lane;
+  constexpr int HC = NH / 2;  // columns of a half
+  if (wid == 0) tc::tmem_alloc(&tslot, T_COLS);
   if (tid == 0) tc::bar_init(&bar, 1);
   stage_w(sm + S_W1, w.w1, NH, FIN);
   stage_w(sm + S_W2, w.w2, NH, NH);
   stage_w(sm + S_W2T, w.w2t, NH, NH);
   stage_w(sm + S_W3, w.w3, NO, NH);
   stage_w(sm + S_W3T, w.w3t, NH, NO);
-  publish();
-  const uint32_t tb = tslot;
   const uint32_t s0 = tc::smem_u32(sm);
   unsigned char* R1 = sm + S_R1;
-  unsigned char* XT = sm + S_XT;
   const float* b1 = w.p + OB1;
   const float* b2 = w.p + OB2;
   const float* b3 = w.p + OB3;
+  const int ntiles = (count + 127) / 128;
+  // copy of a tile's X into R1 (sample-major): a warp copies rows 16 wid .. + 15,
+  // 8 rows x 4 chunks of 16 bytes at a time; rows past the last sample are zero
+  auto copy_x = [&](int tile) {
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      const int r = 16 * wid + 8 * g + (lane & 7), s = tile * 128 + r;
+      const bool in = s < count;
+      const __nv_bfloat16* src = X + (size_t)(in ? (idx ? (long long)idx[s] : off + s) : 0) * FIN + (lane >> 3) * 8;
+      const uint32_t dst = s0 + S_R1 + tc::kmaj(r, (lane >> 3) * 8, FIN);
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + 512u * k), "l"(src + 32 * k),
+                     "r"(in ? 16 : 0)
+                     : "memory");
+    }
+  };
+  if ((int)blockIdx.x < ntiles) copy_x(blockIdx.x);
+  publish();
+  const uint32_t tb = tslot;
   uint32_t ph = 0;
   bool ok = true, any = false;
   float lsum = 0.0f;
+  float sb1[HC], sb2[HC], sb3[NOUT];  // bias-gradient sums of this row's columns over all tiles
+#pragma unroll
+  for (int i = 0; i < HC; ++i) sb1[i] = sb2[i] = 0.0f;
+#pragma unroll
+  for (int o = 0; o < NOUT; ++o) sb3[o] = 0.0f;
   auto sync_mma = [&]() {  // every thread calls it; `ok` ends up the same in all of them
     if (tid == 0) tc::commit(&bar);
     __syncwarp();
@@ -251,78 +295,108 @@ __global__ void __launch_bounds__(128, 1)
     ph ^= 1u;
     tc::fence_after();
   };
-  const int ntiles = (count + 127) / 128;
-  for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-    // ---- stage the sample tile: X (sample-major) into R1, X^T into XT
-    for (int t = tid; t < 128 * (FIN / 8); t += 128) {
-      const int r = t >> 5, c8 = (t & 31) * 8;
-      const int g = tile * 128 + r;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (g < count) v = *reinterpret_cast<const uint4*>(X + (size_t)idx[g] * FIN + c8);
-      *reinterpret_cast<uint4*>(R1 + tc::kmaj(r, c8, FIN)) = v;
-      const uint16_t* e = reinterpret_cast<const uint16_t*>(&v);
+  // a warp's 32 rows x HC columns of the [128 x NH] tile at src, transposed into
+  // the [NH x 128] tile at dst (rows HC half .. of it)
+  auto transpose_half = [&](uint32_t dst, uint32_t src) {
+    __syncwarp();
 #pragma unroll
-      for (int i = 0; i < 8; ++i) *reinterpret_cast<uint16_t*>(XT + tc::kmaj(c8 + i, r, 128)) = e[i];
+    for (int c8 = 0; c8 < HC / 8; ++c8) {
+      const int cg = half * (HC / 8) + c8;
+      transpose4(dst + 128u * (cg * 16 + 4 * q), 128u, src + 128u * (4 * q * (NH / 8) + cg), 16u * NH);
     }
-    const int gr = tile * 128 + tid;
+  };
+  for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+    const int gr = tile * 128 + row;
     const bool valid = gr < count;
     float tgt[NOUT];
 #pragma unroll
-    for (int o = 0; o < NOUT; ++o) tgt[o] = valid ? T[(size_t)idx[gr] * NOUT + o] : 0.0f;
+    for (int o = 0; o < NOUT; ++o) tgt[o] = 0.0f;
+    if (valid && half == 0) {
+      const float4* tp = reinterpret_cast<const float4*>(T + (size_t)(idx ? (long long)idx[gr] : off + gr) * NOUT);
+      const float4 t0 = tp[0], t1 = tp[1];
+      tgt[0] = t0.x; tgt[1] = t0.y; tgt[2] = t0.z; tgt[3] = t0.w;
+      tgt[4] = t1.x; tgt[5] = t1.y; tgt[6] = t1.z; tgt[7] = t1.w;
+    }
+    // ---- X^T (feature-major) of the rows this warp copied
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      const int rg = 2 * wid + g;
+#pragma unroll
+      for (int c8 = 0; c8 < FIN / 8; c8 += 4)
+        transpose4(s0 + S_XT + 128u * (c8 * 16 + rg), 128u * 16, s0 + S_R1 + 128u * (rg * (FIN / 8) + c8), 128u);
+    }
     publish();
     // ---- layer 1
     if (tid == 0) gemm(tb + T_D1, s0 + S_R1, s0 + S_W1, NH, FIN, false);
     sync_mma();
     if (!ok) break;
-    for (int c0 = 0; c0 < NH; c0 += 16) {
+    {  // the next tile's rows, on their way to L2
+      const int s = (tile + (int)gridDim.x) * 128 + (tid >> 1);
+      if (s < count) {
+        const __nv_bfloat16* src = X + (size_t)(idx ? (long long)idx[s] : off + s) * FIN + (tid & 1) * (FIN / 2);
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(src));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(src + FIN / 4));
+      }
+    }
+    float dg1[HC], dg2[HC];
+#pragma unroll
+    for (int c = 0; c < HC; c += 16) {
+      const int c0 = half * HC + c;
       float z[16];
       tc::tmem_ld16(tc::tmem_at(tb + T_D1, q, c0), z);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        float dg;
-        const float h = gelu_t(z[i] + b1[c0 + i], dg);
-        tc::st_bf16(sm + S_H1, tc::kmaj(tid, c0 + i, NH), h);
-        tc::st_bf16(R1 + R_HT, tc::kmaj(c0 + i, tid, 128), h);
-      }
+      for (int i = 0; i < 16; ++i) z[i] = gelu_t(z[i] + b1[c0 + i], dg1[c + i]);
+      store16_bf16(sm + S_H1, row, c0, NH, z);
     }
+    transpose_half(s0 + S_R1 + R_HT, s0 + S_H1);
     publish();
     // ---- layer 2
     if (tid == 0) gemm(tb + T_D2, s0 + S_H1, s0 + S_W2, NH, NH, false);
     sync_mma();
     if (!ok) break;
-    for (int c0 = 0; c0 < NH; c0 += 16) {
+#pragma unroll
+    for (int c = 0; c < HC; c += 16) {
+      const int c0 = half * HC + c;
       float z[16];
       tc::tmem_ld16(tc::tmem_at(tb + T_D2, q, c0), z);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        float dg;
-        const float h = gelu_t(z[i] + b2[c0 + i], dg);
-        tc::st_bf16(sm + S_H2, tc::kmaj(tid, c0 + i, NH), h);
-        tc::st_bf16(R1 + R_HT, tc::kmaj(NH + c0 + i, tid, 128), h);
-      }
+      for (int i = 0; i < 16; ++i) z[i] = gelu_t(z[i] + b2[c0 + i], dg2[c + i]);
+      store16_bf16(sm + S_H2, row, c0, NH, z);
     }
+    transpose_half(s0 + S_R1 + R_HT + NH * 128 * 2, s0 + S_H2);
     publish();
-    // ---- layer 3 and the loss
+    // ---- layer 3 and the loss (outputs 8 .. 15 are padding: the other half writes their zeros)
     if (tid == 0) gemm(tb + T_D3, s0 + S_H2, s0 + S_W3, NO, NH, false);
     sync_mma();
     if (!ok) break;
-    {
+    if (half == 0) {
       float y[16];
       tc::tmem_ld16(tc::tmem_at(tb + T_D3, q, 0), y);
+      uint32_t pk[4];
 #pragma unroll
-      for (int o = 0; o < NO; ++o) {
+      for (int o = 0; o < NOUT; ++o) {
         float dy = 0.0f;
-        if (o < NOUT && valid) {
+        if (valid) {
           const float e = y[o] + b3[o] - tgt[o];
           lsum += e * e;
           dy = gscale * e;
         }
-        tc::st_bf16(R1 + R_DY, tc::kmaj(tid, o, NO), dy);
-        tc::st_bf16(R1 + R_DYT, tc::kmaj(o, tid, 128), dy);
-        float sdy = dy;
-        for (int m = 16; m > 0; m >>= 1) sdy += __shfl_xor_sync(0xffffffffu, sdy, m);
-        if (lane == 0 && o < NOUT) atomicAdd(grad + OB3 + o, sdy);
+        sb3[o] += dy;
+        y[o] = dy;
       }
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const __nv_bfloat162 x = __floats2bfloat162_rn(y[2 * a], y[2 * a + 1]);
+        pk[a] = *reinterpret_cast<const uint32_t*>(&x);
+      }
+      *reinterpret_cast<uint4*>(R1 + R_DY + tc::kmaj(row, 0, NO)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+      __syncwarp();
+      transpose4(s0 + S_R1 + R_DYT + 128u * 4 * q, 128u, s0 + S_R1 + R_DY + 256u * 4 * q, 256u);
+    } else {
+      *reinterpret_cast<uint4*>(R1 + R_DY + tc::kmaj(row, 8, NO)) = make_uint4(0, 0, 0, 0);
+      *reinterpret_cast<uint4*>(R1 + R_DYT + 128 * 16 + 16 * row) = make_uint4(0, 0, 0, 0);
     }
     publish();
     // ---- dH2 = dY W3 ; dW3^T += H2^T dY (rows 64..127 of the stacked H^T)
@@ -332,24 +406,19 @@ __global__ void __launch_bounds__(128, 1)
     }
     sync_mma();
     if (!ok) break;
-    for (int c0 = 0; c0 < NH; c0 += 16) {
-      float dh[16], z[16];
-      tc::tmem_ld16(tc::tmem_at(tb + T_DH2, q, c0), dh);
-      tc::tmem_ld16(tc::tmem_at(tb + T_D2, q, c0), z);
+#pragma unroll
+    for (int c = 0; c < HC; c += 16) {
+      float dz[16];
+      tc::tmem_ld16(tc::tmem_at(tb + T_DH2, q, half * HC + c), dz);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        float dg;
-        gelu_t(z[i] + b2[c0 + i], dg);
-        const float dz = valid ? dh[i] * dg : 0.0f;
-        tc::st_bf16(R1 + R_DZ2, tc::kmaj(tid, c0 + i, NH), dz);
-        tc::st_bf16(sm + S_H1, tc::kmaj(c0 + i, tid, 128), dz);  // dZ2^T (the H1 tile is free)
-        float sd = dz;
-        for (int m = 16; m > 0; m >>= 1) sd += __shfl_xor_sync(0xffffffffu, sd, m);
-        if (lane == 0) red[q][c0 + i] = sd;
+        dz[i] = valid ? dz[i] * dg2[c + i] : 0.0f;
+        sb2[c + i] += dz[i];
       }
+      store16_bf16(R1 + R_DZ2, row, half * HC + c, NH, dz);
     }
+    transpose_half(s0 + S_H1, s0 + S_R1 + R_DZ2);  // dZ2^T (the H1 tile is free)
     publish();
-    if (tid < NH) atomicAdd(grad + OB2 + tid, red[0][tid] + red[1][tid] + red[2][tid] + red[3][tid]);
     // ---- dH1 = dZ2 W2 ; dW2^T += H1^T dZ2 (rows 0..63 of the stacked H^T)
     if (tid == 0) {
       gemm(tb + T_DH1, s0 + S_R1 + R_DZ2, s0 + S_W2T, NH, NH, false);
@@ -357,59 +426,78 @@ __global__ void __launch_bounds__(128, 1)
     }
     sync_mma();
     if (!ok) break;
-    for (int c0 = 0; c0 < NH; c0 += 16) {
-      float dh[16], z[16];
-      tc::tmem_ld16(tc::tmem_at(tb + T_DH1, q, c0), dh);
-      tc::tmem_ld16(tc::tmem_at(tb + T_D1, q, c0), z);
+#pragma unroll
+    for (int c = 0; c < HC; c += 16) {
+      float dz[16];
+      tc::tmem_ld16(tc::tmem_at(tb + T_DH1, q, half * HC + c), dz);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        float dg;
-        gelu_t(z[i] + b1[c0 + i], dg);
-        const float dz = valid ? dh[i] * dg : 0.0f;
-        tc::st_bf16(sm + S_H2, tc::kmaj(c0 + i, tid, 128), dz);  // dZ1^T (the H2 tile is free)
-        float sd = dz;
-        for (int m = 16; m > 0; m >>= 1) sd += __shfl_xor_sync(0xffffffffu, sd, m);
-        if (lane == 0) red1[q][c0 + i] = sd;
+        dz[i] = valid ? dz[i] * dg1[c + i] : 0.0f;
+        sb1[c + i] += dz[i];
       }
+      store16_bf16(R1 + R_DZ2, row, half * HC + c, NH, dz);  // dZ1 in the place of dZ2, whose MMAs are done
     }
+    transpose_half(s0 + S_H2, s0 + S_R1 + R_DZ2);  // dZ1^T (the H2 tile is free)
     publish();
-    if (tid < NH) atomicAdd(grad + OB1 + tid, red1[0][tid] + red1[1][tid] + red1[2][tid] + red1[3][tid]);
-    // ---- dW1^T += X^T dZ1, features 0..127 and 128..255
+    // ---- dW1^T += X^T dZ1, features 0..127 and 128..255, while the next X comes into R1
     if (tid == 0) {
       gemm(tb + T_G1A, s0 + S_XT, s0 + S_H2, NH, 128, any);
       gemm(tb + T_G1B, s0 + S_XT + tc::kmaj(128, 0, 128), s0 + S_H2, NH, 128, any);
     }
+    __syncwarp();
+    if (tile + (int)gridDim.x < ntiles) copy_x(tile + gridDim.x);
     sync_mma();
     any = true;
-    __syncthreads();  // the next tile overwrites R1, XT and the reductions
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   if (!ok) {
     if (tid == 0) atomicExch(err, 1);
     tc::bar_wait(&bar, ph ^ 1u);  // a second bounded wait for MMAs still in flight
   } else if (any) {
     // ---- weight gradients from TMEM: lane = input index, column = output index
-    for (int c0 = 0; c0 < NH; c0 += 16) {
+#pragma unroll
+    for (int c = 0; c < HC; c += 16) {
+      const int c0 = half * HC + c;
       float ga[16], gb[16], g2[16];
       tc::tmem_ld16(tc::tmem_at(tb + T_G1A, q, c0), ga);
       tc::tmem_ld16(tc::tmem_at(tb + T_G1B, q, c0), gb);
       tc::tmem_ld16(tc::tmem_at(tb + T_G2, q, c0), g2);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        atomicAdd(grad + OW1 + (c0 + i) * FIN + tid, ga[i]);
-        atomicAdd(grad + OW1 + (c0 + i) * FIN + 128 + tid, gb[i]);
-        if (tid < NH) atomicAdd(grad + OW2 + (c0 + i) * NH + tid, g2[i]);
+        atomicAdd(grad + OW1 + (c0 + i) * FIN + row, ga[i]);
+        atomicAdd(grad + OW1 + (c0 + i) * FIN + 128 + row, gb[i]);
+        if (row < NH) atomicAdd(grad + OW2 + (c0 + i) * NH + row, g2[i]);
       }
     }
-    float g3[16];
-    tc::tmem_ld16(tc::tmem_at(tb + T_G3, q, 0), g3);
-    if (tid >= NH)
-      for (int o = 0; o < NOUT; ++o) atomicAdd(grad + OW3 + o * NH + (tid - NH), g3[o]);
-    for (int m = 16; m > 0; m >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, m);
-    if (lane == 0) atomicAdd(loss, lsum);
+    auto warp_sum = [](float x) {
+      for (int m = 16; m > 0; m >>= 1) x += __shfl_xor_sync(0xffffffffu, x, m);
+      return x;
+    };
+#pragma unroll
+    for (int i = 0; i < HC; ++i) {
+      const float x1 = warp_sum(sb1[i]), x2 = warp_sum(sb2[i]);
+      if (lane == 0) {
+        atomicAdd(grad + OB1 + half * HC + i, x1);
+        atomicAdd(grad + OB2 + half * HC + i, x2);
+      }
+    }
+    if (half == 0) {
+      float g3[16];
+      tc::tmem_ld16(tc::tmem_at(tb + T_G3, q, 0), g3);
+      if (row >= NH)
+        for (int o = 0; o < NOUT; ++o) atomicAdd(grad + OW3 + o * NH + (row - NH), g3[o]);
+#pragma unroll
+      for (int o = 0; o < NOUT; ++o) {
+        const float x = warp_sum(sb3[o]);
+        if (lane == 0) atomicAdd(grad + OB3 + o, x);
+      }
+      lsum = warp_sum(lsum);
+      if (lane == 0) atomicAdd(loss, lsum);
+    }
   }
   tc::fence_before();
   __syncthreads();
-  if (q == 0) tc::tmem_free(tb, T_COLS);
+  if (wid == 0) tc::tmem_free(tb, T_COLS);
 }
 
 // shared-memory map of the inference kernel: weights, then one 128 x 256 input
@@ -617,11 +705,6 @@ __global__ void k_batch_idx(int* idx, int count, long long n, unsigned long long
   idx[i] = (int)(x % (unsigned long long)n);
 }
 
-__global__ void k_iota(int* idx, int count, long long off) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < count) idx[i] = (int)(off + i);
-}
-
 // ------------------------------------------------------- solver coupling
 // Domain sums of the hydro increments y[0..4] (for a conservative correction):
 // FP64 per thread, then per warp and per block (256 threads), one atomic per
@@ -761,8 +844,8 @@ struct Mlp {
   long long n = 0;
   int* idx = nullptr;
   int idx_cap = 0;
-  float* loss = nullptr;
-  int* err = nullptr;
+  float* loss = nullptr;       // behind the gradient, one copy reads both
+  int* err = nullptr;          // behind the loss
   int step = 0;
   MlpNorm norm{};
   float* ys = nullptr;          // correction of a grid: the network outputs
@@ -810,24 +893,25 @@ int set_smem_once() {
   return MHD_OK;
 }
 
-// gradient of the mean loss over idx[0..count) into m->g, loss sum into m->loss
-int grad_pass(Mlp* m, int count) {
+// gradient of the mean loss over idx[0..count), or samples off .. off + count - 1
+// when idx is null, into m->g, loss sum into m->loss (the float after it)
+int grad_pass(Mlp* m, const int* idx, long long off, int count) {
   int rc = set_smem_once();
   if (rc) return rc;
-  MCK(cudaMemset(m->g, 0, sizeof(float) * NPARAM));
-  MCK(cudaMemset(m->loss, 0, sizeof(float)));
+  MCK(cudaMemsetAsync(m->g, 0, sizeof(float) * (NPARAM + 1), 0));
   const int tiles = (count + 127) / 128;
   const int grid = tiles < m->sms ? tiles : m->sms;
-  k_mlp_train<<<grid, 128, S_TOTAL>>>(m->X, m->T, m->idx, count, 2.0f / ((float)count * NOUT), wview(m), m->g,
+  k_mlp_train<<<grid, 256, S_TOTAL>>>(m->X, m->T, idx, off, count, 2.0f / ((float)count * NOUT), wview(m), m->g,
                                        m->loss, m->err);
   MCK(cudaGetLastError());
   return MHD_OK;
 }
 
+const char* const kGaveUp = "MLP kernel: a tensor-core completion wait gave up";
 int check_err(Mlp* m) {
   int e = 0;
   MCK(cudaMemcpy(&e, m->err, sizeof(int), cudaMemcpyDeviceToHost));
-  if (e) return mfail(MHD_E_TIMEOUT, "MLP kernel: a tensor-core completion wait gave up");
+  if (e) return mfail(MHD_E_TIMEOUT, kGaveUp);
   return MHD_OK;
 }
 }  // namespace
@@ -873,17 +957,18 @@ int mhd_mlp_create(const float* params, void** out) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, dev);
   bool ok = cudaMalloc(&m->p, sizeof(float) * NPARAM) == cudaSuccess &&
-            cudaMalloc(&m->g, sizeof(float) * NPARAM) == cudaSuccess &&
+            cudaMalloc(&m->g, sizeof(float) * (NPARAM + 2)) == cudaSuccess &&
             cudaMalloc(&m->m, sizeof(float) * NPARAM) == cudaSuccess &&
             cudaMalloc(&m->v, sizeof(float) * NPARAM) == cudaSuccess &&
             cudaMalloc(&m->w1, 2 * NH * FIN) == cudaSuccess && cudaMalloc(&m->w2, 2 * NH * NH) == cudaSuccess &&
             cudaMalloc(&m->w2t, 2 * NH * NH) == cudaSuccess && cudaMalloc(&m->w3, 2 * NO * NH) == cudaSuccess &&
-            cudaMalloc(&m->w3t, 2 * NO * NH) == cudaSuccess && cudaMalloc(&m->loss, sizeof(float)) == cudaSuccess &&
-            cudaMalloc(&m->err, sizeof(int)) == cudaSuccess;
+            cudaMalloc(&m->w3t, 2 * NO * NH) == cudaSuccess;
   if (!ok) {
     mhd_mlp_free(m);
     return mfail(MHD_E_NOMEM, "MLP device allocation failed");
   }
+  m->loss = m->g + NPARAM;
+  m->err = reinterpret_cast<int*>(m->loss + 1);
   cudaMemcpy(m->p, params, sizeof(float) * NPARAM, cudaMemcpyHostToDevice);
   cudaMemset(m->m, 0, sizeof(float) * NPARAM);
   cudaMemset(m->v, 0, sizeof(float) * NPARAM);
@@ -947,18 +1032,15 @@ int mhd_mlp_grad(void* h, int64_t offset, int32_t count, float* grad_out, float*
   Mlp* m = (Mlp*)h;
   if (!m || !grad_out || count <= 0 || offset < 0 || offset + count > m->n)
     return mfail(MHD_E_ARG, "bad gradient range");
-  int rc = ensure_idx(m, count);
+  int rc = grad_pass(m, nullptr, offset, count);
   if (rc) return rc;
-  k_iota<<<(count + 255) / 256, 256>>>(m->idx, count, offset);
-  rc = grad_pass(m, count);
-  if (rc) return rc;
-  MCK(cudaDeviceSynchronize());
-  rc = check_err(m);
-  if (rc) return rc;
+  uint32_t tail[2];  // loss sum, error word
+  MCK(cudaMemcpy(tail, m->loss, sizeof(tail), cudaMemcpyDeviceToHost));
+  if (tail[1]) return mfail(MHD_E_TIMEOUT, kGaveUp);
   MCK(cudaMemcpy(grad_out, m->g, sizeof(float) * NPARAM, cudaMemcpyDeviceToHost));
   if (loss_out) {
     float l = 0;
-    MCK(cudaMemcpy(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost));
+    memcpy(&l, tail, sizeof(l));
     *loss_out = l / ((float)count * NOUT);
   }
   return MHD_OK;
@@ -973,7 +1055,7 @@ int mhd_mlp_train(void* h, int32_t iters, int32_t batch, float lr, uint64_t seed
   int lcnt = 0;
   for (int it = 0; it < iters; ++it) {
     k_batch_idx<<<(batch + 255) / 256, 256>>>(m->idx, batch, m->n, seed + (uint64_t)m->step);
-    rc = grad_pass(m, batch);
+    rc = grad_pass(m, m->idx, 0, batch);
     if (rc) return rc;
     m->step += 1;
     const float b1 = 0.9f, b2 = 0.999f;
@@ -1027,8 +1109,7 @@ int mhd_mlp_free(void* h) {
   Mlp* m = (Mlp*)h;
   if (!m) return MHD_OK;
   cudaDeviceSynchronize();
-  void* ptrs[] = {m->p, m->g, m->m, m->v, m->w1, m->w2, m->w2t, m->w3, m->w3t, m->X, m->T, m->idx, m->loss, m->err,
-                  m->ys, m->sums};
+  void* ptrs[] = {m->p, m->g, m->m, m->v, m->w1, m->w2, m->w2t, m->w3, m->w3t, m->X, m->T, m->idx, m->ys, m->sums};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   delete m;

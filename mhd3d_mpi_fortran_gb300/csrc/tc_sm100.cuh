@@ -120,9 +120,5 @@ __device__ __forceinline__ uint32_t tmem_at(uint32_t base, int q, int c) {
   return base + ((uint32_t)(32 * q) << 16) + (uint32_t)c;
 }
 
-__device__ __forceinline__ void st_bf16(unsigned char* tile, uint32_t off, float x) {
-  *reinterpret_cast<__nv_bfloat16*>(tile + off) = __float2bfloat16_rn(x);
-}
-
 }  // namespace tc
 }  // namespace mhd

@@ -172,3 +172,21 @@ def test_grid_inference_equals_matrix_inference_on_a_ragged_grid():
     for k in ("bi", "bj", "bk"):
         got = f1[k][sl] - f0[k][sl]
         assert np.abs(got - ref[k]).max() <= 2e-2 * np.abs(ref[k]).max() + 1e-6, k
+
+
+@pytest.mark.parametrize("off,n", [(0, 1), (3, 127), (0, 129), (5, 128 * 153 + 1)])
+def test_gradient_at_ragged_counts_and_offsets(off, n):
+    """Part of a tile, one row past a tile, and more tiles than CTAs, at an offset:
+    weight and bias gradients against the oracle with the same BF16 rounding
+    points (2e-2: BF16 roundings that the FP32 accumulation order flips)."""
+    p = mo.init_params(11)
+    xb = _features(off + n, 12)
+    t = (np.random.default_rng(13).standard_normal((off + n, mo.NOUT)) * 0.5).astype(np.float32)
+    mlp = learned.MLP(p)
+    mlp.set_data(xb, t)
+    loss, g = mlp.grad(off, n)
+    lref, gref = mo.loss_and_grad(p, mo.bf16_val(xb[off:]), t[off:], bf16=True)
+    assert loss == pytest.approx(lref, rel=1e-3)
+    for (name, a), b in zip(mo.unpack(g).items(), mo.unpack(gref).values()):
+        assert np.linalg.norm(a - b) <= 2e-2 * max(np.linalg.norm(b), 1e-30), name
+    mlp.close()
