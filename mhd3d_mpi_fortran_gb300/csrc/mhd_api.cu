@@ -278,7 +278,7 @@ void carve(Handle* h, Dev<T>& d, char* base) {
   d.dt_mode = h->prm.dt_mode;
   for (int i = 0; i < 3; ++i) d.bc[i] = h->prm.bc[i];
   d.gam = (T)h->prm.gam; d.pdmb = (T)h->prm.pdmb; d.eps = (T)h->prm.eps;
-  d.rgm1 = (T)(1.0 / (h->prm.gam - 1.0));
+  d.rgm1 = T(1) / (d.gam - T(1));
   d.alpha = (T)h->prm.alpha; d.beta = (T)h->prm.beta; d.cfl = (T)h->prm.cfl;
   d.rho = next(); d.vx = next(); d.vy = next(); d.vz = next(); d.p = next();
   d.bi = next(); d.bj = next(); d.bk = next(); d.bx = next(); d.by = next(); d.bz = next();

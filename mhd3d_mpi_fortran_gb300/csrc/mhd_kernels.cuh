@@ -753,8 +753,32 @@ __device__ __forceinline__ float2 add(float2 a, float2 b) { return __fadd2_rn(a,
 __device__ __forceinline__ float2 sub(float2 a, float2 b) { return __ffma2_rn(b, K(-1.0f), a); }  // a - b, one rounding
 __device__ __forceinline__ float2 mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 rcp(float2 a) { return make_float2(__fdividef(1.0f, a.x), __fdividef(1.0f, a.y)); }
-__device__ __forceinline__ float2 rsq(float2 a) { return make_float2(rsqrtf(a.x), rsqrtf(a.y)); }
+// 1/x, 1/sqrt(x) and exp(-x) on the SFU alone: the .ftz forms, which drop the
+// rescaling of subnormal operands and results around each (two to three
+// instructions; a face takes 18 of these).  Same bits for normal numbers; below
+// 1.2e-38 (a pressure, or a tail of erfc or exp that is added to values of order one)
+// they are zero.
+__device__ __forceinline__ float rcp1(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rsq1(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float ex21(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float2 rcp(float2 a) { return make_float2(rcp1(a.x), rcp1(a.y)); }
+__device__ __forceinline__ float2 rsq(float2 a) { return make_float2(rsq1(a.x), rsq1(a.y)); }
+__device__ __forceinline__ float2 exp_neg(float2 a) {
+  a = mul(a, K(-1.4426950408889634f));
+  return make_float2(ex21(a.x), ex21(a.y));
+}
 }  // namespace p2
 
 // corner_pdm of both components from pair-interleaved shared memory.
@@ -872,6 +896,14 @@ inline KArg<T, false> one(const Dev<T>& d) { return KArg<T, false>{d}; }
 constexpr int pass_min_blocks(bool B) { return B ? MHD_BATCH_MINB : 0; }
 
 // ------------------------------------------------------------- small kernels
+// dt of the current step in T (FP32: the copy select_tau rounds once; a
+// conversion per thread ran on the FP64 pipe, 16 cycles a warp).
+template <typename T>
+__device__ __forceinline__ T step_tau(const Scal* sc) {
+  if constexpr (std::is_same<T, float>::value) return sc->tauf;
+  else return sc->tau;
+}
+
 template <typename T>
 __device__ __forceinline__ long long idx3(const Geom& g, int i, int j, int k) {
   return (long long)i + (long long)g.px * ((long long)j + (long long)g.py * (long long)k);
@@ -1101,6 +1133,7 @@ __device__ __forceinline__ void select_tau(Scal* s, int mode) {
     s->tau0 = dt;
   }
   // mode 3: read-only (diagnostics); tau untouched
+  s->tauf = (float)s->tau;
 }
 template <typename T>
 __global__ void k_cfl_final(Dev<T> d, int mode) { select_tau(d.sc, mode); }
@@ -1254,8 +1287,7 @@ __device__ __forceinline__ void pdm_pair_states(const float2* a, float pdmb, flo
 // evaluated with negated coefficients, so exp(z^2 - (-q)) takes the same
 // argument as erfc_pos's exp(-z^2 + q).
 __device__ __forceinline__ float2 half_erfc_lr(float2 x) {
-  const float2 z = make_float2(fabsf(x.x), fabsf(x.y));
-  const float2 t = p2::rcp(p2::fma(p2::K(0.5f), z, p2::K(1.0f)));
+  const float2 t = p2::rcp(make_float2(fmaf(0.5f, fabsf(x.x), 1.0f), fmaf(0.5f, fabsf(x.y), 1.0f)));
   float2 nq = p2::fma(t, p2::K(-0.17087277f), p2::K(0.82215223f));
   nq = p2::fma(t, nq, p2::K(-1.48851587f));
   nq = p2::fma(t, nq, p2::K(1.13520398f));
@@ -1265,8 +1297,7 @@ __device__ __forceinline__ float2 half_erfc_lr(float2 x) {
   nq = p2::fma(t, nq, p2::K(-0.37409196f));
   nq = p2::fma(t, nq, p2::K(-1.00002368f));
   nq = p2::fma(t, nq, p2::K(1.26551223f));
-  const float2 y = p2::fma(z, z, nq);  // z^2 - q
-  const float2 e = make_float2(__expf(-y.x), __expf(-y.y));
+  const float2 e = p2::exp_neg(p2::fma(x, x, nq));  // of x^2 - q
   const float2 h = p2::mul(p2::K(0.5f), p2::mul(t, e));
   const float2 g = p2::sub(p2::K(1.0f), h);
   return make_float2(x.x <= 0.0f ? h.x : g.x, x.y >= 0.0f ? h.y : g.y);
@@ -1276,9 +1307,8 @@ __device__ __forceinline__ float2 half_erfc_lr(float2 x) {
 // formulas of face_flux) with the left state in lane x and the right state
 // in lane y of X[q] = (l[q], r[q]); out = left + right.
 template <int D>
-__device__ __forceinline__ void face_flux_lr(const float2* X, float gam, float* out) {
+__device__ __forceinline__ void face_flux_lr(const float2* X, float rg, float* out) {
   using namespace p2;
-  const float rg = __frcp_rn(gam - 1.0f);
   const float2 r = X[0], u = X[1], v = X[2], w = X[3], pr = X[4], bx = X[5], by = X[6], bz = X[7];
   const float2 vn = X[1 + D], bn = X[5 + D];
   float2 ke = mul(u, u);
@@ -1290,7 +1320,7 @@ __device__ __forceinline__ void face_flux_lr(const float2* X, float gam, float* 
   const float2 ra = rsq(lam);
   const float2 v0 = half_erfc_lr(mul(mul(lam, ra), vn));
   const float2 lv = mul(mul(lam, vn), vn);
-  const float2 b = mul(mul(K(0.5f * 0.56418958354775628f), ra), make_float2(__expf(-lv.x), __expf(-lv.y)));
+  const float2 b = mul(mul(K(0.5f * 0.56418958354775628f), ra), exp_neg(lv));
   const float2 v1 = fma(vn, v0, make_float2(b.x, -b.y));
   float2 f[8];
   f[0] = mul(r, v1);
@@ -1399,7 +1429,7 @@ __device__ __forceinline__ void face_flux(const float* l, const float* r, const 
   float2 X[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) X[q] = make_float2(l[q], r[q]);
-  face_flux_lr<D>(X, d.gam, out);
+  face_flux_lr<D>(X, d.rgm1, out);
 }
 template <int D>
 __device__ __forceinline__ void face_flux(const double* l, const double* r, const Dev<double>& d, double* out) {
@@ -1655,7 +1685,7 @@ __host__ __device__ constexpr size_t flux_t_smem() {
 template <typename T, bool M>
 __device__ __forceinline__ void cell_update_vals(const Dev<T>& d, int c, int cd, const T* dF, const T* du,
                                                  const T* pv, const T* qv, int form, T cw, T den) {
-  const T tau = (T)d.sc->tau;
+  const T tau = step_tau<T>(d.sc);
   const T gm1 = d.gam - T(1);
   T dv[8];
   if (M) {
@@ -2432,7 +2462,8 @@ __global__ void __launch_bounds__(32 * NW, MHD_EMF_STREAM_MINB)
     for (int m = 0; m < 8; ++m) gw[m] = first_a1(s_lo - 4 + m);
     __syncthreads();  // the first step refills the slot of slice s_lo - 4
   }
-#pragma unroll 1
+  // two steps a turn: half of the windows' register moves (256^3 stage 2301 -> 2285 us; four a turn spill)
+#pragma unroll 2
   for (int s = s_lo; s <= s_hi; ++s) {
     const bool more = s < s_hi;
     T bnext = T(0);
@@ -3056,7 +3087,7 @@ __global__ void k_update_b(KArg<T, B> ka, int form, T cw, T den) {
   bool in_x = i < g.ng + g.nx0, in_y = j < g.ng + g.ny0, in_z = k < g.ng + g.nz0;
   long long c = idx3<T>(g, i, j, k);
   const long long sy = g.px, sz = g.plane;
-  const T tau = (T)d.sc->tau;
+  const T tau = step_tau<T>(d.sc);
   const T dx = d.wx[i], dy = d.wy[j], dz = d.wz[k];
   const T rx = d.rwx[i], ry = d.rwy[j], rz = d.rwz[k];
   const T *ei = d.E[0], *ej = d.E[1], *ek = d.E[2];
@@ -3355,7 +3386,7 @@ __global__ void __launch_bounds__(256, pass_min_blocks(B))
   if (i < g.ng + g.nx0 && j < g.ng + g.ny0) {
     const int px = g.px, pl = (int)g.plane;
     const int c = i + px * j + pl * k;
-    const T tau = (T)d.sc->tau;
+    const T tau = step_tau<T>(d.sc);
     const T dx = d.wx[i], dy = d.wy[j], dz = d.wz[k];
     const T rx = d.rwx[i], ry = d.rwy[j], rz = d.rwz[k];
     const T *ei = d.E[0], *ej = d.E[1], *ek = d.E[2];

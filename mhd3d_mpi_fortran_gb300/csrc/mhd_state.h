@@ -39,6 +39,7 @@ struct Scal {
   unsigned int status;           // MHD_ST_* bits
   unsigned int pend_status;      // status bits of the state the next step starts from
   unsigned long long dtnext_bits; // CFL dt of that state (min over cells, +inf when empty)
+  float tauf;                    // tau rounded to FP32, set with it
 };
 // form of an RK first stage that also stores U^n (the input state) for the
 // later stages' combines
@@ -78,7 +79,7 @@ struct Dev {
   int recon, stepop, tvd_shift, dt_mode;
   int bc[3];
   T gam, pdmb, eps, alpha, beta, cfl;
-  T rgm1;      // 1 / (gam - 1)
+  T rgm1;      // 1 / (gam - 1), of gam in T
   // state of the current level; the cell primitives and the face B are
   // double-buffered: the z-flux kernel writes the new primitives into o*, the
   // CT kernel the new face B into ob* (swapped after each stage), so no kernel
