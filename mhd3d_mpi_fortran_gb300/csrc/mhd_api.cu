@@ -88,7 +88,7 @@ struct Handle {
   float* geoT = nullptr;       // FP32 copy of the cell widths
   int* gmap = nullptr;         // ghost-image tables
   bool metric = false;         // curvilinear metric mode (mhd_init_mapped)
-  double* met = nullptr;       // FP64 metric arrays (kMetricArrays x vol)
+  double* met = nullptr;       // metric arrays (room for kMetricArrays x vol in FP64; see metric_to_fp32)
   std::vector<double> nodes;   // host copy of the node coordinates (checkpoints)
   // graphs keyed by (nsteps, starting parity + 2 prepared) -> (exec, parity + 2 prepared after replay)
   std::map<std::pair<int, int>, std::pair<cudaGraphExec_t, int>> graphs;
@@ -304,7 +304,7 @@ void carve(Handle* h, Dev<T>& d, char* base) {
   d.gmap = h->gmap;
   d.partial = nullptr;
   d.counter = nullptr;
-  d.m = Metric{};
+  d.m = Metric<T>{};
   d.tile_td = h->tile_td;
   d.tile_ey = h->tile_ey;
   for (int D = 1; D < 3; ++D) d.seg[D - 1] = sweep_seg(D, g, sweep_cols(D, g));
@@ -316,9 +316,9 @@ void carve(Handle* h, Dev<T>& d, char* base) {
   d.emf = h->prm.emf;
   for (int q = 0; q < 12; ++q) d.ye[q] = (h->prm.emf == MHD_EMF_YEE) ? next() : nullptr;
   if (h->metric) {
-    const double* mb = h->met;
-    auto nm = [&]() { const double* r = mb; mb += n; return r; };
-    Metric& m = d.m;
+    const T* mb = (const T*)h->met;
+    auto nm = [&]() { const T* r = mb; mb += n; return r; };
+    Metric<T>& m = d.m;
     for (int a = 0; a < 3; ++a)
       for (int q = 0; q < 3; ++q) m.nrm[a][q] = nm();
     for (int a = 0; a < 3; ++a) m.am[a] = nm();
@@ -331,10 +331,11 @@ void carve(Handle* h, Dev<T>& d, char* base) {
     m.sa = nm();
     for (int e = 0; e < 3; ++e) m.ge[e] = nm();
     for (int e = 0; e < 3; ++e) m.dl[e] = nm();
+    m.vol64 = sizeof(T) == 8 ? (const double*)m.vol : h->met + (kMetricArrays - 1) * n;
   }
 }
 
-// The writable view of the metric block carved as carve() lays it out.
+// The FP64 metric block as metric_geometry writes it (FP64 handles: as carve() lays it out).
 MetricOut metric_out(Handle* h) {
   const size_t n = (size_t)h->g.vol;
   double* mb = h->met;
@@ -703,6 +704,31 @@ int mhd_init(const mhd_params* prm, const double* rho, const double* vx, const d
   return MHD_OK;
 }
 
+__global__ void k_to_f32(const double* __restrict__ src, float* __restrict__ dst, size_t n) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    dst[i] = (float)src[i];
+}
+
+// FP32 handles: the metric block rounded once, in place.  Every read of an
+// FP64 entry was a conversion on the FP64 pipe (a warp every 16 cycles) and twice
+// the bytes.  FP32 array a ends at or below the end of FP64 array a, so in
+// ascending order, each by way of the flux arrays (scratch before the first step),
+// nothing is overwritten unread; V stays in FP64 behind them for the diagnostics.
+static int metric_to_fp32(Handle* h) {
+  const size_t n = (size_t)h->g.vol;
+  float* tmp = h->df.F[0][0];
+  double* vol64 = (double*)h->df.F[0][2];  // two FP32 arrays
+  const MetricOut m = metric_out(h);
+  CK(cudaMemcpyAsync(vol64, m.vol, n * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
+  for (int a = 0; a < kMetricArrays; ++a) {
+    k_to_f32<<<152 * 8, 256, 0, h->st>>>(h->met + a * n, tmp, n);
+    CK(cudaMemcpyAsync((float*)h->met + a * n, tmp, n * sizeof(float), cudaMemcpyDeviceToDevice, h->st));
+  }
+  CK(cudaMemcpyAsync(h->met + (kMetricArrays - 1) * n, vol64, n * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
+  CK(cudaGetLastError());
+  return wait_stream(h);
+}
+
 // Metric mode: upload the node coordinates, compute the FP64 metric on the
 // device, reject meshes with a non-positive interior cell volume.
 static int setup_metric(Handle* h, const double* const xyz[3]) {
@@ -739,6 +765,7 @@ static int setup_metric(Handle* h, const double* const xyz[3]) {
   }
   cudaFree(dn);
   if (rc) return rc;
+  if (h->fp32 && (rc = metric_to_fp32(h)) != MHD_OK) return rc;
   if (!(vmin > 0.0)) return fail(MHD_E_ARG, "mapped grid has a non-positive cell volume");
   // the Dev views were carved before the metric existed: refresh them
   if (h->fp32) carve<float>(h, h->df, (char*)h->buf);

@@ -913,15 +913,15 @@ __device__ __forceinline__ long long idx3(const Geom& g, int i, int j, int k) {
 // B = sum_a (Phi_a averaged over the two a-faces / V) e_a, e_a the cell's
 // edge vector along a (the oracle's get_bxyz_metric, in its operand order).
 template <typename T>
-__device__ __forceinline__ void cell_b_metric(const Metric& m, long long c, T lo0, T hi0, T lo1, T hi1, T lo2,
+__device__ __forceinline__ void cell_b_metric(const Metric<T>& m, long long c, T lo0, T hi0, T lo1, T hi1, T lo2,
                                               T hi2, T& bx, T& by, T& bz) {
-  const T V = (T)m.vol[c], rV = (T)m.rvol[c];
+  const T V = m.vol[c], rV = m.rvol[c];
   const T p0 = Ops<T>::dw(T(0.5) * (hi0 + lo0), V, rV);
   const T p1 = Ops<T>::dw(T(0.5) * (hi1 + lo1), V, rV);
   const T p2 = Ops<T>::dw(T(0.5) * (hi2 + lo2), V, rV);
-  bx = p0 * (T)m.eb[0][0][c] + p1 * (T)m.eb[1][0][c] + p2 * (T)m.eb[2][0][c];
-  by = p0 * (T)m.eb[0][1][c] + p1 * (T)m.eb[1][1][c] + p2 * (T)m.eb[2][1][c];
-  bz = p0 * (T)m.eb[0][2][c] + p1 * (T)m.eb[1][2][c] + p2 * (T)m.eb[2][2][c];
+  bx = p0 * m.eb[0][0][c] + p1 * m.eb[1][0][c] + p2 * m.eb[2][0][c];
+  by = p0 * m.eb[0][1][c] + p1 * m.eb[1][1][c] + p2 * m.eb[2][1][c];
+  bz = p0 * m.eb[0][2][c] + p1 * m.eb[1][2][c] + p2 * m.eb[2][2][c];
 }
 
 // vf = |v| + |B| / sqrt(rho) of get_eijk_LFM (1766), b2 = |B|^2 (in FP64 with
@@ -991,7 +991,7 @@ __device__ __forceinline__ T cell_dt(const Dev<T>& d, int c, int i, int j, int k
   const T vcfl = cfl_speed<M>(d.gam, r0, p0, u, v, w, a * a + b * b + cc * cc);
   T dt;
   if (M)  // metric mode: 1/dx_a -> |mean area vector of the a-faces| / V
-    dt = O::dv(d.cfl, O::dw(vcfl * (T)d.m.sa[c], (T)d.m.vol[c], (T)d.m.rvol[c]));
+    dt = O::dv(d.cfl, O::dw(vcfl * d.m.sa[c], d.m.vol[c], d.m.rvol[c]));
   else
     dt = O::dv(d.cfl, O::dc(vcfl, d.wx[i], d.rwx[i]) + O::dc(vcfl, d.wy[j], d.rwy[j]) +
                           O::dc(vcfl, d.wz[k], d.rwz[k]));
@@ -1224,7 +1224,7 @@ template <> struct Moments<double> {
 template <> struct Moments<float> {
   // erfc(z) for z >= 0 (Numerical Recipes erfcc)
   static __device__ __forceinline__ float erfc_pos(float z) {
-    float t = __fdividef(1.0f, fmaf(0.5f, z, 1.0f));
+    float t = p2::rcp1(fmaf(0.5f, z, 1.0f));
     float q = fmaf(t, 0.17087277f, -0.82215223f);
     q = fmaf(t, q, 1.48851587f);
     q = fmaf(t, q, -1.13520398f);
@@ -1234,7 +1234,7 @@ template <> struct Moments<float> {
     q = fmaf(t, q, 0.37409196f);
     q = fmaf(t, q, 1.00002368f);
     q = fmaf(t, q, -1.26551223f);
-    return t * __expf(fmaf(-z, z, q));
+    return t * p2::ex21(1.4426950408889634f * fmaf(-z, z, q));
   }
   // 0.5 erfc(-s x) for the left (s=+1) or 0.5 erfc(x) for the right state
   static __device__ __forceinline__ float half_erfc(float x, bool left) {
@@ -1243,17 +1243,17 @@ template <> struct Moments<float> {
     return direct ? h : 1.0f - h;
   }
   static __device__ __forceinline__ void hydro(float lam, float vn, bool left, float& v0, float& v1) {
-    float ra = rsqrtf(lam);
+    float ra = p2::rsq1(lam);
     float a = lam * ra;
     v0 = half_erfc(a * vn, left);
-    float b = (0.5f * 0.56418958354775628f) * ra * __expf(-lam * vn * vn);
+    float b = (0.5f * 0.56418958354775628f) * ra * p2::ex21(1.4426950408889634f * (-lam * vn * vn));
     v1 = left ? fmaf(vn, v0, b) : fmaf(vn, v0, -b);
   }
   static __device__ __forceinline__ float mag(float lam, float vn, bool left) {
-    float a = lam * rsqrtf(lam);
+    float a = lam * p2::rsq1(lam);
     return half_erfc(a * vn, left);
   }
-  static __device__ __forceinline__ float div(float a, float b) { return __fdividef(a, b); }
+  static __device__ __forceinline__ float div(float a, float b) { return a * p2::rcp1(b); }
 };
 
 // ------------------------------------------------ FP32 packed-pair arithmetic
@@ -1481,8 +1481,8 @@ __device__ __forceinline__ void face_flux_n(const T* l, const T* r, const Dev<T>
 template <typename T, int D, bool M>
 __device__ __forceinline__ void any_face_flux(const Dev<T>& d, long long c, const T* L, const T* R, T* out) {
   if (M) {
-    const T n[3] = {(T)d.m.nrm[D][0][c], (T)d.m.nrm[D][1][c], (T)d.m.nrm[D][2][c]};
-    face_flux_n<T>(L, R, d, n, (T)d.m.am[D][c], out);
+    const T n[3] = {d.m.nrm[D][0][c], d.m.nrm[D][1][c], d.m.nrm[D][2][c]};
+    face_flux_n<T>(L, R, d, n, d.m.am[D][c], out);
   } else {
     face_flux<D>(L, R, d, out);
   }
@@ -1689,7 +1689,7 @@ __device__ __forceinline__ void cell_update_vals(const Dev<T>& d, int c, int cd,
   const T gm1 = d.gam - T(1);
   T dv[8];
   if (M) {
-    const T V = (T)d.m.vol[c], rV = (T)d.m.rvol[c];
+    const T V = d.m.vol[c], rV = d.m.rvol[c];
 #pragma unroll
     for (int q = 0; q < 8; ++q) dv[q] = Ops<T>::dw(du[q] + dF[q], V, rV);
   } else {
@@ -2091,7 +2091,7 @@ __device__ __forceinline__ T emf_value(const Dev<T>& d, I c, T v1av, T v2av, T b
   const T b2u = ge0(v1av) ? b2l : b2r;
   const T e = -v1av * b2u + v2av * b1u;
   if (M)  // E.dl: g_e * (convective term) + eta |dl_e| * (resistive term)
-    return (T)d.m.ge[E][c] * e + eta * (T)d.m.dl[E][c] * (b1l + b2r - b1r - b2l);
+    return d.m.ge[E][c] * e + eta * d.m.dl[E][c] * (b1l + b2r - b1r - b2l);
   return e + eta * (b1l + b2r - b1r - b2l);
 }
 
@@ -3061,15 +3061,15 @@ __global__ void k_metric_prep(Dev<T> d, Inp<T> in) {
   const int k = blockIdx.z;
   if (i > g.nx || j > g.ny || k > g.nz) return;
   const long long c = idx3<T>(g, i, j, k);
-  const Metric& m = d.m;
+  const Metric<T>& m = d.m;
   if (i < g.nx && j < g.ny && k < g.nz) {
     const T u = in.vx[c], v = in.vy[c], w = in.vz[c];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) d.mw[a][c] = u * (T)m.nb[a][0][c] + v * (T)m.nb[a][1][c] + w * (T)m.nb[a][2][c];
+    for (int a = 0; a < 3; ++a) d.mw[a][c] = u * m.nb[a][0][c] + v * m.nb[a][1][c] + w * m.nb[a][2][c];
   }
-  if (j < g.ny && k < g.nz) d.mbn[0][c] = Ops<T>::dv(in.bi[c], (T)m.am[0][c]);
-  if (i < g.nx && k < g.nz) d.mbn[1][c] = Ops<T>::dv(in.bj[c], (T)m.am[1][c]);
-  if (i < g.nx && j < g.ny) d.mbn[2][c] = Ops<T>::dv(in.bk[c], (T)m.am[2][c]);
+  if (j < g.ny && k < g.nz) d.mbn[0][c] = Ops<T>::dv(in.bi[c], m.am[0][c]);
+  if (i < g.nx && k < g.nz) d.mbn[1][c] = Ops<T>::dv(in.bj[c], m.am[1][c]);
+  if (i < g.nx && j < g.ny) d.mbn[2][c] = Ops<T>::dv(in.bk[c], m.am[2][c]);
 }
 
 // ------------------------------------------------------------------ update
@@ -3469,7 +3469,7 @@ __global__ void k_diag_partial(Dev<T> d, double* part) {
     int j = (int)(r % g.ny0) + g.ng;
     int k = (int)(r / g.ny0) + g.ng;
     long long c = idx3<T>(g, i, j, k);
-    double dv = M ? d.m.vol[c] : d.dx[i] * d.dy[j] * d.dz[k];
+    double dv = M ? d.m.vol64[c] : d.dx[i] * d.dy[j] * d.dz[k];
     double rr = d.rho[c], u = d.vx[c], v = d.vy[c], w = d.vz[c], pp = d.p[c];
     double a = d.bx[c], b = d.by[c], cc = d.bz[c];
     ms = dd_add(ms, DD{rr * dv, 0.0});

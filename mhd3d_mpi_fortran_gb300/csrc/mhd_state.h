@@ -45,23 +45,25 @@ struct Scal {
 // later stages' combines
 constexpr int FORM_SAVE = -2;
 
-// Curvilinear metric (metric mode only; FP64 in both precisions), computed
-// once on the device from the node coordinates.  Same padded layout as the
-// fields: a face at the index of the cell on its high side (the cell whose
-// low face it is), an edge at the index of its upper cell.
+// Curvilinear metric (metric mode only), computed once on the device in FP64
+// from the node coordinates and held in the precision the step reads it in.  Same
+// padded layout as the fields: a face at the index of the cell on its high side
+// (the cell whose low face it is), an edge at the index of its upper cell.
+template <typename T>
 struct Metric {
-  const double* nrm[3][3];  // unit normals of the low faces [face axis][component]
-  const double* am[3];      // face area magnitudes |A|
-  const double* vol;        // cell volumes V
-  const double* rvol;       // 1/V
-  const double* eb[3][3];   // cell edge vectors (face-centroid differences) [axis][component]
-  const double* nb[3][3];   // mean unit normal of the two a-faces of a cell [axis][component]
-  const double* sa;         // sum over a of |mean area vector of the a-faces| (CFL)
-  const double* ge[3];      // per edge family: g_e = |A1|_e |A2|_e / Vbar_e
-  const double* dl[3];      // per edge family: edge length
+  const T* nrm[3][3];       // unit normals of the low faces [face axis][component]
+  const T* am[3];           // face area magnitudes |A|
+  const T* vol;             // cell volumes V
+  const T* rvol;            // 1/V
+  const T* eb[3][3];        // cell edge vectors (face-centroid differences) [axis][component]
+  const T* nb[3][3];        // mean unit normal of the two a-faces of a cell [axis][component]
+  const T* sa;              // sum over a of |mean area vector of the a-faces| (CFL)
+  const T* ge[3];           // per edge family: g_e = |A1|_e |A2|_e / Vbar_e
+  const T* dl[3];           // per edge family: edge length
+  const double* vol64;      // V in FP64 (diagnostics)
 };
 
-// Raw device arrays the geometry kernels write (the const views above alias them).
+// Raw device arrays the geometry kernels write.
 struct MetricOut {
   double *nrm[3][3], *am[3], *vol, *rvol, *eb[3][3], *nb[3][3], *sa, *ge[3], *dl[3];
 };
@@ -107,7 +109,7 @@ struct Dev {
   unsigned int* counter;
   // metric mode: geometry, and the per-stage normal velocities w^a (cells)
   // and face-normal field b_a = Phi_a/|A_a| (faces) of the EMF
-  Metric m;
+  Metric<T> m;
   T* mw[3];
   T* mbn[3];
   // launch shapes (host side only): y/z face-tile length and EMF shape (ei
