@@ -263,6 +263,12 @@ inline void set_widths(Handle* h, Dev<float>& d) {
   d.rwx = h->geoT + n; d.rwy = h->geoT + n + g.nx; d.rwz = h->geoT + n + g.nx + g.ny;
 }
 
+// Do the streamed EMF families of this grid fill the chip?
+bool emf_streams(const Geom& g) {
+  const int cols = emf_stream_cols(0, g);
+  return (long long)cols * emf_stream_segs(g.nz0, emf_stream_seg(0, g, cols)) >= 256;
+}
+
 template <typename T>
 void carve(Handle* h, Dev<T>& d, char* base) {
   const Geom& g = h->g;
@@ -309,6 +315,7 @@ void carve(Handle* h, Dev<T>& d, char* base) {
   d.tile_ey = h->tile_ey;
   for (int D = 1; D < 3; ++D) d.seg[D - 1] = sweep_seg(D, g, sweep_cols(D, g));
   for (int E = 0; E < 3; ++E) d.eseg[E] = emf_stream_seg(E, g, emf_stream_cols(E, g));
+  d.ctk = ct_planes((long long)((g.nx0 + 31) / 32) * ((g.ny0 + 7) / 8) * g.nz0);
   for (int a = 0; a < 3; ++a) {
     d.mw[a] = h->metric ? next() : nullptr;
     d.mbn[a] = h->metric ? next() : nullptr;
@@ -597,9 +604,7 @@ static int create_handle(const mhd_params* prm, const double* dx, const double* 
   Geom& g = h->g;
   g.nx0 = prm->nx0; g.ny0 = prm->ny0; g.nz0 = prm->nz0;
   {
-    const int cols = emf_stream_cols(0, g);
-    const long long eb = (long long)cols * emf_stream_segs(g.nz0, emf_stream_seg(0, g, cols));
-    h->tile_ey = (h->fp32 && !metric) ? (eb >= 256 ? kEmfStream : 8) : h->fp32 ? 8 : 4;
+h->tile_ey = (h->fp32 && !metric) ? (emf_streams(g) ? kEmfStream : 8) : h->fp32 ? 8 : 4;
   }
   g.nord = prm->nord; g.ng = prm->nord / 2;
   g.nx = g.nx0 + g.nord; g.ny = g.ny0 + g.nord; g.nz = g.nz0 + g.nord;
@@ -1251,13 +1256,15 @@ static bool batchable(Handle* const* hs, int n) {
 // launch holds the blocks of all of them.  Returns the blocks of its ei streams.
 template <typename T>
 static long long batch_segments(std::vector<Dev<T>>& ds) {
-  long long cols[5] = {0, 0, 0, 0, 0}, eb = 0;
+  long long cols[5] = {0, 0, 0, 0, 0}, eb = 0, ct = 0;
   for (const Dev<T>& d : ds) {
     for (int D = 1; D < 3; ++D) cols[D - 1] += sweep_cols(D, d.g);
     for (int E = 0; E < 3; ++E) cols[2 + E] += emf_stream_cols(E, d.g);
+    ct += (long long)((d.g.nx0 + 31) / 32) * ((d.g.ny0 + 7) / 8) * d.g.nz0;
   }
   for (long long& c : cols) c = std::min<long long>(c, INT32_MAX / 2);
   for (Dev<T>& d : ds) {
+    d.ctk = ct_planes(ct);
     for (int D = 1; D < 3; ++D) d.seg[D - 1] = sweep_seg(D, d.g, (int)cols[D - 1]);
     for (int E = 0; E < 3; ++E) d.eseg[E] = emf_stream_seg(E, d.g, (int)cols[2 + E]);
     eb += (long long)emf_stream_cols(0, d.g) * emf_stream_segs(d.g.nz0, d.eseg[0]);

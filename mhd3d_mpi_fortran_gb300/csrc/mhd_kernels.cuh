@@ -926,9 +926,12 @@ __device__ __forceinline__ void cell_b_metric(const Metric<T>& m, long long c, T
 
 // vf = |v| + |B| / sqrt(rho) of get_eijk_LFM (1766), b2 = |B|^2 (in FP64 with
 // the reference's roundings: the edge EMF multiplies the jumps of B by it).
+// FP32: the contraction spelled out, so that every kernel that fills vf gives the same bits.
+__device__ __forceinline__ float sq3(float a, float b, float c) { return fmaf(c, c, fmaf(a, a, __fmul_rn(b, b))); }
+__device__ __forceinline__ double sq3(double a, double b, double c) { return a * a + b * b + c * c; }
 template <typename T>
 __device__ __forceinline__ T vf_val(T u, T v, T w, T b2, T r0) {
-  return sq(u * u + v * v + w * w) + sq(b2 / r0);
+  return sq(sq3(u, v, w)) + sq(b2 / r0);
 }
 // get_bxyz over all cells (incl. ghosts) and vf = |v| + |B|/sqrt(rho).
 template <typename T, bool M>
@@ -952,7 +955,7 @@ __global__ void k_bxyz_vf(Dev<T> d, int want_vf) {
   d.bz[c] = bz;
   if (want_vf) {
     T u = d.vx[c], v = d.vy[c], w = d.vz[c];
-    d.vf[c] = vf_val(u, v, w, bx * bx + by * by + bz * bz, d.rho[c]);
+    d.vf[c] = vf_val(u, v, w, sq3(bx, by, bz), d.rho[c]);
   }
 }
 
@@ -1171,26 +1174,63 @@ __global__ void k_save_prev(Dev<T> d) {
 
 // advance_predictor_ab (3821-3840): Xh = X + tau/tau0/2*(X-Xp), then Xp = X;
 // also vf of the predicted state.
+//
+// 23 arrays read and 23 written: bytes bound it (0.87 GB at 160^3, 128 us).  A
+// thread takes 16 bytes of every array, all of them loaded before the first store,
+// and the padding of the rows is left out (a sixth at nx = 168).
+// 160^3 FP32: 186 -> 143 us.
+template <typename T> struct Vec16 {
+  static constexpr int W = 16 / sizeof(T);
+  uint4 u;
+  __device__ __forceinline__ void load(const T* p) { u = *reinterpret_cast<const uint4*>(p); }
+  __device__ __forceinline__ T get(int i) const {
+    if constexpr (sizeof(T) == 4) return __uint_as_float((&u.x)[i]);
+    else return __hiloint2double((int)(&u.x)[2 * i + 1], (int)(&u.x)[2 * i]);
+  }
+  __device__ __forceinline__ void put(int i, T x) {
+    if constexpr (sizeof(T) == 4) {
+      (&u.x)[i] = __float_as_uint(x);
+    } else {
+      (&u.x)[2 * i] = (unsigned)__double2loint(x);
+      (&u.x)[2 * i + 1] = (unsigned)__double2hiint(x);
+    }
+  }
+  __device__ __forceinline__ void store(T* p) const { *reinterpret_cast<uint4*>(p) = u; }
+};
 template <typename T>
-__global__ void k_predictor_ab(Dev<T> d) {
-  long long n = d.g.vol;
-  T cf = (T)d.sc->ab_coef;
-  T* x[11] = {d.rho, d.vx, d.vy, d.vz, d.p, d.bi, d.bj, d.bk, d.bx, d.by, d.bz};
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n;
-       c += (long long)gridDim.x * blockDim.x) {
+__global__ void __launch_bounds__(256, 2) k_predictor_ab(Dev<T> d) {
+  typedef Vec16<T> V;
+  const Geom& g = d.g;
+  const int nq = (g.nx + V::W) / V::W, u = blockIdx.x * blockDim.x + threadIdx.x;  // x = 0 .. nx of a row
+  if (u >= nq * g.py * g.pz) return;
+  const int c = u / nq * g.px + u % nq * V::W;
+  const T cf = (T)d.sc->ab_coef;
+  const T* x[11] = {d.rho, d.vx, d.vy, d.vz, d.p, d.bi, d.bj, d.bk, d.bx, d.by, d.bz};
+  V xv[11], xp[11], vf;
+#pragma unroll
+  for (int a = 0; a < 11; ++a) {
+    xv[a].load(x[a] + c);
+    xp[a].load(d.q[a] + c);
+  }
+#pragma unroll
+  for (int i = 0; i < V::W; ++i) {
     T hv[11];
 #pragma unroll
     for (int a = 0; a < 11; ++a) {
-      T xv = x[a][c], xp = d.q[a][c];
-      hv[a] = xv + cf * (xv - xp);
-      d.h[a][c] = hv[a];
-      d.q[a][c] = xv;
+      hv[a] = xv[a].get(i) + cf * (xv[a].get(i) - xp[a].get(i));
+      xp[a].put(i, hv[a]);
     }
-    T rr = hv[0];
-    d.vf[c] = (rr > T(0)) ? sq(hv[1] * hv[1] + hv[2] * hv[2] + hv[3] * hv[3]) +
+    const T rr = hv[0];
+    vf.put(i, (rr > T(0)) ? sq(hv[1] * hv[1] + hv[2] * hv[2] + hv[3] * hv[3]) +
                                 sq((hv[8] * hv[8] + hv[9] * hv[9] + hv[10] * hv[10]) / rr)
-                          : T(0);
+                          : T(0));
   }
+#pragma unroll
+  for (int a = 0; a < 11; ++a) {
+    xp[a].store(d.h[a] + c);
+    xv[a].store(d.q[a] + c);
+  }
+  vf.store(d.vf + c);
 }
 
 // ------------------------------------------------------------------ fluxes
@@ -3274,7 +3314,7 @@ __device__ __forceinline__ T fill_bxyz_elem(const Dev<T>& d, int4 bb, int want_v
     d.bz[c] = bz;
     if (want_vf || want_dt) {
       const T u = d.vx[c], v = d.vy[c], w = d.vz[c], r0 = d.rho[c];
-      if (want_vf) d.vf[c] = vf_val(u, v, w, bx * bx + by * by + bz * bz, r0);
+      if (want_vf) d.vf[c] = vf_val(u, v, w, sq3(bx, by, bz), r0);
       if (want_dt) return cell_dt<T, M>(d, c, i, j, k, r0, d.p[c], u, v, w, bx, by, bz, st);
     }
     return T(INFINITY);
@@ -3371,66 +3411,110 @@ __global__ void __launch_bounds__(256, pass_min_blocks(B))
 // face B as U^n of the later combines; dt_next (the last stage) accumulates
 // the CFL dt and status of the new cells for the next step, as k_cfl would
 // compute them at its start.
+//
+// Bytes bound it (20 arrays a cell), and by one cell a thread it waited on them:
+// 24 of 31 cycles a warp on loads at 44 % of DRAM, ei, ej and bk fetched again by
+// the next plane, their face computed twice.  A thread now walks Dev::ctk cells up
+// z: the upper z face and edges of a cell are the lower ones of the next, and
+// the next cell's inputs are loaded before this one's stores.  RK stage: 256^3
+// 2285 -> 2202 us, 32 grids in a batch 2583 -> 2397.
+//
+// A sum that no product before it is contracted into (the faces as they are stored).
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return a + b; }
+template <typename T>
+struct CtIn {  // what cell c reads beyond the carried lower z face and edges
+  T ek00, ek10, ek01, ek11, ei0, ei1, ej0, ej1, bi0, bi1, bj0, bj1, bk;  // e*0, e*1, bk: at the upper z face
+  T qi0, qi1, qj0, qj1, qk;
+  T u, v, w, r, p;
+  __device__ __forceinline__ void load(const Dev<T>& d, int c, int px, int pl, bool comb, bool prim, bool dt) {
+    const T *ei = d.E[0], *ej = d.E[1], *ek = d.E[2];
+    ek00 = ek[c]; ek10 = ek[c + 1]; ek01 = ek[c + px]; ek11 = ek[c + 1 + px];
+    ei0 = ei[c + pl]; ei1 = ei[c + px + pl];
+    ej0 = ej[c + pl]; ej1 = ej[c + 1 + pl];
+    bi0 = d.bi[c]; bi1 = d.bi[c + 1];
+    bj0 = d.bj[c]; bj1 = d.bj[c + px];
+    bk = d.bk[c + pl];
+    if (comb) {
+      qi0 = d.q[5][c]; qi1 = d.q[5][c + 1];
+      qj0 = d.q[6][c]; qj1 = d.q[6][c + px];
+      qk = d.q[7][c + pl];
+    }
+    if (prim) { u = d.ovx[c]; v = d.ovy[c]; w = d.ovz[c]; r = d.orho[c]; }
+    if (dt) p = d.op[c];
+  }
+};
 template <typename T, bool B>
-__global__ void __launch_bounds__(256, pass_min_blocks(B))
-    k_ct_fill(KArg<T, B> ka, int form, T cw, T den, int want_vf, int dt_next) {
+__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 3) k_ct_fill(KArg<T, B> ka, int form, T cw, T den, int want_vf, int dt_next) {
   const int4 bb = ka.blk();
   const auto& d = ka.dev(bb);
   const Geom& g = d.g;
   const int i = g.ng + bb.y * 32 + (threadIdx.x & 31);
   const int j = g.ng + bb.z * 8 + (threadIdx.x >> 5);
-  const int k = g.ng + bb.w;
+  const int k0 = g.ng + bb.w * d.ctk, k1 = min(k0 + d.ctk, g.ng + g.nz0);
   const bool save = form == FORM_SAVE, want_dt = dt_next != 0;
   T m = T(INFINITY);
   unsigned st = 0;
   if (i < g.ng + g.nx0 && j < g.ng + g.ny0) {
     const int px = g.px, pl = (int)g.plane;
-    const int c = i + px * j + pl * k;
+    int c = i + px * j + pl * k0;
     const T tau = step_tau<T>(d.sc);
-    const T dx = d.wx[i], dy = d.wy[j], dz = d.wz[k];
-    const T rx = d.rwx[i], ry = d.rwy[j], rz = d.rwz[k];
-    const T *ei = d.E[0], *ej = d.E[1], *ek = d.E[2];
+    const T dx = d.wx[i], dy = d.wy[j];
+    const T rx = d.rwx[i], ry = d.rwy[j];
     typedef Ops<T> O;
-    auto new_bi = [&](int f) {
-      T b = d.bi[f] - tau * (O::dc(ek[f + px] - ek[f], dy, ry) - O::dc(ej[f + pl] - ej[f], dz, rz));
-      return form >= 0 ? comb(form, cw, d.q[5][f], b, den) : b;
+    // a face from its old value, U^n and the four edges around it (advance_bijk + combine)
+    auto face = [&](T b, T q, T e1, T w1, T r1, T e2, T w2, T r2) {
+      T n;
+      if constexpr (std::is_same<T, float>::value)  // the contraction spelled out: a face has the same bits as a low and as a high one
+        n = fmaf(-tau, fmaf(e1, r1, -(e2 * r2)), b);
+      else
+        n = b - tau * (O::dc(e1, w1, r1) - O::dc(e2, w2, r2));
+      return form >= 0 ? comb(form, cw, q, n, den) : n;
     };
-    auto new_bj = [&](int f) {
-      T b = d.bj[f] - tau * (O::dc(ei[f + pl] - ei[f], dz, rz) - O::dc(ek[f + 1] - ek[f], dx, rx));
-      return form >= 0 ? comb(form, cw, d.q[6][f], b, den) : b;
-    };
-    auto new_bk = [&](int f) {
-      T b = d.bk[f] - tau * (O::dc(ej[f + 1] - ej[f], dx, rx) - O::dc(ei[f + px] - ei[f], dy, ry));
-      return form >= 0 ? comb(form, cw, d.q[7][f], b, den) : b;
-    };
-    const bool lx = i == g.ng + g.nx0 - 1, ly = j == g.ng + g.ny0 - 1, lz = k == g.ng + g.nz0 - 1;
-    if (save) {  // face B^n of the step (this first stage's input) for the later combines
-      d.q[5][c] = d.bi[c];
-      d.q[6][c] = d.bj[c];
-      d.q[7][c] = d.bk[c];
-      if (lx) d.q[5][c + 1] = d.bi[c + 1];
-      if (ly) d.q[6][c + px] = d.bj[c + px];
-      if (lz) d.q[7][c + pl] = d.bk[c + pl];
-    }
-    const T bil = new_bi(c), bih = new_bi(c + 1);
-    const T bjl = new_bj(c), bjh = new_bj(c + px);
-    const T bkl = new_bk(c), bkh = new_bk(c + pl);
-    d.obi[c] = bil;
-    d.obj[c] = bjl;
-    d.obk[c] = bkl;
-    if (lx) d.obi[c + 1] = bih;
-    if (ly) d.obj[c + px] = bjh;
-    if (lz) d.obk[c + pl] = bkh;
-    const T bx = T(0.5) * (bih + bil);
-    const T by = T(0.5) * (bjh + bjl);
-    const T bz = T(0.5) * (bkh + bkl);
-    d.bx[c] = bx;
-    d.by[c] = by;
-    d.bz[c] = bz;
-    if (want_vf || want_dt) {
-      const T u = d.ovx[c], v = d.ovy[c], w = d.ovz[c], r0 = d.orho[c];
-      if (want_vf) d.vf[c] = vf_val(u, v, w, bx * bx + by * by + bz * bz, r0);
-      if (want_dt) m = cell_dt<T, false>(d, c, i, j, k, r0, d.op[c], u, v, w, bx, by, bz, st);
+    const bool lx = i == g.ng + g.nx0 - 1, ly = j == g.ng + g.ny0 - 1;
+    T ei0 = d.E[0][c], ei1 = d.E[0][c + px], ej0 = d.E[1][c], ej1 = d.E[1][c + 1], bk = d.bk[c];
+    const T qk = form >= 0 ? d.q[7][c] : T(0);
+    CtIn<T> a, nx;
+    a.load(d, c, px, pl, form >= 0, want_vf || want_dt, want_dt);
+    T bkl = face(bk, qk, ej1 - ej0, dx, rx, ei1 - ei0, dy, ry);
+    for (int k = k0; k < k1; ++k, c += pl) {
+      if (k + 1 < k1) nx.load(d, c + pl, px, pl, form >= 0, want_vf || want_dt, want_dt);
+      const T dz = d.wz[k], rz = d.rwz[k];
+      const bool lz = k == g.ng + g.nz0 - 1;
+      if (save) {  // face B^n of the step (this first stage's input) for the later combines
+        d.q[5][c] = a.bi0;
+        d.q[6][c] = a.bj0;
+        d.q[7][c] = bk;
+        if (lx) d.q[5][c + 1] = a.bi1;
+        if (ly) d.q[6][c + px] = a.bj1;
+        if (lz) d.q[7][c + pl] = a.bk;
+      }
+      const T bil = face(a.bi0, a.qi0, a.ek01 - a.ek00, dy, ry, a.ej0 - ej0, dz, rz);
+      const T bih = face(a.bi1, a.qi1, a.ek11 - a.ek10, dy, ry, a.ej1 - ej1, dz, rz);
+      const T bjl = face(a.bj0, a.qj0, a.ei0 - ei0, dz, rz, a.ek10 - a.ek00, dx, rx);
+      const T bjh = face(a.bj1, a.qj1, a.ei1 - ei1, dz, rz, a.ek11 - a.ek01, dx, rx);
+      const T bkh = face(a.bk, a.qk, a.ej1 - a.ej0, dx, rx, a.ei1 - a.ei0, dy, ry);
+      d.obi[c] = bil;
+      d.obj[c] = bjl;
+      d.obk[c] = bkl;
+      if (lx) d.obi[c + 1] = bih;
+      if (ly) d.obj[c + px] = bjh;
+      if (lz) d.obk[c + pl] = bkh;
+      const T bx = T(0.5) * add_rn(bih, bil);
+      const T by = T(0.5) * add_rn(bjh, bjl);
+      const T bz = T(0.5) * add_rn(bkh, bkl);
+      d.bx[c] = bx;
+      d.by[c] = by;
+      d.bz[c] = bz;
+      if (want_vf) d.vf[c] = vf_val(a.u, a.v, a.w, sq3(bx, by, bz), a.r);
+      if (want_dt) {
+        const T dt = cell_dt<T, false>(d, c, i, j, k, a.r, a.p, a.u, a.v, a.w, bx, by, bz, st);
+        m = (dt < m) ? dt : m;
+      }
+      ei0 = a.ei0; ei1 = a.ei1; ej0 = a.ej0; ej1 = a.ej1;
+      bk = a.bk;
+      bkl = bkh;
+      a = nx;
     }
   }
   if (want_dt) dt_next_accumulate(d.sc, m, st);
@@ -3584,7 +3668,7 @@ void Launch<T, M>::ct_fill(const Dev<T>& d, int form, double c, double den, bool
     static PerDevice pref_ct, pref_fill;
     prefer_carveout(k_ct_fill<T, false>, 0, pref_ct);
     prefer_carveout(k_fill_bxyz<T, false, false>, 0, pref_fill);
-    k_ct_fill<T, false><<<dim3(fs.nbx, fs.nby, d.g.nz0), 256, 0, st>>>(one(d), form, (T)c, (T)den,
+    k_ct_fill<T, false><<<dim3(fs.nbx, fs.nby, (d.g.nz0 + d.ctk - 1) / d.ctk), 256, 0, st>>>(one(d), form, (T)c, (T)den,
                                                                         want_vf ? 1 : 0, dt_next ? 1 : 0);
     k_fill_bxyz<T, false, false><<<(fs.nshell + 255) / 256, 256, 0, st>>>(one(other_half(d)), want_vf ? 1 : 0, 1,
                                                                          dt_next ? 1 : 0);
@@ -3617,7 +3701,8 @@ void Launch<T, M>::save_prev(const Dev<T>& d, cudaStream_t st) {
 
 template <typename T, bool M>
 void Launch<T, M>::predictor_ab(const Dev<T>& d, cudaStream_t st) {
-  k_predictor_ab<T><<<152 * 8, 256, 0, st>>>(d);
+  const int n = (d.g.nx + Vec16<T>::W) / Vec16<T>::W * d.g.py * d.g.pz;
+  k_predictor_ab<T><<<(n + 255) / 256, 256, 0, st>>>(d);
 }
 
 template <typename T, int RECON, bool M>
@@ -3892,6 +3977,7 @@ void Launch<T, M>::emf(const Dev<T>& d, const Inp<T>& in0, cudaStream_t st) {
   }
   if (d.recon == R_PDM) {
     Prm<T> P = prm_of(d);
+    // (the metric mode keeps the tiles: beside the streams its face tiles ran a third slower)
     if constexpr (std::is_same<T, float>::value && !M) {
       if (d.tile_ey == kEmfStream) {
         emf_pdm_stream<T, M>(d, in, P, st);
@@ -3950,7 +4036,7 @@ dim3 Batch<T>::dims(int fam, const Dev<T>& d, int td, int ey) {
     case BF_EMF_R: return stream ? dim3(EmfRows(g).blocks(), 1, 1) : dim3(0, 0, 0);
     case BF_CT: {  // k_ct_fill: the fill's interior tiles
       const FillShape fs(g);
-      return dim3(fs.nbx, fs.nby, g.nz0);
+      return dim3(fs.nbx, fs.nby, (g.nz0 + d.ctk - 1) / d.ctk);
     }
     default: return dim3((FillShape(g).nshell + 255) / 256, 1, 1);  // BF_FILL: the shell of the new half
   }

@@ -117,6 +117,7 @@ struct Dev {
   // PDM path
   int tile_td, tile_ey;
   int seg[2];        // cells per column segment of the y / z sweeps (sweep_seg)
+  int ctk;           // cells up z per thread of the CT pass (ct_planes)
   int eseg[3];       // edges per segment of the streamed EMF families (emf_stream_seg)
   int emf;           // edge EMF scheme: 0 LFM, 1 Yee
   T* ye[12];         // Yee split electric fields, [x, y, z edges][pp, np, pn, nn] (emf = 1)
@@ -249,6 +250,16 @@ constexpr int kEmfStream = 1;   // EMF-shape value of the slice-streamed EMF fam
 #ifndef MHD_EMF_SEG_MIN
 #define MHD_EMF_SEG_MIN 16
 #endif
+// Cells up z per thread of the CT pass, for a launch of `blocks` blocks at one cell
+// each (of all the grids of a batch): up to 8 while 256 blocks remain.  Stage in us
+// at 1, 2, 4, 8 cells: 32^3 (128 blocks) 25.3 26.1 27.5 30.7; 64^3 (1024) 58.2
+// 58.1 57.2 59.7; 113x75x58 (2320) 92.8 91.5 91.6 90.4; 256^3 2288 2230 2209 2202
+// (16: 2198).
+inline int ct_planes(long long blocks) {
+  int n = 1;
+  while (n < 8 && blocks / (2 * n) >= 256) n *= 2;
+  return n;
+}
 // Blocks of edge columns of streamed family E of a grid.
 inline int emf_stream_cols(int E, const Geom& g) {
   return ((g.nx0 + 31) / 32) * (((E == 2 ? g.nz0 : g.ny0) + MHD_EMF_NW - 1) / MHD_EMF_NW);

@@ -60,3 +60,21 @@ def test_batched_steps_fold_dt_as_single_steps(precision, stepop):
             assert np.array_equal(fa[k], fb[k]), k
         a.close()
         b.close()
+
+
+@pytest.mark.parametrize("precision", [FP32, FP64])
+@pytest.mark.parametrize("shape", [(16, 16, 5), (33, 9, 260), (70, 50, 35), (96, 96, 63)])
+def test_cells_up_z_leave_consistent_faces(shape, precision):
+    """CT passes of 1 to 8 cells a thread, with a ragged last walk: the cell B they
+    leave is the mean of the stored faces bit for bit (a face computed as one
+    cell's high side and the next one's low side is the same value)."""
+    s = state(*shape, 8, 7)
+    with MHDSolver(Params(*shape, stepop=STEP_RK3, precision=precision, tau=1e-4), s) as g:
+        g.step(2)
+        f = g.fetch()
+    t = np.float32 if precision == FP32 else np.float64
+    f = {k: v.astype(t) for k, v in f.items()}
+    half = t(0.5)
+    assert np.array_equal(f["bx"], half * (f["bi"][1:] + f["bi"][:-1]))
+    assert np.array_equal(f["by"], half * (f["bj"][:, 1:] + f["bj"][:, :-1]))
+    assert np.array_equal(f["bz"], half * (f["bk"][:, :, 1:] + f["bk"][:, :, :-1]))
