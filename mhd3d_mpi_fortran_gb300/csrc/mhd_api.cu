@@ -69,7 +69,8 @@ struct Handle {
   Scal* sc = nullptr;          // device scalars
   Scal* sc_h = nullptr;        // pinned mirror
   double* diag = nullptr;      // device diagnostics buffer
-  double* diag_h = nullptr;    // pinned
+  double* diag_h = nullptr;    // pinned, behind sc_h
+  double* stage_h = nullptr;   // pinned room for a small grid's whole frame, behind diag_h; null on others
   Dev<float> df{};
   Dev<double> dd{};
   bool profile = false;
@@ -113,7 +114,9 @@ int wait_stream(Handle* h) {
       cudaEventDestroy(e);
       return fail(MHD_E_TIMEOUT, "device did not finish within the wait bound");
     }
-    std::this_thread::sleep_for(std::chrono::microseconds(el < 0.01 ? 20 : 500));
+    // a 20 us sleep takes about 75: steps and frames of a few ms are polled
+    if (el < 0.01) std::this_thread::yield();
+    else std::this_thread::sleep_for(std::chrono::microseconds(200));
   }
   cudaEventDestroy(e);
   return MHD_OK;
@@ -369,6 +372,23 @@ size_t n_arrays(const mhd_params& p, bool metric) {
   return n;
 }
 
+// The 11 arrays mhd_fetch returns: extents of array a (cell arrays, then bi, bj, bk).
+void frame_extent(const Geom& g, int a, int e[3]) {
+  e[0] = g.nx + (a == 8); e[1] = g.ny + (a == 9); e[2] = g.nz + (a == 10);
+}
+size_t frame_doubles(const Geom& g) {
+  size_t n = 0;
+  for (int a = 0; a < 11; ++a) {
+    int e[3];
+    frame_extent(g, a, e);
+    n += (size_t)e[0] * e[1] * e[2];
+  }
+  return n;
+}
+// A frame of up to this many bytes that goes to pageable arrays is read in one
+// copy and spread by the host: eleven pageable copies of 85 KB took 25 us each.
+constexpr size_t kStageBytes = (size_t)1 << 20;
+
 // host FP64 Fortran array (ex,ey,ez) -> padded T on the host; rows in parallel
 template <typename T>
 void pack(const Geom& g, const double* src, int ex, int ey, int ez, T* dst) {
@@ -394,14 +414,6 @@ __global__ void k_from_f64(const double* __restrict__ src, int ex, int ey, int p
   const int j = blockIdx.y, k = blockIdx.z;
   if (i < ex) dst[i + (long long)px * j + plane * k] = (T)src[i + (long long)ex * (j + (long long)ey * k)];
 }
-template <typename T>
-__global__ void k_to_f64(const T* __restrict__ src, int ex, int ey, int px, long long plane,
-                         double* __restrict__ dst) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y, k = blockIdx.z;
-  if (i < ex) dst[i + (long long)ex * (j + (long long)ey * k)] = (double)src[i + (long long)px * j + plane * k];
-}
-
 template <typename T>
 double* f64_scratch(const Dev<T>& d) {
   return reinterpret_cast<double*>(d.F[0][0]);  // 8 x vol x sizeof(T) bytes, >= one FP64 array
@@ -635,9 +647,16 @@ h->tile_ey = (h->fp32 && !metric) ? (emf_streams(g) ? kEmfStream : 8) : h->fp32 
       cudaMalloc(&h->sc, sizeof(Scal)) != cudaSuccess ||
       cudaMalloc(&h->diag, sizeof(double) * (8 + 5 * 152 * 2)) != cudaSuccess)
     return bail(MHD_E_NOMEM, "device allocation failed");
-  if (cudaMallocHost(&h->sc_h, sizeof(Scal)) != cudaSuccess ||
-      cudaMallocHost(&h->diag_h, sizeof(double) * 8) != cudaSuccess)
-    return bail(MHD_E_NOMEM, "pinned allocation failed");
+  {
+    const size_t head = round_up(sizeof(Scal), 64), frame = frame_doubles(g) * sizeof(double);
+    const bool small = frame <= kStageBytes;
+    char* pin = nullptr;
+    if (cudaMallocHost(&pin, head + 64 + (small ? frame : 0)) != cudaSuccess)
+      return bail(MHD_E_NOMEM, "pinned allocation failed");
+    h->sc_h = (Scal*)pin;
+    h->diag_h = (double*)(pin + head);
+    h->stage_h = small ? (double*)(pin + head + 64) : nullptr;
+  }
   for (int i = 0; i < 16; ++i) cudaEventCreate(&h->ev[i]);
   if (cudaMemsetAsync(h->buf, 0, h->bytes, h->st) != cudaSuccess) return bail(MHD_E_CUDA, "memset failed");
   std::vector<double> geo((size_t)g.nx + g.ny + g.nz);
@@ -1084,40 +1103,115 @@ int mhd_last_timings(void* handle, float out_ms[8]) {
   return MHD_OK;
 }
 
-// Writes the first byte of every page of a caller's output array on all host
-// threads.  A copy into pages the process has not touched yet would take
-// their first-touch faults one at a time inside the copy; already-mapped pages
-// cost one store each.  The array is overwritten right after.
-static void prefault(double* p, size_t bytes) {
-  const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-  char* c = reinterpret_cast<char*>(p);
-  const long long npg = (long long)((bytes + page - 1) / page);
-#pragma omp parallel for schedule(static)
-  for (long long k = 0; k < npg; ++k) c[(size_t)k * page] = 0;
+// Several padded arrays of T to packed FP64 arrays, one after the other at dst.
+template <typename T>
+struct Unpack {
+  const T* src[11];
+  int e[11][3];
+  long long at[11];
+};
+template <typename T>
+__global__ void k_unpack(Unpack<T> u, int px, long long plane, double* __restrict__ dst) {
+  const int a = blockIdx.y, ex = u.e[a][0], ey = u.e[a][1];
+  const int n = ex * ey * u.e[a][2];
+  const T* __restrict__ src = u.src[a];
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    const int i = t % ex, r = t / ex, j = r % ey, k = r / ey;
+    dst[u.at[a] + t] = (double)src[i + (long long)px * j + plane * k];
+  }
 }
 
-// Device-side conversion to FP64, then a copy straight into the caller's arrays.
+// Make the caller's pages present before the copies (a copy into fresh pages
+// faults them one by one): pinned arrays have theirs, few pages go in a plain loop.
+static void prefault(double* const* outs, const size_t* count) {
+  const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  long long first[12] = {0};
+  char* base[11];
+  for (int a = 0; a < 11; ++a) {
+    base[a] = reinterpret_cast<char*>(outs[a]);
+    long long npg = 0;
+    if (outs[a]) {
+      cudaPointerAttributes at;
+      const bool known = cudaPointerGetAttributes(&at, outs[a]) == cudaSuccess;
+      if (!known) cudaGetLastError();
+      if (!known || at.type != cudaMemoryTypeHost) npg = (long long)((count[a] * sizeof(double) + page - 1) / page);
+    }
+    first[a + 1] = first[a] + npg;
+  }
+  const long long total = first[11];
+  auto touch = [&](long long k) {
+    int a = 0;
+    while (k >= first[a + 1]) ++a;
+    base[a][(size_t)(k - first[a]) * page] = 0;
+  };
+  if (total <= 1024) {
+    for (long long k = 0; k < total; ++k) touch(k);
+  } else {
+#pragma omp parallel for schedule(static)
+    for (long long k = 0; k < total; ++k) touch(k);
+  }
+}
+
+// Device-side conversion to FP64, then a copy straight into the caller's arrays
+// (or by way of stage_h).  The converted arrays go to the flux and EMF arrays (F and
+// E are one block) and to dU, scratch between steps, as many at a time as fit.
 template <typename T>
 static int fetch_t(Handle* h, double* const* outs) {
   const Geom& g = h->g;
   Dev<T> d = at_par(dev<T>(h), h->par);
   const T* srcs[11] = {d.rho, d.vx, d.vy, d.vz, d.p, d.bx, d.by, d.bz, d.bi, d.bj, d.bk};
+  size_t count[11];
   int ext[11][3];
-  for (int a = 0; a < 8; ++a) { ext[a][0] = g.nx; ext[a][1] = g.ny; ext[a][2] = g.nz; }
-  ext[8][0] = g.nx + 1; ext[8][1] = g.ny; ext[8][2] = g.nz;
-  ext[9][0] = g.nx; ext[9][1] = g.ny + 1; ext[9][2] = g.nz;
-  ext[10][0] = g.nx; ext[10][1] = g.ny; ext[10][2] = g.nz + 1;
-  double* scratch = f64_scratch(d);
-  for (int a = 0; a < 11; ++a)
-    if (outs[a]) prefault(outs[a], sizeof(double) * (size_t)ext[a][0] * ext[a][1] * ext[a][2]);
   for (int a = 0; a < 11; ++a) {
+    frame_extent(g, a, ext[a]);
+    count[a] = (size_t)ext[a][0] * ext[a][1] * ext[a][2];
+  }
+  double* const room[2] = {f64_scratch(d), reinterpret_cast<double*>(d.dU[0])};
+  const size_t cap[2] = {11 * (size_t)g.vol * sizeof(T) / sizeof(double), 8 * (size_t)g.vol * sizeof(T) / sizeof(double)};
+  bool staged = h->stage_h != nullptr;
+  for (int a = 0; a < 11 && staged; ++a) {
     if (!outs[a]) continue;
-    const int ex = ext[a][0], ey = ext[a][1], ez = ext[a][2];
-    k_to_f64<T><<<dim3((ex + 255) / 256, ey, ez), 256, 0, h->st>>>(srcs[a], ex, ey, g.px, g.plane, scratch);
-    CK(cudaMemcpyAsync(outs[a], scratch, sizeof(double) * (size_t)ex * ey * ez, cudaMemcpyDeviceToHost, h->st));
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, outs[a]) != cudaSuccess) cudaGetLastError();
+    else if (at.type == cudaMemoryTypeHost) staged = false;
+  }
+  if (!staged) prefault(outs, count);
+  size_t done = 0;  // doubles staged so far
+  for (int a = 0, r = 0; a < 11; r ^= 1) {
+    Unpack<T> u;
+    size_t n = 0, most = 0;
+    int m = 0, from[11];
+    for (; a < 11 && (!outs[a] || n + count[a] <= cap[r]); ++a) {
+      if (!outs[a]) continue;
+      u.src[m] = srcs[a];
+      for (int q = 0; q < 3; ++q) u.e[m][q] = ext[a][q];
+      u.at[m] = (long long)n;
+      from[m++] = a;
+      n += count[a];
+      most = std::max(most, count[a]);
+    }
+    if (!m) continue;
+    const unsigned nb = (unsigned)std::min<size_t>((most + 255) / 256, 152 * 16);
+    k_unpack<T><<<dim3(nb, m), 256, 0, h->st>>>(u, g.px, g.plane, room[r]);
+    if (staged) {
+      CK(cudaMemcpyAsync(h->stage_h + done, room[r], sizeof(double) * n, cudaMemcpyDeviceToHost, h->st));
+      done += n;
+      continue;
+    }
+    for (int q = 0; q < m; ++q)
+      CK(cudaMemcpyAsync(outs[from[q]], room[r] + u.at[q], sizeof(double) * count[from[q]], cudaMemcpyDeviceToHost,
+                         h->st));
   }
   CK(cudaGetLastError());
-  return wait_stream(h);
+  const int rc = wait_stream(h);
+  if (rc || !staged) return rc;
+  done = 0;
+  for (int a = 0; a < 11; ++a) {
+    if (!outs[a]) continue;
+    std::memcpy(outs[a], h->stage_h + done, sizeof(double) * count[a]);
+    done += count[a];
+  }
+  return MHD_OK;
 }
 
 int mhd_fetch(void* handle, double* rho, double* vx, double* vy, double* vz, double* p, double* bx,
@@ -1731,7 +1825,6 @@ int mhd_free(void* handle) {
   if (h->sc) cudaFree(h->sc);
   if (h->diag) cudaFree(h->diag);
   if (h->sc_h) cudaFreeHost(h->sc_h);
-  if (h->diag_h) cudaFreeHost(h->diag_h);
   if (h->st) cudaStreamDestroy(h->st);
   if (h->st2) cudaStreamDestroy(h->st2);
   if (h->ev_fork) cudaEventDestroy(h->ev_fork);

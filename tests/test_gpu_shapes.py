@@ -1,5 +1,7 @@
 """Launch shapes that follow the grid: segments and flattened columns of the
 FP32 column sweeps, and the batched step with its dt folded into the last stage."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -78,3 +80,32 @@ def test_cells_up_z_leave_consistent_faces(shape, precision):
     assert np.array_equal(f["bx"], half * (f["bi"][1:] + f["bi"][:-1]))
     assert np.array_equal(f["by"], half * (f["bj"][:, 1:] + f["bj"][:, :-1]))
     assert np.array_equal(f["bz"], half * (f["bk"][:, :, 1:] + f["bk"][:, :, :-1]))
+
+
+@pytest.mark.parametrize("shape,nord,precision", [((8, 8, 8), 8, FP64), ((16, 16, 16), 8, FP32), ((40, 70, 31), 8, FP32),
+                                                  ((56, 120, 64), 4, FP32), ((40, 21, 33), 6, FP64)])
+def test_fetch_paths_agree(shape, nord, precision):
+    """Frames by way of the staging buffer (small grids), straight into fresh pageable
+    arrays, into pinned arrays, and a part of the fields only: the values mhd_init got."""
+    import torch
+    s = state(*shape, nord, 11)
+    f = np.float32 if precision == FP32 else np.float64
+    with MHDSolver(Params(*shape, nord=nord, reconop={8: 1, 6: 3, 4: 5}[nord], precision=precision, tau=1e-4), s) as g:
+        got = g.fetch()
+        pin = g.output_arrays()
+        pin = {k: torch.empty(a.size, dtype=torch.float64, pin_memory=True).numpy().reshape(a.shape, order="F")
+               for k, a in pin.items()}
+        g.fetch(out=pin)
+        some = [None] * 11
+        part = {k: np.zeros_like(got[k]) for k in ("p", "bi", "bk")}
+        for k, a in part.items():
+            some[FIELDS.index(k)] = a.ctypes.data
+        assert g.lib.mhd_fetch(g.h, *[None if q is None else ctypes.cast(q, ctypes.POINTER(ctypes.c_double))
+                                      for q in some]) == 0
+    c = slice(nord // 2, -(nord // 2))
+    for k in ("rho", "vx", "vy", "vz", "p"):
+        assert np.array_equal(got[k][c, c, c], getattr(s, k).astype(f)[c, c, c]), k
+    for k in FIELDS:
+        assert np.array_equal(got[k], pin[k]), k
+    for k, a in part.items():
+        assert np.array_equal(a, got[k]), k
