@@ -84,6 +84,8 @@ struct Handle {
   // cleared when the state changes otherwise between steps (init, load,
   // batched steps)
   bool prepared = false;
+  int launched = 0;              // steps launched kernel by kernel (do_steps)
+  bool no_replay = false;        // a capture of the step failed: keep launching
   int tile_td = 8, tile_ey = 8;  // launch shapes (autotuned for FP32 Cartesian PDM)
   bool tiles_set = false;        // chosen by mhd_set_tiles or an autotuner, not by default
   float* geoT = nullptr;       // FP32 copy of the cell widths
@@ -453,6 +455,30 @@ int init_device(Handle* h) {
   return wait_stream(h);
 }
 
+}  // namespace
+static int graph_for(Handle* h, int nsteps, cudaGraphExec_t* out);
+namespace {
+
+constexpr int kReplayAfter = 6;  // steps launched before the step is captured (a capture takes the time of three)
+
+// The graph of one step from the handle's present state; false when it cannot be made (the
+// step is then launched as before).  The thread's capture mode is relaxed meanwhile, so that a
+// capture the caller has open on a stream of its own is not disturbed.
+bool step_replay(Handle* h, cudaGraphExec_t* ex) {
+  const int par = h->par;
+  const bool prepared = h->prepared;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  const bool ok = graph_for(h, 1, ex) == MHD_OK;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (ok) return true;
+  cudaGetLastError();
+  h->par = par;
+  h->prepared = prepared;
+  h->no_replay = true;
+  return false;
+}
+
 template <typename T>
 int do_steps(Handle* h, int n) {
   if (h->profile) {
@@ -471,7 +497,21 @@ int do_steps(Handle* h, int n) {
     }
     return MHD_OK;
   }
-  for (int s = 0; s < n; ++s) enqueue_any<T>(h, h->par, h->st);
+  // Launched one by one, a stage's kernels wait about 10 us at each fork and join of
+  // the two streams and cost the host 45 us (16^3 deck: 570 us a step against 470
+  // replayed), so that once a handle has stepped a few times its step is captured
+  // and replayed; handles that step less never pay for the capture.
+  for (int s = 0; s < n; ++s) {
+    if (h->launched >= kReplayAfter && !h->no_replay) {
+      cudaGraphExec_t ex = nullptr;
+      if (step_replay(h, &ex)) {
+        CK(cudaGraphLaunch(ex, h->st));
+        continue;
+      }
+    }
+    enqueue_any<T>(h, h->par, h->st);
+    ++h->launched;
+  }
   CK(cudaGetLastError());
   return MHD_OK;
 }
@@ -1046,8 +1086,9 @@ static int graph_for(Handle* h, int nsteps, cudaGraphExec_t* out) {
     else enqueue_any<double>(h, par, h->st);
   }
   CK(cudaStreamEndCapture(h->st, &gr));
-  CK(cudaGraphInstantiate(&ex, gr, 0));
+  const cudaError_t ie = cudaGraphInstantiate(&ex, gr, 0);
   cudaGraphDestroy(gr);
+  CK(ie);
   h->graphs[key] = std::make_pair(ex, par + (h->prepared ? 2 : 0));
   h->par = par;
   *out = ex;
@@ -1121,22 +1162,19 @@ __global__ void k_unpack(Unpack<T> u, int px, long long plane, double* __restric
   }
 }
 
-// Make the caller's pages present before the copies (a copy into fresh pages
-// faults them one by one): pinned arrays have theirs, few pages go in a plain loop.
+// Writes the first byte of every page of the caller's output arrays, on all host
+// threads unless they are few.  A copy into pages that are not mapped (fresh ones,
+// or those the system has unmapped to sample their use, pinned ones included)
+// would take their faults one at a time inside the copy: without this a 256^3
+// frame of 9 ms took 80 about every half second, with it 25.  The arrays are
+// overwritten right after.
 static void prefault(double* const* outs, const size_t* count) {
   const size_t page = (size_t)sysconf(_SC_PAGESIZE);
   long long first[12] = {0};
   char* base[11];
   for (int a = 0; a < 11; ++a) {
     base[a] = reinterpret_cast<char*>(outs[a]);
-    long long npg = 0;
-    if (outs[a]) {
-      cudaPointerAttributes at;
-      const bool known = cudaPointerGetAttributes(&at, outs[a]) == cudaSuccess;
-      if (!known) cudaGetLastError();
-      if (!known || at.type != cudaMemoryTypeHost) npg = (long long)((count[a] * sizeof(double) + page - 1) / page);
-    }
-    first[a + 1] = first[a] + npg;
+    first[a + 1] = first[a] + (outs[a] ? (long long)((count[a] * sizeof(double) + page - 1) / page) : 0);
   }
   const long long total = first[11];
   auto touch = [&](long long k) {

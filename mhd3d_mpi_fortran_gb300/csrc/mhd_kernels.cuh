@@ -971,7 +971,7 @@ __device__ __forceinline__ float cfl_sqrt(float x) { return x > 0.0f ? x * rsqrt
 template <bool M>
 __device__ __forceinline__ float cfl_speed(float gam, float r0, float p0, float u, float v, float w, float b2) {
   typedef Ops<float> O;
-  const float vv = cfl_sqrt(u * u + v * v + w * w);
+  const float vv = cfl_sqrt(sq3(u, v, w));
   const float valf = O::dv(cfl_sqrt(b2), cfl_sqrt(r0));
   const float vs = cfl_sqrt(O::dv(gam * p0, r0));
   return vv + cfl_sqrt(valf * valf + vs * vs);
@@ -991,7 +991,7 @@ template <typename T, bool M>
 __device__ __forceinline__ T cell_dt(const Dev<T>& d, int c, int i, int j, int k, T r0, T p0, T u, T v, T w, T a,
                                      T b, T cc, unsigned& st) {
   typedef Ops<T> O;
-  const T vcfl = cfl_speed<M>(d.gam, r0, p0, u, v, w, a * a + b * b + cc * cc);
+  const T vcfl = cfl_speed<M>(d.gam, r0, p0, u, v, w, sq3(a, b, cc));
   T dt;
   if (M)  // metric mode: 1/dx_a -> |mean area vector of the a-faces| / V
     dt = O::dv(d.cfl, O::dw(vcfl * d.m.sa[c], d.m.vol[c], d.m.rvol[c]));

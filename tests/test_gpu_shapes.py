@@ -109,3 +109,25 @@ def test_fetch_paths_agree(shape, nord, precision):
         assert np.array_equal(got[k], pin[k]), k
     for k, a in part.items():
         assert np.array_equal(a, got[k]), k
+
+
+@pytest.mark.parametrize("precision,stepop,dt_mode", [(FP32, 1, 0), (FP32, STEP_RK2, DT_CFL), (FP32, STEP_RK3, 0),
+                                                      (FP64, STEP_RK3, DT_CFL), (FP64, 1, 0)])
+def test_replayed_steps_equal_launched_ones(precision, stepop, dt_mode):
+    """A handle's later steps replay a captured step: 13 steps in calls of 1, 9
+    and 3 (with a tile change between, which drops the captures in FP32) against
+    a handle that runs them as one graph, bit for bit."""
+    shape = (24, 18, 21)
+    s = state(*shape, 8, 5)
+    prm = Params(*shape, precision=precision, stepop=stepop, dt_mode=dt_mode, tau=1e-4)
+    with MHDSolver(prm, s) as g, MHDSolver(prm, s) as h:
+        tg = g.step(1)
+        tg = g.step(9)
+        if precision == FP32:
+            g.set_tiles(8, 8)
+        tg = g.step(3)
+        th = h.step(13, graph=True)  # one capture of all 13
+        fg, fh = g.fetch(), h.fetch()
+    assert tg == th
+    for k in FIELDS:
+        assert np.array_equal(fg[k], fh[k]), k
