@@ -1162,32 +1162,22 @@ __global__ void k_unpack(Unpack<T> u, int px, long long plane, double* __restric
   }
 }
 
-// Writes the first byte of every page of the caller's output arrays, on all host
-// threads unless they are few.  A copy into pages that are not mapped (fresh ones,
-// or those the system has unmapped to sample their use, pinned ones included)
-// would take their faults one at a time inside the copy: without this a 256^3
-// frame of 9 ms took 80 about every half second, with it 25.  The arrays are
-// overwritten right after.
-static void prefault(double* const* outs, const size_t* count) {
+// Writes the first byte of every page of one of the caller's output arrays, on
+// all host threads unless they are few.  A copy into pages that are not mapped
+// (fresh ones, or those the system has unmapped to sample their use, pinned ones
+// included) would take their faults one at a time inside the copy: without this a
+// 256^3 frame of 9 ms took 80 about every half second, with it 25.  Each array is
+// touched just before its copy is queued, while the copy before it runs.
+static void prefault(double* p, size_t bytes) {
   const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-  long long first[12] = {0};
-  char* base[11];
-  for (int a = 0; a < 11; ++a) {
-    base[a] = reinterpret_cast<char*>(outs[a]);
-    first[a + 1] = first[a] + (outs[a] ? (long long)((count[a] * sizeof(double) + page - 1) / page) : 0);
+  char* c = reinterpret_cast<char*>(p);
+  const long long npg = (long long)((bytes + page - 1) / page);
+  if (npg <= 128) {
+    for (long long k = 0; k < npg; ++k) c[(size_t)k * page] = 0;
+    return;
   }
-  const long long total = first[11];
-  auto touch = [&](long long k) {
-    int a = 0;
-    while (k >= first[a + 1]) ++a;
-    base[a][(size_t)(k - first[a]) * page] = 0;
-  };
-  if (total <= 1024) {
-    for (long long k = 0; k < total; ++k) touch(k);
-  } else {
 #pragma omp parallel for schedule(static)
-    for (long long k = 0; k < total; ++k) touch(k);
-  }
+  for (long long k = 0; k < npg; ++k) c[(size_t)k * page] = 0;
 }
 
 // Device-side conversion to FP64, then a copy straight into the caller's arrays
@@ -1213,7 +1203,6 @@ static int fetch_t(Handle* h, double* const* outs) {
     if (cudaPointerGetAttributes(&at, outs[a]) != cudaSuccess) cudaGetLastError();
     else if (at.type == cudaMemoryTypeHost) staged = false;
   }
-  if (!staged) prefault(outs, count);
   size_t done = 0;  // doubles staged so far
   for (int a = 0, r = 0; a < 11; r ^= 1) {
     Unpack<T> u;
@@ -1236,9 +1225,11 @@ static int fetch_t(Handle* h, double* const* outs) {
       done += n;
       continue;
     }
-    for (int q = 0; q < m; ++q)
-      CK(cudaMemcpyAsync(outs[from[q]], room[r] + u.at[q], sizeof(double) * count[from[q]], cudaMemcpyDeviceToHost,
-                         h->st));
+    for (int q = 0; q < m; ++q) {
+      const size_t bytes = sizeof(double) * count[from[q]];
+      prefault(outs[from[q]], bytes);
+      CK(cudaMemcpyAsync(outs[from[q]], room[r] + u.at[q], bytes, cudaMemcpyDeviceToHost, h->st));
+    }
   }
   CK(cudaGetLastError());
   const int rc = wait_stream(h);
