@@ -1425,21 +1425,42 @@ struct GaussArg {
   __device__ __forceinline__ double bell(double z) const { return poly(row + 4, z); }
 };
 
+// a = sqrt(r / q) and ia = sqrt(q / r) for the two lam of a face state, q = 2 p and
+// q = 2 p + B^2, by one rsqrt each.  The product r q must be a normal number for that:
+// where either is not (p = 0, a product below 1e-307 or above 1e308, a negative p,
+// NaN) the quotient decides, as the reference writes it.  p = 0 so gives a =
+// inf, ia = 0 and with them finite moments of a gas that moves.
+__device__ __forceinline__ void lam_roots(double r, double q, double qm, double& a, double& ia, double& am) {
+  const double m = q * r, mm = qm * r;
+  const unsigned lo = 0x00200000u, n = 0x7fe00000u - lo;  // high words of 2^-1021 .. 2^1023
+  if ((unsigned)__double2hiint(m) - lo < n && (unsigned)__double2hiint(mm) - lo < n) {
+    const double s = rsqrt(m);
+    a = r * s;
+    ia = q * s;
+    am = r * rsqrt(mm);
+  } else {
+    a = sqrt(r / q);
+    ia = 1.0 / a;
+    am = sqrt(r / qm);
+  }
+}
+
 // One side (left: + moments) of the FP64 flux through a face normal to axis D:
-// the formulas of face_flux with sqrt(lam) = rho / sqrt(2 p rho), the shared
-// products formed once and fused operations.  About 85 operations of the
-// FP64 pipe; as written in the reference, with two divisions, a root, an exp
-// and two erfc per side, about 240.
+// the formulas of face_flux with lam_roots, the shared products formed once and
+// fused operations.  About 85 operations of the FP64 pipe; as written in the
+// reference, with two divisions, a root, an exp and two erfc per side, about 240.
 template <int D>
 __device__ __forceinline__ void face_side64(const double* q, const Dev<double>& dv, bool left, double* f) {
   const double r = q[0], u = q[1], v = q[2], w = q[3], p = q[4], x = q[5], y = q[6], z = q[7];
   const double vn = q[1 + D], bn = q[5 + D];
-  const double ke = fma(u, u, fma(v, v, w * w)), p2 = p + p;
-  const double s = rsqrt(p2 * r);
-  const double a = (r * s) * vn;
+  const double ke = fma(u, u, fma(v, v, w * w)), p2 = p + p, b2 = fma(x, x, fma(y, y, z * z));
+  double a, ia, am;
+  lam_roots(r, p2, p2 + b2, a, ia, am);
+  a *= vn;
+  am *= vn;
   const GaussArg ga(dv.gtab, a);
   const double v0 = ga.half_erfc(a, left);
-  const double b = (p2 * s) * ga.bell(a);
+  const double b = ia * ga.bell(a);
   const double v1 = fma(vn, v0, left ? b : -b);
   const double m = r * v1, pv = p * v0;
   f[0] = m;
@@ -1448,8 +1469,6 @@ __device__ __forceinline__ void face_side64(const double* q, const Dev<double>& 
   f[3] = m * w;
   f[1 + D] += pv;
   f[4] = fma(fma(0.5 * ke, r, p * (dv.rgm1 + 0.5)), v1, (0.5 * vn) * pv);
-  const double b2 = fma(x, x, fma(y, y, z * z));
-  const double am = (r * rsqrt((p2 + b2) * r)) * vn;
   const double m0 = GaussArg(dv.gtab, am).half_erfc(am, left);
   const double t = -bn * m0;
   f[5] = x * t;
