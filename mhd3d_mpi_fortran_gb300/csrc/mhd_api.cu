@@ -606,23 +606,39 @@ int mhd_device_info(int32_t out[4]) {
 void mhd::gauss_table(double* out) {
   // With e(z) = exp(-z^2) / (2 sqrt(pi)): e' = -2 z e gives e's Taylor
   // coefficients about c by a_{n+1} = -2 (c a_n + a_{n-1}) / (n + 1), and
-  // (0.5 erfc)' = -2 e gives those of 0.5 erfc from them.
+  // (0.5 erfc)' = -2 e gives those of 0.5 erfc from them.  The powers above the
+  // last kept one are then exchanged, from the highest down, for the lower ones of
+  // the Chebyshev polynomial of their degree on |d| <= h: the k-th costs its value /
+  // 2^(k-1) at most, 7e-17 of either function in the last row (4e-13 if they were left out).
+  constexpr int N = kGaussTerms, K = 20;
+  const long double h = 1.0L / 64;
+  long double cheb[K][K] = {{1.0L}, {0.0L, 1.0L}};
+  for (int k = 2; k < K; ++k)
+    for (int j = 0; j <= k; ++j) cheb[k][j] = (j ? 2.0L * cheb[k - 1][j - 1] : 0.0L) - cheb[k - 2][j];
+  auto row = [&](long double* a, double* o) {  // a[n]: coefficient of d^n
+    long double hk = 1.0L;
+    for (int k = 0; k < K; ++k, hk *= h) a[k] *= hk;
+    for (int k = K - 1; k >= N; --k)
+      for (int j = 0; j < k; ++j) a[j] -= a[k] / cheb[k][k] * cheb[k][j];
+    hk = 1.0L;
+    for (int k = 0; k < N; ++k, hk *= h) o[k] = (double)(a[k] / hk);
+  };
   for (unsigned i = 0; i < kGaussRows; ++i) {
     const long double c = i / 32.0L;
-    long double a[8], prev = 0.0L;
-    a[0] = std::exp(-c * c) / (2.0L * std::sqrt(3.14159265358979323846264338327950288L));
-    for (int n = 0; n < 7; ++n) {
-      a[n + 1] = -2.0L * (c * a[n] + prev) / (n + 1);
-      prev = a[n];
+    long double e[K], g[K], prev = 0.0L;
+    e[0] = std::exp(-c * c) / (2.0L * std::sqrt(3.14159265358979323846264338327950288L));
+    g[0] = 0.5L * std::erfc(c);
+    for (int n = 0; n + 1 < K; ++n) {
+      e[n + 1] = -2.0L * (c * e[n] + prev) / (n + 1);
+      g[n + 1] = -2.0L * e[n] / (n + 1);
+      prev = e[n];
     }
-    double* h = out + 16 * i;
-    h[0] = (double)(0.5L * std::erfc(c));
-    for (int n = 0; n < 7; ++n) h[n + 1] = (double)(-2.0L * a[n] / (n + 1));
-    for (int n = 0; n < 8; ++n) h[8 + n] = (double)a[n];
+    row(g, out + 2 * N * i);
+    row(e, out + 2 * N * i + N);
   }
 }
 
-static size_t geo_doubles(const Geom& g) { return 2 * ((size_t)g.nx + g.ny + g.nz) + 16 * (size_t)kGaussRows; }
+static size_t geo_doubles(const Geom& g) { return 2 * ((size_t)g.nx + g.ny + g.nz) + 2 * kGaussTerms * (size_t)kGaussRows; }
 
 // Cell widths (dx | dy | dz), their reciprocals and the Gaussian rows to h->geo.
 static bool upload_geo(Handle* h, std::vector<double> geo) {
@@ -630,7 +646,7 @@ static bool upload_geo(Handle* h, std::vector<double> geo) {
   geo.resize(geo_doubles(h->g));
   for (size_t i = 0; i < n; ++i) geo[n + i] = 1.0 / geo[i];
   static const std::vector<double> rows = [] {
-    std::vector<double> r(16 * (size_t)kGaussRows);
+    std::vector<double> r(2 * kGaussTerms * (size_t)kGaussRows);
     gauss_table(r.data());
     return r;
   }();

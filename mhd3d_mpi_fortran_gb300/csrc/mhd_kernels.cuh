@@ -1386,43 +1386,56 @@ __device__ __forceinline__ void face_flux_lr(const float2* X, float rg, float* o
 }
 
 // ------------------------------------------------------- FP64 moments
-// 0.5 erfc(|z|) and exp(-z^2) / (2 sqrt(pi)) from one table of Taylor
-// polynomials (d.gtab: row i about c = i / 32, eight coefficients of each;
-// gauss_table() fills it).  CUDA's erfc and exp take about 60 and 20 operations
-// of the FP64 pipe; here the row index and the offset from its centre take
-// three and each polynomial seven.  The offset is at most 1/64, where the first
-// term left out is below 5e-17 of either function's largest value; beyond
-// |z| = 6.5 both are below 1e-19 and are taken as zero (NaN stays NaN).
-// In v1 = v v0 +- b the two terms cancel in the tails, so that an absolute error of
-// this size is what the moments carried before as well.
+// 0.5 erfc(|z|) and exp(-z^2) / (2 sqrt(pi)) from one table of polynomials
+// (d.gtab: row i about c = i / 32, ten coefficients of each; gauss_table() fills it).
+// CUDA's erfc and exp take about 60 and 20 operations of the FP64 pipe; here the
+// row index and the offset from its centre take three and each polynomial nine.
+// Both are good to 3e-16 of their own value: a stream that leaves a face
+// sends v v0 +- b through it, whose terms cancel to 1 / 2 z^2, and a dense one may
+// feed a thin cell with it.  Beyond |z| = 6.5 the tails come from erfc and exp; where the
+// result is 1 less a tail they are below its rounding and taken as zero (NaN stays NaN).
+static __device__ __noinline__ double half_erfc_far(double az) { return 0.5 * erfc(az); }
+static __device__ __noinline__ double bell_far(double az) {  // z^2 in two parts
+  const double s = az * az, e = 0.28209479177387814 * exp(-s);
+  return s < INFINITY ? fma(-e, fma(az, az, -s), e) : 0.0;
+}
 struct GaussArg {
   const double2* row;
   double d;
-  int far;  // 0: in the table, 1: beyond it, 2: NaN
-  __device__ __forceinline__ GaussArg(const double* tab, double z) {
+  int far;      // 0: in the table, 1: beyond it, 2: NaN
+  bool direct;  // the side that a tail is the moment of: z <= 0 for the left (+ moments), z >= 0 for the right state
+  __device__ __forceinline__ GaussArg(const double* tab, double z, bool left) {
     const double az = abs_bits(z);
     const double t = fma(az, 32.0, 6755399441055744.0);  // 1.5 * 2^52: the nearest integer in the low word
     d = fma(t - 6755399441055744.0, -0.03125, az);
     const int hi = __double2hiint(az);
     far = hi < 0x401a0000 ? 0 : hi <= 0x7ff00000 ? 1 : 2;
+    direct = (__double2hiint(z) < 0) == left;
     const unsigned i = (unsigned)__double2loint(t);
-    row = reinterpret_cast<const double2*>(tab) + (i < kGaussRows ? i : kGaussRows - 1) * 8;
+    row = reinterpret_cast<const double2*>(tab) + (i < kGaussRows ? i : kGaussRows - 1) * kGaussTerms;
   }
-  __device__ __forceinline__ double poly(const double2* q, double z) const {
-    const double2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2), e = __ldg(q + 3);
-    double s = fma(e.y, d, e.x);
-    s = fma(fma(s, d, c.y), d, c.x);
-    s = fma(fma(s, d, b.y), d, b.x);
-    s = fma(fma(s, d, a.y), d, a.x);
-    return far == 0 ? s : far == 1 ? 0.0 : z;
+  __device__ __forceinline__ double poly(const double2* q) const {
+    static_assert(kGaussTerms == 10, "five pairs of coefficients");
+    double2 a = __ldg(q + 4);
+    double s = fma(a.y, d, a.x);
+#pragma unroll
+    for (int k = 3; k >= 0; --k) {
+      a = __ldg(q + k);
+      s = fma(fma(s, d, a.y), d, a.x);
+    }
+    return s;
   }
-  // 0.5 erfc(-z) for the left (+ moment) or 0.5 erfc(z) for the right state
-  __device__ __forceinline__ double half_erfc(double z, bool left) const {
-    const double h = poly(row, z);
-    const bool direct = (__double2hiint(z) < 0) == left;
+  // 0.5 erfc(-z) for the left or 0.5 erfc(z) for the right state
+  __device__ __forceinline__ double half_erfc(double z) const {
+    double h = poly(row);
+    if (far) h = far == 2 ? z : direct ? half_erfc_far(abs_bits(z)) : 0.0;
     return direct ? h : 1.0 - h;
   }
-  __device__ __forceinline__ double bell(double z) const { return poly(row + 4, z); }
+  __device__ __forceinline__ double bell(double z) const {
+    double e = poly(row + kGaussTerms / 2);
+    if (far) e = far == 2 ? z : direct ? bell_far(abs_bits(z)) : 0.0;
+    return e;
+  }
 };
 
 // a = sqrt(r / q) and ia = sqrt(q / r) for the two lam of a face state, q = 2 p and
@@ -1458,8 +1471,8 @@ __device__ __forceinline__ void face_side64(const double* q, const Dev<double>& 
   lam_roots(r, p2, p2 + b2, a, ia, am);
   a *= vn;
   am *= vn;
-  const GaussArg ga(dv.gtab, a);
-  const double v0 = ga.half_erfc(a, left);
+  const GaussArg ga(dv.gtab, a, left);
+  const double v0 = ga.half_erfc(a);
   const double b = ia * ga.bell(a);
   const double v1 = fma(vn, v0, left ? b : -b);
   const double m = r * v1, pv = p * v0;
@@ -1469,7 +1482,7 @@ __device__ __forceinline__ void face_side64(const double* q, const Dev<double>& 
   f[3] = m * w;
   f[1 + D] += pv;
   f[4] = fma(fma(0.5 * ke, r, p * (dv.rgm1 + 0.5)), v1, (0.5 * vn) * pv);
-  const double m0 = GaussArg(dv.gtab, am).half_erfc(am, left);
+  const double m0 = GaussArg(dv.gtab, am, left).half_erfc(am);
   const double t = -bn * m0;
   f[5] = x * t;
   f[6] = y * t;

@@ -102,7 +102,7 @@ struct Dev {
   const double *dx, *dy, *dz;  // FP64 cell widths (ghost-inclusive, 1-D)
   const T *wx, *wy, *wz;       // the same widths in T (FP32 path: converted once)
   const T *rwx, *rwy, *rwz;    // reciprocal widths
-  const double* gtab;          // Taylor rows of the Gaussian moments (FP64; gauss_table)
+  const double* gtab;          // polynomial rows of the Gaussian moments (FP64; gauss_table)
   Scal* sc;
   const int* gmap;             // per-axis ghost-image tables (cell x,y,z; face x,y,z), each n+2
   unsigned int* partial;       // per-block scratch of the CFL reduction
@@ -226,10 +226,11 @@ int mlp_correct(void* h, Dev<float>& d, cudaStream_t st);
 // MHD_E_TIMEOUT if an MLP kernel recorded a wait that gave up, else MHD_OK.
 int mlp_status(void* h);
 
-// Rows of Dev::gtab: row i holds the Taylor coefficients about c = i / 32 of
-// 0.5 erfc(c + d) (eight) and of exp(-(c + d)^2) / (2 sqrt(pi)) (eight), up to c = 6.5.
+// Rows of Dev::gtab: row i holds polynomials in d, |d| <= 1/64, for 0.5 erfc(c + d)
+// and exp(-(c + d)^2) / (2 sqrt(pi)) about c = i / 32, kGaussTerms coefficients of each, up to c = 6.5.
 constexpr unsigned kGaussRows = 32 * 13 / 2 + 1;
-void gauss_table(double* out);  // kGaussRows * 16 values (host)
+constexpr int kGaussTerms = 10;
+void gauss_table(double* out);  // kGaussRows * 2 * kGaussTerms values (host)
 // Dev::recon of PDM with pdmb <= 0 (the general limiter; R_PDMG of the kernels).
 constexpr int kReconPdmGeneral = 6;
 // Tile lengths the autotuner tries (FP32 Cartesian PDM).

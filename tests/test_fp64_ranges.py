@@ -1,8 +1,10 @@
 """FP64 step at the ends of its range, against the oracle."""
+import ctypes
+
 import numpy as np
 import pytest
 
-from mhd3d_mpi_fortran_gb300 import MHDSolver, ics
+from mhd3d_mpi_fortran_gb300 import MHDSolver, abi, ics
 from mhd3d_mpi_fortran_gb300.abi import Params
 
 RECONS = [1, 2, 3, 4, 5]
@@ -72,3 +74,58 @@ def test_pressure_times_density_beyond_the_range(scale):
         b *= np.sqrt(scale)
     fo = fluxes_match(Params(12, 9, 10, tau=1e-3), s)
     assert np.isfinite(fo[0][0]).all()
+
+
+@pytest.mark.gpu
+def test_tails_of_the_moments():
+    """Two streams that leave a face: only the tails of the moments cross it.  Constant states on
+    either side (so that the face states are the cells'), one argument z = sqrt(rho / 2p) |v| per
+    row from 0.3 to 25; mass flux and magnetic stress relative to 40 digits.  The bound: z is off by
+    5 half units of rounding, which a tail takes 2 z^2 times, and v v0 and b cancel to 1 / 2z^2."""
+    mp = pytest.importorskip("mpmath")
+    n = 64
+    s = ics.empty_state(ics.grid(16, n, 8))
+    z = np.geomspace(0.3, 25.0, n)
+    row = np.ones(s.vx.shape[1])
+    row[4:-4] = z
+    left = (np.arange(s.vx.shape[0]) < 12).reshape(-1, 1, 1)
+    s.rho[...] = np.where(left, 1.0, 2.0 ** -10)
+    s.p[...] = np.where(left, 0.7, 1.3 * 2.0 ** -10)
+    s.vx[...] = np.where(left, -1.0, 1.0) * np.sqrt(2 * s.p / s.rho) * row.reshape(1, -1, 1)
+    s.bj[...] = 0.4
+    with MHDSolver(Params(16, n, 8, tau=1e-3), s) as g:
+        f = g.debug_fluxes()[0]
+    mp.mp.dps = 40
+    for j in range(n):
+        mass = stress = 0
+        for side, i in ((1, 11), (-1, 12)):
+            rho, p, v, b2 = (mp.mpf(float(a)) for a in (s.rho[i, 4 + j, 4], s.p[i, 4 + j, 4], s.vx[i, 4 + j, 4], 0.4 ** 2))
+            a, am = mp.sqrt(rho / (2 * p)), mp.sqrt(rho / (2 * p + b2))
+            mass += rho * (v * mp.erfc(-side * a * v) / 2 + side * mp.exp(-(a * v) ** 2) / (2 * a * mp.sqrt(mp.pi)))
+            stress += b2 / 2 * mp.erfc(-side * am * v) / 2
+        for got, ref, k in ((f[0], mass, 0), (f[5], stress, 5)):
+            err = abs(float((mp.mpf(float(got[8, j, 3])) - ref) / ref))
+            assert err <= 4e-15 * (1 + z[j] ** 2), (z[j], k, err)
+
+
+def test_table_rows_of_the_library():
+    """The rows that the library uploads, as the kernels evaluate them: relative errors of the
+    polynomials, the last row's outer edge included (1.1e-16: first terms left out and coefficients;
+    as much again for the roundings of the evaluation)."""
+    mp = pytest.importorskip("mpmath")
+    lib = abi.load()
+    fill = lib._ZN3mhd11gauss_tableEPd
+    fill.argtypes, fill.restype = [ctypes.c_void_p], None
+    out = np.zeros((209, 20))
+    fill(out.ctypes.data)
+    mp.mp.dps = 30
+    r = np.random.default_rng(1)
+    for i in range(0, 209, 3):
+        c = i / 32.0
+        for d in np.concatenate([[-1 / 64, 1 / 64, 0.0], r.uniform(-1 / 64, 1 / 64, 5)]):
+            h = e = 0.0
+            for k in range(9, -1, -1):
+                h, e = h * d + out[i, k], e * d + out[i, 10 + k]
+            x = mp.mpf(c) + mp.mpf(d)
+            assert abs(h / (mp.erfc(x) / 2) - 1) <= 3.3e-16, (c, d)
+            assert abs(e / (mp.exp(-x * x) / (2 * mp.sqrt(mp.pi))) - 1) <= 3.3e-16, (c, d)
