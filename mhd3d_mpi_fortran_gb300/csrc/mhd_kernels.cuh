@@ -967,7 +967,9 @@ __device__ __forceinline__ double cfl_sqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float cfl_sqrt(float x) { return x > 0.0f ? x * rsqrtf(x) : 0.0f; }
 
 // |v| + fast speed sqrt(B^2 / rho + gam p / rho); FP64 takes one root and one
-// reciprocal for the second term (three roots and two divisions as written in get_dt).
+// reciprocal for the second term (three roots and two divisions as written in get_dt) of a
+// cell with p >= 0 and a positive rho whose reciprocal is a normal number.  In any other
+// cell the three roots decide what is NaN, and with it out of the minimum.
 template <bool M>
 __device__ __forceinline__ float cfl_speed(float gam, float r0, float p0, float u, float v, float w, float b2) {
   typedef Ops<float> O;
@@ -978,7 +980,7 @@ __device__ __forceinline__ float cfl_speed(float gam, float r0, float p0, float 
 }
 template <bool M>
 __device__ __forceinline__ double cfl_speed(double gam, double r0, double p0, double u, double v, double w, double b2) {
-  if (M) {
+  if (M || !ge0(p0) || (unsigned)__double2hiint(r0) - 0x00200000u >= 0x7fc00000u - 0x00200000u) {
     const double valf = sqrt(b2) / sqrt(r0), vs = sqrt(gam * p0 / r0);
     return sqrt(u * u + v * v + w * w) + sqrt(valf * valf + vs * vs);
   }

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from mhd3d_mpi_fortran_gb300 import MHDSolver, abi, ics
-from mhd3d_mpi_fortran_gb300.abi import Params
+from mhd3d_mpi_fortran_gb300.abi import DT_CFL, Params
 
 RECONS = [1, 2, 3, 4, 5]
 
@@ -129,3 +129,21 @@ def test_table_rows_of_the_library():
             x = mp.mpf(c) + mp.mpf(d)
             assert abs(h / (mp.erfc(x) / 2) - 1) <= 3.3e-16, (c, d)
             assert abs(e / (mp.exp(-x * x) / (2 * mp.sqrt(mp.pi))) - 1) <= 3.3e-16, (c, d)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("vals", [dict(p=-0.5), dict(rho=-0.5), dict(rho=-0.5, p=-0.5), dict(rho=0.0), dict(p=0.0),
+                                  dict(rho=0.0, p=0.0)])
+def test_cfl_dt_of_unphysical_cells(vals):
+    """A cell of negative or zero density or pressure in a strong field, where its dt would be the
+    smallest: the speed is NaN where get_dt's three roots give NaN, and drops out."""
+    from oracle.oracle import OracleSolver
+    s = flow(12, 9, 10)
+    s.bi[7:9, 6, 6] = 8.0
+    for k, x in vals.items():
+        getattr(s, k)[7, 6, 6] = x
+    prm = Params(12, 9, 10, dt_mode=DT_CFL, tau=1e-3)
+    with MHDSolver(prm, s) as g:
+        got = g.diagnostics()["dt_cfl"]
+    ref = OracleSolver(prm, s).diagnostics()["dt_cfl"]
+    assert np.isfinite(ref) and got == pytest.approx(ref, rel=1e-14)
