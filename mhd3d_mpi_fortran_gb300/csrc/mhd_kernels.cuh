@@ -481,7 +481,13 @@ __device__ __forceinline__ void weno_both(float fm3, float fm2, float fm1, float
 // plus a small correction (half a unit of rounding).  48 operations of the FP64
 // pipe per state, as the reference writes it about 150: one division instead
 // of nine, the weights 1 : 6 : 3 over e^2 brought to their common denominator
-// after scaling by a power of two (integer pipe).
+// after scaling by a power of two (integer pipe).  Beside a jump whose indicator is 2^450
+// times those of the smooth candidates the scaled squares of these vanish: there the
+// weights are the quotients.
+static __device__ __noinline__ double weno_mix_far(double e0, double e1, double e2, double g0, double g1, double g2) {
+  const double a0 = 1.0 / (e0 * e0), a1 = 6.0 / (e1 * e1), a2 = 3.0 / (e2 * e2);
+  return (a0 * g0 + a1 * g1 + a2 * g2) / (6.0 * (a0 + a1 + a2));
+}
 __device__ __forceinline__ double weno_mix(double e0, double e1, double e2, double g0, double g1, double g2) {
   const int x0 = __double2hiint(e0), x1 = __double2hiint(e1), x2 = __double2hiint(e2);
   const int sh = (max(x0, max(x1, x2)) & 0x7ff00000) - 0x3ff00000;
@@ -489,8 +495,9 @@ __device__ __forceinline__ double weno_mix(double e0, double e1, double e2, doub
   const double s1 = __hiloint2double(max(x1 - sh, 0x00100000), __double2loint(e1));
   const double s2 = __hiloint2double(max(x2 - sh, 0x00100000), __double2loint(e2));
   const double d0 = s0 * s0, d1 = s1 * s1, d2 = s2 * s2;
-  const double a0 = d1 * d2, a1 = (6.0 * d0) * d2, a2 = (3.0 * d0) * d1;
-  return fma(a0, g0, fma(a1, g1, a2 * g2)) / (6.0 * (a0 + a1 + a2));
+  const double a0 = d1 * d2, a1 = (6.0 * d0) * d2, a2 = (3.0 * d0) * d1, sum = a0 + a1 + a2;
+  if (__double2hiint(sum) < (1023 - 900) << 20) return weno_mix_far(e0, e1, e2, g0, g1, g2);
+  return fma(a0, g0, fma(a1, g1, a2 * g2)) / (6.0 * sum);
 }
 // S = 1 for the left state, -1 for the right one (the stencil mirrored): near
 // cell a1, the cell b0 across the face, the first differences dm behind a1 and

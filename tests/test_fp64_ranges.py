@@ -147,3 +147,14 @@ def test_cfl_dt_of_unphysical_cells(vals):
         got = g.diagnostics()["dt_cfl"]
     ref = OracleSolver(prm, s).diagnostics()["dt_cfl"]
     assert np.isfinite(ref) and got == pytest.approx(ref, rel=1e-14)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("recon", [3, 4])
+def test_weno_weights_beside_a_huge_jump(recon):
+    """Smoothness indicators 1e166 apart: the smooth candidates keep their weights."""
+    s = flow(16, 9, 10)
+    s.vz[8:] = 1e80
+    s.vz[:8] = 0.3
+    fo = fluxes_match(Params(16, 9, 10, reconop=recon, tau=1e-3), s)
+    assert all(np.isfinite(q).all() for q in fo[0])
