@@ -64,7 +64,6 @@ struct Handle {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   void* buf = nullptr;
   size_t bytes = 0;
-  void* fz = nullptr;          // FP64: five z-flux arrays (Dev::fz), null when there was no room
   double* geo = nullptr;       // FP64: dx | dy | dz, their reciprocals, the Gaussian moment rows (Dev::gtab)
   Scal* sc = nullptr;          // device scalars
   Scal* sc_h = nullptr;        // pinned mirror
@@ -300,12 +299,11 @@ void carve(Handle* h, Dev<T>& d, char* base) {
   for (int i = 0; i < 11; ++i) d.q[i] = (i < nq) ? next() : nullptr;
   for (int i = 0; i < 11; ++i) d.h[i] = (h->prm.stepop == MHD_STEP_AB2) ? next() : nullptr;
   // x-face fluxes only: the y / z faces are consumed inside the sweeps / face
-  // tiles, or (FP64) go to dead arrays and fz; the kernel-level debug entry point
+  // tiles, or (FP64, k_faces) go to dead arrays; the kernel-level debug entry point
   // gives them scratch of its own
   for (int q = 0; q < 8; ++q) d.F[0][q] = next();
   for (int ax = 1; ax < 3; ++ax)
     for (int q = 0; q < 8; ++q) d.F[ax][q] = nullptr;
-  for (int q = 0; q < 5; ++q) d.fz[q] = h->fz ? (T*)h->fz + q * n : nullptr;
   for (int e = 0; e < 3; ++e) d.E[e] = next();
   d.vf = next();
   d.dx = h->geo; d.dy = h->geo + g.nx; d.dz = h->geo + g.nx + g.ny;
@@ -751,15 +749,6 @@ h->tile_ey = (h->fp32 && !metric) ? (emf_streams(g) ? kEmfStream : 8) : h->fp32 
   s.pend_status = 0;
   if (cudaMemcpy(h->sc, &s, sizeof(Scal), cudaMemcpyHostToDevice) != cudaSuccess)
     return bail(MHD_E_CUDA, "scalar upload failed");
-  if (!h->fp32) {  // z-flux arrays, where they take a quarter of the free memory at most (the face tiles need none)
-    const size_t want = 5 * (size_t)g.vol * sizeof(double);
-    size_t avail = 0, total = 0;
-    if (want < ((size_t)64 << 20) || (cudaMemGetInfo(&avail, &total) == cudaSuccess && want <= avail / 4))
-      if (cudaMalloc(&h->fz, want) != cudaSuccess) {
-        h->fz = nullptr;
-        cudaGetLastError();
-      }
-  }
   if (h->fp32) carve<float>(h, h->df, (char*)h->buf);
   else carve<double>(h, h->dd, (char*)h->buf);
   *out = h;
@@ -1865,7 +1854,6 @@ int mhd_free(void* handle) {
     if (h->ev[i]) cudaEventDestroy(h->ev[i]);
   for (cudaEvent_t e : h->pool) cudaEventDestroy(e);
   if (h->buf) cudaFree(h->buf);
-  if (h->fz) cudaFree(h->fz);
   if (h->geo) cudaFree(h->geo);
   if (h->geoT) cudaFree(h->geoT);
   if (h->gmap) cudaFree(h->gmap);

@@ -1649,18 +1649,20 @@ __global__ void k_flux(KArg<T, B> ka, Inp<T> in0, Prm<T> P) {
 // bounds the faces, so the fluxes' traffic is free, no face is computed twice
 // (the y / z tiles recompute one of nine), the lanes are full whatever the
 // extents (nx0 = 16 left half of a tile's idle), and 16^3 cells are spread over
-// every SM (blocks of 64 faces while there are few).  The y fluxes take the
-// place of dU, the z fluxes the other half's face B, dead until CT writes it, and
-// five arrays of their own (Dev::fz; without them, on a grid that leaves no room,
-// the tiles run).
-template <typename T, int D>
-__device__ __forceinline__ T* face_flux_ptr(const Dev<T>& d, int q) {
+// every SM (blocks of 64 faces while there are few).  The fluxes take arrays that
+// are dead meanwhile: y those of dU, z the other half's, face B until CT writes it and
+// the primitives until the update does.
+template <int D>
+__device__ __forceinline__ double* face_flux_ptr(const Dev<double>& d, int q) {
   if (D == 0) return d.F[0][q];
   if (D == 1) return d.dU[q];
-  return q == 0 ? d.obi : q == 1 ? d.obj : q == 2 ? d.obk : d.fz[q < 3 ? 0 : q - 3];
+  double* const z[8] = {d.orho, d.ovx, d.ovy, d.ovz, d.op, d.obi, d.obj, d.obk};
+  return z[q];
 }
-template <typename T, int RECON, int D, bool M>
-__device__ __forceinline__ void face_one(const Dev<T>& d, const Inp<T>& in, const Prm<T>& P, int t, int ni, int nj) {
+template <int RECON, int D, bool M>
+__device__ __forceinline__ void face_one(const Dev<double>& d, const Inp<double>& in, const Prm<double>& P, int t,
+                                         int ni, int nj) {
+  typedef double T;
   const Geom& g = d.g;
   const int i = t % ni, r = t / ni, j = r % nj, k = r / nj;
   const int c = i + g.ng + g.px * (j + g.ng + g.py * (k + g.ng));
@@ -1670,18 +1672,18 @@ __device__ __forceinline__ void face_one(const Dev<T>& d, const Inp<T>& in, cons
   face_states<T, RECON, M>(src, c, s, P, L, R);
   any_face_flux<T, D, M>(d, c, L, R, out);
 #pragma unroll
-  for (int q = 0; q < 8; ++q) face_flux_ptr<T, D>(d, q)[c] = out[q];
+  for (int q = 0; q < 8; ++q) face_flux_ptr<D>(d, q)[c] = out[q];
 }
-template <typename T, int RECON, bool M>
-__global__ void __launch_bounds__(128) k_faces(Dev<T> d, Inp<T> in, Prm<T> P) {
+template <int RECON, bool M>
+__global__ void __launch_bounds__(128) k_faces(Dev<double> d, Inp<double> in, Prm<double> P) {
   const Geom& g = d.g;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n0 = (g.nx0 + 1) * g.ny0 * g.nz0, n1 = g.nx0 * (g.ny0 + 1) * g.nz0, n2 = g.nx0 * g.ny0 * (g.nz0 + 1);
-  if (t < n0) return face_one<T, RECON, 0, M>(d, in, P, t, g.nx0 + 1, g.ny0);
+  unsigned t = blockIdx.x * blockDim.x + threadIdx.x;  // each axis fits an int, the three together may not
+  const unsigned n0 = (g.nx0 + 1) * g.ny0 * g.nz0, n1 = g.nx0 * (g.ny0 + 1) * g.nz0, n2 = g.nx0 * g.ny0 * (g.nz0 + 1);
+  if (t < n0) return face_one<RECON, 0, M>(d, in, P, t, g.nx0 + 1, g.ny0);
   t -= n0;
-  if (t < n1) return face_one<T, RECON, 1, M>(d, in, P, t, g.nx0, g.ny0 + 1);
+  if (t < n1) return face_one<RECON, 1, M>(d, in, P, t, g.nx0, g.ny0 + 1);
   t -= n1;
-  if (t < n2) face_one<T, RECON, 2, M>(d, in, P, t, g.nx0, g.ny0);
+  if (t < n2) face_one<RECON, 2, M>(d, in, P, t, g.nx0, g.ny0);
 }
 
 // Stage combine of the RK steps (mhd3d3.f90:3674-3702, 3745-3788):
@@ -1830,26 +1832,40 @@ __device__ __forceinline__ void cell_update(const Dev<T>& d, int c, int cd, cons
   cell_update_vals<T, M>(d, c, cd, dF, du, pv, qv, form, cw, den);
 }
 
-// The update after k_faces: the flux divergence in the tiles' order, then cell_update_vals.
-template <typename T, bool M>
-__global__ void __launch_bounds__(128) k_update_faces(Dev<T> d, int form, T cw, T den) {
+// The update after k_faces: the flux divergence in the tiles' order, then
+// cell_update_vals, which puts a cell's new primitives where the z fluxes of its low face
+// lie.  So a block owns whole columns, TX of them, and walks them in slabs of TZ cells:
+// every thread has read both faces of its cell before any writes, and the next slab's
+// low faces are beyond what this one writes.  TZ = 32 (or what nz0 needs) by 128 / TZ
+// columns, a sector of x.  Bytes and latency bound it; PDM stage in us at one cell a thread
+// with the z fluxes in arrays of their own, and at TZ = 8, 16, 32, 64: 16^3 48.8, 53.4
+// 48.6 48.4 48.4; 64^3 898.6, 908.8 909.6 899.1 900.3 (256 or 512 threads: no faster).
+template <bool M>
+__global__ void __launch_bounds__(128) k_update_faces(Dev<double> d, int form, double cw, double den) {
+  typedef double T;
   const Geom& g = d.g;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= g.nx0 * g.ny0 * g.nz0) return;
-  const int i = t % g.nx0 + g.ng, r = t / g.nx0, j = r % g.ny0 + g.ng, k = r / g.ny0 + g.ng;
-  const int c = i + g.px * (j + g.py * k), sy = g.px, sz = (int)g.plane;
-  T du[8], dF[8], pv[5], qv[5];
+  const int nbx = (g.nx0 + blockDim.x - 1) / blockDim.x;
+  const int i0 = blockIdx.x % nbx * blockDim.x + threadIdx.x, j = blockIdx.x / nbx + g.ng, i = i0 + g.ng;
+  const int sy = g.px, sz = (int)g.plane;
+  for (int k0 = 0; k0 < g.nz0; k0 += blockDim.y) {
+    const int k = k0 + threadIdx.y + g.ng, c = i + g.px * (j + g.py * k);
+    const bool in = i0 < g.nx0 && k < g.ng + g.nz0;
+    T du[8], dF[8], pv[5], qv[5];
+    if (in) {
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const T *fx = face_flux_ptr<T, 0>(d, q), *fy = face_flux_ptr<T, 1>(d, q), *fz = face_flux_ptr<T, 2>(d, q);
-    const T dx = fx[c + 1] - fx[c], dy = fy[c + sy] - fy[c];
-    du[q] = M ? dx + dy : Ops<T>::dc(dx, d.wx[i], d.rwx[i]) + Ops<T>::dc(dy, d.wy[j], d.rwy[j]);
-    dF[q] = fz[c + sz] - fz[c];
+      for (int q = 0; q < 8; ++q) {
+        const T *fx = face_flux_ptr<0>(d, q), *fy = face_flux_ptr<1>(d, q), *fz = face_flux_ptr<2>(d, q);
+        const T dx = fx[c + 1] - fx[c], dy = fy[c + sy] - fy[c];
+        du[q] = M ? dx + dy : Ops<T>::dc(dx, d.wx[i], d.rwx[i]) + Ops<T>::dc(dy, d.wy[j], d.rwy[j]);
+        dF[q] = fz[c + sz] - fz[c];
+      }
+      pv[0] = d.rho[c]; pv[1] = d.vx[c]; pv[2] = d.vy[c]; pv[3] = d.vz[c]; pv[4] = d.p[c];
+#pragma unroll
+      for (int q = 0; q < 5; ++q) qv[q] = (form >= 0) ? d.q[q][c] : T(0);
+    }
+    __syncthreads();
+    if (in) cell_update_vals<T, M>(d, c, k, dF, du, pv, qv, form, cw, den);
   }
-  pv[0] = d.rho[c]; pv[1] = d.vx[c]; pv[2] = d.vy[c]; pv[3] = d.vz[c]; pv[4] = d.p[c];
-#pragma unroll
-  for (int q = 0; q < 5; ++q) qv[q] = (form >= 0) ? d.q[q][c] : T(0);
-  cell_update_vals<T, M>(d, c, k, dF, du, pv, qv, form, cw, den);
 }
 
 template <typename T, int RECON, int D, bool M, bool B, int TDV = TD>
@@ -3819,17 +3835,19 @@ void hydro_r(const Dev<T>& d, const Inp<T>& in, int part, int form, double c, do
              cudaStream_t st) {
   Prm<T> P = prm_of(d);
   const Geom& g = d.g;
-  if (std::is_same<T, double>::value && d.fz[0]) {
+  if constexpr (std::is_same<T, double>::value) {
     if (part == 0) {
-      const int n = (g.nx0 + 1) * g.ny0 * g.nz0 + g.nx0 * (g.ny0 + 1) * g.nz0 + g.nx0 * g.ny0 * (g.nz0 + 1);
-      const int nt = n < 4 * 152 * 128 ? 64 : 128;
-      k_faces<T, RECON, M><<<(n + nt - 1) / nt, nt, 0, st>>>(d, in, P);
+      const unsigned n = (unsigned)((g.nx0 + 1) * g.ny0 * g.nz0) + g.nx0 * (g.ny0 + 1) * g.nz0 +
+                         g.nx0 * g.ny0 * (g.nz0 + 1);
+      const unsigned nt = n < 4 * 152 * 128 ? 64 : 128;
+      k_faces<RECON, M><<<(n + nt - 1) / nt, nt, 0, st>>>(d, in, P);
     } else if (part == 2) {
-      k_update_faces<T, M><<<(g.nx0 * g.ny0 * g.nz0 + 127) / 128, 128, 0, st>>>(d, form, (T)c, (T)den);
+      int tz = 1;
+      while (tz < 32 && tz < g.nz0) tz *= 2;
+      const dim3 b(128 / tz, tz);
+      k_update_faces<M><<<(g.nx0 + b.x - 1) / b.x * g.ny0, b, 0, st>>>(d, form, c, den);
     }
-    return;
-  }
-  if (part == 0) {
+  } else if (part == 0) {
     const int n0 = (g.nx0 + 1) * g.ny0 * g.nz0;
     static PerDevice pref;
     prefer_carveout(k_flux<T, RECON, 0, M, false>, 0, pref);

@@ -96,7 +96,6 @@ struct Dev {
   // AB predicted half step {rho, vx, vy, vz, p, bi, bj, bk, bx, by, bz}
   T* h[11];
   T* F[3][8];  // face fluxes [axis][rho, rvx, rvy, rvz, eng, s_x, s_y, s_z]
-  T* fz[5];    // FP64: five of the z-face fluxes (k_faces), null when the face tiles run
   T* E[3];     // edge EMFs ei, ej, ek
   T* vf;       // |v| + |B|/sqrt(rho) of the stage input
   const double *dx, *dy, *dz;  // FP64 cell widths (ghost-inclusive, 1-D)
