@@ -281,8 +281,7 @@ void carve(Handle* h, Dev<T>& d, char* base) {
   auto next = [&]() { T* r = a; a += n; return r; };
   d.g = g;
   d.recon = h->prm.reconop;
-  // the fast PDM limiter needs a positive constant (in T); any other takes the general form
-  if (d.recon == MHD_RECON_PDM && !((T)h->prm.pdmb > T(0))) d.recon = kReconPdmGeneral;
+  if (d.recon == MHD_RECON_PDM && !pdm_signless((T)h->prm.pdmb)) d.recon = kReconPdmGeneral;
   d.stepop = h->prm.stepop;
   d.tvd_shift = h->prm.tvd_shift;
   d.dt_mode = h->prm.dt_mode;
@@ -1369,8 +1368,7 @@ struct BatchBufs {
 // Cartesian, PDM, the same RK stepper, dt mode and limiter constants.
 static bool batchable(Handle* const* hs, int n) {
   const mhd_params& a = hs[0]->prm;
-  if (hs[0]->metric || a.reconop != MHD_RECON_PDM || !((hs[0]->fp32 ? (double)(float)a.pdmb : a.pdmb) > 0.0) ||
-      a.emf != MHD_EMF_LFM ||
+  if (hs[0]->metric || a.reconop != MHD_RECON_PDM || a.emf != MHD_EMF_LFM ||
       (a.stepop != MHD_STEP_RK2 && a.stepop != MHD_STEP_RK3))
     return false;
   for (int i = 1; i < n; ++i) {

@@ -26,8 +26,8 @@
 
 namespace mhd {
 
-// R_PDMG: PDM with a limiter constant pdmb that is not positive (carve() picks
-// it), evaluated as the reference writes the limiter; R_PDM needs pdmb > 0.
+// R_PDMG: PDM with a limiter constant for which the sign-free form (R_PDM) does not hold
+// (pdm_signless; carve() picks it), evaluated as the reference writes the limiter, in the same kernels.
 enum { R_PDM = 1, R_TVD = 2, R_WENO = 3, R_MPWENO = 4, R_TVDMC = 5, R_PDMG = 6 };
 enum { BC_PERIODIC = 0, BC_EVEN = 1, BC_REFLECT = 2, BC_OUTFLOW = 3 };
 enum { EMF_LFM = 0, EMF_YEE = 1 };
@@ -735,12 +735,19 @@ __device__ __forceinline__ double2 corner_quad2(double2 q, double2 far1, double2
   return make_double2(corner_quad(q.x, far1.x, far2.x, q.x - out1.x, q.x - out2.x, pd, vi.x),
                       corner_quad(q.y, far1.y, far2.y, q.y - out1.y, q.y - out2.y, pd, vi.y));
 }
-// corner_pdm_vals<R_PDM> of both components.
-template <typename T>
+// corner_pdm_vals of both components.
+template <typename T, int RECON>
 __device__ __forceinline__ void corner_pdm_vals2(
     typename Pr<T>::V m11, typename Pr<T>::V m21, typename Pr<T>::V m12, typename Pr<T>::V m01, typename Pr<T>::V p11,
     typename Pr<T>::V m02, typename Pr<T>::V m10, typename Pr<T>::V m20, typename Pr<T>::V m1p, typename Pr<T>::V c0,
     typename Pr<T>::V p10, typename Pr<T>::V p01, typename Pr<T>::V vi, T pd, T& r0, T& r1) {
+  if constexpr (RECON != R_PDM) {
+    r0 = corner_pdm_vals<T, RECON>(m11.x, m21.x, m12.x, m01.x, p11.x, m02.x, m10.x, m20.x, m1p.x, c0.x, p10.x, p01.x,
+                                   vi.x, pd);
+    r1 = corner_pdm_vals<T, RECON>(m11.y, m21.y, m12.y, m01.y, p11.y, m02.y, m10.y, m20.y, m1p.y, c0.y, p10.y, p01.y,
+                                   vi.y, pd);
+    return;
+  }
   typedef typename Pr<T>::V V;
   const V v00 = corner_quad2(m11, m01, m10, m21, m12, pd, vi);
   const V v10 = corner_quad2(m01, m11, c0, p11, m02, pd, vi);
@@ -789,14 +796,14 @@ __device__ __forceinline__ float2 exp_neg(float2 a) {
 }  // namespace p2
 
 // corner_pdm of both components from pair-interleaved shared memory.
-template <typename T>
+template <typename T, int RECON>
 __device__ __forceinline__ void corner_pdm_pair(const typename Pr<T>::V* __restrict__ v, int c, int s1, int s2,
                                                 typename Pr<T>::V vi, T pd, T& r0, T& r1) {
   typedef typename Pr<T>::V V;
   const V m11 = v[c - s1 - s2], m21 = v[c - 2 * s1 - s2], m12 = v[c - s1 - 2 * s2], m01 = v[c - s2];
   const V p11 = v[c + s1 - s2], m02 = v[c - 2 * s2], m10 = v[c - s1], m20 = v[c - 2 * s1];
   const V m1p = v[c - s1 + s2], c0 = v[c], p10 = v[c + s1], p01 = v[c + s2];
-  corner_pdm_vals2<T>(m11, m21, m12, m01, p11, m02, m10, m20, m1p, c0, p10, p01, vi, pd, r0, r1);
+  corner_pdm_vals2<T, RECON>(m11, m21, m12, m01, p11, m02, m10, m20, m1p, c0, p10, p01, vi, pd, r0, r1);
 }
 
 // Limited corner value of v at the edge whose two transverse axes have
@@ -1315,12 +1322,35 @@ template <> struct Moments<float> {
 // kernel (x faces, y / z face tiles and column sweeps, batched or not) goes
 // through these functions, so they agree bit for bit.
 
+// pdm2 of two fields (lanes .x and .y), for any pdmb: the differences on the
+// packed pipe, the clamp and the limiter per lane.
+__device__ __forceinline__ float2 pdm_general_lim(float fii, float dfl, float dfr, float dfm, float df0, float dfp) {
+  const float sm = sgn1(dfm), s0 = sgn1(df0), sp = sgn1(dfp);
+  const float qm = fabsf(sm + s0), qp = fabsf(s0 + sp);
+  return make_float2(fii - s0 * mx(0.0f, fabsf(dfl) - qm * fabsf(dfm)),
+                     fii + s0 * mx(0.0f, fabsf(dfr) - qp * fabsf(dfp)));
+}
+__device__ __forceinline__ void pdm_pair_general(float2 fm2, float2 fm1, float2 f0, float2 fp1, float2 fi, float pdmb,
+                                                 float2& lr0, float2& lr1) {
+  const float2 kp = p2::K(pdmb);
+  const float2 dfm = p2::mul(kp, p2::sub(fm1, fm2));
+  const float2 df0 = p2::mul(kp, p2::sub(f0, fm1));
+  const float2 dfp = p2::mul(kp, p2::sub(fp1, f0));
+  const float2 fii = make_float2(mx(mn(fm1.x, f0.x), mn(fi.x, mx(fm1.x, f0.x))),
+                                 mx(mn(fm1.y, f0.y), mn(fi.y, mx(fm1.y, f0.y))));
+  const float2 dfl = p2::sub(fii, fm1), dfr = p2::sub(f0, fii);
+  lr0 = pdm_general_lim(fii.x, dfl.x, dfr.x, dfm.x, df0.x, dfp.x);
+  lr1 = pdm_general_lim(fii.y, dfl.y, dfr.y, dfm.y, df0.y, dfp.y);
+}
+
 // PDM face states of two fields (lanes .x and .y) from their 8-tap windows (tap
 // m = cell c+m-4 for the face at the low side of cell c): pdm_states with the
 // differences on the packed pipe, the clamps and thresholds per lane.  lr0 /
 // lr1 are the (left, right) states of lane x / lane y.
+template <int RECON>
 __device__ __forceinline__ void pdm_pair_states(const float2* a, float pdmb, float2& lr0, float2& lr1) {
   const float2 fi = tap8p(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7]);
+  if constexpr (RECON != R_PDM) return pdm_pair_general(a[2], a[3], a[4], a[5], fi, pdmb, lr0, lr1);
   const float2 fm2 = a[2], fm1 = a[3], f0 = a[4], fp1 = a[5], k = p2::K(pdmb + pdmb);
   const float2 Dl = p2::mul(k, p2::sub(fm1, fm2)), Dr = p2::mul(k, p2::sub(f0, fp1));
   const float2 x = make_float2(clamp2(fm1.x, f0.x, fi.x), clamp2(fm1.y, f0.y, fi.y));
@@ -1589,7 +1619,7 @@ __device__ __forceinline__ void recon_win(const T* w, const Prm<T>& P, T& fl, T&
 // c along stride s (recon_face per field); FP32 PDM on field pairs.
 template <typename T, int RECON, bool M, typename I>
 __device__ __forceinline__ void face_states(const T* const* src, I c, I s, const Prm<T>& P, T* L, T* R) {
-  if constexpr (std::is_same<T, float>::value && RECON == R_PDM && MHD_RECON_PACKED) {
+  if constexpr (std::is_same<T, float>::value && is_pdm(RECON) && MHD_RECON_PACKED) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const float *fa = src[2 * q], *fb = src[2 * q + 1];
@@ -1597,7 +1627,7 @@ __device__ __forceinline__ void face_states(const T* const* src, I c, I s, const
 #pragma unroll
       for (int m = 0; m < 8; ++m) a[m] = make_float2(fa[c + (m - 4) * s], fb[c + (m - 4) * s]);
       float2 lr0, lr1;
-      pdm_pair_states(a, P.pdmb, lr0, lr1);
+      pdm_pair_states<RECON>(a, P.pdmb, lr0, lr1);
       L[2 * q] = lr0.x; R[2 * q] = lr0.y;
       L[2 * q + 1] = lr1.x; R[2 * q + 1] = lr1.y;
     }
@@ -2106,11 +2136,11 @@ __global__ void __launch_bounds__(128, kSweepMinB)
       asm volatile("cp.async.commit_group;" ::: "memory");
     }
     T L[8], R[8], F[8];
-    if constexpr (std::is_same<T, float>::value && RECON == R_PDM && MHD_RECON_PACKED) {
+    if constexpr (std::is_same<T, float>::value && is_pdm(RECON) && MHD_RECON_PACKED) {
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         float2 lr0, lr1;
-        pdm_pair_states(w[q], P.pdmb, lr0, lr1);
+        pdm_pair_states<RECON>(w[q], P.pdmb, lr0, lr1);
         L[2 * q] = lr0.x; R[2 * q] = lr0.y;
         L[2 * q + 1] = lr1.x; R[2 * q + 1] = lr1.y;
       }
@@ -2268,7 +2298,7 @@ inline dim3 emf_grid(int E, const Geom& g, int tx, int ty, int tz) {
               emf_edge_tiles(ez, tz, emf_merges(E, 2)));
 }
 
-template <typename T, int E, int TX, int TY, int TZ, bool M>
+template <typename T, int RECON, int E, int TX, int TY, int TZ, bool M>
 __device__ __forceinline__ void emf_pdm_tile(const Dev<T>& d, const Inp<T>& in, const Prm<T>& P, int ox, int oy,
                                              int oz) {
   constexpr int A1 = (E + 1) % 3, A2 = (E + 2) % 3;
@@ -2345,12 +2375,12 @@ __device__ __forceinline__ void emf_pdm_tile(const Dev<T>& d, const Inp<T>& in, 
     constexpr int GS = G2;
     const V vi = tap8p(gg[0], gg[GS], gg[2 * GS], gg[3 * GS], gg[4 * GS], gg[5 * GS], gg[6 * GS], gg[7 * GS]);
     T v1av, v2av;
-    corner_pdm_pair<T>(sv, cv, S1, S2, vi, P.pdmb, v1av, v2av);
+    corner_pdm_pair<T, RECON>(sv, cv, S1, S2, vi, P.pdmb, v1av, v2av);
     const int c = gx + g.px * (gy + g.py * gz);
     const int s1 = st[A1], s2 = st[A2];
     T b1l, b1r, b2l, b2r;
-    recon_edge<T, R_PDM>(fb[A1], c, s2, P, b1l, b1r);
-    recon_edge<T, R_PDM>(fb[A2], c, s1, P, b2l, b2r);
+    recon_edge<T, RECON>(fb[A1], c, s2, P, b1l, b1r);
+    recon_edge<T, RECON>(fb[A2], c, s1, P, b2l, b2r);
     const T* vf = d.vf;
     const T eta = eta4(vf[c - s1 - s2], vf[c - s2], vf[c], vf[c - s1]);
     d.E[E][c] = emf_value<T, E, M>(d, c, v1av, v2av, b1l, b1r, b2l, b2r, eta);
@@ -2371,7 +2401,7 @@ template <typename T>
 constexpr int emf_min_blocks(int E, int NT, bool B) {
   return !MHD_EMF_FULL_OCC ? 1 : sizeof(T) == 8 ? 1024 / NT : !B ? 2048 / NT : (E == 0 ? 1024 / NT : 1536 / NT);
 }
-template <typename T, int E, int TX, int TY, int TZ, int NT, bool M, bool B>
+template <typename T, int RECON, int E, int TX, int TY, int TZ, int NT, bool M, bool B>
 __global__ void __launch_bounds__(NT, emf_min_blocks<T>(E, NT, B))
     k_emf_pdm(KArg<T, B> ka, Inp<T> in0, Prm<T> P) {
   const int4 bb = ka.blk();
@@ -2380,7 +2410,7 @@ __global__ void __launch_bounds__(NT, emf_min_blocks<T>(E, NT, B))
   const Geom& g = d.g;
   const int ox = g.ng + bb.y * TX, oy = g.ng + bb.z * TY, oz = g.ng + bb.w * TZ;
   if constexpr (E == 0) {
-    emf_pdm_tile<T, E, TX, TY, TZ, M>(d, in, P, ox, oy, oz);
+    emf_pdm_tile<T, RECON, E, TX, TY, TZ, M>(d, in, P, ox, oy, oz);
   } else {
     // transverse axes a1, a2: is this block the widened last tile of the axis?
     constexpr int A1 = (E + 1) % 3, A2 = (E + 2) % 3;
@@ -2391,27 +2421,27 @@ __global__ void __launch_bounds__(NT, emf_min_blocks<T>(E, NT, B))
     const bool w2 = tl[A2] > 1 && n0[A2] - org[A2] == tl[A2];
     constexpr int X1 = A1 == 0, Y1 = A1 == 1, Z1 = A1 == 2, X2 = A2 == 0, Y2 = A2 == 1, Z2 = A2 == 2;
     if (w1 && w2)
-      emf_pdm_tile<T, E, TX + X1 + X2, TY + Y1 + Y2, TZ + Z1 + Z2, M>(d, in, P, ox, oy, oz);
+      emf_pdm_tile<T, RECON, E, TX + X1 + X2, TY + Y1 + Y2, TZ + Z1 + Z2, M>(d, in, P, ox, oy, oz);
     else if (w1)
-      emf_pdm_tile<T, E, TX + X1, TY + Y1, TZ + Z1, M>(d, in, P, ox, oy, oz);
+      emf_pdm_tile<T, RECON, E, TX + X1, TY + Y1, TZ + Z1, M>(d, in, P, ox, oy, oz);
     else if (w2)
-      emf_pdm_tile<T, E, TX + X2, TY + Y2, TZ + Z2, M>(d, in, P, ox, oy, oz);
+      emf_pdm_tile<T, RECON, E, TX + X2, TY + Y2, TZ + Z2, M>(d, in, P, ox, oy, oz);
     else
-      emf_pdm_tile<T, E, TX, TY, TZ, M>(d, in, P, ox, oy, oz);
+      emf_pdm_tile<T, RECON, E, TX, TY, TZ, M>(d, in, P, ox, oy, oz);
   }
 }
 
-template <typename T, int E, int TX, int TY, int TZ, int NT, bool M>
+template <typename T, int RECON, int E, int TX, int TY, int TZ, int NT, bool M>
 void launch_emf_pdm(const Dev<T>& d, const Inp<T>& in, const Prm<T>& P, cudaStream_t st) {
   constexpr size_t bytes = emf_pdm_smem<T, E, TX, TY, TZ>();
   static PerDevice attr;
   unsigned long long bit = 0;
   if (attr.need(bit)) {
-    cudaFuncSetAttribute(k_emf_pdm<T, E, TX, TY, TZ, NT, M, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_emf_pdm<T, RECON, E, TX, TY, TZ, NT, M, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)bytes);
     attr.mark(bit);
   }
-  k_emf_pdm<T, E, TX, TY, TZ, NT, M, false><<<emf_grid(E, d.g, TX, TY, TZ), NT, bytes, st>>>(one(d), in, P);
+  k_emf_pdm<T, RECON, E, TX, TY, TZ, NT, M, false><<<emf_grid(E, d.g, TX, TY, TZ), NT, bytes, st>>>(one(d), in, P);
 }
 
 // ------------------------------------------------------ streamed PDM EMF
@@ -2462,7 +2492,7 @@ __device__ __forceinline__ void cp_async_zfill(uint32_t dst, const T* src, bool 
 #ifndef MHD_EMF_STREAM_MINB
 #define MHD_EMF_STREAM_MINB 3
 #endif
-template <typename T, int E, int NW, bool M, bool B>
+template <typename T, int RECON, int E, int NW, bool M, bool B>
 __global__ void __launch_bounds__(32 * NW, MHD_EMF_STREAM_MINB)
     k_emf_stream(KArg<T, B> ka, Inp<T> in0, Prm<T> P) {
   const int4 bb = ka.blk();
@@ -2603,13 +2633,14 @@ __global__ void __launch_bounds__(32 * NW, MHD_EMF_STREAM_MINB)
       m10 = sm1[0]; m20 = sm2[0]; m1p = sm1[1]; c0 = s00[0]; p10 = sp1[0]; p01 = s00[1];
     }
     T v1av, v2av;
-    corner_pdm_vals2<T>(m11, m21, m12, m01, p11, m02, m10, m20, m1p, c0, p10, p01, vi, P.pdmb, v1av, v2av);
+    corner_pdm_vals2<T, RECON>(m11, m21, m12, m01, p11, m02, m10, m20, m1p, c0, p10, p01, vi, P.pdmb, v1av, v2av);
     // face B: across the slice from the staged slice, along S from the window
     constexpr int BS = SA2 ? TS : 1;
     const T* bb = br + (s & 1) * NS + oi;
     T sl, sr, wl, wr;
-    recon_pdm8<T, R_PDM, true>(bb[-4 * BS], bb[-3 * BS], bb[-2 * BS], bb[-BS], bb[0], bb[BS], bb[2 * BS], bb[3 * BS], P.pdmb, sl, sr);
-    recon_pdm8<T, R_PDM, true>(bw[0], bw[1], bw[2], bw[3], bw[4], bw[5], bw[6], bw[7], P.pdmb, wl, wr);
+    recon_pdm8<T, RECON, true>(bb[-4 * BS], bb[-3 * BS], bb[-2 * BS], bb[-BS], bb[0], bb[BS], bb[2 * BS], bb[3 * BS],
+                               P.pdmb, sl, sr);
+    recon_pdm8<T, RECON, true>(bw[0], bw[1], bw[2], bw[3], bw[4], bw[5], bw[6], bw[7], P.pdmb, wl, wr);
     const T* f0 = fr + (s & 3) * NS + oi;
     const T* fm = fr + ((s - 1) & 3) * NS + oi;
     T eta;
@@ -2653,7 +2684,7 @@ constexpr size_t emf_rows_smem() {
                    c = emf_pdm_smem<T, 1, 1, 8, 32>();
   return a > b ? (a > c ? a : c) : (b > c ? b : c);
 }
-template <typename T, bool M, bool B>
+template <typename T, int RECON, bool M, bool B>
 __global__ void __launch_bounds__(256) k_emf_rows(KArg<T, B> ka, Inp<T> in0, Prm<T> P) {
   const int4 bb = ka.blk();
   const auto& d = ka.dev(bb);
@@ -2663,18 +2694,18 @@ __global__ void __launch_bounds__(256) k_emf_rows(KArg<T, B> ka, Inp<T> in0, Prm
   int b = bb.y;
   if (b < r.bi) {
     const int nbx = (g.nx0 + 31) / 32, bx = b % nbx, bz = b / nbx;
-    emf_pdm_tile<T, 0, 32, 1, 8, M>(d, in, P, g.ng + 32 * bx, g.ng + g.ny0, g.ng + 8 * bz);
+    emf_pdm_tile<T, RECON, 0, 32, 1, 8, M>(d, in, P, g.ng + 32 * bx, g.ng + g.ny0, g.ng + 8 * bz);
     return;
   }
   b -= r.bi;
   if (b < r.bk) {
     const int nby = (g.ny0 + 32) / 32, by = b % nby, bz = b / nby;
-    emf_pdm_tile<T, 2, 1, 32, 8, M>(d, in, P, g.ng + g.nx0, g.ng + 32 * by, g.ng + 8 * bz);
+    emf_pdm_tile<T, RECON, 2, 1, 32, 8, M>(d, in, P, g.ng + g.nx0, g.ng + 32 * by, g.ng + 8 * bz);
     return;
   }
   b -= r.bk;
   const int nby = (g.ny0 + 7) / 8, by = b % nby, bz = b / nby;
-  emf_pdm_tile<T, 1, 1, 8, 32, M>(d, in, P, g.ng + g.nx0, g.ng + 8 * by, g.ng + 32 * bz);
+  emf_pdm_tile<T, RECON, 1, 1, 8, 32, M>(d, in, P, g.ng + g.nx0, g.ng + 8 * by, g.ng + 32 * bz);
 }
 
 // blocks of streamed family E on one grid (x tiles, warp-axis tiles, segments)
@@ -2683,30 +2714,31 @@ inline dim3 emf_stream_grid(int E, const Geom& g, int seg) {
   return dim3((g.nx0 + 31) / 32, (nW0 + MHD_EMF_NW - 1) / MHD_EMF_NW,
               emf_stream_segs(nS0, seg));
 }
-template <typename T, int E, bool M, bool B>
+template <typename T, int RECON, int E, bool M, bool B>
 void stream_attr() {
   static PerDevice attr;
   unsigned long long bit = 0;
   if (attr.need(bit)) {
-    cudaFuncSetAttribute(k_emf_stream<T, E, MHD_EMF_NW, M, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_emf_stream<T, RECON, E, MHD_EMF_NW, M, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)EmfStream<T, E, MHD_EMF_NW>::smem);
     attr.mark(bit);
   }
 }
-template <typename T, int E, bool M>
+template <typename T, int RECON, int E, bool M>
 void launch_emf_stream(const Dev<T>& d, const Inp<T>& in, const Prm<T>& P, cudaStream_t st) {
   typedef EmfStream<T, E, MHD_EMF_NW> K;
-  stream_attr<T, E, M, false>();
-  k_emf_stream<T, E, MHD_EMF_NW, M, false><<<emf_stream_grid(E, d.g, d.eseg[E]), K::NT, K::smem, st>>>(one(d), in, P);
+  stream_attr<T, RECON, E, M, false>();
+  k_emf_stream<T, RECON, E, MHD_EMF_NW, M, false>
+      <<<emf_stream_grid(E, d.g, d.eseg[E]), K::NT, K::smem, st>>>(one(d), in, P);
 }
 
-template <typename T, bool M>
+template <typename T, int RECON, bool M>
 void emf_pdm_stream(const Dev<T>& d, const Inp<T>& in, const Prm<T>& P, cudaStream_t st) {
-  launch_emf_stream<T, 0, M>(d, in, P, st);
-  launch_emf_stream<T, 1, M>(d, in, P, st);
-  launch_emf_stream<T, 2, M>(d, in, P, st);
+  launch_emf_stream<T, RECON, 0, M>(d, in, P, st);
+  launch_emf_stream<T, RECON, 1, M>(d, in, P, st);
+  launch_emf_stream<T, RECON, 2, M>(d, in, P, st);
   static_assert(emf_rows_smem<T>() <= 48 * 1024, "k_emf_rows fits the default shared-memory limit");
-  k_emf_rows<T, M, false><<<EmfRows(d.g).blocks(), 256, emf_rows_smem<T>(), st>>>(one(d), in, P);
+  k_emf_rows<T, RECON, M, false><<<EmfRows(d.g).blocks(), 256, emf_rows_smem<T>(), st>>>(one(d), in, P);
 }
 
 // ------------------------------------------------------------- WENO EMF
@@ -3049,7 +3081,7 @@ __device__ __forceinline__ void emf64_weno(const Dev<double>& d, const Inp<doubl
   }
 }
 
-template <int E, bool M>
+template <int RECON, int E, bool M>
 __device__ __forceinline__ void emf64_pdm(const Dev<double>& d, const Inp<double>& in, const Prm<double>& P,
                                           const Tile64& w, int blk, double* sv) {
   constexpr int A1 = (E + 1) % 3, A2 = (E + 2) % 3;
@@ -3081,11 +3113,11 @@ __device__ __forceinline__ void emf64_pdm(const Dev<double>& d, const Inp<double
       const double* q = sg + ((k * te + e) * c2 + f2) * t1 + f1;
       const double vi = tap8(q[0], q[t1], q[2 * t1], q[3 * t1], q[4 * t1], q[5 * t1], q[6 * t1], q[7 * t1]);
       const double* v = sv + ((k * te + e) * c2 + f2 + 4) * c1 + f1 + 4;
-      sq[t] = corner_pdm<double, R_PDM>(v, 0, 1, c1, vi, P.pdmb);
+      sq[t] = corner_pdm<double, RECON>(v, 0, 1, c1, vi, P.pdmb);
     } else {
       const int s = k == 2 ? st2 : st1;
       double l, rr;
-      recon_edge<double, R_PDM>(k == 2 ? fb[A1] : fb[A2], p.org + e * p.se + f1 * st1 + f2 * st2, s, P, l, rr);
+      recon_edge<double, RECON>(k == 2 ? fb[A1] : fb[A2], p.org + e * p.se + f1 * st1 + f2 * st2, s, P, l, rr);
       sq[(2 * k - 2) * ned + u] = l;
       sq[(2 * k - 1) * ned + u] = rr;
     }
@@ -3109,7 +3141,7 @@ __global__ void __launch_bounds__(256) k_emf64(Dev<double> d, Inp<double> in, Pr
   auto tile = [&](auto fam, int blk) {
     constexpr int E = decltype(fam)::value;
     if constexpr (is_weno(RECON)) emf64_weno<RECON, E, M>(d, in, P, w.f[E], blk, sm);
-    else emf64_pdm<E, M>(d, in, P, w.f[E], blk, sm);
+    else emf64_pdm<RECON, E, M>(d, in, P, w.f[E], blk, sm);
   };
   if (b < w.blocks[0]) return tile(std::integral_constant<int, 0>{}, b);
   b -= w.blocks[0];
@@ -3805,7 +3837,7 @@ void launch_flux_t(const Dev<T>& d, const Inp<T>& in, const Prm<T>& P, int form,
 // for the FP32 Cartesian PDM path (chosen by the autotuner), 8 elsewhere.
 template <typename T, int RECON, bool M>
 constexpr bool tunable() {
-  return std::is_same<T, float>::value && RECON == R_PDM && !M;
+  return std::is_same<T, float>::value && is_pdm(RECON) && !M;
 }
 
 inline dim3 sweep_grid(int D, const Geom& g, int seg) {
@@ -3815,9 +3847,9 @@ inline dim3 sweep_grid(int D, const Geom& g, int seg) {
 
 template <typename T, int RECON, int D, bool M>
 void flux_t_any(const Dev<T>& d, const Inp<T>& in, const Prm<T>& P, int form, T c, T den, int ab, cudaStream_t st) {
-  if constexpr (std::is_same<T, float>::value && !M && RECON != R_PDMG) {
-    if (d.tile_td == kSweepTile) {  // column sweeps (every FP32 Cartesian reconstruction with a register window)
-      static PerDevice pref;  // 4 blocks of 27 KB static shared memory
+  if constexpr (std::is_same<T, float>::value && !M) {
+    if (d.tile_td == kSweepTile) {  // column sweeps
+      static PerDevice pref;  // 4 blocks of 20 (y) or 22 KB (z) static shared memory
       prefer_carveout(k_flux_sweep<T, D, false, RECON>, 50, pref);
       k_flux_sweep<T, D, false, RECON><<<sweep_grid(D, d.g, d.seg[D - 1]), dim3(32, 4), 0, st>>>(one(d), in, P, form, c, den);
       return;
@@ -4017,6 +4049,28 @@ template <typename T> struct EiTile { static constexpr int Y = MHD_EI_TILE; };
 constexpr int ei_x(int y) { return y == 8 ? MHD_EI_X : 32; }
 template <> struct EiTile<double> { static constexpr int Y = 4; };
 
+template <typename T, int RECON, bool M>
+void emf_pdm(const Dev<T>& d, const Inp<T>& in, cudaStream_t st) {
+  Prm<T> P = prm_of(d);
+  // (the metric mode keeps the tiles: beside the streams its face tiles ran a third slower)
+  if constexpr (std::is_same<T, float>::value && !M) {
+    if (d.tile_ey == kEmfStream) {
+      emf_pdm_stream<T, RECON, M>(d, in, P, st);
+      return;
+    }
+  }
+  if constexpr (std::is_same<T, double>::value) {
+    launch_emf64<RECON, M>(d, in, P, st);
+  } else {
+    if (!M && d.tile_ey == 4)
+      launch_emf_pdm<T, RECON, 0, 32, 4, 4, 512, M>(d, in, P, st);
+    else
+      launch_emf_pdm<T, RECON, 0, ei_x(EiTile<T>::Y), EiTile<T>::Y, EiTile<T>::Y, 512, M>(d, in, P, st);
+    launch_emf_pdm<T, RECON, 1, 32, 1, kPT, 32 * kPT, M>(d, in, P, st);
+    launch_emf_pdm<T, RECON, 2, 32, kPT, 1, 32 * kPT, M>(d, in, P, st);
+  }
+}
+
 template <typename T, bool M>
 void Launch<T, M>::emf(const Dev<T>& d, const Inp<T>& in0, cudaStream_t st) {
   if constexpr (!M) {  // Yee: Cartesian only (checked at mhd_init)
@@ -4034,29 +4088,9 @@ void Launch<T, M>::emf(const Dev<T>& d, const Inp<T>& in0, cudaStream_t st) {
     in.vx = d.mw[0]; in.vy = d.mw[1]; in.vz = d.mw[2];
     in.bi = d.mbn[0]; in.bj = d.mbn[1]; in.bk = d.mbn[2];
   }
-  if (d.recon == R_PDM) {
-    Prm<T> P = prm_of(d);
-    // (the metric mode keeps the tiles: beside the streams its face tiles ran a third slower)
-    if constexpr (std::is_same<T, float>::value && !M) {
-      if (d.tile_ey == kEmfStream) {
-        emf_pdm_stream<T, M>(d, in, P, st);
-        return;
-      }
-    }
-    if constexpr (std::is_same<T, double>::value) {
-      launch_emf64<R_PDM, M>(d, in, P, st);
-    } else {
-      if (!M && d.tile_ey == 4)
-        launch_emf_pdm<T, 0, 32, 4, 4, 512, M>(d, in, P, st);
-      else
-        launch_emf_pdm<T, 0, ei_x(EiTile<T>::Y), EiTile<T>::Y, EiTile<T>::Y, 512, M>(d, in, P, st);
-      launch_emf_pdm<T, 1, 32, 1, kPT, 32 * kPT, M>(d, in, P, st);
-      launch_emf_pdm<T, 2, 32, kPT, 1, 32 * kPT, M>(d, in, P, st);
-    }
-    return;
-  }
   switch (d.recon) {
-    case R_PDMG: emf_r<T, R_PDMG, M>(d, in, st); break;
+    case R_PDM: emf_pdm<T, R_PDM, M>(d, in, st); break;
+    case R_PDMG: emf_pdm<T, R_PDMG, M>(d, in, st); break;
     case R_TVD: emf_r<T, R_TVD, M>(d, in, st); break;
     case R_WENO: emf_weno<T, R_WENO, M>(d, in, st); break;
     case R_MPWENO: emf_weno<T, R_MPWENO, M>(d, in, st); break;
@@ -4118,7 +4152,7 @@ void set_smem(K kernel, size_t bytes) {
 }
 
 // Batched EMF families with ei tile Y (edges along y and z per block).
-template <typename T, int Y>
+template <typename T, int RECON, int Y>
 void batch_emf(const BatchView& v, const Dev<T>* tab, const Prm<T>& P, cudaStream_t st) {
   constexpr int X = ei_x(Y);
   constexpr size_t si = emf_pdm_smem<T, 0, X, Y, Y>();
@@ -4127,54 +4161,91 @@ void batch_emf(const BatchView& v, const Dev<T>* tab, const Prm<T>& P, cudaStrea
   static PerDevice attr;
   unsigned long long bit = 0;
   if (attr.need(bit)) {
-    set_smem(k_emf_pdm<T, 0, X, Y, Y, 512, false, true>, si);
-    set_smem(k_emf_pdm<T, 1, 32, 1, kPT, 32 * kPT, false, true>, sj);
-    set_smem(k_emf_pdm<T, 2, 32, kPT, 1, 32 * kPT, false, true>, sk);
+    set_smem(k_emf_pdm<T, RECON, 0, X, Y, Y, 512, false, true>, si);
+    set_smem(k_emf_pdm<T, RECON, 1, 32, 1, kPT, 32 * kPT, false, true>, sj);
+    set_smem(k_emf_pdm<T, RECON, 2, 32, kPT, 1, 32 * kPT, false, true>, sk);
     attr.mark(bit);
   }
   const Inp<T> none{};
-  k_emf_pdm<T, 0, X, Y, Y, 512, false, true><<<v.nblk[BF_EMF_I], 512, si, st>>>(
+  k_emf_pdm<T, RECON, 0, X, Y, Y, 512, false, true><<<v.nblk[BF_EMF_I], 512, si, st>>>(
       KArg<T, true>{tab, v.map[BF_EMF_I]}, none, P);
-  k_emf_pdm<T, 1, 32, 1, kPT, 32 * kPT, false, true><<<v.nblk[BF_EMF_J], 32 * kPT, sj, st>>>(
+  k_emf_pdm<T, RECON, 1, 32, 1, kPT, 32 * kPT, false, true><<<v.nblk[BF_EMF_J], 32 * kPT, sj, st>>>(
       KArg<T, true>{tab, v.map[BF_EMF_J]}, none, P);
-  k_emf_pdm<T, 2, 32, kPT, 1, 32 * kPT, false, true><<<v.nblk[BF_EMF_K], 32 * kPT, sk, st>>>(
+  k_emf_pdm<T, RECON, 2, 32, kPT, 1, 32 * kPT, false, true><<<v.nblk[BF_EMF_K], 32 * kPT, sk, st>>>(
       KArg<T, true>{tab, v.map[BF_EMF_K]}, none, P);
 }
 
 // Batched slice-streamed EMF families and their boundary rows.
-template <typename T>
+template <typename T, int RECON>
 void batch_emf_stream(const BatchView& v, const Dev<T>* tab, const Prm<T>& P, cudaStream_t st) {
-  stream_attr<T, 0, false, true>();
-  stream_attr<T, 1, false, true>();
-  stream_attr<T, 2, false, true>();
+  stream_attr<T, RECON, 0, false, true>();
+  stream_attr<T, RECON, 1, false, true>();
+  stream_attr<T, RECON, 2, false, true>();
   const Inp<T> none{};
   constexpr int NT = 32 * MHD_EMF_NW;
-  k_emf_stream<T, 0, MHD_EMF_NW, false, true><<<v.nblk[BF_EMF_I], NT, EmfStream<T, 0, MHD_EMF_NW>::smem, st>>>(
+  k_emf_stream<T, RECON, 0, MHD_EMF_NW, false, true><<<v.nblk[BF_EMF_I], NT, EmfStream<T, 0, MHD_EMF_NW>::smem, st>>>(
       KArg<T, true>{tab, v.map[BF_EMF_I]}, none, P);
-  k_emf_stream<T, 1, MHD_EMF_NW, false, true><<<v.nblk[BF_EMF_J], NT, EmfStream<T, 1, MHD_EMF_NW>::smem, st>>>(
+  k_emf_stream<T, RECON, 1, MHD_EMF_NW, false, true><<<v.nblk[BF_EMF_J], NT, EmfStream<T, 1, MHD_EMF_NW>::smem, st>>>(
       KArg<T, true>{tab, v.map[BF_EMF_J]}, none, P);
-  k_emf_stream<T, 2, MHD_EMF_NW, false, true><<<v.nblk[BF_EMF_K], NT, EmfStream<T, 2, MHD_EMF_NW>::smem, st>>>(
+  k_emf_stream<T, RECON, 2, MHD_EMF_NW, false, true><<<v.nblk[BF_EMF_K], NT, EmfStream<T, 2, MHD_EMF_NW>::smem, st>>>(
       KArg<T, true>{tab, v.map[BF_EMF_K]}, none, P);
-  k_emf_rows<T, false, true><<<v.nblk[BF_EMF_R], 256, emf_rows_smem<T>(), st>>>(
+  k_emf_rows<T, RECON, false, true><<<v.nblk[BF_EMF_R], 256, emf_rows_smem<T>(), st>>>(
       KArg<T, true>{tab, v.map[BF_EMF_R]}, none, P);
 }
 
 // Batched y / z face tiles of length TDV.
-template <typename T, int TDV>
+template <typename T, int RECON, int TDV>
 void batch_flux_t(const BatchView& v, const Dev<T>* tab, const Prm<T>& P, int form, T c, T den, cudaStream_t st) {
   constexpr size_t sf = flux_t_smem<T, TDV>();
   static PerDevice attr;
   unsigned long long bit = 0;
   if (attr.need(bit)) {
-    set_smem(k_flux_t<T, R_PDM, 1, false, true, TDV>, sf);
-    set_smem(k_flux_t<T, R_PDM, 2, false, true, TDV>, sf);
+    set_smem(k_flux_t<T, RECON, 1, false, true, TDV>, sf);
+    set_smem(k_flux_t<T, RECON, 2, false, true, TDV>, sf);
     attr.mark(bit);
   }
   const Inp<T> none{};
-  k_flux_t<T, R_PDM, 1, false, true, TDV><<<v.nblk[BF_FLUX_Y], dim3(32, TDV + 1), sf, st>>>(
+  k_flux_t<T, RECON, 1, false, true, TDV><<<v.nblk[BF_FLUX_Y], dim3(32, TDV + 1), sf, st>>>(
       KArg<T, true>{tab, v.map[BF_FLUX_Y]}, none, P, -1, T(0), T(1), 0);
-  k_flux_t<T, R_PDM, 2, false, true, TDV><<<v.nblk[BF_FLUX_Z], dim3(32, TDV + 1), sf, st>>>(
+  k_flux_t<T, RECON, 2, false, true, TDV><<<v.nblk[BF_FLUX_Z], dim3(32, TDV + 1), sf, st>>>(
       KArg<T, true>{tab, v.map[BF_FLUX_Z]}, none, P, form, c, den, 0);
+}
+
+// Parts 1 (EMF families) and 2 (face fluxes and the conserved update) of Batch::parts.
+template <typename T, int RECON>
+void batch_emf_and_faces(const BatchView& v, const Dev<T>* tab, const Prm<T>& P, int which, int form, T c, T den,
+                         cudaStream_t st) {
+  constexpr bool F32 = std::is_same<T, float>::value;
+  if (which & 1) {
+    if constexpr (F32) {
+      if (v.tile_ey == kEmfStream) batch_emf_stream<T, RECON>(v, tab, P, st);
+      else if (v.tile_ey == 4) batch_emf<T, RECON, 4>(v, tab, P, st);
+      else batch_emf<T, RECON, EiTile<T>::Y>(v, tab, P, st);
+    } else {
+      batch_emf<T, RECON, EiTile<T>::Y>(v, tab, P, st);
+    }
+  }
+  if (which & 2) {
+    const Inp<T> none{};
+    k_flux<T, RECON, 0, false, true>
+        <<<v.nblk[BF_FLUX_X], 128, 0, st>>>(KArg<T, true>{tab, v.map[BF_FLUX_X]}, none, P);
+    if constexpr (F32) {
+      if (v.tile_td == kSweepTile) {
+        k_flux_sweep<T, 1, true, RECON><<<v.nblk[BF_FLUX_Y], dim3(32, 4), 0, st>>>(
+            KArg<T, true>{tab, v.map[BF_FLUX_Y]}, none, P, -1, T(0), T(1));
+        k_flux_sweep<T, 2, true, RECON><<<v.nblk[BF_FLUX_Z], dim3(32, 4), 0, st>>>(
+            KArg<T, true>{tab, v.map[BF_FLUX_Z]}, none, P, form, c, den);
+      } else if (v.tile_td == 4) {
+        batch_flux_t<T, RECON, 4>(v, tab, P, form, c, den, st);
+      } else if (v.tile_td == 16) {
+        batch_flux_t<T, RECON, 16>(v, tab, P, form, c, den, st);
+      } else {
+        batch_flux_t<T, RECON, TD>(v, tab, P, form, c, den, st);
+      }
+    } else {
+      batch_flux_t<T, RECON, TD>(v, tab, P, form, c, den, st);
+    }
+  }
 }
 
 template <typename T>
@@ -4183,34 +4254,8 @@ void Batch<T>::parts(const BatchView& v, int sel, int which, int form, double c,
   // the batch shares the deck's limiter constants (checked when it is built)
   Prm<T> P;
   P.pdmb = (T)v.pdmb; P.eps = (T)v.eps; P.alpha = (T)v.alpha; P.beta = (T)v.beta; P.tvd_shift = v.tvd_shift;
-  constexpr bool F32 = std::is_same<T, float>::value;
-  if (which & 1) {  // EMF families
-    if constexpr (F32) {
-      if (v.tile_ey == kEmfStream) {
-        batch_emf_stream<T>(v, tab, P, st);
-        return parts(v, sel, which & ~1, form, c, den, st);
-      }
-    }
-    if (F32 && v.tile_ey == 4) batch_emf<T, 4>(v, tab, P, st);
-    else batch_emf<T, EiTile<T>::Y>(v, tab, P, st);
-  }
-  if (which & 2) {  // face fluxes and the conserved update
-    const Inp<T> none{};
-    k_flux<T, R_PDM, 0, false, true><<<v.nblk[BF_FLUX_X], 128, 0, st>>>(KArg<T, true>{tab, v.map[BF_FLUX_X]}, none,
-                                                                       P);
-    if constexpr (F32) {
-      if (v.tile_td == kSweepTile) {
-        k_flux_sweep<T, 1, true><<<v.nblk[BF_FLUX_Y], dim3(32, 4), 0, st>>>(KArg<T, true>{tab, v.map[BF_FLUX_Y]}, none,
-                                                                             P, -1, T(0), T(1));
-        k_flux_sweep<T, 2, true><<<v.nblk[BF_FLUX_Z], dim3(32, 4), 0, st>>>(KArg<T, true>{tab, v.map[BF_FLUX_Z]}, none,
-                                                                             P, form, (T)c, (T)den);
-        return parts(v, sel, which & 4, form, c, den, st);
-      }
-    }
-    if (F32 && v.tile_td == 4) batch_flux_t<T, F32 ? 4 : TD>(v, tab, P, form, (T)c, (T)den, st);
-    else if (F32 && v.tile_td == 16) batch_flux_t<T, F32 ? 16 : TD>(v, tab, P, form, (T)c, (T)den, st);
-    else batch_flux_t<T, TD>(v, tab, P, form, (T)c, (T)den, st);
-  }
+  if (pdm_signless(P.pdmb)) batch_emf_and_faces<T, R_PDM>(v, tab, P, which, form, (T)c, (T)den, st);
+  else batch_emf_and_faces<T, R_PDMG>(v, tab, P, which, form, (T)c, (T)den, st);
   if (which & 4) {  // face-B update + bxyz + vf (interior), then the ghost shell of the half the stage wrote
     const int dt_next = (which & 8) ? 1 : 0;
     k_ct_fill<T, true><<<v.nblk[BF_CT], 256, 0, st>>>(KArg<T, true>{tab, v.map[BF_CT]}, form, (T)c, (T)den, 1, dt_next);

@@ -230,7 +230,10 @@ int mlp_status(void* h);
 constexpr unsigned kGaussRows = 32 * 13 / 2 + 1;
 constexpr int kGaussTerms = 10;
 void gauss_table(double* out);  // kGaussRows * 2 * kGaussTerms values (host)
-// Dev::recon of PDM with pdmb <= 0 (the general limiter; R_PDMG of the kernels).
+// Does the sign-free form of the PDM limiter hold for this constant (in the precision
+// of the step)?  It needs pdmb > 0.
+template <typename T> inline bool pdm_signless(T pdmb) { return pdmb > T(0); }
+// Dev::recon of PDM with any other constant (the general limiter; R_PDMG of the kernels).
 constexpr int kReconPdmGeneral = 6;
 // Tile lengths the autotuner tries (FP32 Cartesian PDM).
 constexpr int kSweepTile = 32;  // face-shape value of the column sweeps
