@@ -4,6 +4,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <cmath>
 #include <string>
 #include <vector>
 
@@ -231,8 +232,9 @@ constexpr unsigned kGaussRows = 32 * 13 / 2 + 1;
 constexpr int kGaussTerms = 10;
 void gauss_table(double* out);  // kGaussRows * 2 * kGaussTerms values (host)
 // Does the sign-free form of the PDM limiter hold for this constant (in the precision
-// of the step)?  It needs pdmb > 0.
-template <typename T> inline bool pdm_signless(T pdmb) { return pdmb > T(0); }
+// of the step)?  It needs pdmb > 0 and a finite 2 pdmb, its factor of the slopes
+// (a slope of zero times infinity would be NaN).
+template <typename T> inline bool pdm_signless(T pdmb) { return pdmb > T(0) && std::isfinite(pdmb + pdmb); }
 // Dev::recon of PDM with any other constant (the general limiter; R_PDMG of the kernels).
 constexpr int kReconPdmGeneral = 6;
 // Tile lengths the autotuner tries (FP32 Cartesian PDM).
