@@ -127,7 +127,9 @@ int mhd_step(void* handle, double* tau_inout, uint32_t* status);
 
 /* n steps back to back without host synchronisation in between (the driver's
  * inner `do nt=1,nts` loop, mhd3d3.f90:3284-3288).  status accumulates;
- * tau_out is output only (the dt of the last step). */
+ * tau_out is output only (the dt of the last step).  mhd_step, mhd_step_n and
+ * mhd_step_corrected launch a handle's first steps kernel by kernel and replay
+ * a captured step after those (same results). */
 int mhd_step_n(void* handle, int32_t nsteps, double* tau_out, uint32_t* status);
 
 /* Copy the current state back into ghost-inclusive FP64 Fortran arrays.  Any
@@ -160,8 +162,9 @@ int mhd_set_tau(void* handle, double tau);
 int mhd_set_profiling(void* handle, int32_t on);
 int mhd_last_timings(void* handle, float out_ms[8]);
 
-/* Enqueue nsteps (graph-replayed when use_graph != 0) between two CUDA events
- * recorded on the handle's stream; *ms = their elapsed device time. */
+/* Enqueue nsteps between two CUDA events recorded on the handle's stream, one
+ * replay of their graph when use_graph != 0, else launched kernel by kernel;
+ * *ms = their elapsed device time. */
 int mhd_time_steps(void* handle, int32_t nsteps, int32_t use_graph, float* ms);
 
 int mhd_free(void* handle);

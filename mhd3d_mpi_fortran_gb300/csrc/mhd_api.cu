@@ -476,8 +476,9 @@ bool step_replay(Handle* h, cudaGraphExec_t* ex) {
   return false;
 }
 
+// replay: a step may be replayed from a capture once the handle has run a few.
 template <typename T>
-int do_steps(Handle* h, int n) {
+int do_steps(Handle* h, int n, bool replay = true) {
   if (h->profile) {
     for (int i = 0; i < 8; ++i) h->tms[i] = 0;
     Rec r;
@@ -499,7 +500,7 @@ int do_steps(Handle* h, int n) {
   // replayed), so that once a handle has stepped a few times its step is captured
   // and replayed; handles that step less never pay for the capture.
   for (int s = 0; s < n; ++s) {
-    if (h->launched >= kReplayAfter && !h->no_replay) {
+    if (replay && h->launched >= kReplayAfter && !h->no_replay) {
       cudaGraphExec_t ex = nullptr;
       if (step_replay(h, &ex)) {
         CK(cudaGraphLaunch(ex, h->st));
@@ -1114,7 +1115,7 @@ int mhd_time_steps(void* handle, int32_t nsteps, int32_t use_graph, float* ms) {
   if (use_graph) {
     CK(cudaGraphLaunch(ex, h->st));
   } else {
-    int rc = h->fp32 ? do_steps<float>(h, nsteps) : do_steps<double>(h, nsteps);
+    int rc = h->fp32 ? do_steps<float>(h, nsteps, false) : do_steps<double>(h, nsteps, false);
     if (rc) return rc;
   }
   CK(cudaEventRecord(h->ev[1], h->st));

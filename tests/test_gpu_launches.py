@@ -82,7 +82,25 @@ def test_every_limiter_constant_takes_the_same_kernels(precision, n):
         assert child("limited", precision, n, pdmb) == some, pdmb
 
 
-PROGRAMS = {f.__name__: f for f in (limited,)}
+def timed(precision):
+    """Two timings of three steps without a graph, the second after more steps."""
+    with MHDSolver(Params(24, 16, 12, precision=precision, tau=1e-4), state((24, 16, 12))) as g:
+        g.time_steps(2)
+        one = traced(lambda: g.time_steps(3))
+        g.step(9)
+        return one, traced(lambda: g.time_steps(3))
+
+
+@pytest.mark.parametrize("precision", [FP32, FP64])
+def test_time_steps_without_a_graph_launches_the_kernels(precision):
+    """Steps timed without a graph are launched one by one, however many the handle has run."""
+    one, many = child("timed", precision)
+    assert sum(one[0].values()) > 0 and one[0] == many[0]
+    for k in ("cudaGraphLaunch", "cudaGraphInstantiate", "cudaStreamBeginCapture"):
+        assert not any(c.startswith(k) for c in many[1]), k
+
+
+PROGRAMS = {f.__name__: f for f in (limited, timed)}
 
 if __name__ == "__main__":
     name, *args = json.loads(sys.argv[1])
