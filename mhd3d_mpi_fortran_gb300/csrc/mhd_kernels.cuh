@@ -769,9 +769,9 @@ __device__ __forceinline__ float2 mul(float2 a, float2 b) { return __fmul2_rn(a,
 __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 // 1/x, 1/sqrt(x) and exp(-x) on the SFU alone: the .ftz forms, which drop the
 // rescaling of subnormal operands and results around each (two to three
-// instructions; a face takes 18 of these).  Same bits for normal numbers; below
-// 1.2e-38 (a pressure, or a tail of erfc or exp that is added to values of order one)
-// they are zero.
+// instructions; a face takes 18 of these).  Same bits for normal numbers; a
+// tail of erfc or exp below 1.2e-38 is zero, and an operand below it counts as zero: the
+// reciprocals and roots of lam check for that (lam_roots).
 __device__ __forceinline__ float rcp1(float x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -782,6 +782,17 @@ __device__ __forceinline__ float rsq1(float x) {
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
+// the same with subnormal operands
+__device__ __forceinline__ float rcp1s(float x) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rsq1s(float x) {
+  float r;
+  asm("rsqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 __device__ __forceinline__ float ex21(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -789,6 +800,25 @@ __device__ __forceinline__ float ex21(float x) {
 }
 __device__ __forceinline__ float2 rcp(float2 a) { return make_float2(rcp1(a.x), rcp1(a.y)); }
 __device__ __forceinline__ float2 rsq(float2 a) { return make_float2(rsq1(a.x), rsq1(a.y)); }
+// lam = r / q, ra = 1 / sqrt(lam), a = sqrt(lam) of two values of each of two q.  a ra is one,
+// to a few roundings, unless an operand was flushed (or lam is zero, infinite or NaN):
+// the forms with the rescaling decide then.  The check takes five instructions on the FMA
+// pipe, which has room, where the rescaling of eight operands takes about 20 on any.
+__device__ __forceinline__ void lam_roots(float2 r, float2 q, float2 qm, float2& lam, float2& ra, float2& a, float2& am) {
+  lam = mul(r, rcp(q));
+  ra = rsq(lam);
+  a = mul(lam, ra);
+  float2 lm = mul(r, rcp(qm)), rm = rsq(lm);
+  am = mul(lm, rm);
+  const float2 one = mul(mul(a, ra), mul(am, rm));
+  if (!(one.x * one.y < 2.0f)) {
+    lam = mul(r, make_float2(rcp1s(q.x), rcp1s(q.y)));
+    ra = make_float2(rsq1s(lam.x), rsq1s(lam.y));
+    a = mul(lam, ra);
+    lm = mul(r, make_float2(rcp1s(qm.x), rcp1s(qm.y)));
+    am = mul(lm, make_float2(rsq1s(lm.x), rsq1s(lm.y)));
+  }
+}
 __device__ __forceinline__ float2 exp_neg(float2 a) {
   a = mul(a, K(-1.4426950408889634f));
   return make_float2(ex21(a.x), ex21(a.y));
@@ -1299,17 +1329,17 @@ template <> struct Moments<float> {
     return direct ? h : 1.0f - h;
   }
   static __device__ __forceinline__ void hydro(float lam, float vn, bool left, float& v0, float& v1) {
-    float ra = p2::rsq1(lam);
+    float ra = p2::rsq1s(lam);
     float a = lam * ra;
     v0 = half_erfc(a * vn, left);
     float b = (0.5f * 0.56418958354775628f) * ra * p2::ex21(1.4426950408889634f * (-lam * vn * vn));
     v1 = left ? fmaf(vn, v0, b) : fmaf(vn, v0, -b);
   }
   static __device__ __forceinline__ float mag(float lam, float vn, bool left) {
-    float a = lam * p2::rsq1(lam);
+    float a = lam * p2::rsq1s(lam);
     return half_erfc(a * vn, left);
   }
-  static __device__ __forceinline__ float div(float a, float b) { return a * p2::rcp1(b); }
+  static __device__ __forceinline__ float div(float a, float b) { return a * p2::rcp1s(b); }
 };
 
 // ------------------------------------------------ FP32 packed-pair arithmetic
@@ -1395,9 +1425,12 @@ __device__ __forceinline__ void face_flux_lr(const float2* X, float rg, float* o
   ke = fma(w, w, ke);
   const float2 leng = fma(pr, K(rg), mul(mul(K(0.5f), r), ke));
   // hydro moments, lam = rho / (2 p)
-  const float2 lam = mul(r, rcp(mul(K(2.0f), pr)));
-  const float2 ra = rsq(lam);
-  const float2 v0 = half_erfc_lr(mul(mul(lam, ra), vn));
+  float2 lb = mul(bx, bx);
+  lb = fma(by, by, lb);
+  lb = fma(bz, bz, lb);
+  float2 lam, ra, a, am;
+  lam_roots(r, mul(K(2.0f), pr), fma(K(2.0f), pr, lb), lam, ra, a, am);
+  const float2 v0 = half_erfc_lr(mul(a, vn));
   const float2 lv = mul(mul(lam, vn), vn);
   const float2 b = mul(mul(K(0.5f * 0.56418958354775628f), ra), exp_neg(lv));
   const float2 v1 = fma(vn, v0, make_float2(b.x, -b.y));
@@ -1410,11 +1443,7 @@ __device__ __forceinline__ void face_flux_lr(const float2* X, float rg, float* o
   f[1 + D] = fma(pr, v0, f[1 + D]);
   f[4] = fma(mul(mul(K(0.5f), pr), vn), v0, f[4]);
   // magnetic stress, lam = rho / (2 p + B^2)
-  float2 lb = mul(bx, bx);
-  lb = fma(by, by, lb);
-  lb = fma(bz, bz, lb);
-  const float2 lm = mul(r, rcp(fma(K(2.0f), pr, lb)));
-  const float2 m0 = half_erfc_lr(mul(mul(lm, rsq(lm)), vn));
+  const float2 m0 = half_erfc_lr(mul(am, vn));
   const float2 nm0 = mul(K(-1.0f), m0);
   const float2 hb = mul(K(0.5f), lb);
   f[5] = (D == 0) ? mul(sub(hb, mul(bx, bx)), m0) : mul(mul(bx, bn), nm0);
