@@ -579,7 +579,7 @@ def run_ours(a):
         "scaling": "weak", "vs_baseline": None, "dtype": "f32",
         "data": "synthetic: seeded Gaussian-random solenoidal turbulence, k^-2 on 2<=k<=8, 256^3 periodic",
         "config": bench_config(n, a.recon),
-        "launch": {"precision": "FP32 state/fluxes, FP64 metric and sums", "graph": graph,
+        "launch": {"precision": "FP32 state and fluxes, FP64 sums", "graph": graph,
                    "tiles": {"face_tile_len": tiles[0], "ei_emf_tile": tiles[1]},
                    "parallelism": "replicas" if ws > 1 else "single GPU"},
         "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": hbm, "unit": "GB/s",

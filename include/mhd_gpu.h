@@ -158,7 +158,9 @@ int mhd_set_tau(void* handle, double tau);
  * with CUDA events on the handle's stream (no extra synchronisation);
  * mhd_last_timings then returns the summed device time of the last
  * mhd_step_n call in ms: [x fluxes, y fluxes, z fluxes + conserved update,
- * emf, face-B update, fill + bxyz, dt (+ save / predictor), unused]. */
+ * emf, face-B update, fill + bxyz, dt (+ save / predictor), unused].  FP64
+ * handles compute the faces of all axes in one launch: the first slot holds
+ * them, the second nothing and the third the conserved update. */
 int mhd_set_profiling(void* handle, int32_t on);
 int mhd_last_timings(void* handle, float out_ms[8]);
 

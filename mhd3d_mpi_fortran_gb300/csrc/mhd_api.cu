@@ -135,8 +135,8 @@ Inp<T> half_inp(const Dev<T>& d) {
 
 // Launch-family recorder: in profile mode every family is bracketed by a pair
 // of CUDA events on the stream (no synchronisation); pairs are resolved after
-// the call.  Families: 0 x fluxes, 1 y fluxes (+x divergence), 2 z fluxes +
-// conserved update, 3 emf, 4 ct (face B) with the fill + bxyz that follows it
+// the call.  Families: 0 x fluxes (FP64: the faces of all axes), 1 y fluxes (+x
+// divergence; FP64: nothing), 2 z fluxes + conserved update (FP64: the update), 3 emf, 4 ct (face B) with the fill + bxyz that follows it
 // (one fused family since both run in Launch::ct_fill), 5 unused, 6
 // dt/save/predict.
 struct Rec {
@@ -177,7 +177,7 @@ Dev<T> at_par(const Dev<T>& base, int par) {
 
 // The EMF families and the face-flux kernels of a stage read the same stage
 // input and write disjoint arrays (E; F, dU and the other half of the
-// primitives), so the EMF runs on the side stream between a fork and a join
+// primitives, in FP64 of the face B too), so the EMF runs on the side stream between a fork and a join
 // event while the fluxes run on st; CT, which reads both, follows the join.
 // In graph capture the fork and join become the graph's dependencies.  The
 // family recorder (profile mode) keeps one stream so that its event pairs
@@ -385,7 +385,9 @@ size_t frame_doubles(const Geom& g) {
   return n;
 }
 // A frame of up to this many bytes that goes to pageable arrays is read in one
-// copy and spread by the host: eleven pageable copies of 85 KB took 25 us each.
+// copy and spread by the host: eleven pageable copies cost 12 us each whatever they hold,
+// the host's copy 65 us a MB.  Fetch of an FP64 frame in us, staged / eleven copies: 0.37 MB 70 /
+// 132, 0.71 MB 89 / 134, 1.23 MB 120 / 139, 1.56 MB 141 / 141, 1.95 MB 165 / 144, 5.7 MB 403 / 166.
 constexpr size_t kStageBytes = (size_t)1 << 20;
 
 // host FP64 Fortran array (ex,ey,ez) -> padded T on the host; rows in parallel
@@ -456,7 +458,11 @@ int init_device(Handle* h) {
 static int graph_for(Handle* h, int nsteps, cudaGraphExec_t* out);
 namespace {
 
-constexpr int kReplayAfter = 6;  // steps launched before the step is captured (a capture takes the time of three)
+// Steps launched before the step is captured.  A capture costs the call that makes it 75 to
+// 150 us (handles whose steps flip the halves make two), and a replayed step saves, in us: 16^3 FP64 deck 77 of 597,
+// 32^3 37 of 104, 64^3 18 of 155, 128^3 43 of 722, 256^3 129 of 4622, 64^3 FP64 16 of 1863.  It is made up for
+// within one to six steps, so a handle that has run six is taken to run as many again.
+constexpr int kReplayAfter = 6;
 
 // The graph of one step from the handle's present state; false when it cannot be made (the
 // step is then launched as before).  The thread's capture mode is relaxed meanwhile, so that a
@@ -672,9 +678,7 @@ static int create_handle(const mhd_params* prm, const double* dx, const double* 
   h->tile_td = (h->fp32 && !metric) ? kSweepTile : 8;
   Geom& g = h->g;
   g.nx0 = prm->nx0; g.ny0 = prm->ny0; g.nz0 = prm->nz0;
-  {
-h->tile_ey = (h->fp32 && !metric) ? (emf_streams(g) ? kEmfStream : 8) : h->fp32 ? 8 : 4;
-  }
+  h->tile_ey = (h->fp32 && !metric) ? (emf_streams(g) ? kEmfStream : 8) : h->fp32 ? 8 : 4;
   g.nord = prm->nord; g.ng = prm->nord / 2;
   g.nx = g.nx0 + g.nord; g.ny = g.ny0 + g.nord; g.nz = g.nz0 + g.nord;
   g.px = (int)round_up((size_t)g.nx + 1, 32);

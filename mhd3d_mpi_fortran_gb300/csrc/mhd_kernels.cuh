@@ -1,21 +1,27 @@
 // Device kernels of the per-timestep MHD update.  Included by exactly one
-// translation unit per precision: mhd_fp64.cu (built with -fmad=false so that
-// every FP64 expression is rounded exactly as the reference writes it) and
-// mhd_fp32.cu (FMA contraction on, the performance path).
+// translation unit per precision: mhd_fp64.cu (built with -fmad=false: FP64
+// products are fused only where the code says so, and the edge EMF and metric mode
+// round as the reference does) and mhd_fp32.cu (FMA contraction on, the performance path).
 //
 // Kernel map (reference routine -> kernel):
-//   get_bxyz (mhd3d3.f90:2118-2128) + vf of get_eijk_LFM (1766)  -> k_bxyz_vf
-//   get_dt   (1608-1639) + diag_rho_neg/diag_overflow (3143-3160) -> k_cfl, k_cfl_final
-//   advance_previous (3794-3819)                                  -> k_save_prev
+//   get_bxyz (mhd3d3.f90:2118-2128) + vf of get_eijk_LFM (1766)  -> k_ct_fill,
+//     k_fill_bxyz (k_bxyz_vf at init)
+//   get_dt   (1608-1639) + diag_rho_neg/diag_overflow (3143-3160) -> cell_dt in k_ct_fill
+//     and k_fill_bxyz or in k_cfl, k_cfl_final
+//   advance_previous (3794-3819) -> FORM_SAVE of the first stage (metric mode: k_cfl)
 //   advance_predictor_ab (3821-3840)                              -> k_predictor_ab
 //   get_flux_stress + get_v_face + reconstruct_3d (2385-2615, 833-1596)
-//     -> k_flux (x faces), k_flux_t<D=1> (y faces, x+y divergence),
-//        k_flux_t<D=2> (z faces + the conserved update below)
-//   get_eijk_LFM + get_vav_center2corner + interp2_* (1754-2116, 926-1067) -> k_emf
+//     -> FP32: k_flux (x faces), k_flux_sweep or k_flux_t of D = 1 (y faces, x+y
+//        divergence) and D = 2 (z faces + the conserved update below);
+//        FP64: k_faces (all axes), batches as FP32 tiles
+//   get_eijk_LFM + get_vav_center2corner + interp2_* (1754-2116, 926-1067)
+//     -> FP32: k_emf_stream + k_emf_rows or k_emf_pdm (PDM), k_emf_weno, k_emf (TVD);
+//        FP64: k_emf64 (PDM, WENO), k_emf (TVD), k_emf_pdm (batches)
+//   get_eijk_Yee (1654-1752)                                      -> k_yee_split, k_emf_yee
 //   get_conserve + advance_corrector1/2 + RK combines (1641-1650, 3842-3907,
-//     3670-3697, 3741-3783)                                       -> k_flux_t<D=2>
-//   advance_bijk + B combines (3909-3933, 3698-3702, 3784-3788)   -> k_update_b
-//   fill_hydro_mpi / fill_mag_mpi (781-819, 346-616)              -> k_fill
+//     3670-3697, 3741-3783) -> cell_update_vals in the z faces (FP64: k_update_faces)
+//   advance_bijk + B combines (3909-3933, 3698-3702, 3784-3788) -> k_ct_fill (metric: k_update_b)
+//   fill_hydro_mpi / fill_mag_mpi (781-819, 346-616) -> k_fill_bxyz (k_fill at init)
 #pragma once
 #include <cuda_runtime.h>
 #include <type_traits>
@@ -1197,25 +1203,6 @@ template <typename T>
 __global__ void k_cfl_final_batch(const Dev<T>* __restrict__ tab, int ngrids, int mode) {
   const int gi = blockIdx.x * blockDim.x + threadIdx.x;
   if (gi < ngrids) select_tau(tab[gi].sc, mode);
-}
-
-// advance_previous for RK (3794-3819): U^n of the stage combines.
-template <typename T>
-__global__ void k_save_prev(Dev<T> d) {
-  long long n = d.g.vol;
-  T gm1 = d.gam - T(1);
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n;
-       c += (long long)gridDim.x * blockDim.x) {
-    T r = d.rho[c], u = d.vx[c], v = d.vy[c], w = d.vz[c];
-    d.q[0][c] = r;
-    d.q[1][c] = r * u;
-    d.q[2][c] = r * v;
-    d.q[3][c] = r * w;
-    d.q[4][c] = T(0.5) * r * (u * u + v * v + w * w) + d.p[c] / gm1;
-    d.q[5][c] = d.bi[c];
-    d.q[6][c] = d.bj[c];
-    d.q[7][c] = d.bk[c];
-  }
 }
 
 // advance_predictor_ab (3821-3840): Xh = X + tau/tau0/2*(X-Xp), then Xp = X;
@@ -3813,11 +3800,6 @@ void Launch<T, M>::cfl_folded(const Dev<T>& d, int mode, bool recompute, cudaStr
 }
 
 template <typename T, bool M>
-void Launch<T, M>::save_prev(const Dev<T>& d, cudaStream_t st) {
-  k_save_prev<T><<<152 * 8, 256, 0, st>>>(d);
-}
-
-template <typename T, bool M>
 void Launch<T, M>::predictor_ab(const Dev<T>& d, cudaStream_t st) {
   const int n = (d.g.nx + Vec16<T>::W) / Vec16<T>::W * d.g.py * d.g.pz;
   k_predictor_ab<T><<<(n + 255) / 256, 256, 0, st>>>(d);
@@ -4063,7 +4045,7 @@ void emf_r(const Dev<T>& d, const Inp<T>& in, cudaStream_t st) {
   k_emf<T, RECON, 2, M><<<grid3(g.nx0 + 1, g.ny0 + 1, g.nz0, b), b, 0, st>>>(d, in, P);
 }
 
-// ei tile cross-section: 8 x 8 edges in FP32, 4 x 4 in FP64; its length along
+// ei tile cross-section: 8 x 8 edges in FP32, 4 x 4 in FP64 (batches); its length along
 // the edge axis is ei_x() below.
 #ifndef MHD_EI_TILE
 #define MHD_EI_TILE 8

@@ -162,7 +162,6 @@ struct Launch {
   // recompute, from a dt pass over the current state instead (first step,
   // or after the state changed between steps)
   static void cfl_folded(const Dev<T>& d, int mode, bool recompute, cudaStream_t st);
-  static void save_prev(const Dev<T>& d, cudaStream_t st);
   static void predictor_ab(const Dev<T>& d, cudaStream_t st);
   // face fluxes of all three axes into F (kernel-level debug entry point)
   static void fluxes(const Dev<T>& d, const Inp<T>& in, cudaStream_t st);
