@@ -109,6 +109,7 @@ template <> struct Div<float> {
 // blast is symmetric to the last bit, and where two slopes tie the corner
 // limiter's choice follows the rounding (8 faces of bk move by 1e-7 of 1e-6 in
 // the second step after a change of 1e-16).
+static __device__ __noinline__ double quot_far(double a, double b) { return a / b; }
 template <typename T> struct Ops;
 template <> struct Ops<double> {
   static __device__ __forceinline__ double dw(double a, double w, double) { return a / w; }     // metric mode: a / V
@@ -116,10 +117,12 @@ template <> struct Ops<double> {
   static __device__ __forceinline__ double dv(double a, double b) { return a / b; }
   static __device__ __forceinline__ double rcp(double b) { return 1.0 / b; }  // used with dvr below
   // a / b from rb = 1 / b and one residual correction (Markstein's theorem:
-  // the rounding of the division when a rb is within one unit of it)
+  // the rounding of the division when a rb is within one unit of it).  Where rb or
+  // a rb is beyond the range (a subnormal, zero or infinite b) the correction is
+  // NaN, and the quotient divides.
   static __device__ __forceinline__ double dvr(double a, double b, double rb) {
-    const double q = a * rb;
-    return fma(fma(-q, b, a), rb, q);
+    const double q = a * rb, r = fma(fma(-q, b, a), rb, q);
+    return (__double2hiint(r) & 0x7ff00000) < 0x7ff00000 ? r : quot_far(a, b);
   }
 };
 template <> struct Ops<float> {
