@@ -135,10 +135,10 @@ Inp<T> half_inp(const Dev<T>& d) {
 
 // Launch-family recorder: in profile mode every family is bracketed by a pair
 // of CUDA events on the stream (no synchronisation); pairs are resolved after
-// the call.  Families: 0 x fluxes (FP64: the faces of all axes), 1 y fluxes (+x
-// divergence; FP64: nothing), 2 z fluxes + conserved update (FP64: the update), 3 emf, 4 ct (face B) with the fill + bxyz that follows it
-// (one fused family since both run in Launch::ct_fill), 5 unused, 6
-// dt/save/predict.
+// the call.  Families: 0 x fluxes (FP64: the faces of all axes), 1 y fluxes (+ x
+// divergence; FP64: nothing), 2 z fluxes + conserved update (FP64: the update),
+// 3 emf, 4 ct (face B) with the fill + bxyz that follows it (one fused family
+// since both run in Launch::ct_fill), 5 unused, 6 dt/save/predict.
 struct Rec {
   Handle* h = nullptr;
   cudaStream_t st = nullptr;
