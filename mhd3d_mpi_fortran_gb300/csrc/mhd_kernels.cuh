@@ -176,12 +176,16 @@ __device__ __forceinline__ double tap8_fused(double a0, double a1, double a2, do
 // integer pipe), so minima and maxima run on order-preserving integer images
 // of the values, and the face fluxes take the state as x held within the two
 // intervals at once (within(): one rounding of c + D).
-// NaN: the near cells reach the result as in the reference's form, a NaN that
-// is only in the interpolant is dropped by the clamp there as here.
+// NaN: of a face's two states one is NaN where one is in the reference's form, and a NaN
+// that is only in the interpolant is dropped by the clamp there as here (the larger near
+// cell remains).  A right state whose far cell alone is NaN is NaN here and the near cell
+// there: sums over both sides or all quadrants do not show it; the Yee EMF, which takes
+// one side, passes the near cell as the other bound of the clamp (lim).
 template <typename T> struct Sel;
 template <> struct Sel<float> {
   typedef float K;
   static __device__ __forceinline__ K key(float x) { return x; }
+  static __device__ __forceinline__ K interp(float x) { return x; }
   static __device__ __forceinline__ float val(K k) { return k; }
   static __device__ __forceinline__ K mn(K a, K b) { return fminf(a, b); }
   static __device__ __forceinline__ K mx(K a, K b) { return fmaxf(a, b); }
@@ -211,6 +215,10 @@ template <> struct Sel<double> {
   typedef long long K;  // ordered as the doubles are: negative values with the magnitude bits inverted
   static __device__ __forceinline__ K flip(K b) { return b ^ ((b >> 63) & 0x7fffffffffffffffLL); }
   static __device__ __forceinline__ K key(double x) { return flip(__double_as_longlong(x)); }
+  // of an interpolant: a NaN of either sign is beyond infinity
+  static __device__ __forceinline__ K interp(double x) {
+    return (unsigned)__double2hiint(x) > 0xfff00000u ? 0x7fffffffffffffffLL : key(x);
+  }
   static __device__ __forceinline__ double val(K k) { return __longlong_as_double(flip(k)); }
   static __device__ __forceinline__ K mn(K a, K b) { return a < b ? a : b; }
   static __device__ __forceinline__ K mx(K a, K b) { return a > b ? a : b; }
@@ -235,8 +243,8 @@ __device__ __forceinline__ float shrink(float d, float D) {  // d and D of one s
   return copysignf(Sel<float>::mx_nan(m, 0.0f), d);
 }
 __device__ __forceinline__ void pdm_states(float fm2, float fm1, float f0, float fp1, float fi, float pdmb, float& fl,
-                                           float& fr) {
-  const float k = pdmb + pdmb, x = clamp2(fm1, f0, fi);
+                                           float& fr, float lim) {
+  const float k = pdmb + pdmb, x = clamp2(lim, f0, fi);
   const float dl = x - fm1, dr = x - f0;
   fl = x - (dl - shrink(dl, k * (fm1 - fm2)));
   fr = x - (dr - shrink(dr, k * (f0 - fp1)));
@@ -248,11 +256,11 @@ __device__ __forceinline__ double within(long long lo, long long hi, long long c
   return S::keep_nan(S::val(S::mx3(lo, S::mn(c, o), S::mn3(hi, S::mx(c, o), x))), out);
 }
 __device__ __forceinline__ void pdm_states_fused(double fm2, double fm1, double f0, double fp1, double fi, double pdmb,
-                                                 double& fl, double& fr) {
+                                                 double& fl, double& fr, double lim) {
   typedef Sel<double> S;
   const double k = pdmb + pdmb;
-  const long long a = S::key(fm1), b = S::key(f0), x = S::key(fi);
-  const long long lo = S::mn(a, b), hi = S::mx(a, b);
+  const long long a = S::key(fm1), b = S::key(f0), x = S::interp(fi), m = S::key(lim);
+  const long long lo = S::mn(m, b), hi = S::mx(m, b);
   fl = within(lo, hi, a, fma(k, fm1 - fm2, fm1), x);
   fr = within(lo, hi, b, fma(k, f0 - fp1, f0), x);
 }
@@ -282,9 +290,10 @@ template <int N> __device__ __forceinline__ double div_by(double x) {
 __device__ __forceinline__ double abs_bits(double x) {
   return __hiloint2double(__double2hiint(x) & 0x7fffffff, __double2loint(x));
 }
-// a >= b for |a|, |b| (integer comparison of the magnitudes)
+// a >= b for |a|, |b| (integer comparison of the magnitudes), false where either is NaN
 __device__ __forceinline__ bool abs_ge(double a, double b) {
-  return (__double_as_longlong(a) & 0x7fffffffffffffffLL) >= (__double_as_longlong(b) & 0x7fffffffffffffffLL);
+  const long long x = __double_as_longlong(a) & 0x7fffffffffffffffLL;
+  return x >= (__double_as_longlong(b) & 0x7fffffffffffffffLL) && (int)(x >> 32) <= 0x7ff00000;
 }
 __device__ __forceinline__ bool abs_ge(float a, float b) { return fabsf(a) >= fabsf(b); }
 // x >= 0 (-0.0 counts)
@@ -315,7 +324,8 @@ struct Edge64 {
   // 0; - when the far cell is the larger.  2 |dn| is exact, so the fused
   // difference rounds as the reference's product and difference do.
   static __device__ __forceinline__ double limited(double near, double fii, double dn, bool up) {
-    const double m = (__double2hiint(dn) >= 0) == up ? abs_bits(dn) : 0.0;
+    const int hd = __double2hiint(dn);
+    const double m = (hd >= 0) == up || (hd & 0x7fffffff) > 0x7ff00000 ? abs_bits(dn) : 0.0;  // (NaN stays)
     const double t = fma(-2.0, m, abs_bits(near - fii));
     const int h = __double2hiint(t);
     const bool neg = (unsigned)h - 0x80000000u <= 0x7ff00000u;  // below zero (not NaN)
@@ -325,7 +335,7 @@ struct Edge64 {
   static __device__ __forceinline__ void states(double fm2, double fm1, double f0, double fp1, double fi, double pdmb,
                                                 double& fl, double& fr) {
     const S::K a = S::key(fm1), b = S::key(f0);
-    const double fii = clamp(a, b, S::key(fi));
+    const double fii = clamp(a, b, S::interp(fi));
     fl = limited(fm1, fii, pdmb * (fm1 - fm2), b >= a);
     fr = limited(f0, fii, pdmb * (f0 - fp1), a > b);
   }
@@ -591,12 +601,12 @@ constexpr bool is_pdm(int recon) { return recon == R_PDM || recon == R_PDMG; }
 template <typename T, int RECON = R_PDM, bool EDGE = false>
 __device__ __forceinline__ void recon_pdm8(T a0, T a1, T a2, T a3, T a4, T a5, T a6, T a7, T pdmb, T& fl, T& fr) {
   if constexpr (RECON == R_PDM && std::is_same<T, double>::value && !EDGE) {
-    pdm_states_fused(a2, a3, a4, a5, tap8_fused(a0, a1, a2, a3, a4, a5, a6, a7), pdmb, fl, fr);
+    pdm_states_fused(a2, a3, a4, a5, tap8_fused(a0, a1, a2, a3, a4, a5, a6, a7), pdmb, fl, fr, a3);
   } else {
     const T fi = tap8(a0, a1, a2, a3, a4, a5, a6, a7);
     if constexpr (RECON != R_PDM) pdm2(a2, a3, a4, a5, fi, pdmb, fl, fr);
     else if constexpr (std::is_same<T, double>::value) Edge64::states(a2, a3, a4, a5, fi, pdmb, fl, fr);
-    else pdm_states(a2, a3, a4, a5, fi, pdmb, fl, fr);
+    else pdm_states(a2, a3, a4, a5, fi, pdmb, fl, fr, a3);
   }
 }
 
@@ -642,7 +652,7 @@ __device__ __forceinline__ double corner_quad(double q, double far1, double far2
   typedef Sel<double> S;
   const bool b = abs_ge(e1, e2);
   const S::K c = S::key(q), f = S::key(b ? far1 : far2);
-  return Edge64::limited(q, Edge64::clamp(c, f, S::key(vi)), pd * (b ? e1 : e2), f > c);
+  return Edge64::limited(q, Edge64::clamp(c, f, S::interp(vi)), pd * (b ? e1 : e2), f > c);
 }
 // The reference's form, for any pdmb (R_PDMG): one half of pdm2 with the clamp
 // pair (lo, hi) = (fm1, f0), the cell `outer` beyond the near end and the side
@@ -3964,6 +3974,21 @@ __global__ void k_yee_split(Dev<T> d, Inp<T> in) {
 // moment; the edge EMF is epp + enp + epn + enn.  ei: y then z, ej: z then x,
 // ek: x then y (reconstruct_3d dirs 5/6, 6/4, 4/5).  Only the rows the
 // second pass reads are reconstructed in the first.
+// PDM state of one side from 8 taps.  The other side does not enter the sum, so a NaN is kept
+// to the states that have it in the reference's form: the left one of a NaN on either side of
+// the face, the right one of a NaN in its own cell.
+__device__ __forceinline__ bool nan_bits(double x) { return (__double2hiint(x) & 0x7fffffff) > 0x7ff00000; }
+__device__ __forceinline__ bool nan_bits(float x) { return x != x; }
+template <typename T>
+__device__ __forceinline__ T pdm_one(const T* a, T pdmb, bool left) {
+  const T lim = nan_bits(a[3]) ? a[4] : a[3];
+  T l, r;
+  if constexpr (std::is_same<T, double>::value)
+    pdm_states_fused(a[2], a[3], a[4], a[5], tap8_fused(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7]), pdmb, l, r, lim);
+  else
+    pdm_states(a[2], a[3], a[4], a[5], tap8(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7]), pdmb, l, r, lim);
+  return !left ? r : nan_bits(a[4]) ? a[4] : l;
+}
 template <typename T, int RECON, int E>
 __global__ void k_emf_yee(Dev<T> d, Prm<T> P) {
   const Geom& g = d.g;
@@ -3990,14 +4015,26 @@ __global__ void k_emf_yee(Dev<T> d, Prm<T> P) {
     for (int m = 0; m < 8; ++m) {
       q[m] = T(0);
       if (m >= M0 && m <= M1) {
-        T l, r;
-        recon_face<T, RECON>(f, c + (m - 4) * sB, sA, P, l, r);
-        q[m] = left1 ? l : r;
+        const int e = c + (m - 4) * sB;
+        if constexpr (RECON == R_PDM) {
+          T a[8];
+#pragma unroll
+          for (int t = 0; t < 8; ++t) a[t] = f[e + (t - 4) * sA];
+          q[m] = pdm_one(a, P.pdmb, left1);
+        } else {
+          T l, r;
+          recon_face<T, RECON>(f, e, sA, P, l, r);
+          q[m] = left1 ? l : r;
+        }
       }
     }
-    T l, r;
-    recon_win<T, RECON, 0>(q, P, l, r);
-    part[s] = left2 ? l : r;
+    if constexpr (RECON == R_PDM) {
+      part[s] = pdm_one(q, P.pdmb, left2);
+    } else {
+      T l, r;
+      recon_win<T, RECON, 0>(q, P, l, r);
+      part[s] = left2 ? l : r;
+    }
   }
   d.E[E][c] = part[0] + part[1] + part[2] + part[3];
 }
